@@ -166,6 +166,8 @@ struct pspin_state {
     float2* d_spins = nullptr;
     double *d_E = nullptr, *d_beta = nullptr, *d_target = nullptr, *d_drift = nullptr, *d_e2 = nullptr,
            *d_e4 = nullptr;
+    double* d_epart = nullptr;          // per-CTA partial energies
+    int energy_splits = 1;
     long long *d_acc = nullptr, *d_prop = nullptr;
     uint64_t* d_key = nullptr;
     int2* d_entries = nullptr;
@@ -243,7 +245,7 @@ static void free_state(pspin_state* s) {
     if (!s) return;
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     void* ptrs[] = {s->d_samples, s->d_units, s->d_spins, s->d_E, s->d_beta, s->d_target, s->d_drift,
-                    s->d_e2, s->d_e4, s->d_acc, s->d_prop, s->d_key, s->d_entries, s->d_chunk_start, s->d_site_chunks,
+                    s->d_e2, s->d_e4, s->d_epart, s->d_acc, s->d_prop, s->d_key, s->d_entries, s->d_chunk_start, s->d_site_chunks,
                     s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status,
                     s->d_beta_sched, s->d_perm, s->d_drand, s->d_ex_acc, s->d_ex_prop, s->d_trace,
                     s->d_tc_w, s->d_tc_x, s->d_tc_f, s->d_tc_ws, s->d_tc_h, s->d_f64_h, s->d_tc_e,
@@ -727,8 +729,10 @@ static int run_energy(pspin_state* s, double* e2, double* e4, bool overwrite, bo
     p.energy = overwrite ? s->d_E : nullptr;
     p.drift = overwrite ? s->d_drift : nullptr;
     p.target = renorm ? s->d_target : nullptr;
+    p.partial = s->d_epart;
+    p.max_splits = s->energy_splits;
     CK(launch_energy(p, (int)s->units.size(), s->max_N, s->st));
-    s->kernel_launches++;
+    s->kernel_launches += renorm ? 3 : 2;
     return PSPIN_OK;
 }
 
@@ -1012,11 +1016,13 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         return bail(fail(PSPIN_ERR_ARG, "N=%d with %d replicas per lane needs more shared memory than a CTA has",
                          s->max_N, s->rpl));
 
+    s->energy_splits = energy_max_splits((int)s->units.size());
     if ((rc = dalloc(&s->d_samples, n)) || (rc = dalloc(&s->d_units, s->units.size())) ||
         (rc = dalloc(&s->d_spins, (size_t)s->spin_total)) || (rc = dalloc(&s->d_E, s->R_tot)) ||
         (rc = dalloc(&s->d_beta, s->R_tot)) || (rc = dalloc(&s->d_target, s->R_tot)) ||
         (rc = dalloc(&s->d_drift, s->R_tot)) || (rc = dalloc(&s->d_e2, s->R_tot)) ||
-        (rc = dalloc(&s->d_e4, s->R_tot)) || (rc = dalloc(&s->d_acc, s->R_tot)) ||
+        (rc = dalloc(&s->d_e4, s->R_tot)) ||
+        (rc = dalloc(&s->d_epart, energy_partial_doubles((int)s->units.size(), s->energy_splits))) || (rc = dalloc(&s->d_acc, s->R_tot)) ||
         (rc = dalloc(&s->d_prop, s->R_tot)) || (rc = dalloc(&s->d_key, s->R_tot)) ||
         (rc = dalloc(&s->d_entries, (size_t)ent_total)) || (rc = dalloc(&s->d_site_chunks, (size_t)split_total)) ||
         (rc = dalloc(&s->d_chunk_start, (size_t)chunk_total + 1)) ||

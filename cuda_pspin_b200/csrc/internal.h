@@ -165,7 +165,11 @@ struct EnergyParams {
     double* drift;            // |E_running - E_fp64| before the overwrite (when energy set)
     const double* target;     // constraint target per replica (renormalise when non-null)
     int renorm_only;          // 1: renormalise and return (energies come from elsewhere)
+    double* partial;          // [n_units][max_splits][32][2]: (e2, e4) of each CTA's share of the tables
+    int max_splits;           // most CTAs per unit
 };
+int energy_max_splits(int n_units);
+size_t energy_partial_doubles(int n_units, int max_splits);
 cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStream_t st);
 
 struct ExchangeParams {

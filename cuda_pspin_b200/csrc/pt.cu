@@ -5,25 +5,18 @@
 namespace pspin {
 
 // ---------------------------------------------------------------------
-// FP64 energies of every replica of one unit.
-//
-// The chain's energy (mc.cu:323-405): E2 = -sum_{i<j} Re[g_ij a_i conj a_j]
-// (diagonal excluded), E4 = -sum over active (q,ch) Re[g f_ch(a)] with the
-// channel conjugation patterns of mc.cu:389-391.  Amplitudes are the FP32
-// ones the sweep evolves, upcast.  With a target, each replica is first
-// rescaled in FP64 to sum|a|^2 = target (sphere) or sum|a|^4 = target
-// (cube) and the rescaled amplitudes are stored back.
+// Projection of every replica of one unit onto its constraint, in FP64:
+// sum|a|^2 = target (sphere) or sum|a|^4 = target (cube), the rescaled
+// amplitudes stored back as FP32.
 // ---------------------------------------------------------------------
-__global__ void __launch_bounds__(256) energy_kernel(const EnergyParams P) {
-    extern __shared__ float2 esm[];
+__global__ void __launch_bounds__(256) renorm_kernel(const EnergyParams P) {
+    extern __shared__ float2 rsm[];
     const Unit U = P.units[blockIdx.x];
     const SampleDev S = P.samples[U.sample];
     const int N = S.N, R = S.R;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    float2* sp = esm;                                                      // [N][32]
-    double* red = reinterpret_cast<double*>(esm + (size_t)N * kRepBlock);  // [nw][32][2]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2* sp = rsm;                                                      // [N][32]
     __shared__ double scale_s[kRepBlock];
-
     for (int idx = threadIdx.x; idx < N * kRepBlock; idx += blockDim.x) {
         const int site = idx >> 5, l = idx & 31;
         float2 v = make_float2(0.f, 0.f);
@@ -31,92 +24,217 @@ __global__ void __launch_bounds__(256) energy_kernel(const EnergyParams P) {
         sp[idx] = v;
     }
     __syncthreads();
-
-    if (P.target != nullptr) {
-        if (warp == 0) {
-            double s = 0.0;
-            for (int site = 0; site < N; site++) {
-                const float2 a = sp[site * kRepBlock + lane];
-                const double r2 = (double)a.x * a.x + (double)a.y * a.y;
-                s += (S.variant == 0) ? r2 : r2 * r2;
-            }
-            double sc = 1.0;
-            if (lane < U.rep_count && s > 0.0) {
-                const double t = P.target[S.rep_off + U.rep_begin + lane];
-                sc = (S.variant == 0) ? sqrt(t / s) : sqrt(sqrt(t / s));
-            }
-            scale_s[lane] = sc;
+    if (warp == 0) {
+        double s = 0.0;
+        for (int site = 0; site < N; site++) {
+            const float2 a = sp[site * kRepBlock + lane];
+            const double r2 = (double)a.x * a.x + (double)a.y * a.y;
+            s += (S.variant == 0) ? r2 : r2 * r2;
         }
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < N * kRepBlock; idx += blockDim.x) {
-            const int site = idx >> 5, l = idx & 31;
-            const double sc = scale_s[l];
-            const float2 a = sp[idx];
-            const float2 b = make_float2((float)(a.x * sc), (float)(a.y * sc));
-            sp[idx] = b;
-            if (l < U.rep_count) P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + l] = b;
+        double sc = 1.0;
+        if (lane < U.rep_count && s > 0.0) {
+            const double t = P.target[S.rep_off + U.rep_begin + lane];
+            sc = (S.variant == 0) ? sqrt(t / s) : sqrt(sqrt(t / s));
         }
-        if (P.renorm_only) return;
-        __syncthreads();
+        scale_s[lane] = sc;
     }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < N * kRepBlock; idx += blockDim.x) {
+        const int site = idx >> 5, l = idx & 31;
+        const double sc = scale_s[l];
+        const float2 a = sp[idx];
+        if (l < U.rep_count)
+            P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + l] = make_float2((float)(a.x * sc), (float)(a.y * sc));
+    }
+}
+
+// ---------------------------------------------------------------------
+// FP64 energies of every replica.
+//
+// The chain's energy (mc.cu:323-405): E2 = -sum_{i<j} Re[g_ij a_i conj a_j]
+// (diagonal excluded), E4 = -sum over active (q,ch) Re[g f_ch(a)] with the
+// channel conjugation patterns of mc.cu:389-391.  Amplitudes are the FP32
+// ones the sweep evolves, upcast.
+//
+// Site i is unconjugated in every channel and runs fastest in the table of a
+// dense sample, so a run of entries with the same (j, k, l, ch) costs
+// Y = sum g a_i, two FP64 FMA per entry, and one product Y a_j a_k a_l (with
+// the channel's conjugations) per run; a table in any other order is correct
+// with runs of one entry.  One entry as a product of four amplitudes of its
+// own had cost 8 conversions and ~13 FP64 operations.  The amplitudes are
+// upcast once per CTA into shared memory (kDouble: up to N = kDoubleN; above,
+// FP32 upcast at each use), so an entry is bound by its shared-memory reads
+// (16-byte broadcast + 512-byte row: 5 wavefronts a warp).
+//
+// Lanes are replicas; a unit's table is cut over `splits` CTAs of 8 warps, so
+// few units still fill the chip; each CTA writes one partial per replica and
+// energy_sum_kernel adds them in a fixed order.  768 units of a 256-sample
+// batch (N 24..64, fully connected, 96 replicas): 45 ms before, 5.5 ms now;
+// two units at N=128 (10.7 M entries): 728 ms before, 0.94 ms now.
+// ---------------------------------------------------------------------
+constexpr int kDoubleN = 192;      // amplitudes as double2 up to here: 96 KB of shared memory a CTA
+constexpr int kEnergyWarps = 8;
+
+// CTAs sharing a sample's table: at least 1024 entries for each of their warps
+__host__ __device__ inline int energy_splits(int64_t nq, int max_splits) {
+    const int64_t want = nq / (kEnergyWarps * 1024) + 1;
+    return (int)(want < max_splits ? want : max_splits);
+}
+
+template <bool kDouble>
+__global__ void __launch_bounds__(32 * kEnergyWarps) energy_kernel(const EnergyParams P) {
+    extern __shared__ __align__(16) unsigned char esm[];
+    const Unit U = P.units[blockIdx.x];
+    const SampleDev S = P.samples[U.sample];
+    const int splits = energy_splits(S.nq, P.max_splits), split = blockIdx.y;
+    if (split >= splits) return;
+    const int N = S.N, R = S.R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int nw = kEnergyWarps;
+    __shared__ Q64 stage_all[nw][32];
+    static_assert(sizeof(Q64) == sizeof(double2), "the partial sums reuse the staging rows");
+    Q64* stage = stage_all[warp];
+    double2* spd = reinterpret_cast<double2*>(esm);                        // [N][32]
+    float2* spf = reinterpret_cast<float2*>(esm);
+    for (int idx = threadIdx.x; idx < N * kRepBlock; idx += blockDim.x) {
+        const int site = idx >> 5, l = idx & 31;
+        float2 v = make_float2(0.f, 0.f);
+        if (l < U.rep_count) v = P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + l];
+        if (kDouble) spd[idx] = make_double2(v.x, v.y);
+        else spf[idx] = v;
+    }
+    __syncthreads();
+    auto amp = [&](int site) {
+        if (kDouble) return spd[site * kRepBlock + lane];
+        const float2 v = spf[site * kRepBlock + lane];
+        return make_double2(v.x, v.y);
+    };
 
     double e2 = 0.0, e4 = 0.0;
     if (S.h2_active) {
         const int64_t npair = (int64_t)N * (N - 1) / 2;
-        for (int64_t pidx = warp; pidx < npair; pidx += nw) {
+        for (int64_t pidx = split * nw + warp; pidx < npair; pidx += (int64_t)splits * nw) {
             // pair index -> (i<j), row-major over j
-            int j = (int)((1.0 + sqrt(1.0 + 8.0 * (double)pidx)) * 0.5);
+            int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)pidx)) * 0.5f);
             while ((int64_t)j * (j - 1) / 2 > pidx) j--;
             while ((int64_t)(j + 1) * j / 2 <= pidx) j++;
             const int i = (int)(pidx - (int64_t)j * (j - 1) / 2);
             const double g = __ldg(P.g2 + S.g2_off + (int64_t)i * N + j);
             if (g == 0.0) continue;
-            const float2 ai = sp[i * kRepBlock + lane], aj = sp[j * kRepBlock + lane];
+            const double2 ai = amp(i), aj = amp(j);
             // -Re[g a_i conj(a_j)]
-            e2 -= g * ((double)ai.x * aj.x + (double)ai.y * aj.y);
+            e2 -= g * (ai.x * aj.x + ai.y * aj.y);
         }
     }
-    const Q64* __restrict__ Q = P.quartets + S.q_off;
-    for (int64_t t = warp; t < S.nq; t += nw) {
-        const Q64 q = Q[t];
-        const int l = q.lch & 0x3FFF, ch = q.lch >> 14;
-        const float2 fi = sp[q.i * kRepBlock + lane], fj = sp[q.j * kRepBlock + lane];
-        const float2 fk = sp[q.k * kRepBlock + lane], fl = sp[l * kRepBlock + lane];
-        double ix = fi.x, iy = fi.y, jx = fj.x, jy = fj.y, kx = fk.x, ky = fk.y, lx = fl.x, ly = fl.y;
-        // conjugations: ch0 {k,l}, ch1 {j,k}, ch2 {j,l} (mc.cu:389-391)
-        if (ch == 0) { ky = -ky; ly = -ly; }
-        else if (ch == 1) { jy = -jy; ky = -ky; }
-        else { jy = -jy; ly = -ly; }
-        const double ax = ix * jx - iy * jy, ay = ix * jy + iy * jx;   // s0 s1
-        const double bx = kx * lx - ky * ly, by = kx * ly + ky * lx;   // s2 s3
-        e4 -= q.g * (ax * bx - ay * by);
+    // this warp's contiguous share of the table, 32 entries at a time: the
+    // next 32 are in flight while these are summed
+    const int64_t workers = (int64_t)splits * nw, me = (int64_t)split * nw + warp;
+    const int64_t t0 = S.nq * me / workers, t1 = S.nq * (me + 1) / workers;
+    const int4* __restrict__ Q = reinterpret_cast<const int4*>(P.quartets + S.q_off);
+    int4 mine = make_int4(0, 0, 0, 0);
+    if (t0 + lane < t1) mine = __ldg(Q + t0 + lane);
+    for (int64_t t = t0; t < t1; t += 32) {
+        const int n = (int)(t1 - t < 32 ? t1 - t : 32);
+        reinterpret_cast<int4*>(stage)[lane] = mine;
+        const int4 cur = mine;
+        if (t + 32 + lane < t1) mine = __ldg(Q + t + 32 + lane);
+        // starts of the runs of equal (j, k, l, ch)
+        const unsigned kl = (unsigned)cur.y, kj = (unsigned)cur.x >> 16;
+        const unsigned pkl = __shfl_up_sync(0xffffffffu, kl, 1), pkj = __shfl_up_sync(0xffffffffu, kj, 1);
+        unsigned starts = __ballot_sync(0xffffffffu, lane < n && (lane == 0 || kl != pkl || kj != pkj));
+        __syncwarp();
+        while (starts) {
+            const int b = __ffs(starts) - 1;
+            starts &= starts - 1;
+            const int e = starts ? __ffs(starts) - 1 : n;
+            double yx = 0.0, yy = 0.0;
+#pragma unroll 4
+            for (int u = b; u < e; u++) {
+                const Q64 q = stage[u];
+                const double2 a = amp(q.i);
+                yx = fma(q.g, a.x, yx);
+                yy = fma(q.g, a.y, yy);
+            }
+            const Q64 q = stage[b];
+            const int ch = q.lch >> 14;
+            double2 aj = amp(q.j), ak = amp(q.k), al = amp(q.lch & 0x3FFF);
+            // conjugations: ch0 {k,l}, ch1 {j,k}, ch2 {j,l} (mc.cu:389-391)
+            if (ch != 0) aj.y = -aj.y;
+            if (ch != 2) ak.y = -ak.y;
+            if (ch != 1) al.y = -al.y;
+            const double bx = ak.x * al.x - ak.y * al.y, by = ak.x * al.y + ak.y * al.x;   // s2 s3
+            const double ax = yx * aj.x - yy * aj.y, ay = yx * aj.y + yy * aj.x;           // sum g s0 s1
+            e4 -= ax * bx - ay * by;
+        }
+        __syncwarp();
     }
-    red[(warp * kRepBlock + lane) * 2] = e2;
-    red[(warp * kRepBlock + lane) * 2 + 1] = e4;
+    double2* red = reinterpret_cast<double2*>(&stage_all[0][0]);          // [nw][32], each warp its own staging rows
+    red[warp * kRepBlock + lane] = make_double2(e2, e4);
     __syncthreads();
-    if (warp == 0 && lane < U.rep_count) {
+    if (warp == 0) {
         double s2 = 0.0, s4 = 0.0;
         for (int w = 0; w < nw; w++) {
-            s2 += red[(w * kRepBlock + lane) * 2];
-            s4 += red[(w * kRepBlock + lane) * 2 + 1];
+            const double2 v = red[w * kRepBlock + lane];
+            s2 += v.x;
+            s4 += v.y;
         }
-        const int64_t gr = S.rep_off + U.rep_begin + lane;
-        if (P.e2) P.e2[gr] = s2;
-        if (P.e4) P.e4[gr] = s4;
-        if (P.energy) {
-            if (P.drift) P.drift[gr] = fabs(P.energy[gr] - (s2 + s4));
-            P.energy[gr] = s2 + s4;
-        }
+        double2* out = reinterpret_cast<double2*>(P.partial);             // [units][max_splits][32]
+        out[((int64_t)blockIdx.x * P.max_splits + split) * kRepBlock + lane] = make_double2(s2, s4);
     }
 }
 
+__global__ void __launch_bounds__(kRepBlock) energy_sum_kernel(const EnergyParams P) {
+    const Unit U = P.units[blockIdx.x];
+    const SampleDev S = P.samples[U.sample];
+    const int lane = threadIdx.x;
+    if (lane >= U.rep_count) return;
+    const int splits = energy_splits(S.nq, P.max_splits);
+    const double2* part = reinterpret_cast<const double2*>(P.partial) + (int64_t)blockIdx.x * P.max_splits * kRepBlock + lane;
+    double s2 = 0.0, s4 = 0.0;
+#pragma unroll 8
+    for (int q = 0; q < splits; q++) {
+        const double2 v = part[(int64_t)q * kRepBlock];
+        s2 += v.x;
+        s4 += v.y;
+    }
+    const int64_t gr = S.rep_off + U.rep_begin + lane;
+    if (P.e2) P.e2[gr] = s2;
+    if (P.e4) P.e4[gr] = s4;
+    if (P.energy) {
+        if (P.drift) P.drift[gr] = fabs(P.energy[gr] - (s2 + s4));
+        P.energy[gr] = s2 + s4;
+    }
+}
+
+// most CTAs a unit's table is cut into: 16 CTAs per SM over all units
+int energy_max_splits(int n_units) {
+    int sms = 0, dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        sms = 148;
+    const int want = n_units > 0 ? (16 * sms + n_units - 1) / n_units : 1;
+    return want < 1 ? 1 : (want > 256 ? 256 : want);
+}
+
+size_t energy_partial_doubles(int n_units, int max_splits) { return (size_t)n_units * max_splits * kRepBlock * 2; }
+
 cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStream_t st) {
     if (n_units <= 0) return cudaSuccess;
-    const int threads = 256;
-    const size_t smem = (size_t)max_N * kRepBlock * sizeof(float2) + (size_t)(threads / 32) * kRepBlock * 2 * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(energy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e;
+    if (p.target != nullptr) {
+        const size_t smem = (size_t)max_N * kRepBlock * sizeof(float2);
+        e = cudaFuncSetAttribute(renorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        renorm_kernel<<<n_units, 256, smem, st>>>(p);
+        if ((e = cudaGetLastError()) != cudaSuccess || p.renorm_only) return e;
+    }
+    const bool dbl = max_N <= kDoubleN;
+    const size_t smem = (size_t)max_N * kRepBlock * (dbl ? sizeof(double2) : sizeof(float2));
+    auto kern = dbl ? energy_kernel<true> : energy_kernel<false>;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    energy_kernel<<<n_units, threads, smem, st>>>(p);
+    kern<<<dim3((unsigned)n_units, (unsigned)p.max_splits), 32 * kEnergyWarps, smem, st>>>(p);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    energy_sum_kernel<<<n_units, kRepBlock, 0, st>>>(p);
     return cudaGetLastError();
 }
 
