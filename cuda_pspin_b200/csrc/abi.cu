@@ -46,15 +46,12 @@ struct LearnParams {
 cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, int n_units, int max_N, cudaStream_t st,
                                  int* max_clusters);
 size_t learned_smem_bytes_host(int N, int warps, int C);
-cudaError_t launch_mlp_fwd_bwd(const float* w, const float* records, const int* index, int n, float* save,
-                               float* loss, cudaStream_t st);
-cudaError_t launch_mlp_grad(const float* save, int n, float* grad, cudaStream_t st);
-cudaError_t launch_adam(float* w, float* m, float* v, const float* g, __nv_bfloat16* wbf, float lr, int t,
-                        cudaStream_t st);
+cudaError_t launch_mlp_train(float* w, const float* records, unsigned long long filled, uint64_t key, uint32_t step,
+                             int n, float* partial, float* loss, float* grad, float* m, float* v, __nv_bfloat16* wbf,
+                             float lr, int adam_step, cudaStream_t st);
+size_t mlp_partial_floats();
 cudaError_t launch_to_bf16(const float* w, __nv_bfloat16* wbf, cudaStream_t st);
-cudaError_t launch_sample_index(int* idx, int n, unsigned long long filled, uint64_t key, uint32_t step,
-                                cudaStream_t st);
-constexpr int kMlpParamsHost = 6426, kRecordFloatsHost = 11, kSaveFloatsHost = 8 + 4 * 64 + 26;
+constexpr int kMlpParamsHost = 6426, kRecordFloatsHost = 11;
 cudaError_t dev_fmc_mask(uint8_t* mask, const double* omega, int N, double gamma, cudaStream_t st);
 cudaError_t launch_cube_normalize_many(double* all, int N, int nsamples, cudaStream_t st);
 cudaError_t dev_g2_build(const double* normals, int N, const double* omega, double gamma, double* g2,
@@ -210,9 +207,8 @@ struct pspin_state {
     unsigned long long* d_rec_count = nullptr;
     int rec_cap = 0;
     float rec_prob = 0.f;
-    float *d_save = nullptr, *d_loss = nullptr;
-    int* d_idx = nullptr;
-    int save_cap = 0;
+    float *d_mlp_part = nullptr, *d_loss = nullptr;   // partial gradients, per-record losses of a batch
+    int loss_cap = 0;
     int adam_t = 0;
     uint64_t learn_seed = 0;
 
@@ -250,7 +246,7 @@ static void free_state(pspin_state* s) {
                     s->d_beta_sched, s->d_perm, s->d_drand, s->d_ex_acc, s->d_ex_prop, s->d_trace,
                     s->d_tc_w, s->d_tc_x, s->d_tc_f, s->d_tc_ws, s->d_tc_h, s->d_f64_h, s->d_tc_e,
                     s->d_w32, s->d_adam_m, s->d_adam_v, s->d_grad, s->d_wbf, s->d_records, s->d_rec_count,
-                    s->d_save, s->d_loss, s->d_idx, s->d_obs_E, s->d_obs_q, s->d_pair_chunks, s->d_site_chunks_g, s->d_nbmask,
+                    s->d_mlp_part, s->d_loss, s->d_obs_E, s->d_obs_q, s->d_pair_chunks, s->d_site_chunks_g, s->d_nbmask,
                     s->d_units_k[0], s->d_units_k[1]};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -2208,18 +2204,14 @@ extern "C" int pspin_learn_params(pspin_state* s, float* get, const float* set) 
     return PSPIN_OK;
 }
 
-static int ensure_save(pspin_state* s, int n) {
-    if (n <= s->save_cap) return PSPIN_OK;
-    cudaFree(s->d_save);
+static int ensure_batch(pspin_state* s, int n) {
+    if (!s->d_mlp_part) TRY(dalloc(&s->d_mlp_part, mlp_partial_floats()));
+    if (n <= s->loss_cap) return PSPIN_OK;
     cudaFree(s->d_loss);
-    cudaFree(s->d_idx);
-    s->d_save = nullptr; s->d_loss = nullptr; s->d_idx = nullptr;
-    s->save_cap = 0;
-    int rc;
-    if ((rc = dalloc(&s->d_save, (size_t)n * kSaveFloatsHost)) || (rc = dalloc(&s->d_loss, n)) ||
-        (rc = dalloc(&s->d_idx, n)))
-        return rc;
-    s->save_cap = n;
+    s->d_loss = nullptr;
+    s->loss_cap = 0;
+    TRY(dalloc(&s->d_loss, n));
+    s->loss_cap = n;
     return PSPIN_OK;
 }
 
@@ -2232,14 +2224,13 @@ extern "C" int pspin_learn_train(pspin_state* s, int steps, int batch, float lr,
     CK(cudaStreamSynchronize(s->st));
     const unsigned long long filled = cnt < (unsigned long long)s->rec_cap ? cnt : (unsigned long long)s->rec_cap;
     if (filled == 0) return fail(PSPIN_ERR_STATE, "no training records yet");
-    TRY(ensure_save(s, batch));
+    TRY(ensure_batch(s, batch));
     for (int it = 0; it < steps; it++) {
-        CK(launch_sample_index(s->d_idx, batch, filled, s->learn_seed ^ 0x5eedULL, (uint32_t)s->adam_t, s->st));
-        CK(launch_mlp_fwd_bwd(s->d_w32, s->d_records, s->d_idx, batch, s->d_save, s->d_loss, s->st));
-        CK(launch_mlp_grad(s->d_save, batch, s->d_grad, s->st));
         s->adam_t++;
-        CK(launch_adam(s->d_w32, s->d_adam_m, s->d_adam_v, s->d_grad, s->d_wbf, lr, s->adam_t, s->st));
-        s->kernel_launches += 4;
+        CK(launch_mlp_train(s->d_w32, s->d_records, filled, s->learn_seed ^ 0x5eedULL, (uint32_t)(s->adam_t - 1), batch,
+                            s->d_mlp_part, s->d_loss, s->d_grad, s->d_adam_m, s->d_adam_v, s->d_wbf, lr, s->adam_t,
+                            s->st));
+        s->kernel_launches += 2;
     }
     if (mean_loss) {
         std::vector<float> l(batch);
@@ -2272,13 +2263,14 @@ extern "C" int pspin_learn_records(pspin_state* s, int64_t* n_recorded, float* o
 extern "C" int pspin_learn_loss_grad(pspin_state* s, const float* records, int n, double* loss, float* grad) {
     if (!s || !records || n < 1) return fail(PSPIN_ERR_ARG, "bad arguments");
     if (!s->d_w32) return fail(PSPIN_ERR_STATE, "pspin_learn_init has not been called");
-    TRY(ensure_save(s, n));
+    TRY(ensure_batch(s, n));
     float* d_rec = nullptr;
     TRY(dalloc(&d_rec, (size_t)n * kRecordFloatsHost));
     cudaError_t e = cudaMemcpyAsync(d_rec, records, (size_t)n * kRecordFloatsHost * sizeof(float),
                                     cudaMemcpyHostToDevice, s->st);
-    if (e == cudaSuccess) e = launch_mlp_fwd_bwd(s->d_w32, d_rec, nullptr, n, s->d_save, s->d_loss, s->st);
-    if (e == cudaSuccess) e = launch_mlp_grad(s->d_save, n, s->d_grad, s->st);
+    if (e == cudaSuccess)
+        e = launch_mlp_train(s->d_w32, d_rec, 0, 0, 0, n, s->d_mlp_part, s->d_loss, s->d_grad, nullptr, nullptr, nullptr,
+                             0.f, 0, s->st);
     std::vector<float> l(n);
     if (e == cudaSuccess) e = cudaMemcpyAsync(l.data(), s->d_loss, n * sizeof(float), cudaMemcpyDeviceToHost, s->st);
     if (e == cudaSuccess && grad)

@@ -548,74 +548,260 @@ cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, int
 }
 
 // ------------------------------------------------------------------ training
-// Per record: forward and backward through the network (FP32 master
-// weights); activations and deltas saved for the per-parameter reduction.
-constexpr int kSaveFloats = kMlpIn + 2 * kMlpHidden + 2 * kMlpHidden + kMlpOut;   // f, h1, h2, d1, d2, d3
+// Forward, backward and gradient of one minibatch in one kernel (FP32 master
+// weights).  A CTA of 8 warps takes tiles of 32 records, lane = record: the
+// warps share each layer's units, activations and deltas stay in shared
+// memory (rows of kTrainRow words, one per unit), and the tile's contribution
+// to every parameter's gradient is added to registers (a thread owns a 4 x 4
+// patch of W2 and its share of the rest).  kTrainCtas CTAs at most, each
+// taking every kTrainCtas-th tile, then one partial gradient per CTA: the
+// summation order depends on the batch size alone.  With one thread per
+// record and activations in global memory, and one thread per parameter
+// summing over all records, a step at batch 4096 took 525 us on 32 and 26
+// blocks; 27 us + 5 us (sum and Adam).
+constexpr int kTrainCtas = 296;                 // two per SM
+constexpr int kTrainRow = 36;                   // 32 records + 4: rows 16-byte aligned, float4 reads conflict-free
+constexpr int kTrainRows = kMlpIn + 4 * kMlpHidden + 2 * kMlpOut;    // f, h1, h2, d1, d2, out, d3
+constexpr int kTrainWeights = (kMlpParams + 3) & ~3;
+constexpr size_t kTrainSmem = (size_t)(kTrainWeights + kTrainRows * kTrainRow + 3 * 32) * sizeof(float);
 
-__global__ void mlp_fwd_bwd_kernel(const float* __restrict__ w, const float* __restrict__ records,
-                                   const int* __restrict__ index, int n, float* __restrict__ save,
-                                   float* __restrict__ loss) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    const float* rec = records + (int64_t)(index ? index[b] : b) * kRecordFloats;
-    float* sv = save + (int64_t)b * kSaveFloats;
-    float* f = sv;
-    float* h1 = f + kMlpIn;
-    float* h2 = h1 + kMlpHidden;
-    float* d1 = h2 + kMlpHidden;
-    float* d2 = d1 + kMlpHidden;
-    float* d3 = d2 + kMlpHidden;
-    for (int i = 0; i < kMlpIn; i++) f[i] = rec[i];
-    float out[kMlpOut];
-    mlp_forward_rows(w, f, h1, h2, out);
-    loss[b] = loss_output_grad(out, rec[kMlpIn], rec[kMlpIn + 1], rec[kMlpIn + 2], d3);
-    for (int i = 0; i < kMlpHidden; i++) {
-        float s = 0.f;
-        for (int o = 0; o < kMlpOut; o++) s = fmaf(w[kOffW3 + o * kMlpHidden + i], d3[o], s);
-        d2[i] = s * (1.0f - h2[i] * h2[i]);
+__global__ void __launch_bounds__(256, 2) mlp_train_kernel(const float* __restrict__ wg, const float* __restrict__ records,
+                                                           unsigned long long filled, uint32_t key0, uint32_t key1,
+                                                           uint32_t step, int n, float* __restrict__ partial,
+                                                           float* __restrict__ loss) {
+    extern __shared__ __align__(16) float tsm[];
+    float* w = tsm;
+    float* f = w + kTrainWeights;
+    float* h1 = f + kMlpIn * kTrainRow;
+    float* h2 = h1 + kMlpHidden * kTrainRow;
+    float* d1 = h2 + kMlpHidden * kTrainRow;
+    float* d2 = d1 + kMlpHidden * kTrainRow;
+    float* ot = d2 + kMlpHidden * kTrainRow;
+    float* d3 = ot + kMlpOut * kTrainRow;
+    float* lp = d3 + kMlpOut * kTrainRow;       // [3][32] parts of log q
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int ti = tid >> 4, tj = tid & 15;
+    for (int i = tid; i < kMlpParams; i += 256) w[i] = wg[i];
+    float g2[4][4], g3[2][4], g1[4];            // W2 patch; W3 patch; W1 column or biases
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+        g1[a] = 0.f;
+#pragma unroll
+        for (int b = 0; b < 4; b++) g2[a][b] = 0.f;
     }
-    for (int i = 0; i < kMlpHidden; i++) {
-        float s = 0.f;
-        for (int o = 0; o < kMlpHidden; o++) s = fmaf(w[kOffW2 + o * kMlpHidden + i], d2[o], s);
-        d1[i] = s * (1.0f - h1[i] * h1[i]);
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+#pragma unroll
+        for (int b = 0; b < 4; b++) g3[a][b] = 0.f;
+    __syncthreads();
+    const int tiles = (n + 31) / 32;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int b = tile * 32 + lane;
+        const bool on = b < n;
+        // the record: entry b, or a draw from the ring's `filled` entries
+        const float* rec = records;
+        if (on) {
+            int64_t at = b;
+            if (filled > 0) {
+                const U4 r = philox4x32_10(U4{(uint32_t)b, step, 0x74726e00u, 0u}, key0, key1);
+                at = (int)(((uint64_t)r.x * filled) >> 32);
+            }
+            rec = records + at * kRecordFloats;
+        }
+        f[warp * kTrainRow + lane] = on ? rec[warp] : 0.f;             // 8 warps, 8 features
+        __syncthreads();
+        {   // hidden 1: units 8 warp .. + 7
+            float z[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) z[q] = w[kOffB1 + warp * 8 + q];
+#pragma unroll
+            for (int i = 0; i < kMlpIn; i++) {
+                const float x = f[i * kTrainRow + lane];
+#pragma unroll
+                for (int q = 0; q < 8; q++) z[q] = fmaf(w[kOffW1 + (warp * 8 + q) * kMlpIn + i], x, z[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) h1[(warp * 8 + q) * kTrainRow + lane] = tanhf(z[q]);
+        }
+        __syncthreads();
+        {   // hidden 2
+            float z[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) z[q] = w[kOffB2 + warp * 8 + q];
+#pragma unroll 4
+            for (int i = 0; i < kMlpHidden; i += 4) {
+                float x[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) x[u] = h1[(i + u) * kTrainRow + lane];
+#pragma unroll
+                for (int q = 0; q < 8; q++) {
+                    const float4 c = *reinterpret_cast<const float4*>(w + kOffW2 + (warp * 8 + q) * kMlpHidden + i);
+                    z[q] = fmaf(c.x, x[0], z[q]);
+                    z[q] = fmaf(c.y, x[1], z[q]);
+                    z[q] = fmaf(c.z, x[2], z[q]);
+                    z[q] = fmaf(c.w, x[3], z[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) h2[(warp * 8 + q) * kTrainRow + lane] = tanhf(z[q]);
+        }
+        __syncthreads();
+        {   // outputs warp, warp + 8, ...
+            float z[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) z[q] = warp + 8 * q < kMlpOut ? w[kOffB3 + warp + 8 * q] : 0.f;
+#pragma unroll 4
+            for (int i = 0; i < kMlpHidden; i += 4) {
+                float x[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) x[u] = h2[(i + u) * kTrainRow + lane];
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (warp + 8 * q < kMlpOut) {
+                        const float4 c = *reinterpret_cast<const float4*>(w + kOffW3 + (warp + 8 * q) * kMlpHidden + i);
+                        z[q] = fmaf(c.x, x[0], z[q]);
+                        z[q] = fmaf(c.y, x[1], z[q]);
+                        z[q] = fmaf(c.z, x[2], z[q]);
+                        z[q] = fmaf(c.w, x[3], z[q]);
+                    }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (warp + 8 * q < kMlpOut) ot[(warp + 8 * q) * kTrainRow + lane] = z[q];
+        }
+        __syncthreads();
+        if (warp < 3) {   // the loss: warp 0 the Beta law, warps 1 and 2 a site each
+            auto out = [&](int o) { return ot[o * kTrainRow + lane]; };
+            auto grad = [&](int o, float v) { d3[o * kTrainRow + lane] = on ? v : 0.f; };
+            const float x = on ? rec[kMlpIn + warp] : 0.5f;
+            lp[warp * 32 + lane] = warp == 0 ? loss_beta_grad(out, grad, x) : loss_site_grad(warp - 1, out, grad, x);
+        }
+        __syncthreads();
+        if (warp == 7 && on) loss[b] = -((lp[lane] + lp[32 + lane]) + lp[64 + lane]);
+        {   // deltas of hidden 2
+            float z[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) z[q] = 0.f;
+#pragma unroll 2
+            for (int o = 0; o < kMlpOut; o++) {
+                const float x = d3[o * kTrainRow + lane];
+                const float4* c = reinterpret_cast<const float4*>(w + kOffW3 + o * kMlpHidden + warp * 8);
+                const float4 c0 = c[0], c1 = c[1];
+                z[0] = fmaf(c0.x, x, z[0]); z[1] = fmaf(c0.y, x, z[1]); z[2] = fmaf(c0.z, x, z[2]); z[3] = fmaf(c0.w, x, z[3]);
+                z[4] = fmaf(c1.x, x, z[4]); z[5] = fmaf(c1.y, x, z[5]); z[6] = fmaf(c1.z, x, z[6]); z[7] = fmaf(c1.w, x, z[7]);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const float h = h2[(warp * 8 + q) * kTrainRow + lane];
+                d2[(warp * 8 + q) * kTrainRow + lane] = z[q] * (1.0f - h * h);
+            }
+        }
+        __syncthreads();
+        {   // deltas of hidden 1
+            float z[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) z[q] = 0.f;
+#pragma unroll 4
+            for (int o = 0; o < kMlpHidden; o++) {
+                const float x = d2[o * kTrainRow + lane];
+                const float4* c = reinterpret_cast<const float4*>(w + kOffW2 + o * kMlpHidden + warp * 8);
+                const float4 c0 = c[0], c1 = c[1];
+                z[0] = fmaf(c0.x, x, z[0]); z[1] = fmaf(c0.y, x, z[1]); z[2] = fmaf(c0.z, x, z[2]); z[3] = fmaf(c0.w, x, z[3]);
+                z[4] = fmaf(c1.x, x, z[4]); z[5] = fmaf(c1.y, x, z[5]); z[6] = fmaf(c1.z, x, z[6]); z[7] = fmaf(c1.w, x, z[7]);
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const float h = h1[(warp * 8 + q) * kTrainRow + lane];
+                d1[(warp * 8 + q) * kTrainRow + lane] = z[q] * (1.0f - h * h);
+            }
+        }
+        __syncthreads();
+        // the tile's gradient: rows ti + 16a (deltas) x columns tj + 16c (activations), summed over the 32 records
+        auto row4 = [](const float* p, int r, int b4) { return *reinterpret_cast<const float4*>(p + r * kTrainRow + b4); };
+        auto dot4 = [](const float4 d, const float4 x, float s) {
+            return fmaf(d.w, x.w, fmaf(d.z, x.z, fmaf(d.y, x.y, fmaf(d.x, x.x, s))));
+        };
+        const float4 one = make_float4(1.f, 1.f, 1.f, 1.f);
+#pragma unroll 2
+        for (int b4 = 0; b4 < 32; b4 += 4) {
+            float4 xa[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) xa[c] = row4(h1, tj + 16 * c, b4);
+#pragma unroll
+            for (int a = 0; a < 4; a++) {
+                const float4 d = row4(d2, ti + 16 * a, b4);
+#pragma unroll
+                for (int c = 0; c < 4; c++) g2[a][c] = dot4(d, xa[c], g2[a][c]);
+                if (tj == 9) g1[a] = dot4(d, one, g1[a]);                                  // b2
+            }
+#pragma unroll
+            for (int c = 0; c < 4; c++) xa[c] = row4(h2, tj + 16 * c, b4);
+#pragma unroll
+            for (int a = 0; a < 2; a++)
+                if (ti + 16 * a < kMlpOut) {
+                    const float4 d = row4(d3, ti + 16 * a, b4);
+#pragma unroll
+                    for (int c = 0; c < 4; c++) g3[a][c] = dot4(d, xa[c], g3[a][c]);
+                    if (tj == 10) g1[a] = dot4(d, one, g1[a]);                             // b3
+                }
+            if (tj <= 8) {                                                                  // W1, b1
+                const float4 x = tj < 8 ? row4(f, tj, b4) : one;
+#pragma unroll
+                for (int a = 0; a < 4; a++) g1[a] = dot4(row4(d1, ti + 16 * a, b4), x, g1[a]);
+            }
+        }
+        __syncthreads();
     }
+    float* out = partial + (size_t)blockIdx.x * kMlpParams;
+#pragma unroll
+    for (int a = 0; a < 4; a++) {
+#pragma unroll
+        for (int c = 0; c < 4; c++) out[kOffW2 + (ti + 16 * a) * kMlpHidden + tj + 16 * c] = g2[a][c];
+        if (tj < 8) out[kOffW1 + (ti + 16 * a) * kMlpIn + tj] = g1[a];
+        if (tj == 8) out[kOffB1 + ti + 16 * a] = g1[a];
+        if (tj == 9) out[kOffB2 + ti + 16 * a] = g1[a];
+    }
+#pragma unroll
+    for (int a = 0; a < 2; a++)
+        if (ti + 16 * a < kMlpOut) {
+#pragma unroll
+            for (int c = 0; c < 4; c++) out[kOffW3 + (ti + 16 * a) * kMlpHidden + tj + 16 * c] = g3[a][c];
+            if (tj == 10) out[kOffB3 + ti + 16 * a] = g1[a];
+        }
 }
 
-// gradient of the mean loss, one thread per parameter, summed over records
-// in a fixed order (deterministic)
-__global__ void mlp_grad_reduce_kernel(const float* __restrict__ save, int n, float* __restrict__ grad) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kMlpParams) return;
-    // saved layout per record: f | h1 | h2 | d1 | d2 | d3
-    constexpr int F0 = 0, H1 = kMlpIn, H2 = H1 + kMlpHidden, D1 = H2 + kMlpHidden, D2 = D1 + kMlpHidden,
-                  D3 = D2 + kMlpHidden;
-    int dofs, aofs = 0, ai = -1;   // delta index; activation index (ai < 0: bias)
-    if (p < kOffB1) { dofs = D1 + p / kMlpIn; aofs = F0; ai = p % kMlpIn; }
-    else if (p < kOffW2) { dofs = D1 + (p - kOffB1); }
-    else if (p < kOffB2) { const int q = p - kOffW2; dofs = D2 + q / kMlpHidden; aofs = H1; ai = q % kMlpHidden; }
-    else if (p < kOffW3) { dofs = D2 + (p - kOffB2); }
-    else if (p < kOffB3) { const int q = p - kOffW3; dofs = D3 + q / kMlpHidden; aofs = H2; ai = q % kMlpHidden; }
-    else { dofs = D3 + (p - kOffB3); }
+// Sums the CTAs' partial gradients (8 threads per parameter, fixed order),
+// divides by the batch and, for a training step, applies Adam.
+struct AdamParams {
+    float *w, *m, *v;
+    __nv_bfloat16* wbf;
+    float lr, b1, b2, eps, c1, c2;
+};
+
+__global__ void __launch_bounds__(256) mlp_grad_adam_kernel(const float* __restrict__ partial, int parts, int n,
+                                                            float* __restrict__ grad, const AdamParams A) {
+    __shared__ float sums[8][33];
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + x;
     float s = 0.f;
-    for (int b = 0; b < n; b++) {
-        const float* sv = save + (int64_t)b * kSaveFloats;
-        s = fmaf(sv[dofs], ai >= 0 ? sv[aofs + ai] : 1.0f, s);
-    }
-    grad[p] = s / (float)n;
-}
-
-__global__ void adam_kernel(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v,
-                            const float* __restrict__ g, __nv_bfloat16* __restrict__ wbf, float lr, float b1,
-                            float b2, float eps, float c1, float c2) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= kMlpParams) return;
-    const float gp = g[p];
-    const float mp = b1 * m[p] + (1.0f - b1) * gp, vp = b2 * v[p] + (1.0f - b2) * gp * gp;
-    m[p] = mp;
-    v[p] = vp;
-    const float wp = w[p] - lr * (mp / c1) / (sqrtf(vp / c2) + eps);
-    w[p] = wp;
-    wbf[p] = __float2bfloat16_rn(wp);
+    if (p < kMlpParams)
+#pragma unroll 8
+        for (int c = y; c < parts; c += 8) s += partial[(size_t)c * kMlpParams + p];
+    sums[y][x] = s;
+    __syncthreads();
+    if (y != 0 || p >= kMlpParams) return;
+    s = sums[0][x];
+#pragma unroll
+    for (int q = 1; q < 8; q++) s += sums[q][x];
+    const float gp = s / (float)n;
+    grad[p] = gp;
+    if (A.w == nullptr) return;
+    const float mp = A.b1 * A.m[p] + (1.0f - A.b1) * gp, vp = A.b2 * A.v[p] + (1.0f - A.b2) * gp * gp;
+    A.m[p] = mp;
+    A.v[p] = vp;
+    const float wp = A.w[p] - A.lr * (mp / A.c1) / (sqrtf(vp / A.c2) + A.eps);
+    A.w[p] = wp;
+    A.wbf[p] = __float2bfloat16_rn(wp);
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ w, __nv_bfloat16* __restrict__ wbf) {
@@ -623,38 +809,31 @@ __global__ void to_bf16_kernel(const float* __restrict__ w, __nv_bfloat16* __res
     if (p < kMlpParams) wbf[p] = __float2bfloat16_rn(w[p]);
 }
 
-__global__ void sample_index_kernel(int* __restrict__ idx, int n, unsigned long long filled, uint32_t k0, uint32_t k1,
-                                    uint32_t step) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= n) return;
-    const U4 r = philox4x32_10(U4{(uint32_t)b, step, 0x74726e00u, 0u}, k0, k1);
-    idx[b] = (int)(((uint64_t)r.x * filled) >> 32);
-}
+size_t mlp_partial_floats() { return (size_t)kTrainCtas * kMlpParams; }
 
-cudaError_t launch_mlp_fwd_bwd(const float* w, const float* records, const int* index, int n, float* save,
-                               float* loss, cudaStream_t st) {
-    mlp_fwd_bwd_kernel<<<(n + 127) / 128, 128, 0, st>>>(w, records, index, n, save, loss);
-    return cudaGetLastError();
-}
-cudaError_t launch_mlp_grad(const float* save, int n, float* grad, cudaStream_t st) {
-    mlp_grad_reduce_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(save, n, grad);
-    return cudaGetLastError();
-}
-cudaError_t launch_adam(float* w, float* m, float* v, const float* g, __nv_bfloat16* wbf, float lr, int t,
-                        cudaStream_t st) {
-    const float b1 = 0.9f, b2 = 0.999f;
-    adam_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(w, m, v, g, wbf, lr, b1, b2, 1e-8f,
-                                                          1.0f - powf(b1, (float)t), 1.0f - powf(b2, (float)t));
+// Loss and gradient of the mean -log q_L over n records: entries 0..n-1, or
+// (filled > 0) n draws from the ring's first `filled` entries; partial: the
+// CTAs' partial gradients [mlp_partial_floats()].  adam_step > 0: then one
+// Adam step (the adam_step-th) on w, m, v and the BF16 copy.
+cudaError_t launch_mlp_train(float* w, const float* records, unsigned long long filled, uint64_t key, uint32_t step,
+                             int n, float* partial, float* loss, float* grad, float* m, float* v, __nv_bfloat16* wbf,
+                             float lr, int adam_step, cudaStream_t st) {
+    const int tiles = (n + 31) / 32, ctas = tiles < kTrainCtas ? tiles : kTrainCtas;
+    cudaError_t e = cudaFuncSetAttribute(mlp_train_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
+    if (e != cudaSuccess) return e;
+    mlp_train_kernel<<<ctas, 256, kTrainSmem, st>>>(w, records, filled, (uint32_t)key, (uint32_t)(key >> 32), step, n,
+                                                    partial, loss);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    AdamParams A{};
+    if (adam_step > 0) {
+        const float b1 = 0.9f, b2 = 0.999f;
+        A = AdamParams{w, m, v, wbf, lr, b1, b2, 1e-8f, 1.0f - powf(b1, (float)adam_step), 1.0f - powf(b2, (float)adam_step)};
+    }
+    mlp_grad_adam_kernel<<<(kMlpParams + 31) / 32, 256, 0, st>>>(partial, ctas, n, grad, A);
     return cudaGetLastError();
 }
 cudaError_t launch_to_bf16(const float* w, __nv_bfloat16* wbf, cudaStream_t st) {
     to_bf16_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(w, wbf);
     return cudaGetLastError();
 }
-cudaError_t launch_sample_index(int* idx, int n, unsigned long long filled, uint64_t key, uint32_t step,
-                                cudaStream_t st) {
-    sample_index_kernel<<<(n + 255) / 256, 256, 0, st>>>(idx, n, filled, (uint32_t)key, (uint32_t)(key >> 32), step);
-    return cudaGetLastError();
-}
-
 }  // namespace pspin

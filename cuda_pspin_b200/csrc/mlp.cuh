@@ -49,31 +49,6 @@ __device__ __forceinline__ void pair_features(float2 ai, float2 aj, float2 hi, f
     f[7] = logf(beta > 1e-30f ? beta : 1e-30f);
 }
 
-// Forward pass of one record with FP32 weights; the hidden activations go to
-// the record's rows h1[64], h2[64] (which the backward pass reads) and are
-// read back from there.  (A variant holding them in per-thread arrays gave
-// wrong outputs for the second site's mixture under nvcc 12.9 -O3; this form
-// is checked against float64 autograd.)
-__device__ __forceinline__ void mlp_forward_rows(const float* __restrict__ w, const float* f, float* h1, float* h2,
-                                                 float* out) {
-    for (int o = 0; o < kMlpHidden; o++) {
-        float z = w[kOffB1 + o];
-#pragma unroll
-        for (int i = 0; i < kMlpIn; i++) z = fmaf(w[kOffW1 + o * kMlpIn + i], f[i], z);
-        h1[o] = tanhf(z);
-    }
-    for (int o = 0; o < kMlpHidden; o++) {
-        float z = w[kOffB2 + o];
-        for (int i = 0; i < kMlpHidden; i++) z = fmaf(w[kOffW2 + o * kMlpHidden + i], h1[i], z);
-        h2[o] = tanhf(z);
-    }
-    for (int o = 0; o < kMlpOut; o++) {
-        float z = w[kOffB3 + o];
-        for (int i = 0; i < kMlpHidden; i++) z = fmaf(w[kOffW3 + o * kMlpHidden + i], h2[i], z);
-        out[o] = z;
-    }
-}
-
 __device__ __forceinline__ float softplusf(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
 
@@ -291,40 +266,45 @@ __device__ __forceinline__ float digammaf_series(float x) {
     return r + logf(x) - 0.5f / x - i2 * (1.0f / 12.0f - i2 * (1.0f / 120.0f - i2 / 252.0f));
 }
 
-// d(-log q_L)/d(outputs) for one record; returns -log q_L
-__device__ __forceinline__ float loss_output_grad(const float* o, float t, float psi_i, float psi_j, float* g) {
-    ProposalParams p;
-    decode_outputs(o, p);
-    float loss = -log_learned_density(p, t, psi_i, psi_j);
-    const float dab = digammaf_series(p.a + p.b);
-    g[0] = -(logf(t) - digammaf_series(p.a) + dab) * sigmoidf(o[0]);
-    g[1] = -(log1pf(-t) - digammaf_series(p.b) + dab) * sigmoidf(o[1]);
-    const float psis[2] = {psi_i, psi_j};
-    #pragma unroll
-    for (int s = 0; s < 2; s++) {
-        const float* q = o + 2 + 12 * s;
-        float* gq = g + 2 + 12 * s;
-        float v[4], m = -1e30f;
-        #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            v[k] = logf(p.w[s][k]) + p.kappa[s][k] * cosf(psis[s] - p.mu[s][k]) - log_i0f(p.kappa[s][k]);
-            m = fmaxf(m, v[k]);
-        }
-        float z = 0.f;
-        #pragma unroll
-        for (int k = 0; k < 4; k++) { v[k] = expf(v[k] - m); z += v[k]; }
-        #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float rk = v[k] / z;          // responsibility
-            const float kap = p.kappa[s][k], dpsi = psis[s] - p.mu[s][k];
-            gq[k] = p.w[s][k] - rk;
-            gq[4 + k] = -rk * kap * sinf(dpsi);
-            const float ratio = cyl_bessel_i1f(kap) / cyl_bessel_i0f(kap);
-            const float sg = sigmoidf(q[8 + k]);
-            gq[8 + k] = -rk * (cosf(dpsi) - ratio) * kKappaMax * sg * (1.0f - sg);
-        }
+// One record's -log q_L = -((log Beta + site 0) + site 1) and its gradient in
+// the outputs, in the three parts that are independent given the outputs
+// o[row * stride] (gradients to g[row * gstride]); each returns its part of
+// log q_L.
+template <class Out, class Grad>
+__device__ __forceinline__ float loss_beta_grad(Out out, Grad grad, float t) {
+    const float a = decode_beta_param(out(0)), b = decode_beta_param(out(1));
+    const float dab = digammaf_series(a + b);
+    grad(0, -(logf(t) - digammaf_series(a) + dab) * sigmoidf(out(0)));
+    grad(1, -(log1pf(-t) - digammaf_series(b) + dab) * sigmoidf(out(1)));
+    return log_beta_pdf(t, a, b);
+}
+
+template <class Out, class Grad>
+__device__ __forceinline__ float loss_site_grad(int s, Out out, Grad grad, float psi) {
+    float q[12], w[4], mu[4], kappa[4];
+#pragma unroll
+    for (int o = 0; o < 12; o++) q[o] = out(2 + 12 * s + o);
+    decode_site(q, w, mu, kappa);
+    float v[4], m = -1e30f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        v[k] = logf(w[k]) + kappa[k] * cosf(psi - mu[k]) - log_i0f(kappa[k]);
+        m = fmaxf(m, v[k]);
     }
-    return loss;
+    float z = 0.f;
+#pragma unroll
+    for (int k = 0; k < 4; k++) { v[k] = expf(v[k] - m); z += v[k]; }
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float rk = v[k] / z;          // responsibility
+        const float dpsi = psi - mu[k];
+        grad(2 + 12 * s + k, w[k] - rk);
+        grad(2 + 12 * s + 4 + k, -rk * kappa[k] * sinf(dpsi));
+        const float ratio = cyl_bessel_i1f(kappa[k]) / cyl_bessel_i0f(kappa[k]);
+        const float sg = sigmoidf(q[8 + k]);
+        grad(2 + 12 * s + 8 + k, -rk * (cosf(dpsi) - ratio) * kKappaMax * sg * (1.0f - sg));
+    }
+    return log_vm_mix_site(w, mu, kappa, psi);
 }
 
 }  // namespace pspin
