@@ -153,6 +153,8 @@ struct pspin_state {
     int warps2 = 8, cluster2 = 1;       // block shape of the two-pass (learned / fields) sweep
     int rpl = 1;                        // replicas per lane of the plain CTA / cluster sweep
     std::vector<Unit> units_k[2];       // blocks of 64 and 96 replicas (rpl 2, 3)
+    RingPlan plan{};                    // of the current block shape (plan_key: warps, cluster, rpl it was made for)
+    int plan_key[3] = {0, 0, 0};
     int64_t spin_total = 0;
     cudaStream_t st = nullptr;
     int device = 0;
@@ -732,6 +734,8 @@ static int run_energy(pspin_state* s, double* e2, double* e4, bool overwrite, bo
     return PSPIN_OK;
 }
 
+static int current_plan(pspin_state* s);
+
 extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, const pspin_options* opt,
                                   pspin_state** out) {
     if (!cfgs || n <= 0 || !out) return fail(PSPIN_ERR_ARG, "pspin_create_batch: bad arguments");
@@ -1008,7 +1012,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
     }
     if (sweep_smem_bytes(s->max_N, s->warps) > 227 * 1024)
         return bail(fail(PSPIN_ERR_ARG, "N=%d needs more shared memory than a CTA has", s->max_N));
-    if (s->rpl > 1 && s->cluster >= 1 && multi_smem_bytes_host(s->max_N, s->warps, s->cluster, s->rpl) > 227 * 1024)
+    if (s->rpl > 1 && s->cluster >= 1 && current_plan(s) != PSPIN_OK)
         return bail(fail(PSPIN_ERR_ARG, "N=%d with %d replicas per lane needs more shared memory than a CTA has",
                          s->max_N, s->rpl));
 
@@ -1100,6 +1104,23 @@ extern "C" int pspin_total_replicas(const pspin_state* s) { return s ? s->R_tot 
 extern "C" int pspin_num_samples(const pspin_state* s) { return s ? s->S : 0; }
 
 // ------------------------------------------------------------------ sweeps
+// replica blocks of K replicas per lane
+static int n_units_of(const pspin_state* s, int K) {
+    return (int)(K > 1 ? s->units_k[K - 2].size() : s->units.size());
+}
+static const Unit* units_dev(const pspin_state* s, int K) { return K > 1 ? s->d_units_k[K - 2] : s->d_units; }
+
+// how the current block shape's chains are spread over the machine
+static int current_plan(pspin_state* s) {
+    const int key[3] = {s->warps, s->cluster, s->rpl};
+    if (std::memcmp(key, s->plan_key, sizeof(key)) == 0) return PSPIN_OK;
+    if (!plan_sweep_ring(s->plan, s->warps, s->cluster, n_units_of(s, s->rpl), s->variant, s->max_N, s->rpl))
+        return fail(PSPIN_ERR_CUDA, "block shape %d warps x %d CTAs with %d replicas per lane does not fit at N=%d", s->warps,
+                    s->cluster, s->rpl, s->max_N);
+    std::memcpy(s->plan_key, key, sizeof(key));
+    return PSPIN_OK;
+}
+
 // Enqueues one step: a sweep launch of nsweeps sweeps, the exchange launch
 // (which advances the device sweep counter) and, after an exchange, the
 // observable recorder.  No host bookkeeping, so a sequence of steps can be
@@ -1135,14 +1156,10 @@ static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t 
     p.cluster = s->proposal == PSPIN_PROPOSAL_PLAIN ? s->cluster : s->cluster2;
     if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0) {
         CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, s->st));
-    } else if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->rpl > 1) {
-        const std::vector<Unit>& u = s->units_k[s->rpl - 2];
-        p.units = s->d_units_k[s->rpl - 2];
-        CK(launch_sweep_multi(p, (int)u.size(), s->variant, s->max_N, s->rpl, s->st, nullptr));
-    } else if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 1) {
-        CK(launch_sweep_cluster(p, (int)s->units.size(), s->variant, s->max_N, s->st, nullptr));
     } else if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
-        CK(launch_sweep(p, (int)s->units.size(), s->variant, s->max_N, s->st));
+        TRY(current_plan(s));
+        p.units = units_dev(s, s->rpl);
+        CK(launch_sweep_ring(p, s->plan, n_units_of(s, s->rpl), s->variant, s->max_N, s->rpl, s->st));
     } else {
         if (!s->d_site_chunks_g || !s->d_pair_chunks)
             return fail(PSPIN_ERR_STATE, "two-pass sweep without its group-format lists (pspin_set_proposal builds them)");
@@ -1241,6 +1258,7 @@ static int graph_steps(const pspin_state* s) {
 // same move and pair streams as direct launches would.
 static int capture_graph(pspin_state* s, int G) {
     drop_graph(s);
+    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0) TRY(current_plan(s));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
     int rc = PSPIN_OK;
@@ -1319,40 +1337,19 @@ static bool shape_fits(pspin_state* s, int warps, int cluster, int K = 1) {
         return K == 1 && s->proposal == PSPIN_PROPOSAL_PLAIN &&
                resident_smem_bytes_host(s->max_N, s->max_site_entries, warps) <= 227 * 1024;
     if (cluster * warps > kSplit) return false;
-    if (K > 1) {
-        if (s->proposal != PSPIN_PROPOSAL_PLAIN) return false;
-        if (multi_smem_bytes_host(s->max_N, warps, cluster, K) > 227 * 1024) return false;
-        SweepParams p{};
-        p.warps = warps;
-        p.cluster = cluster;
-        int n = 0;
-        if (launch_sweep_multi(p, (int)s->units_k[K - 2].size(), s->variant, s->max_N, K, s->st, &n) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return n > 0;
+    if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
+        RingPlan r;
+        return plan_sweep_ring(r, warps, cluster, n_units_of(s, K), s->variant, s->max_N, K);
     }
-    if (s->proposal != PSPIN_PROPOSAL_PLAIN) {
-        if (learned_smem_bytes_host(s->max_N, warps, cluster) > 227 * 1024) return false;
-        if (cluster == 1) return true;
-        SweepParams p{};
-        p.warps = warps;
-        p.cluster = cluster;
-        LearnParams lp{};
-        int n = 0;
-        if (launch_learned_sweep(p, lp, (int)s->units.size(), s->max_N, s->st, &n) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        return n > 0;
-    }
-    if (cluster == 1) return sweep_smem_bytes(s->max_N, warps) <= 227 * 1024;
-    if (cluster_smem_bytes_host(s->max_N, warps, cluster) > 227 * 1024) return false;
+    if (K > 1) return false;
+    if (learned_smem_bytes_host(s->max_N, warps, cluster) > 227 * 1024) return false;
+    if (cluster == 1) return true;
     SweepParams p{};
     p.warps = warps;
     p.cluster = cluster;
+    LearnParams lp{};
     int n = 0;
-    if (launch_sweep_cluster(p, (int)s->units.size(), s->variant, s->max_N, s->st, &n) != cudaSuccess) {
+    if (launch_learned_sweep(p, lp, (int)s->units.size(), s->max_N, s->st, &n) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -55,7 +55,7 @@ namespace pspin {
 constexpr int kSplit = 32;        // parts per site list (warps per unit divide it)
 constexpr int kGroupMax = 32;     // max data entries after one header
 constexpr int kStage = 256;       // max entries per TMA chunk (2 KB)
-constexpr int kStages = 3;        // chunks in flight per warp
+constexpr int kStages = 3;        // chunks in flight per warp (set-up's limit on N)
 constexpr int kRepBlock = 32;     // replicas per unit (one per lane)
 
 // Status word bits raised by the sweep kernels.  A CTA (or cluster) whose
@@ -115,8 +115,9 @@ struct SweepParams {
     const uint32_t* nbmask;           // per sample: row m = sites sharing a quartet (or a g2 term) with m
     const long long* sweep_counter;   // global sweep index at launch start
     int nsweeps;
-    int warps;                        // warps per unit (divides 32)
-    int cluster;                      // CTAs per unit (sweep_cluster_kernel), 1: sweep_kernel
+    int warps;                        // block shape: warps per CTA (divides 32) ...
+    int cluster;                      //   ... and CTAs per unit, which fix the summation order of the fields
+    int exec, chains, stages;         // sweep_ring_kernel: the RingPlan the launch runs with
     // trace
     int trace_sample, trace_rep, trace_cap;
     long long trace_sweep0;
@@ -126,26 +127,26 @@ struct SweepParams {
     int stall_move;                   // tests: move index of the stall wait (-1: none)
 };
 
-// shared memory bytes of one sweep CTA: amplitudes, per-warp field
-// partials, per-warp chunk rings, ring mbarriers
-#ifdef __CUDACC__
-__host__ __device__
-#endif
+// Shared memory that one replica block of a sample needs at least: the limit
+// on N at set-up (amplitudes, per-warp field partials, rings and barriers).
 inline size_t sweep_smem_bytes(int N, int warps) {
     return (size_t)(N + 1) * kRepBlock * sizeof(float2) + (size_t)warps * kRepBlock * sizeof(float4) +
            (size_t)warps * kStages * kStage * sizeof(int2) + (size_t)warps * kStages * sizeof(uint64_t);
 }
 
+// How sweep_ring_kernel spreads a unit's chains: over exec CTAs of `chains`
+// chain warps, each with a ring of `stages` chunks; lat: the form for few
+// units.
+struct RingPlan {
+    int exec, chains, stages, lat;
+};
+constexpr size_t kRingSmemMax = 227 * 1024 - 64;   // (the kernel's static shared memory)
+bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int variant, int max_N, int K);
+
 // kernels (launchers are host functions in the .cu files)
-cudaError_t launch_sweep(const SweepParams& p, int n_units, int variant, int max_N, cudaStream_t st);
-cudaError_t launch_sweep_cluster(const SweepParams& p, int n_units, int variant, int max_N, cudaStream_t st,
-                                 int* max_clusters);
-size_t cluster_smem_bytes_host(int N, int warps, int C);
-// the CTA / cluster kernel with K = 2 or 3 replicas per lane (units of up to
-// 32K replicas of one sample); cluster 1 launches no cluster
-cudaError_t launch_sweep_multi(const SweepParams& p, int n_units, int variant, int max_N, int K, cudaStream_t st,
-                               int* max_clusters);
-size_t multi_smem_bytes_host(int N, int warps, int C, int K);
+// units of up to 32K replicas, K = 1, 2, 3 replicas per lane
+cudaError_t launch_sweep_ring(const SweepParams& p, const RingPlan& r, int n_units, int variant, int max_N, int K,
+                              cudaStream_t st);
 // the list-resident kernel; warps > 1 runs batches of consecutive moves that
 // commute (no site of one in the other's quartet neighbourhood) on separate
 // warps, with the neighbour masks `nbmask`

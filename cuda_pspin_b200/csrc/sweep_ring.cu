@@ -1,0 +1,535 @@
+// sweep_ring.cu -- the plain pair-rotation Metropolis sweep (dense sphere and
+// sparse cube) with the site lists streamed through shared memory.
+//
+// Replaces mc_sweep_kernel (mc.cu:66-318) and mc_sparse_sweep_kernel
+// (mc_sparse.cu:63-253).  Same move set, same Metropolis rule; different
+// organisation:
+//
+//  * One unit = up to 32K replicas of one sample (K = 1, 2, 3): lane l holds
+//    replicas l, 32 + l, 64 + l of the unit, amplitudes [site][K][32] float2.
+//    All replicas of a sample propose on the same pair at the same step (the
+//    pair stream belongs to the sample, not to the replica), so a staged
+//    coupling, one broadcast shared-memory read, serves the lane's K replicas.
+//    Pair choice does not depend on the state, so every replica still runs a
+//    random-scan Metropolis chain with the reference's stationary law.
+//  * dE from local fields.  E is affine in a_i for fixed other sites, so
+//      E(a_i',a_j') - E(a_i,a_j) = -Re[da_i h_i(a_j')] - Re[da_j h_j(a_i)]
+//    exactly, where h_i(a_j') is site i's field evaluated with the proposed
+//    a_j, which therefore sits in j's slot during the field pass.
+//  * Summation tree.  A list is cut in 32 balanced parts; with W warps per CTA
+//    and C CTAs per block (the block shape of the options) a list has C*W
+//    chains of 32/(C*W) consecutive parts, each summed in list order, then the
+//    chains of a CTA in order, then the CTAs in order.  The shape fixes that
+//    order, hence the chain of states; how the 2*C*W chains of a move (two
+//    lists) are spread over the machine does not.
+//  * A move's 2*C*W chains run on X CTAs (a thread-block cluster for X > 1),
+//    one warp per chain, so the two lists of a move are read at once.  The
+//    remaining warps of a CTA are K deciders and one producer:
+//      producer: lane l follows chain l through the (state-independent) pair
+//        schedule and keeps its ring of TMA copies (cp.async.bulk, one mbarrier
+//        per slot) full, moves ahead of the readers; no chain warp looks
+//        anything up;
+//      chain warp: reads its chunks, sends its partial field of each replica to
+//        every CTA's exchange buffer (st.async, completion counted in bytes on
+//        the receiving decider's mbarrier; a plain store and an arrival where
+//        the unit is one CTA), then waits for the CTA's deciders;
+//      decider k: while the chains run, the random words, sines and cosines of
+//        the next move for its 32 replicas; when its mbarrier has all 2*C*W
+//        partials, the sum in tree order, the Metropolis decision, the next
+//        proposal, and both into its CTA's copy of the amplitudes.
+//    Every CTA's decider k takes the same decision on the same numbers, so the
+//    copies agree and a move costs one hop between CTAs and one CTA barrier.
+//    With every warp deciding for itself and fetching its own chunks (8 warps
+//    reading list i, then list j), the benchmark's launch ran the FMA pipe at
+//    37 % and a move of a one-sample run cost 8 us of waiting.
+//  * All waits are bounded; a chain whose copy does not arrive sends a marked
+//    partial, so every CTA of the unit leaves at the same move, and nothing is
+//    written back.
+//  * FP32 amplitudes and fields; the running energy is FP64.
+#include "sweep_common.cuh"
+#include "../../include/pspin.h"
+
+namespace pspin {
+
+constexpr int kMaxChains = 16;            // chain warps per CTA
+constexpr int kLatChains = 4;             // up to here a CTA is one chain per SM sub-partition
+constexpr uint32_t kAbortMark = 0x7fc0dead;   // a NaN no arithmetic here produces: this chain gave up
+
+// Shared memory of one CTA: amplitudes [N+1][K][32] float2; rings
+// [chains][stages][kStage] int2; exchange buffer [2][T][K][32] float2 (T =
+// 2*C*W chains of a move); mbarriers full, empty [chains][stages], partials
+// [2][K]; ring tags [chains][stages] int2.
+struct RingLayout {
+    size_t ring, xbuf, bars, tags, total;
+};
+__host__ __device__ inline RingLayout ring_layout(int N, int T, int chains, int stages, int K) {
+    RingLayout L;
+    L.ring = (size_t)(N + 1) * K * kRepBlock * sizeof(float2);
+    L.xbuf = L.ring + (size_t)chains * stages * kStage * sizeof(int2);
+    L.bars = L.xbuf + (size_t)2 * T * K * kRepBlock * sizeof(float2);
+    L.tags = L.bars + (size_t)(2 * chains * stages + 2 * K) * sizeof(uint64_t);
+    L.total = L.tags + (size_t)chains * stages * sizeof(int2);
+    return L;
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+    return ra;
+}
+// 8 bytes into a CTA of the cluster, counted on that CTA's mbarrier
+__device__ __forceinline__ void st_async_f2(uint32_t addr, float2 v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "r"(bar)
+                 : "memory");
+}
+// named barrier 1: deciders arrive, chain warps wait ("the state of the next move is in place")
+__device__ __forceinline__ void state_arrive(int threads) {
+    asm volatile("bar.arrive 1, %0;" ::"r"(threads) : "memory");
+}
+__device__ __forceinline__ void state_wait(int threads) {
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+}
+
+// kLat: few blocks, at most kLatChains chain warps a CTA, so a warp has its
+// sub-partition's issue slots and registers to itself and deep batches of
+// loads in flight carry it; otherwise 16 chain warps share the SM.
+template <int VARIANT, int K, bool kLat>
+__global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 32, 1)
+    sweep_ring_kernel(const SweepParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int X = P.exec, c = P.chains, stages = P.stages;
+    const uint32_t rank = X > 1 ? cluster_rank() : 0u;
+    const Unit U = P.units[blockIdx.x / X];
+    const SampleDev S = P.samples[U.sample];
+    const int N = S.N, R = S.R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int CW = P.cluster * P.warps, T = 2 * CW;
+    constexpr int KB = K * kRepBlock;
+    const RingLayout Lo = ring_layout(N, T, c, stages, K);
+    float2* sp = reinterpret_cast<float2*>(smem_raw);
+    float2* xbuf = reinterpret_cast<float2*>(smem_raw + Lo.xbuf);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + Lo.bars);
+    uint64_t* empty = full + c * stages;
+    uint64_t* xbar = empty + c * stages;
+    int2* tags = reinterpret_cast<int2*>(smem_raw + Lo.tags);
+    __shared__ volatile int stop;
+    __shared__ __align__(8) uint64_t stall_bar;      // test hook: nothing arrives on it
+
+    if (threadIdx.x == 0) {
+        for (int q = 0; q < 2 * c * stages; q++) mbar_init(full + q, 1);
+        // partials: bytes of every chain's st.async (armed by the decider), or
+        // one arrival per chain where the unit is a single CTA
+        for (int q = 0; q < 2 * K; q++) mbar_init(xbar + q, X > 1 ? 1u : (uint32_t)T);
+        mbar_init(&stall_bar, 1);
+        stop = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_async_shared();
+    }
+    load_block_amplitudes(sp, P.spins + S.spin_off + U.rep_begin, R, N, KB, U.rep_count);   // column k*32 + lane
+    for (int idx = threadIdx.x; idx < KB; idx += blockDim.x) sp[(size_t)N * KB + idx] = make_float2(1.f, 0.f);
+
+    const long long sweep0 = *P.sweep_counter;
+    const int steps = N / 2, total = P.nsweeps * steps;
+    const int state_threads = (c + K) * 32;
+    const bool decider = warp >= c && warp < c + K;
+    const int k = warp - c;                          // decider's replica group
+    const int rr = k * kRepBlock + lane;
+    const bool active = decider && rr < U.rep_count;
+    const int64_t gr = S.rep_off + U.rep_begin + rr;
+
+    // the deciders' pending move
+    double E = 0.0, beta_d = 0.0;
+    float beta = 0.f, cu = 0.f;
+    int nacc = 0, nprop = 0, ci0 = 0, cj0 = 0;
+    uint32_t k0 = 0, k1 = 0;
+    float2 cai = make_float2(0.f, 0.f), caj = cai, cain = cai, cajn = cai;
+    float tt[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    auto pair_of = [&](int m, int& i0, int& j0) {
+        pair_pick(S.pair_key0, S.pair_key1, (uint64_t)(sweep0 + m / steps), (uint32_t)(m % steps), N, i0, j0);
+    };
+    auto draw = [&](int m) {
+        move_trig<VARIANT>(move_words(k0, k1, (uint64_t)(sweep0 + m / steps), (uint32_t)(m % steps)), tt);
+    };
+    auto amp = [&](int site) -> float2& { return sp[(site * K + k) * kRepBlock + lane]; };
+    if (active) {
+        beta_d = P.beta[gr];
+        beta = (float)beta_d;
+        const uint64_t key = P.key[gr];
+        k0 = (uint32_t)key;
+        k1 = (uint32_t)(key >> 32);
+        E = P.energy[gr];
+    }
+    __syncthreads();
+    if (decider && total > 0) {
+        pair_of(0, ci0, cj0);
+        draw(0);
+        cai = amp(ci0);
+        caj = amp(cj0);
+        propose_with<VARIANT>(cai, caj, tt, cain, cajn);
+        cu = tt[6];
+        amp(cj0) = cajn;                             // h_i is evaluated at the proposed a_j
+    }
+    if (X > 1) cluster_sync();                       // every CTA's barriers and state are in place
+    else __syncthreads();
+
+    if (warp < c) {
+        // ------------------------------------------------------------ chain warp
+        const int g = (int)rank * c + warp;          // chain g of the move: list g & 1, chain g >> 1 of that list
+        uint64_t* fb = full + warp * stages;
+        uint64_t* eb = empty + warp * stages;
+        const int2* tg = tags + warp * stages;
+        const int2* ring = reinterpret_cast<const int2*>(smem_raw + Lo.ring) + (size_t)warp * stages * kStage;
+        float2* my_x = xbuf + (size_t)((g & 1) * CW + (g >> 1)) * KB + lane;
+        uint32_t slot = 0, phase = 0;
+        for (int m = 0; m < total; m++) {
+            if (m > 0) {
+                __syncwarp();
+                state_wait(state_threads);
+                if (__any_sync(0xffffffffu, stop != 0)) break;
+            }
+            float hx[K], hy[K];
+#pragma unroll
+            for (int q = 0; q < K; q++) hx[q] = hy[q] = 0.f;
+            bool ok = true;
+            if (m == P.stall_move) ok = stall_wait(&stall_bar, P.status, P.wait_clocks);
+            for (bool last = false; ok && !last;) {
+                ok = ring_wait(fb + slot, phase, P.status, P.wait_clocks);
+                if (!ok) break;
+                const int2 t = tg[slot];             // {entries, last chunk of this move}
+                const int2* chunk = ring + slot * kStage;
+                last = t.y != 0;
+                if (K == 1 && kLat) {
+                    if (S.fc_tiles) accumulate_tiles(chunk, t.x, sp, lane, hx[0], hy[0]);
+                    else accumulate_records<4>(chunk, t.x, sp, lane, hx[0], hy[0]);
+                } else {
+                    if (S.fc_tiles) accumulate_tiles_k<K, kLat ? 4 : 2>(chunk, t.x, sp, lane, hx, hy);
+                    else accumulate_records_k<K>(chunk, t.x, sp, lane, hx, hy);
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(eb + slot);
+                if (++slot == (uint32_t)stages) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+            }
+            const uint32_t par = (uint32_t)(m & 1);
+            const float mark = __uint_as_float(kAbortMark);
+            if (!ok)
+#pragma unroll
+                for (int u = 0; u < K; u++) hx[u] = mark;
+            if (X > 1) {
+                const uint32_t dx = smem_u32(my_x) + par * (uint32_t)(T * KB * sizeof(float2));
+                const uint32_t db = smem_u32(xbar + par * K);
+                for (int q = 0; q < X; q++) {
+                    const uint32_t rx = map_rank(dx, (uint32_t)q), rb = map_rank(db, (uint32_t)q);
+#pragma unroll
+                    for (int u = 0; u < K; u++)
+                        st_async_f2(rx + u * (uint32_t)(kRepBlock * sizeof(float2)), make_float2(hx[u], hy[u]),
+                                    rb + u * (uint32_t)sizeof(uint64_t));
+                }
+            } else {
+                float2* dst = my_x + (size_t)par * T * KB;
+#pragma unroll
+                for (int u = 0; u < K; u++) dst[u * kRepBlock] = make_float2(hx[u], hy[u]);
+                __syncwarp();
+                if (lane < K) mbar_arrive(xbar + par * K + lane);
+            }
+        }
+    } else if (decider) {
+        // ------------------------------------------------------------ decider
+        const long long limit = 2 * P.wait_clocks + kDrainClocks;   // beyond any chain's own bounded wait
+        for (int m = 0; m < total; m++) {
+            const uint32_t par = (uint32_t)(m & 1);
+            uint64_t* bar = xbar + par * K + k;
+            if (X > 1 && lane == 0) mbar_expect_tx(bar, (uint32_t)(T * kRepBlock * sizeof(float2)));
+            // the next move's draw, and its sites' amplitudes in the state the
+            // chains are reading (move m's decision can change only ci0, cj0)
+            int ni0 = 0, nj0 = 0;
+            float2 nai = make_float2(0.f, 0.f), naj = nai;
+            if (m + 1 < total) {
+                pair_of(m + 1, ni0, nj0);
+                nai = amp(ni0);
+                naj = amp(nj0);
+                draw(m + 1);
+            }
+            bool ok = __all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(m >> 1) & 1u, P.status, limit));
+            // partials in tree order: a CTA's chains, then the CTAs
+            float2 hi = make_float2(0.f, 0.f), hj = hi;
+            const float2* xi = xbuf + ((size_t)par * T * K + k) * kRepBlock + lane;
+            const float2* xj = xi + (size_t)CW * KB;
+            for (int q = 0; q < P.cluster; q++) {
+                float2 pi = make_float2(0.f, 0.f), pj = pi;
+                for (int w0 = 0; w0 < P.warps; w0 += 4) {
+                    float2 vi[4], vj[4];
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (w0 + u < P.warps) {
+                            vi[u] = xi[(size_t)(q * P.warps + w0 + u) * KB];
+                            vj[u] = xj[(size_t)(q * P.warps + w0 + u) * KB];
+                            ok = ok && __float_as_uint(vi[u].x) != kAbortMark && __float_as_uint(vj[u].x) != kAbortMark;
+                        }
+#pragma unroll
+                    for (int u = 0; u < 4; u++)
+                        if (w0 + u < P.warps) {
+                            if (w0 + u == 0) {
+                                pi = vi[u];
+                                pj = vj[u];
+                            } else {
+                                pi.x += vi[u].x; pi.y += vi[u].y;
+                                pj.x += vj[u].x; pj.y += vj[u].y;
+                            }
+                        }
+                }
+                if (q == 0) {
+                    hi = pi;
+                    hj = pj;
+                } else {
+                    hi.x += pi.x; hi.y += pi.y;
+                    hj.x += pj.x; hj.y += pj.y;
+                }
+            }
+            if (!__all_sync(0xffffffffu, ok)) {      // every CTA of the unit reads the same marks
+                stop = 1;
+                __threadfence_block();
+                __syncwarp();
+                if (m + 1 < total) state_arrive(state_threads);
+                break;
+            }
+            const float dix = __fsub_rn(cain.x, cai.x), diy = __fsub_rn(cain.y, cai.y);
+            const float djx = __fsub_rn(cajn.x, caj.x), djy = __fsub_rn(cajn.y, caj.y);
+            const float dE = -fmaf(dix, hi.x, -diy * hi.y) - fmaf(djx, hj.x, -djy * hj.y);
+            // mc.cu:288-297: beta == 0 accepts everything; otherwise dE <= 0 or u < exp(-beta dE)
+            bool accept;
+            if (beta_d == 0.0) accept = true;
+            else accept = (dE <= 0.f) || (cu < expf(-beta * dE));
+            const float2 ai_post = accept ? cain : cai, aj_post = accept ? cajn : caj;
+            const int pi0 = ci0, pj0 = cj0;
+            const float2 pai = cai, paj = caj, pain = cain, pajn = cajn;
+            const float pu = cu;
+            // the next proposal and the final values of the state it reads
+            if (m + 1 < total) {
+                cai = ni0 == pi0 ? ai_post : (ni0 == pj0 ? aj_post : nai);
+                caj = nj0 == pi0 ? ai_post : (nj0 == pj0 ? aj_post : naj);
+                ci0 = ni0;
+                cj0 = nj0;
+                propose_with<VARIANT>(cai, caj, tt, cain, cajn);
+                cu = tt[6];
+                amp(pi0) = ai_post;
+                amp(pj0) = aj_post;
+                amp(cj0) = cajn;                     // h_i of move m+1 is evaluated at its proposed a_j
+                __syncwarp();
+                state_arrive(state_threads);
+            } else {
+                amp(pi0) = ai_post;
+                amp(pj0) = aj_post;
+            }
+            // bookkeeping, behind the chains' next pass
+            if (accept) {
+                E += (double)dE;
+                nacc++;
+            }
+            nprop++;
+            if (rank == 0 && P.trace != nullptr && U.sample == P.trace_sample && U.rep_begin + rr == P.trace_rep &&
+                active) {
+                const long long idx = (sweep0 + m / steps - P.trace_sweep0) * steps + m % steps;
+                if (idx >= 0 && idx < P.trace_cap) {
+                    pspin_move_record* rec = reinterpret_cast<pspin_move_record*>(P.trace) + idx;
+                    rec->i0 = pi0; rec->j0 = pj0;
+                    rec->ai_old[0] = pai.x; rec->ai_old[1] = pai.y;
+                    rec->aj_old[0] = paj.x; rec->aj_old[1] = paj.y;
+                    rec->ai_new[0] = pain.x; rec->ai_new[1] = pain.y;
+                    rec->aj_new[0] = pajn.x; rec->aj_new[1] = pajn.y;
+                    rec->dE = dE;
+                    rec->accepted = accept ? 1 : 0;
+                    rec->log_q_ratio = 0.f;
+                    rec->log_u = logf(pu);
+                }
+            }
+        }
+    } else if (warp == c + K) {
+        // ------------------------------------------------------------ producer: lane = chain of this CTA
+        const int g = (int)rank * c + lane;
+        const bool mine = lane < c;
+        const int part0 = (g >> 1) * (kSplit / CW), part1 = part0 + kSplit / CW;
+        const int* lists = P.site_chunks + S.split_off;
+        int2* tg = tags + lane * stages;
+        unsigned char* ring = smem_raw + Lo.ring + (size_t)lane * stages * kStage * sizeof(int2);
+        int m = 0, cur = 0, end = 0;                 // the next copy: chunk cur of [cur, end) of move m
+        int64_t b = 0, e = 0;
+        auto open = [&]() {                          // move m's chunks
+            int i0, j0;
+            pair_of(m, i0, j0);
+            const int* sc = lists + ((g & 1) ? j0 : i0) * (kSplit + 1);
+            cur = __ldg(sc + part0);
+            end = __ldg(sc + part1);
+        };
+        auto bounds = [&]() {
+            if (cur < end) {
+                b = __ldg(P.chunk_start + cur);
+                e = __ldg(P.chunk_start + cur + 1);
+            }
+        };
+        bool more = mine && total > 0;
+        if (more) {
+            open();
+            bounds();
+        }
+        uint32_t issued = 0, slot = 0, phase = 1;    // phase of the slot's last release
+        while (__any_sync(0xffffffffu, more) && !__any_sync(0xffffffffu, stop != 0)) {
+            bool did = false;
+            if (more && (issued < (uint32_t)stages || mbar_test_wait(empty + lane * stages + slot, phase))) {
+                uint64_t* fb = full + lane * stages + slot;
+                if (cur < end) {
+                    const uint32_t bytes = (uint32_t)((e - b) * sizeof(int2));
+                    tg[slot] = make_int2((int)(e - b), cur + 1 == end);
+                    mbar_expect_tx(fb, bytes);
+                    bulk_g2s(ring + slot * kStage * sizeof(int2), P.entries + b, bytes, fb);
+                    cur++;
+                } else {                             // no entries in this chain's parts
+                    tg[slot] = make_int2(0, 1);
+                    mbar_arrive(fb);
+                }
+                issued++;
+                if (++slot == (uint32_t)stages) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+                if (cur >= end) {
+                    more = ++m < total;
+                    if (more) open();
+                }
+                if (more) bounds();
+                did = true;
+            }
+            if (!__any_sync(0xffffffffu, did)) __nanosleep(40);
+        }
+        // copies still in flight after an abort (each slot's last one): none may
+        // land after the CTA has gone
+        if (mine && stop)
+            for (uint32_t q = 0; q < (uint32_t)stages && q < issued; q++) {
+                const uint32_t i = issued - 1 - q;
+                if (!mbar_wait(full + lane * stages + i % stages, (i / stages) & 1u, P.status, kDrainClocks, kStatusDrain)) break;
+            }
+        __syncwarp();
+    }
+
+    __syncthreads();                                 // every final write before the write-back
+    if (rank == 0 && !stop) {
+        for (int idx = threadIdx.x; idx < N * KB; idx += blockDim.x) {
+            const int site = idx / KB, r = idx % KB;
+            if (r < U.rep_count) P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + r] = sp[idx];
+        }
+        if (active) {
+            P.energy[gr] = E;
+            P.accepted[gr] += nacc;
+            P.proposed[gr] += nprop;
+        }
+    }
+    if (X > 1) cluster_sync();                       // no CTA leaves while a store may still target it
+}
+
+template <int VARIANT, int K, bool kLat>
+static cudaError_t ring_launch(const SweepParams& p, int n_units, size_t smem, cudaStream_t st, int* max_clusters) {
+    auto kern = sweep_ring_kernel<VARIANT, K, kLat>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && p.exec > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(n_units * p.exec));
+    cfg.blockDim = dim3((unsigned)(32 * (p.chains + K + 1)));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.exec;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.exec > 1 ? 1 : 0;
+    if (max_clusters) {
+        if (p.exec > 1) return cudaOccupancyMaxActiveClusters(max_clusters, kern, &cfg);
+        int blocks = 0, sms = 0, dev = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, (int)cfg.blockDim.x, smem);
+        if (e == cudaSuccess) e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        *max_clusters = blocks * sms;
+        return e;
+    }
+    e = cudaLaunchKernelEx(&cfg, kern, p);
+    if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+static cudaError_t ring_dispatch(SweepParams p, const RingPlan& r, int n_units, int variant, int max_N, int K,
+                                 cudaStream_t st, int* max_clusters) {
+    p.exec = r.exec;
+    p.chains = r.chains;
+    p.stages = r.stages;
+    const size_t smem = ring_layout(max_N, 2 * p.cluster * p.warps, p.chains, p.stages, K).total;
+    const bool lat = r.lat != 0;
+#define PSPIN_RING(V, KK) (lat ? ring_launch<V, KK, true>(p, n_units, smem, st, max_clusters) \
+                               : ring_launch<V, KK, false>(p, n_units, smem, st, max_clusters))
+    if (variant == 0) return K == 1 ? PSPIN_RING(0, 1) : K == 2 ? PSPIN_RING(0, 2) : PSPIN_RING(0, 3);
+    return K == 1 ? PSPIN_RING(1, 1) : K == 2 ? PSPIN_RING(1, 2) : PSPIN_RING(1, 3);
+#undef PSPIN_RING
+}
+
+// Spreads the 2*C*W chains of a unit's move over X CTAs.  16 chains fill an SM
+// (four per sub-partition); with few units the chains go to more CTAs, down to
+// one chain per sub-partition, as long as all clusters are resident at once: a
+// launch that leaves SMs idle is bound by the time of one chain.  Three ring
+// slots per chain where they fit, else two, else more CTAs.
+bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int variant, int max_N, int K) {
+    if (warps < 1 || cluster < 1 || cluster > 16 || kSplit % (cluster * warps) != 0 || K < 1 || K > 3) return false;
+    const int T = 2 * cluster * warps;
+    SweepParams p{};
+    p.warps = warps;
+    p.cluster = cluster;
+    auto resident = [&](int X, int stages, int lat) {
+        if (X > 16 || X > T || T / X > kMaxChains || (lat && T / X > kLatChains)) return 0;
+        if (ring_layout(max_N, T, T / X, stages, K).total > kRingSmemMax) return 0;
+        const RingPlan q{X, T / X, stages, lat};
+        int n = 0;
+        if (ring_dispatch(p, q, n_units, variant, max_N, K, nullptr, &n) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return n;
+    };
+    const int x_fill = T > kMaxChains ? T / kMaxChains : 1;
+    for (int stages = 3; stages >= 2; stages--)
+        for (int X = 16; X >= 1; X /= 2)
+            for (int lat = 1; lat >= 0; lat--)
+                if (X <= T && (X <= T / kLatChains || X == x_fill) && resident(X, stages, lat) >= n_units) {
+                    r = RingPlan{X, T / X, stages, lat};
+                    return true;
+                }
+    for (int X = x_fill; X <= 16 && X <= T; X *= 2)
+        for (int stages = 3; stages >= 2; stages--)
+            if (resident(X, stages, 0) > 0) {
+                r = RingPlan{X, T / X, stages, 0};
+                return true;
+            }
+    return false;
+}
+
+cudaError_t launch_sweep_ring(const SweepParams& p, const RingPlan& r, int n_units, int variant, int max_N, int K,
+                              cudaStream_t st) {
+    if (n_units <= 0) return cudaSuccess;
+    return ring_dispatch(p, r, n_units, variant, max_N, K, st, nullptr);
+}
+
+}  // namespace pspin

@@ -1,0 +1,33 @@
+"""How a move's chains are spread over CTAs does not change the chain: a
+sample alone (few units: many CTAs, at most four chains each, or one CTA)
+and the same sample among enough others to fill the machine (16 chains per
+CTA) give the same amplitudes, energies and counters bit for bit, for every
+block shape, list format and number of replicas per lane.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("warps,cluster,lanes", [(1, 1, 1), (2, 1, 3), (8, 1, 1), (8, 1, 2), (4, 2, 1), (1, 4, 3), (8, 2, 3),
+                                                 (2, 16, 1), (4, 8, 2), (8, 4, 3)])
+@pytest.mark.parametrize("kw", [dict(N=12, nrep=33, fmc_mode=0), dict(N=21, nrep=70, fmc_mode=2, gamma=0.15),
+                                dict(N=40, nrep=40, fmc_mode=1, gamma=1.0, sparse=True)])
+def test_plan_does_not_change_the_chain(warps, cluster, lanes, kw):
+    import cuda_pspin_b200 as ps
+    kw = dict(kw)
+    variant = ps.PSPIN_SPARSE if kw.pop("sparse", False) else ps.PSPIN_DENSE
+    out = []
+    for copies in (1, 90):
+        cfgs = [ps.default_config(seed=50 + k, T=0.5, **kw) for k in range(copies)]
+        opts = ps.make_options(warps_per_unit=warps, cluster_size=cluster, replicas_per_lane=lanes, disorder_stream=True)
+        with ps.Engine(cfgs, variant, opts) as eng:
+            eng.fill_betas(2.0)
+            eng.sweep(3)
+            E, acc, prop = eng.get_results()
+            R = cfgs[0].nrep
+            out.append((eng.get_spins()[0], E[:R], acc[:R], prop[:R]))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][2].sum() > 0
