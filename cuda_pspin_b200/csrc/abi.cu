@@ -136,7 +136,9 @@ struct SampleHost {
     int64_t site_entries = 0;
     double exec_flops_lists = 0.0;   // FP32 ops per replica to accumulate all N site lists once
     int64_t g4_off = -1;             // dense: into d_g4re / d_mask
-    int fc_tiles = 0;                // site lists are fully connected tiles (else group records)
+    int64_t stored_entries = 0;      // of the lists as stored (tiles differ from the nominal size)
+    int fc = 0;                      // fully connected in channel 0
+    int tiles = 0;                   // site lists are dense tiles (else group records)
     int single_groups = 0;           // group records, every group of one entry
     int64_t nq_dense = 0;
 };
@@ -885,13 +887,17 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
             std::vector<double>().swap(g4h[k]);
             std::vector<uint8_t>().swap(maskh[k]);
         }
-        h.fc_tiles = fc ? 1 : 0;
-        if (!fc) build_site_lists(N, h.g2re.data(), h.h2_active, qsv[k], lists[k], true);
-        h.single_groups = (!fc && records_single_groups(lists[k])) ? 1 : 0;
+        if (!fc)
+            build_site_lists(N, h.g2re.data(), h.h2_active, qsv[k], lists[k], kRecords,
+                             variant == PSPIN_DENSE && !s->opt.generic_lists);
+        h.fc = fc ? 1 : 0;
+        h.tiles = lists[k].tiles ? 1 : 0;
+        h.single_groups = records_single_groups(lists[k]) ? 1 : 0;
         build_q64(qsv[k], q64[k]);
         std::vector<QuartetRec>().swap(qsv[k]);
-        h.site_entries = (int64_t)lists[k].entries.size();
-        h.exec_flops_lists = list_exec_flops(lists[k], N, fc, !fc);
+        h.site_entries = lists[k].nominal;
+        h.stored_entries = (int64_t)lists[k].entries.size();
+        h.exec_flops_lists = list_exec_flops(lists[k], N);
     }
 
     const auto t_p3 = clk();
@@ -906,7 +912,8 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         d.R = h.R;
         d.h2_active = h.h2_active;
         d.variant = variant;
-        d.fc_tiles = h.fc_tiles;
+        d.tiles = h.tiles;
+        d.tiles_g = h.tiles;
         d.single_groups = h.single_groups;
         d.spin_off = spin_off;
         d.rep_off = rep_off;
@@ -926,7 +933,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         split_total += (int64_t)h.N * (kSplit + 1);
         q_total += d.nq;
         g2_total += (int64_t)h.N * h.N;
-        ent_total += h.site_entries;
+        ent_total += h.stored_entries;
         chunk_total += (int64_t)lists[k].chunk_start.size();
     }
     if (chunk_total >= (1ll << 31)) return bail(fail(PSPIN_ERR_ARG, "too many list chunks"));
@@ -992,7 +999,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
     if (s->warps < 0) return bail(fail(PSPIN_ERR_ARG, "warps_per_unit must be 1, 2, 4 or 8"));
     if (s->opt.wait_limit_clocks < 0 || s->opt.test_stall_move < 0)
         return bail(fail(PSPIN_ERR_ARG, "wait_limit_clocks and test_stall_move must be >= 0"));
-    for (const SampleHost& h : s->hs) s->max_site_entries = std::max<int64_t>(s->max_site_entries, h.site_entries);
+    for (const SampleHost& h : s->hs) s->max_site_entries = std::max<int64_t>(s->max_site_entries, h.stored_entries);
     {
         const int c = s->opt.cluster_size == 0 ? 1 : s->opt.cluster_size;
         s->warps2 = s->warps;
@@ -2018,10 +2025,10 @@ extern "C" int pspin_local_fields(pspin_state* s, int sample, int method, double
 // Pair sub-lists for the two-pass sweep: rebuilt from the FP64 quartet table
 // (same couplings, rounded to FP32 like the site lists) and appended to the
 // entry and chunk arrays; d_pair_chunks indexes them per sample.  The site
-// lists of samples without tiles are appended as well in the group format
-// (header + entries: the same groups and arithmetic as the records), which
-// the two-pass kernel reads faster; d_site_chunks_g indexes them like
-// d_site_chunks (tile samples keep their tiles).
+// lists are appended as well with the parts balanced by the group format
+// (header + entries), as tiles or, where those do not pay, as groups, which the
+// two-pass kernel reads faster than records; d_site_chunks_g indexes them like
+// d_site_chunks (fully connected samples keep their tiles).
 static int ensure_pair_lists(pspin_state* s) {
     if (s->d_pair_chunks) return PSPIN_OK;
     const int n = s->S;
@@ -2043,7 +2050,10 @@ static int ensure_pair_lists(pspin_state* s) {
         }
         std::vector<Q64>().swap(q[k]);
         build_pair_lists(s->hs[k].N, s->hs[k].g2re.data(), s->hs[k].h2_active, recs, pl[k]);
-        if (!s->hs[k].fc_tiles) build_site_lists(s->hs[k].N, s->hs[k].g2re.data(), s->hs[k].h2_active, recs, gl[k], false);
+        // a fully connected sample keeps its tiles (their parts are the same here)
+        if (!(s->hs[k].tiles && s->hs[k].fc))
+            build_site_lists(s->hs[k].N, s->hs[k].g2re.data(), s->hs[k].h2_active, recs, gl[k], kGroups,
+                             s->hs[k].tiles != 0);
     }
     int64_t ent_new = 0, chunk_new = 0, idx_total = 0, split_total = 0;
     for (int k = 0; k < n; k++) {
@@ -2061,6 +2071,7 @@ static int ensure_pair_lists(pspin_state* s) {
     std::vector<int64_t> cs((size_t)chunk_new + 1);
     std::vector<int> pc((size_t)idx_total);
     std::vector<int64_t> pair_off(n);
+    std::vector<int> tiles_g(n);
     int64_t eoff = 0, coff = 0, ioff = 0;
     for (int k = 0; k < n; k++) {
         std::copy(pl[k].entries.begin(), pl[k].entries.end(), ent.begin() + eoff);
@@ -2080,6 +2091,7 @@ static int ensure_pair_lists(pspin_state* s) {
             eoff += (int64_t)gl[k].entries.size();
             coff += (int64_t)gl[k].chunk_start.size();
         }
+        tiles_g[k] = gl[k].entries.empty() ? s->sd[k].tiles : (int)gl[k].tiles;
         gl[k] = SiteLists();
     }
     cs[chunk_new] = s->ent_total + ent_new;
@@ -2095,7 +2107,10 @@ static int ensure_pair_lists(pspin_state* s) {
         return rc;
     }
     std::vector<SampleDev> sd = s->sd;
-    for (int k = 0; k < n; k++) sd[k].pair_off = pair_off[k];
+    for (int k = 0; k < n; k++) {
+        sd[k].pair_off = pair_off[k];
+        sd[k].tiles_g = tiles_g[k];
+    }
     cudaError_t e = cudaMemcpyAsync(d_ent, s->d_entries, s->ent_total * sizeof(int2), cudaMemcpyDeviceToDevice, s->st);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(d_ent + s->ent_total, ent.data(), ent.size() * sizeof(int2), cudaMemcpyHostToDevice, s->st);

@@ -9,17 +9,17 @@
 //                                           (i64), beta (f64), RNG key (u64),
 //                                           constraint target (f64)
 //   site lists int2   [sum_s entries_s]     per sample, per site: groups of
-//                                           terms with the same (p, o1), one
-//                                           16-byte record {g (f32 bits), o2,
-//                                           p<<16|o1, last} per term (or the
-//                                           fully connected tiles below), packed
+//                                           terms with the same (p, o1), as
+//                                           dense tiles of up to 8 groups, or
+//                                           one 16-byte record {g (f32 bits),
+//                                           o2, p<<16|o1, last} per term, packed
 //                                           in TMA chunks of <= 256 entries that
-//                                           hold whole groups, start 16-byte
-//                                           aligned and have an even length.
-//                                           The pair sub-lists of the two-pass
-//                                           sweep keep the group format: a
-//                                           header {len, p<<16|o1} and len data
-//                                           entries {g, o2}
+//                                           hold whole groups or tiles, start
+//                                           16-byte aligned and have an even
+//                                           length.  The pair sub-lists of the
+//                                           two-pass sweep keep the group
+//                                           format: a header {len, p<<16|o1} and
+//                                           len data entries {g, o2}
 //   chunk starts int64 [n_chunks + 1]       entry offset of every chunk
 //   site chunks int32 [sum_s N_s * 33]      first chunk of each of the 32
 //                                           balanced parts of a site's list
@@ -37,15 +37,15 @@
 // every energy change of site m alone as -Re[da_m h_m].  2-body terms fold
 // in with p = o1 = N, a virtual site whose amplitude is 1.
 //
-// Fully connected tiles.  When every quartet is active in channel 0, a
-// quartet enters site m's field as g a_p conj(a_outer) conj(a_inner) with a
-// contiguous range of inner sites shared by every partner p of one outer
-// site: if m is among the two smallest sites of the quartet, outer = o1 > m,
-// p < o1 and inner in (o1, N); otherwise outer = o2 < m, p > o2 and inner in
-// [0, o2).  A tile is a 16-byte header {outer | lo<<16, hi, p0 | p1<<16,
-// p2 | p3<<16} and hi-lo rows of 4 couplings (one per partner; padding
-// partners are the virtual site with zero couplings), so one gathered
-// a_inner feeds 8 FFMA.
+// Dense tiles.  When every quartet is active in channel 0, a quartet enters
+// site m's field as g a_p conj(a_outer) conj(a_inner) with a contiguous range
+// of inner sites shared by every partner p of one outer site: if m is among
+// the two smallest sites of the quartet, outer = o1 > m, p < o1 and inner in
+// (o1, N); otherwise outer = o2 < m, p > o2 and inner in [0, o2).  Under a
+// frequency mask the inner sites of a group lie in an interval that moves
+// slowly with o1 (the sites are sorted by frequency), so neighbouring groups
+// of one partner overlap.  Either way a tile holds several groups as columns
+// over one inner range (layout.cpp), so one gathered a_inner feeds 8 or 16 FMA.
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -72,7 +72,8 @@ struct SampleDev {
     int R;                 // replicas of this sample
     int h2_active;
     int variant;           // 0 sphere (dense), 1 smoothed cube (sparse)
-    int fc_tiles;          // 1: site lists are fully connected tiles (see below), 0: group records
+    int tiles;             // 1: site lists are dense tiles (layout.cpp), 0: group records
+    int tiles_g;           // the same of the two-pass sweep's site lists (else groups)
     int single_groups;     // group records only, every group of one entry (each record ends its group)
     int64_t spin_off;      // float2 index of site 0, replica 0
     int64_t rep_off;       // index into the per-replica arrays

@@ -279,8 +279,8 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
                 if (!ok_wait) break;               // stop consuming and issuing; abort in reduce()
                 const int n = (int)(__ldg(P.chunk_start + c + 1) - __ldg(P.chunk_start + c));
                 const int k2 = 2 * (which & 1);
-                if (which < 2 && S.fc_tiles)      // unrolled by 2: the kernel is held to 80 registers
-                    accumulate_tiles<2>(ring + slot * kStage, n, sp, lane, h[k2], h[k2 + 1]);
+                if (which < 2 && S.tiles_g)       // small unrolls: the kernel is held to 80 registers
+                    accumulate_tiles_1<2, 2, false>(ring + slot * kStage, n, sp, lane, h[k2], h[k2 + 1]);
                 else accumulate_chunk(ring + slot * kStage, n, sp, lane, h[k2], h[k2 + 1]);
                 consumed++;
                 __syncwarp();

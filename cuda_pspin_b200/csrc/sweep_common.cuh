@@ -2,6 +2,8 @@
 // the per-warp TMA rings that stream site-list chunks into shared memory,
 // and the field accumulation over one staged chunk.
 #pragma once
+#include <type_traits>
+
 #include "internal.h"
 #include "rng.cuh"
 
@@ -343,107 +345,160 @@ __device__ __forceinline__ void accumulate_records(const int2* __restrict__ R2, 
     }
 }
 
-// Field contribution of the fully connected tiles in one staged chunk
-// (16-byte records: header, then rows of 4 couplings).  One gathered
-// a_inner feeds four partners: 8 FFMA per shared-memory gather.  The rows
-// are unrolled by kUnroll (more gathers in flight per warp; the summation
-// order is the same for every kUnroll).
-template <int kUnroll = 8>
-__device__ __forceinline__ void accumulate_tiles(const int2* __restrict__ R2, int n,
-                                                 const float2* __restrict__ sp, int lane,
-                                                 float& hx, float& hy) {
-    const int4* __restrict__ R = reinterpret_cast<const int4*>(R2);
-    const int n16 = n >> 1;
-    int e = 0;
-    while (e < n16) {
-        const int4 hd = R[e];
-        const int outer = hd.x & 0xFFFF, lo = hd.x >> 16, hi = hd.y;
-        const float2 ao = sp[outer * kRepBlock + lane];
-        float y0x = 0.f, y0y = 0.f, y1x = 0.f, y1y = 0.f, y2x = 0.f, y2y = 0.f, y3x = 0.f, y3y = 0.f;
-        const float4* __restrict__ C = reinterpret_cast<const float4*>(R + e + 1);
-        const float2* __restrict__ A = sp + lo * kRepBlock + lane;
-        const int len = hi - lo;
-#pragma unroll kUnroll
-        for (int t = 0; t < len; t++) {
-            const float4 c = C[t];
-            const float2 a = A[t * kRepBlock];
-            y0x = fmaf(c.x, a.x, y0x); y0y = fmaf(-c.x, a.y, y0y);
-            y1x = fmaf(c.y, a.x, y1x); y1y = fmaf(-c.y, a.y, y1y);
-            y2x = fmaf(c.z, a.x, y2x); y2y = fmaf(-c.z, a.y, y2y);
-            y3x = fmaf(c.w, a.x, y3x); y3y = fmaf(-c.w, a.y, y3y);
-        }
-        // h += sum_k a_pk conj(a_outer) Y_k
-        const int pk[4] = {hd.z & 0xFFFF, hd.z >> 16, hd.w & 0xFFFF, hd.w >> 16};
-        const float yx[4] = {y0x, y1x, y2x, y3x}, yy[4] = {y0y, y1y, y2y, y3y};
+// ---------------------------------------------------------------- dense tiles
+// Field contribution of the tiles in one staged chunk (layout.cpp), for a
+// block of 32K replicas stored [site][K][32] (replica k*32 + lane of the block
+// at sp[(site*K + k)*32 + lane]).  A row is one broadcast read of its 4 or 8
+// couplings and one gathered amplitude per replica for 8 or 16 FMA per
+// replica; then each column's sum enters the field in column order,
+//   h += a_p conj(a_o) Y,
+// the arithmetic of accumulate_chunk on the columns' groups, operation for
+// operation (a zero coupling leaves Y as it is, and a column without a group,
+// the virtual site's, adds zero).
+//
+// Rows come in blocks of kUnroll, loads first, then the rest of 4, 2, 1.  The
+// products are paired FMA over two columns (fma.rn.f32x2, the rounding of two
+// single ones; couplings are neighbours in the row, the amplitude's two
+// components are duplicated): an outer product's single FMA reads three new
+// registers and issues at 1.25 cycles, so pairs cost the FMA pipe nothing and
+// free half the issue slots for the loads.  With four warps a sub-partition,
+// cycles per tile and warp, single -> paired: K = 3, 4 x 20 1045 -> 880, 8 x 32
+// 2550 -> 2180; K = 1, 8 x 20 740 -> 645.  kLat, for a warp with a sub-partition
+// to itself: the next tile's header and the columns' amplitudes are loaded ahead
+// of the rows.  (Double-buffered row blocks with masked ends took 1.6 times as
+// long: the masks cost more than the latency they hid.)
+template <int K, int P, int kUnroll>
+struct TileBlock {
+    float4 c[kUnroll][P / 4];
+    float2 a[kUnroll][K];
+    __device__ __forceinline__ void load(const float4* __restrict__ C, const float2* __restrict__ A, int t) {
 #pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float2 ap = sp[pk[k] * kRepBlock + lane];
-            const float px = fmaf(ap.x, ao.x, ap.y * ao.y);
-            const float py = fmaf(ap.y, ao.x, -ap.x * ao.y);
-            hx = fmaf(px, yx[k], fmaf(-py, yy[k], hx));
-            hy = fmaf(px, yy[k], fmaf(py, yx[k], hy));
+        for (int u = 0; u < kUnroll; u++) {
+#pragma unroll
+            for (int w = 0; w < P / 4; w++) c[u][w] = C[(t + u) * (P / 4) + w];
+#pragma unroll
+            for (int k = 0; k < K; k++) a[u][k] = A[((t + u) * K + k) * kRepBlock];
         }
-        e += 1 + len;
     }
-}
-
-// ---------------------------------------------------------------- K replicas per lane
-// The same accumulations for a block of 32K replicas stored [site][K][32]
-// (replica k*32 + lane of the block at sp[(site*K + k)*32 + lane]): each
-// staged coupling is read once and used for the lane's K replicas.  The
-// summation order per replica is that of accumulate_tiles /
-// accumulate_records.
-template <int K, int kUnroll>
-__device__ __forceinline__ void accumulate_tiles_k(const int2* __restrict__ R2, int n,
-                                                   const float2* __restrict__ sp, int lane,
-                                                   float (&hx)[K], float (&hy)[K]) {
-    const int4* __restrict__ R = reinterpret_cast<const int4*>(R2);
-    const int n16 = n >> 1;
-    int e = 0;
-    while (e < n16) {
-        const int4 hd = R[e];
-        const int outer = hd.x & 0xFFFF, lo = hd.x >> 16, hi = hd.y;
-        float y[K][8];
+    __device__ __forceinline__ void add(float2 (&y)[K][P]) const {
 #pragma unroll
-        for (int k = 0; k < K; k++)
-#pragma unroll
-            for (int q = 0; q < 8; q++) y[k][q] = 0.f;
-        const float4* __restrict__ C = reinterpret_cast<const float4*>(R + e + 1);
-        const float2* __restrict__ A = sp + (size_t)lo * K * kRepBlock + lane;
-        const int len = hi - lo;
-#pragma unroll kUnroll
-        for (int t = 0; t < len; t++) {
-            const float4 c = C[t];
+        for (int u = 0; u < kUnroll; u++)
 #pragma unroll
             for (int k = 0; k < K; k++) {
-                const float2 a = A[(t * K + k) * kRepBlock];
-                y[k][0] = fmaf(c.x, a.x, y[k][0]); y[k][1] = fmaf(-c.x, a.y, y[k][1]);
-                y[k][2] = fmaf(c.y, a.x, y[k][2]); y[k][3] = fmaf(-c.y, a.y, y[k][3]);
-                y[k][4] = fmaf(c.z, a.x, y[k][4]); y[k][5] = fmaf(-c.z, a.y, y[k][5]);
-                y[k][6] = fmaf(c.w, a.x, y[k][6]); y[k][7] = fmaf(-c.w, a.y, y[k][7]);
-            }
-        }
-        const int pk[4] = {hd.z & 0xFFFF, hd.z >> 16, hd.w & 0xFFFF, hd.w >> 16};
+                const float2 dx = make_float2(a[u][k].x, a[u][k].x), dy = make_float2(a[u][k].y, a[u][k].y);
 #pragma unroll
-        for (int k = 0; k < K; k++) {
-            const float2 ao = sp[(outer * K + k) * kRepBlock + lane];
-#pragma unroll
-            for (int q = 0; q < 4; q++) {
-                const float2 ap = sp[(pk[q] * K + k) * kRepBlock + lane];
-                const float px = fmaf(ap.x, ao.x, ap.y * ao.y);
-                const float py = fmaf(ap.y, ao.x, -ap.x * ao.y);
-                hx[k] = fmaf(px, y[k][2 * q], fmaf(-py, y[k][2 * q + 1], hx[k]));
-                hy[k] = fmaf(px, y[k][2 * q + 1], fmaf(py, y[k][2 * q], hy[k]));
+                for (int w = 0; w < P / 4; w++) {
+                    const float2 g0 = make_float2(c[u][w].x, c[u][w].y), g1 = make_float2(c[u][w].z, c[u][w].w);
+                    y[k][4 * w + 0] = __ffma2_rn(g0, dx, y[k][4 * w + 0]);
+                    y[k][4 * w + 1] = __ffma2_rn(g0, dy, y[k][4 * w + 1]);
+                    y[k][4 * w + 2] = __ffma2_rn(g1, dx, y[k][4 * w + 2]);
+                    y[k][4 * w + 3] = __ffma2_rn(g1, dy, y[k][4 * w + 3]);
+                }
             }
+    }
+};
+
+template <int K, int P, int kUnroll, bool kLat>
+__device__ __forceinline__ void tile_body(const int4 h0, const int4 h1, const int4* __restrict__ T,
+                                          const float2* __restrict__ sp, int lane, float (&hx)[K], float (&hy)[K]) {
+    const int shared = h0.x & 0xFFFF, lo = h0.y & 0xFFFF, rows = (h0.y >> 16) & 0xFF;
+    const bool shared_p = (h0.x & (2 << 16)) != 0;
+    int v[P];
+    v[0] = h0.z & 0xFFFF; v[1] = h0.z >> 16; v[2] = h0.w & 0xFFFF; v[3] = h0.w >> 16;
+    if (P == 8) {
+        v[P - 4] = h1.x & 0xFFFF; v[P - 3] = h1.x >> 16; v[P - 2] = h1.y & 0xFFFF; v[P - 1] = h1.y >> 16;
+    }
+    const float4* __restrict__ C = reinterpret_cast<const float4*>(T + P / 4);
+    const float2* __restrict__ A = sp + (size_t)lo * K * kRepBlock + lane;
+    float2 y[K][P];      // columns q, q+1 (q even): [q] their Re sums, [q + 1] their -Im sums
+#pragma unroll
+    for (int k = 0; k < K; k++)
+#pragma unroll
+        for (int q = 0; q < P; q++) y[k][q] = make_float2(0.f, 0.f);
+    constexpr bool kEarly = kLat && K == 1;       // registers for the columns' amplitudes
+    float2 f[K], x[kEarly ? P : 1];
+    if (kEarly)
+#pragma unroll
+        for (int q = 0; q < P; q++) x[q] = sp[v[q] * kRepBlock + lane];
+    int t = 0;
+#pragma unroll 1
+    for (; t + kUnroll <= rows; t += kUnroll) {
+        TileBlock<K, P, kUnroll> b;
+        b.load(C, A, t);
+        b.add(y);
+    }
+    auto rest = [&](auto count) {
+        constexpr int n = decltype(count)::value;
+        if (kUnroll > n && (rows & n)) {
+            TileBlock<K, P, n> b;
+            b.load(C, A, t);
+            b.add(y);
+            t += n;
         }
-        e += 1 + len;
+    };
+    rest(std::integral_constant<int, 4>{});
+    rest(std::integral_constant<int, 2>{});
+    rest(std::integral_constant<int, 1>{});
+#pragma unroll
+    for (int k = 0; k < K; k++) f[k] = sp[(shared * K + k) * kRepBlock + lane];
+    auto fold = [&](const float2 ap, const float2 ao, int k, int q) {
+        const float px = fmaf(ap.x, ao.x, ap.y * ao.y);
+        const float py = fmaf(ap.y, ao.x, -ap.x * ao.y);
+        const int q0 = q & ~1;
+        const float yr = q & 1 ? y[k][q0].y : y[k][q0].x, yi = q & 1 ? y[k][q0 + 1].y : y[k][q0 + 1].x;
+        hx[k] = fmaf(px, yr, fmaf(py, yi, hx[k]));
+        hy[k] = fmaf(-px, yi, fmaf(py, yr, hy[k]));
+    };
+    auto column = [&](int k, int q) { return kEarly ? x[kEarly ? q : 0] : sp[(v[q] * K + k) * kRepBlock + lane]; };
+    if (shared_p) {
+#pragma unroll
+        for (int q = 0; q < P; q++)
+#pragma unroll
+            for (int k = 0; k < K; k++) fold(f[k], column(k, q), k, q);
+    } else {
+#pragma unroll
+        for (int q = 0; q < P; q++)
+#pragma unroll
+            for (int k = 0; k < K; k++) fold(column(k, q), f[k], k, q);
     }
 }
 
-// One record at a time (accumulate_records_k for one replica per lane).
-__device__ __forceinline__ void accumulate_records_1(const int2* __restrict__ R2, int n,
-                                                     const float2* __restrict__ sp, int lane, float& hx, float& hy);
+// k4, k8: rows per block in 4- and 8-column tiles
+template <int K, int k4, int k8, bool kLat>
+__device__ __forceinline__ void accumulate_tiles(const int2* __restrict__ R2, int n, const float2* __restrict__ sp,
+                                                 int lane, float (&hx)[K], float (&hy)[K]) {
+    const int4* __restrict__ R = reinterpret_cast<const int4*>(R2);
+    const int n16 = n >> 1;
+    const int4 none = make_int4(0, 0, 0, 0);
+    int e = 0;
+    int4 h0 = n16 > 0 ? R[0] : none, h1 = kLat && n16 > 1 ? R[1] : none;
+    while (e < n16) {
+        const int rows = (h0.y >> 16) & 0xFF;
+        const bool wide = (h0.x & (1 << 16)) != 0;
+        const int4* T = R + e;
+        const int4 c0 = h0, c1 = kLat ? h1 : (wide ? T[1] : none);
+        e += wide ? 2 + 2 * rows : 1 + rows;
+        if (kLat) {
+            h0 = e < n16 ? R[e] : none;
+            h1 = e + 1 < n16 ? R[e + 1] : none;
+        }
+        if (wide) tile_body<K, 8, k8, kLat>(c0, c1, T, sp, lane, hx, hy);
+        else tile_body<K, 4, k4, kLat>(c0, c1, T, sp, lane, hx, hy);
+        if (!kLat && e < n16) h0 = R[e];
+    }
+}
 
+// one replica per lane
+template <int k4, int k8, bool kLat>
+__device__ __forceinline__ void accumulate_tiles_1(const int2* __restrict__ R2, int n, const float2* __restrict__ sp,
+                                                   int lane, float& hx, float& hy) {
+    float hx1[1] = {hx}, hy1[1] = {hy};
+    accumulate_tiles<1, k4, k8, kLat>(R2, n, sp, lane, hx1, hy1);
+    hx = hx1[0];
+    hy = hy1[0];
+}
+
+// Group records for K replicas per lane, one record at a time.
 template <int K>
 __device__ __forceinline__ void accumulate_records_k(const int2* __restrict__ R2, int n,
                                                      const float2* __restrict__ sp, int lane,
@@ -478,44 +533,6 @@ __device__ __forceinline__ void accumulate_records_k(const int2* __restrict__ R2
             }
         }
     }
-}
-
-__device__ __forceinline__ void accumulate_records_1(const int2* __restrict__ R2, int n,
-                                                     const float2* __restrict__ sp, int lane, float& hx, float& hy) {
-    float hx1[1] = {hx}, hy1[1] = {hy};
-    accumulate_records_k<1>(R2, n, sp, lane, hx1, hy1);
-    hx = hx1[0];
-    hy = hy1[0];
-}
-
-// The field partials of the C CTAs x W warps of a block, summed in the fixed
-// order the cluster kernels use -- each CTA's warps in order, then the CTAs
-// in rank order -- from slots buf[(q*W + w) * stride], with the loads of
-// four slots in flight before their additions (the same additions in the
-// same order as one load per addition).
-__device__ __forceinline__ void add4v(float4& a, const float4 b) {
-    a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
-}
-__device__ __forceinline__ float4 sum_partials(const float4* buf, int C, int W, int stride) {
-    float4 hs = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int q = 0; q < C; q++) {
-        float4 part = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int w0 = 0; w0 < W; w0 += 4) {
-            float4 v[4];
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (w0 + u < W) v[u] = buf[(size_t)(q * W + w0 + u) * stride];
-#pragma unroll
-            for (int u = 0; u < 4; u++)
-                if (w0 + u < W) {
-                    if (w0 + u == 0) part = v[u];
-                    else add4v(part, v[u]);
-                }
-        }
-        if (q == 0) hs = part;
-        else add4v(hs, part);
-    }
-    return hs;
 }
 
 // ---------------------------------------------------------------- clusters

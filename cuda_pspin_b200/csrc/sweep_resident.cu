@@ -215,9 +215,9 @@ __global__ void __launch_bounds__(256) sweep_resident_kernel(const SweepParams P
                 __syncwarp();
                 float hix = 0.f, hiy = 0.f, hjx = 0.f, hjy = 0.f;
                 const int2 ri = rng_site[i0], rj = rng_site[j0];
-                if (S.fc_tiles) {
-                    accumulate_tiles(L + ri.x, ri.y - ri.x, sp, lane, hix, hiy);
-                    accumulate_tiles(L + rj.x, rj.y - rj.x, sp, lane, hjx, hjy);
+                if (S.tiles) {
+                    accumulate_tiles_1<8, 4, true>(L + ri.x, ri.y - ri.x, sp, lane, hix, hiy);
+                    accumulate_tiles_1<8, 4, true>(L + rj.x, rj.y - rj.x, sp, lane, hjx, hjy);
                 } else if (S.single_groups) {
                     accumulate_records<4, true>(L + ri.x, ri.y - ri.x, sp, lane, hix, hiy);
                     accumulate_records<4, true>(L + rj.x, rj.y - rj.x, sp, lane, hjx, hjy);

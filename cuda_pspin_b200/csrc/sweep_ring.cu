@@ -29,16 +29,19 @@
 //        schedule and keeps its ring of TMA copies (cp.async.bulk, one mbarrier
 //        per slot) full, moves ahead of the readers; no chain warp looks
 //        anything up;
-//      chain warp: reads its chunks, sends its partial field of each replica to
-//        every CTA's exchange buffer (st.async, completion counted in bytes on
-//        the receiving decider's mbarrier; a plain store and an arrival where
-//        the unit is one CTA), then waits for the CTA's deciders;
+//      chain warp: reads its chunks, leaves its partial field of each replica in
+//        the CTA's shared memory, then waits for the CTA's deciders;
 //      decider k: while the chains run, the random words, sines and cosines of
-//        the next move for its 32 replicas; when its mbarrier has all 2*C*W
-//        partials, the sum in tree order, the Metropolis decision, the next
-//        proposal, and both into its CTA's copy of the amplitudes.
+//        the next move for its 32 replicas; when the CTA's chains have arrived,
+//        their sums (of the tree's groups that lie in this CTA whole, else the
+//        partials as they are) go to every CTA of the unit (st.async, counted in
+//        bytes on the receiving decider's mbarrier); when all have come, the rest
+//        of the tree, the Metropolis decision, the next proposal, and both into
+//        its CTA's copy of the amplitudes.
 //    Every CTA's decider k takes the same decision on the same numbers, so the
-//    copies agree and a move costs one hop between CTAs and one CTA barrier.
+//    copies agree and a move costs one hop between CTAs and two barriers in one.
+//    (Every chain sending its partial to all CTAs: 64 partials of 256 bytes into
+//    each of 16 CTAs and 4000 cycles to sum them at N=32.)
 //    With every warp deciding for itself and fetching its own chunks (8 warps
 //    reading list i, then list j), the benchmark's launch ran the FMA pipe at
 //    37 % and a move of a one-sample run cost 8 us of waiting.
@@ -53,21 +56,34 @@ namespace pspin {
 
 constexpr int kMaxChains = 16;            // chain warps per CTA
 constexpr int kLatChains = 4;             // up to here a CTA is one chain per SM sub-partition
-constexpr uint32_t kAbortMark = 0x7fc0dead;   // a NaN no arithmetic here produces: this chain gave up
+// A CTA one of whose chains gave up sends this NaN, which no arithmetic here
+// produces, in place of its messages.
+constexpr uint32_t kAbortMark = 0x7fc0dead;
+__device__ __forceinline__ bool is_marked(const float2 v) { return __float_as_uint(v.x) == kAbortMark; }
 
 // Shared memory of one CTA: amplitudes [N+1][K][32] float2; rings
-// [chains][stages][kStage] int2; exchange buffer [2][T][K][32] float2 (T =
-// 2*C*W chains of a move); mbarriers full, empty [chains][stages], partials
-// [2][K]; ring tags [chains][stages] int2.
+// [chains][stages][kStage] int2; the chains' partials [chains][K][32] float2;
+// exchange buffer [2][messages][K][32] float2 (messages: see ring_messages);
+// mbarriers full, empty [chains][stages], chains' arrival, messages [2][K]; ring
+// tags [chains][stages] int2.
 struct RingLayout {
-    size_t ring, xbuf, bars, tags, total;
+    size_t ring, part, xbuf, bars, tags, total;
 };
-__host__ __device__ inline RingLayout ring_layout(int N, int T, int chains, int stages, int K) {
+// What a unit's CTAs exchange per move: the sums of the tree's 2*C groups of W
+// chains where a CTA holds whole groups, else the 2*C*W chains.
+__host__ __device__ inline int ring_messages(int warps, int cluster, int chains) {
+    return chains % warps == 0 ? 2 * cluster : 2 * cluster * warps;
+}
+__host__ __device__ inline RingLayout ring_layout(int N, int warps, int cluster, int chains, int stages, int K) {
     RingLayout L;
-    L.ring = (size_t)(N + 1) * K * kRepBlock * sizeof(float2);
-    L.xbuf = L.ring + (size_t)chains * stages * kStage * sizeof(int2);
-    L.bars = L.xbuf + (size_t)2 * T * K * kRepBlock * sizeof(float2);
-    L.tags = L.bars + (size_t)(2 * chains * stages + 2 * K) * sizeof(uint64_t);
+    const size_t row = (size_t)K * kRepBlock * sizeof(float2);
+    L.ring = (size_t)(N + 1) * row;
+    L.part = L.ring + (size_t)chains * stages * kStage * sizeof(int2);
+    L.xbuf = L.part + (size_t)chains * row;
+    // one CTA holds every group: nothing is exchanged
+    const bool alone = chains == 2 * cluster * warps;
+    L.bars = L.xbuf + (alone ? 0 : (size_t)2 * ring_messages(warps, cluster, chains) * row);
+    L.tags = L.bars + (size_t)(2 * chains * stages + 1 + 2 * K) * sizeof(uint64_t);
     L.total = L.tags + (size_t)chains * stages * sizeof(int2);
     return L;
 }
@@ -103,6 +119,49 @@ __device__ __forceinline__ void state_wait(int threads) {
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
+// Partial fields from buf[q * group + w * stride] in tree order: a CTA's W
+// chains, then the C CTAs.  Eight loads in flight before their additions.
+// `ok` is cleared where a value is marked.
+template <int W>
+__device__ __forceinline__ float2 tree_sum_w(const float2* __restrict__ buf, int C, int stride, int group, bool& ok) {
+    constexpr int G = 8 / W;
+    float2 h = make_float2(0.f, 0.f);
+#pragma unroll 1
+    for (int q0 = 0; q0 < C; q0 += G) {
+        float2 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            v[u] = make_float2(0.f, 0.f);
+            if (u < W || q0 + u / W < C) v[u] = buf[(q0 + u / W) * group + (u % W) * stride];
+        }
+#pragma unroll
+        for (int g = 0; g < G; g++) {
+            float2 p = v[g * W];
+            ok = ok && !is_marked(p);
+#pragma unroll
+            for (int w = 1; w < W; w++) {
+                p.x += v[g * W + w].x;
+                p.y += v[g * W + w].y;
+                ok = ok && !is_marked(v[g * W + w]);
+            }
+            if (q0 + g == 0) h = p;
+            else if (q0 + g < C) {
+                h.x += p.x;
+                h.y += p.y;
+            }
+        }
+    }
+    return h;
+}
+__device__ __forceinline__ float2 tree_sum(const float2* __restrict__ buf, int C, int W, int stride, int group, bool& ok) {
+    switch (W) {
+        case 1: return tree_sum_w<1>(buf, C, stride, group, ok);
+        case 2: return tree_sum_w<2>(buf, C, stride, group, ok);
+        case 4: return tree_sum_w<4>(buf, C, stride, group, ok);
+        default: return tree_sum_w<8>(buf, C, stride, group, ok);
+    }
+}
+
 // kLat: few blocks, at most kLatChains chain warps a CTA, so a warp has its
 // sub-partition's issue slots and registers to itself and deep batches of
 // loads in flight carry it; otherwise 16 chain warps share the SM.
@@ -116,25 +175,26 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     const SampleDev S = P.samples[U.sample];
     const int N = S.N, R = S.R;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int CW = P.cluster * P.warps, T = 2 * CW;
+    const int CW = P.cluster * P.warps;
     constexpr int KB = K * kRepBlock;
-    const RingLayout Lo = ring_layout(N, T, c, stages, K);
+    const RingLayout Lo = ring_layout(N, P.warps, P.cluster, c, stages, K);
     float2* sp = reinterpret_cast<float2*>(smem_raw);
+    float2* part = reinterpret_cast<float2*>(smem_raw + Lo.part);
     float2* xbuf = reinterpret_cast<float2*>(smem_raw + Lo.xbuf);
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + Lo.bars);
     uint64_t* empty = full + c * stages;
-    uint64_t* xbar = empty + c * stages;
+    uint64_t* cbar = empty + c * stages;
+    uint64_t* xbar = cbar + 1;
     int2* tags = reinterpret_cast<int2*>(smem_raw + Lo.tags);
-    __shared__ volatile int stop;
+    __shared__ volatile int stop, gave_up;           // the unit aborts; a chain of this CTA gave up
     __shared__ __align__(8) uint64_t stall_bar;      // test hook: nothing arrives on it
 
     if (threadIdx.x == 0) {
         for (int q = 0; q < 2 * c * stages; q++) mbar_init(full + q, 1);
-        // partials: bytes of every chain's st.async (armed by the decider), or
-        // one arrival per chain where the unit is a single CTA
-        for (int q = 0; q < 2 * K; q++) mbar_init(xbar + q, X > 1 ? 1u : (uint32_t)T);
+        mbar_init(cbar, (uint32_t)c);                // every chain of the CTA
+        for (int q = 0; q < 2 * K; q++) mbar_init(xbar + q, 1);   // bytes, armed by the decider
         mbar_init(&stall_bar, 1);
-        stop = 0;
+        stop = gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_shared();
     }
@@ -187,12 +247,11 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
 
     if (warp < c) {
         // ------------------------------------------------------------ chain warp
-        const int g = (int)rank * c + warp;          // chain g of the move: list g & 1, chain g >> 1 of that list
+        float2* mine = part + (size_t)warp * KB + lane;
         uint64_t* fb = full + warp * stages;
         uint64_t* eb = empty + warp * stages;
         const int2* tg = tags + warp * stages;
         const int2* ring = reinterpret_cast<const int2*>(smem_raw + Lo.ring) + (size_t)warp * stages * kStage;
-        float2* my_x = xbuf + (size_t)((g & 1) * CW + (g >> 1)) * KB + lane;
         uint32_t slot = 0, phase = 0;
         for (int m = 0; m < total; m++) {
             if (m > 0) {
@@ -212,10 +271,10 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 const int2* chunk = ring + slot * kStage;
                 last = t.y != 0;
                 if (K == 1 && kLat) {
-                    if (S.fc_tiles) accumulate_tiles(chunk, t.x, sp, lane, hx[0], hy[0]);
+                    if (S.tiles) accumulate_tiles<K, 8, 4, true>(chunk, t.x, sp, lane, hx, hy);
                     else accumulate_records<4>(chunk, t.x, sp, lane, hx[0], hy[0]);
                 } else {
-                    if (S.fc_tiles) accumulate_tiles_k<K, kLat ? 4 : 2>(chunk, t.x, sp, lane, hx, hy);
+                    if (S.tiles) accumulate_tiles<K, 2, 2, kLat>(chunk, t.x, sp, lane, hx, hy);
                     else accumulate_records_k<K>(chunk, t.x, sp, lane, hx, hy);
                 }
                 __syncwarp();
@@ -225,36 +284,23 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                     phase ^= 1u;
                 }
             }
-            const uint32_t par = (uint32_t)(m & 1);
-            const float mark = __uint_as_float(kAbortMark);
-            if (!ok)
 #pragma unroll
-                for (int u = 0; u < K; u++) hx[u] = mark;
-            if (X > 1) {
-                const uint32_t dx = smem_u32(my_x) + par * (uint32_t)(T * KB * sizeof(float2));
-                const uint32_t db = smem_u32(xbar + par * K);
-                for (int q = 0; q < X; q++) {
-                    const uint32_t rx = map_rank(dx, (uint32_t)q), rb = map_rank(db, (uint32_t)q);
-#pragma unroll
-                    for (int u = 0; u < K; u++)
-                        st_async_f2(rx + u * (uint32_t)(kRepBlock * sizeof(float2)), make_float2(hx[u], hy[u]),
-                                    rb + u * (uint32_t)sizeof(uint64_t));
-                }
-            } else {
-                float2* dst = my_x + (size_t)par * T * KB;
-#pragma unroll
-                for (int u = 0; u < K; u++) dst[u * kRepBlock] = make_float2(hx[u], hy[u]);
-                __syncwarp();
-                if (lane < K) mbar_arrive(xbar + par * K + lane);
-            }
+            for (int u = 0; u < K; u++)
+                mine[u * kRepBlock] = make_float2(hx[u], hy[u]);
+            if (!ok) gave_up = 1;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(cbar);
         }
     } else if (decider) {
         // ------------------------------------------------------------ decider
         const long long limit = 2 * P.wait_clocks + kDrainClocks;   // beyond any chain's own bounded wait
+        const int W = P.warps, C = P.cluster;
+        const bool grouped = c % W == 0;
+        const int msgs = ring_messages(W, C, c), local = grouped ? c / W : c;
         for (int m = 0; m < total; m++) {
             const uint32_t par = (uint32_t)(m & 1);
             uint64_t* bar = xbar + par * K + k;
-            if (X > 1 && lane == 0) mbar_expect_tx(bar, (uint32_t)(T * kRepBlock * sizeof(float2)));
+            if (X > 1 && lane == 0) mbar_expect_tx(bar, (uint32_t)(msgs * kRepBlock * sizeof(float2)));
             // the next move's draw, and its sites' amplitudes in the state the
             // chains are reading (move m's decision can change only ci0, cj0)
             int ni0 = 0, nj0 = 0;
@@ -265,42 +311,28 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 naj = amp(nj0);
                 draw(m + 1);
             }
-            bool ok = __all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(m >> 1) & 1u, P.status, limit));
-            // partials in tree order: a CTA's chains, then the CTAs
-            float2 hi = make_float2(0.f, 0.f), hj = hi;
-            const float2* xi = xbuf + ((size_t)par * T * K + k) * kRepBlock + lane;
-            const float2* xj = xi + (size_t)CW * KB;
-            for (int q = 0; q < P.cluster; q++) {
-                float2 pi = make_float2(0.f, 0.f), pj = pi;
-                for (int w0 = 0; w0 < P.warps; w0 += 4) {
-                    float2 vi[4], vj[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                        if (w0 + u < P.warps) {
-                            vi[u] = xi[(size_t)(q * P.warps + w0 + u) * KB];
-                            vj[u] = xj[(size_t)(q * P.warps + w0 + u) * KB];
-                            ok = ok && __float_as_uint(vi[u].x) != kAbortMark && __float_as_uint(vj[u].x) != kAbortMark;
-                        }
-#pragma unroll
-                    for (int u = 0; u < 4; u++)
-                        if (w0 + u < P.warps) {
-                            if (w0 + u == 0) {
-                                pi = vi[u];
-                                pj = vj[u];
-                            } else {
-                                pi.x += vi[u].x; pi.y += vi[u].y;
-                                pj.x += vj[u].x; pj.y += vj[u].y;
-                            }
-                        }
+            bool ok = __all_sync(0xffffffffu, mbar_wait(cbar, (uint32_t)m & 1u, P.status, limit) && gave_up == 0);
+            const float2* mine = part + k * kRepBlock + lane;
+            int gw = W;                              // values per group still to be summed
+            if (X > 1) {
+                // this CTA's messages to every CTA
+                const uint32_t dx = smem_u32(xbuf + ((par * msgs + rank * local) * K + k) * kRepBlock + lane);
+                const uint32_t db = smem_u32(bar);
+#pragma unroll 1
+                for (int u = 0; u < local; u++) {
+                    bool none = true;
+                    float2 v = grouped ? tree_sum(mine + u * W * KB, 1, W, KB, 0, none) : mine[u * KB];
+                    if (!ok) v.x = __uint_as_float(kAbortMark);
+                    for (int q = 0; q < X; q++)
+                        st_async_f2(map_rank(dx + u * (uint32_t)(KB * sizeof(float2)), (uint32_t)q), v,
+                                    map_rank(db, (uint32_t)q));
                 }
-                if (q == 0) {
-                    hi = pi;
-                    hj = pj;
-                } else {
-                    hi.x += pi.x; hi.y += pi.y;
-                    hj.x += pj.x; hj.y += pj.y;
-                }
+                ok = ok && __all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(m >> 1) & 1u, P.status, limit));
+                mine = xbuf + (par * msgs * K + k) * kRepBlock + lane;
+                if (grouped) gw = 1;
             }
+            const float2 hi = tree_sum(mine, C, gw, KB, 2 * gw * KB, ok);
+            const float2 hj = tree_sum(mine + gw * KB, C, gw, KB, 2 * gw * KB, ok);
             if (!__all_sync(0xffffffffu, ok)) {      // every CTA of the unit reads the same marks
                 stop = 1;
                 __threadfence_block();
@@ -316,9 +348,23 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
             if (beta_d == 0.0) accept = true;
             else accept = (dE <= 0.f) || (cu < expf(-beta * dE));
             const float2 ai_post = accept ? cain : cai, aj_post = accept ? cajn : caj;
+            if (rank == 0 && P.trace != nullptr && U.sample == P.trace_sample && U.rep_begin + rr == P.trace_rep &&
+                active) {
+                const long long idx = (sweep0 + m / steps - P.trace_sweep0) * steps + m % steps;
+                if (idx >= 0 && idx < P.trace_cap) {
+                    pspin_move_record* rec = reinterpret_cast<pspin_move_record*>(P.trace) + idx;
+                    rec->i0 = ci0; rec->j0 = cj0;
+                    rec->ai_old[0] = cai.x; rec->ai_old[1] = cai.y;
+                    rec->aj_old[0] = caj.x; rec->aj_old[1] = caj.y;
+                    rec->ai_new[0] = cain.x; rec->ai_new[1] = cain.y;
+                    rec->aj_new[0] = cajn.x; rec->aj_new[1] = cajn.y;
+                    rec->dE = dE;
+                    rec->accepted = accept ? 1 : 0;
+                    rec->log_q_ratio = 0.f;
+                    rec->log_u = logf(cu);
+                }
+            }
             const int pi0 = ci0, pj0 = cj0;
-            const float2 pai = cai, paj = caj, pain = cain, pajn = cajn;
-            const float pu = cu;
             // the next proposal and the final values of the state it reads
             if (m + 1 < total) {
                 cai = ni0 == pi0 ? ai_post : (ni0 == pj0 ? aj_post : nai);
@@ -342,28 +388,14 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 nacc++;
             }
             nprop++;
-            if (rank == 0 && P.trace != nullptr && U.sample == P.trace_sample && U.rep_begin + rr == P.trace_rep &&
-                active) {
-                const long long idx = (sweep0 + m / steps - P.trace_sweep0) * steps + m % steps;
-                if (idx >= 0 && idx < P.trace_cap) {
-                    pspin_move_record* rec = reinterpret_cast<pspin_move_record*>(P.trace) + idx;
-                    rec->i0 = pi0; rec->j0 = pj0;
-                    rec->ai_old[0] = pai.x; rec->ai_old[1] = pai.y;
-                    rec->aj_old[0] = paj.x; rec->aj_old[1] = paj.y;
-                    rec->ai_new[0] = pain.x; rec->ai_new[1] = pain.y;
-                    rec->aj_new[0] = pajn.x; rec->aj_new[1] = pajn.y;
-                    rec->dE = dE;
-                    rec->accepted = accept ? 1 : 0;
-                    rec->log_q_ratio = 0.f;
-                    rec->log_u = logf(pu);
-                }
-            }
         }
     } else if (warp == c + K) {
         // ------------------------------------------------------------ producer: lane = chain of this CTA
-        const int g = (int)rank * c + lane;
+        // chain g of the move: the groups alternate between the lists, group 2q
+        // the W chains of CTA q of the tree in list i, 2q + 1 in list j
+        const int g = (int)rank * c + lane, W = P.warps, list = (g / W) & 1;
         const bool mine = lane < c;
-        const int part0 = (g >> 1) * (kSplit / CW), part1 = part0 + kSplit / CW;
+        const int part0 = (g / (2 * W) * W + g % W) * (kSplit / CW), part1 = part0 + kSplit / CW;
         const int* lists = P.site_chunks + S.split_off;
         int2* tg = tags + lane * stages;
         unsigned char* ring = smem_raw + Lo.ring + (size_t)lane * stages * kStage * sizeof(int2);
@@ -372,7 +404,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         auto open = [&]() {                          // move m's chunks
             int i0, j0;
             pair_of(m, i0, j0);
-            const int* sc = lists + ((g & 1) ? j0 : i0) * (kSplit + 1);
+            const int* sc = lists + (list ? j0 : i0) * (kSplit + 1);
             cur = __ldg(sc + part0);
             end = __ldg(sc + part1);
         };
@@ -478,7 +510,7 @@ static cudaError_t ring_dispatch(SweepParams p, const RingPlan& r, int n_units, 
     p.exec = r.exec;
     p.chains = r.chains;
     p.stages = r.stages;
-    const size_t smem = ring_layout(max_N, 2 * p.cluster * p.warps, p.chains, p.stages, K).total;
+    const size_t smem = ring_layout(max_N, p.warps, p.cluster, p.chains, p.stages, K).total;
     const bool lat = r.lat != 0;
 #define PSPIN_RING(V, KK) (lat ? ring_launch<V, KK, true>(p, n_units, smem, st, max_clusters) \
                                : ring_launch<V, KK, false>(p, n_units, smem, st, max_clusters))
@@ -500,7 +532,7 @@ bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int varia
     p.cluster = cluster;
     auto resident = [&](int X, int stages, int lat) {
         if (X > 16 || X > T || T / X > kMaxChains || (lat && T / X > kLatChains)) return 0;
-        if (ring_layout(max_N, T, T / X, stages, K).total > kRingSmemMax) return 0;
+        if (ring_layout(max_N, warps, cluster, T / X, stages, K).total > kRingSmemMax) return 0;
         const RingPlan q{X, T / X, stages, lat};
         int n = 0;
         if (ring_dispatch(p, q, n_units, variant, max_N, K, nullptr, &n) != cudaSuccess) {

@@ -31,3 +31,26 @@ def test_plan_does_not_change_the_chain(warps, cluster, lanes, kw):
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
     assert out[0][2].sum() > 0
+
+
+@pytest.mark.parametrize("kw", [dict(N=12, nrep=33, fmc_mode=2, gamma=0.3), dict(N=33, nrep=40, fmc_mode=2, gamma=0.1),
+                                dict(N=40, nrep=8, fmc_mode=2, gamma=0.004), dict(N=64, nrep=20, fmc_mode=2, gamma=0.1),
+                                dict(N=24, nrep=5, fmc_mode=1, gamma=2.0), dict(N=70, nrep=4, fmc_mode=2, gamma=0.9)])
+@pytest.mark.parametrize("warps,cluster,lanes", [(8, 1, 1), (2, 16, 1), (8, 2, 3), (4, 1, 2)])
+def test_tiles_equal_records(kw, warps, cluster, lanes):
+    """A masked sample's lists as dense tiles (few and many terms per group,
+    groups longer than 32 terms, columns of one and of eight) and as per-term
+    records (generic_lists) give the same chain bit for bit."""
+    import cuda_pspin_b200 as ps
+    out = []
+    for generic in (False, True):
+        c = ps.default_config(seed=17, T=0.5, **kw)
+        opts = ps.make_options(warps_per_unit=warps, cluster_size=cluster, replicas_per_lane=lanes, generic_lists=generic)
+        with ps.Engine(c, ps.PSPIN_DENSE, opts) as eng:
+            eng.fill_betas(2.0)
+            eng.sweep(2)
+            E, acc, prop = eng.get_results()
+            out.append((eng.get_spins()[0], E, acc, prop))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][2].sum() > 0
