@@ -155,8 +155,11 @@ struct pspin_state {
     int warps2 = 8, cluster2 = 1;       // block shape of the two-pass (learned / fields) sweep
     int rpl = 1;                        // replicas per lane of the plain CTA / cluster sweep
     std::vector<Unit> units_k[2];       // blocks of 64 and 96 replicas (rpl 2, 3)
-    RingPlan plan{};                    // of the current block shape (plan_key: warps, cluster, rpl it was made for)
-    int plan_key[3] = {0, 0, 0};
+    // of the current block shape, for launches without and with exchanges inside
+    // (plan_key: warps, cluster, rpl, exchanging replicas it was made for)
+    RingPlan plan[2] = {};
+    int plan_key[2][4] = {};
+    int* d_queue = nullptr;             // task counter, then tasks finished per replica block
     int64_t spin_total = 0;
     cudaStream_t st = nullptr;
     int device = 0;
@@ -246,7 +249,7 @@ static void free_state(pspin_state* s) {
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     void* ptrs[] = {s->d_samples, s->d_units, s->d_spins, s->d_E, s->d_beta, s->d_target, s->d_drift,
                     s->d_e2, s->d_e4, s->d_epart, s->d_acc, s->d_prop, s->d_key, s->d_entries, s->d_chunk_start, s->d_site_chunks,
-                    s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status,
+                    s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status, s->d_queue,
                     s->d_beta_sched, s->d_perm, s->d_drand, s->d_ex_acc, s->d_ex_prop, s->d_trace,
                     s->d_tc_w, s->d_tc_x, s->d_tc_f, s->d_tc_ws, s->d_tc_h, s->d_f64_h, s->d_tc_e,
                     s->d_w32, s->d_adam_m, s->d_adam_v, s->d_grad, s->d_wbf, s->d_records, s->d_rec_count,
@@ -736,7 +739,7 @@ static int run_energy(pspin_state* s, double* e2, double* e4, bool overwrite, bo
     return PSPIN_OK;
 }
 
-static int current_plan(pspin_state* s);
+static int current_plan(pspin_state* s, int pt_slots);
 
 extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, const pspin_options* opt,
                                   pspin_state** out) {
@@ -1019,7 +1022,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
     }
     if (sweep_smem_bytes(s->max_N, s->warps) > 227 * 1024)
         return bail(fail(PSPIN_ERR_ARG, "N=%d needs more shared memory than a CTA has", s->max_N));
-    if (s->rpl > 1 && s->cluster >= 1 && current_plan(s) != PSPIN_OK)
+    if (s->rpl > 1 && s->cluster >= 1 && current_plan(s, 0) != PSPIN_OK)
         return bail(fail(PSPIN_ERR_ARG, "N=%d with %d replicas per lane needs more shared memory than a CTA has",
                          s->max_N, s->rpl));
 
@@ -1036,7 +1039,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         (rc = dalloc(&s->d_q64, (size_t)std::max<int64_t>(q_total, 1))) ||
         (rc = dalloc(&s->d_g2, (size_t)g2_total)) || (rc = dalloc(&s->d_sweep_counter, 1)) ||
         (rc = dalloc(&s->d_nbmask, (size_t)std::max<int64_t>(nb_total, 1))) ||
-        (rc = dalloc(&s->d_status, 1)) || (rc = dalloc(&s->d_units_k[0], s->units_k[0].size())) ||
+        (rc = dalloc(&s->d_status, 1)) || (rc = dalloc(&s->d_queue, s->units.size() + 1)) || (rc = dalloc(&s->d_units_k[0], s->units_k[0].size())) ||
         (rc = dalloc(&s->d_units_k[1], s->units_k[1].size())))
         return bail(rc);
     auto up = [&](void* dst, const void* src, size_t bytes) -> int {
@@ -1117,14 +1120,15 @@ static int n_units_of(const pspin_state* s, int K) {
 }
 static const Unit* units_dev(const pspin_state* s, int K) { return K > 1 ? s->d_units_k[K - 2] : s->d_units; }
 
-// how the current block shape's chains are spread over the machine
-static int current_plan(pspin_state* s) {
-    const int key[3] = {s->warps, s->cluster, s->rpl};
-    if (std::memcmp(key, s->plan_key, sizeof(key)) == 0) return PSPIN_OK;
-    if (!plan_sweep_ring(s->plan, s->warps, s->cluster, n_units_of(s, s->rpl), s->variant, s->max_N, s->rpl))
+// How the current block shape's chains are spread over the machine, in launches
+// without (pt_slots 0) or with exchanges inside.
+static int current_plan(pspin_state* s, int pt_slots) {
+    const int w = pt_slots > 0, key[4] = {s->warps, s->cluster, s->rpl, pt_slots};
+    if (std::memcmp(key, s->plan_key[w], sizeof(key)) == 0) return PSPIN_OK;
+    if (!plan_sweep_ring(s->plan[w], s->warps, s->cluster, n_units_of(s, s->rpl), s->variant, s->max_N, s->rpl, pt_slots))
         return fail(PSPIN_ERR_CUDA, "block shape %d warps x %d CTAs with %d replicas per lane does not fit at N=%d", s->warps,
                     s->cluster, s->rpl, s->max_N);
-    std::memcpy(s->plan_key, key, sizeof(key));
+    std::memcpy(s->plan_key[w], key, sizeof(key));
     return PSPIN_OK;
 }
 
@@ -1132,7 +1136,7 @@ static int current_plan(pspin_state* s) {
 // (which advances the device sweep counter) and, after an exchange, the
 // observable recorder.  No host bookkeeping, so a sequence of steps can be
 // captured in a CUDA graph; e0/e1 (optional) bracket the sweep kernel.
-static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t e0, cudaEvent_t e1) {
+static SweepParams sweep_params(pspin_state* s, int nsweeps) {
     SweepParams p{};
     p.samples = s->d_samples;
     p.units = s->d_units;
@@ -1159,27 +1163,31 @@ static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t 
     p.status = s->d_status;
     p.wait_clocks = s->opt.wait_limit_clocks > 0 ? (long long)s->opt.wait_limit_clocks : kWaitClocks;
     p.stall_move = s->opt.test_stall_move > 0 ? s->opt.test_stall_move - 1 : -1;
-    if (e0) CK(cudaEventRecord(e0, s->st));
     p.cluster = s->proposal == PSPIN_PROPOSAL_PLAIN ? s->cluster : s->cluster2;
-    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0) {
-        CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, s->st));
-    } else if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
-        TRY(current_plan(s));
-        p.units = units_dev(s, s->rpl);
-        CK(launch_sweep_ring(p, s->plan, n_units_of(s, s->rpl), s->variant, s->max_N, s->rpl, s->st));
-    } else {
-        if (!s->d_site_chunks_g || !s->d_pair_chunks)
-            return fail(PSPIN_ERR_STATE, "two-pass sweep without its group-format lists (pspin_set_proposal builds them)");
-        LearnParams lp{};
-        lp.mode = s->proposal;
-        lp.w = s->d_wbf;
-        lp.records = s->d_records;
-        lp.rec_count = s->d_rec_count;
-        lp.rec_cap = s->rec_cap;
-        lp.rec_prob = s->rec_prob;
-        CK(launch_learned_sweep(p, lp, (int)s->units.size(), s->max_N, s->st, nullptr));
+    return p;
+}
+
+// The ring kernel on the current block shape.  Launches of several sweeps on more
+// units than run at once, and launches with exchanges inside, are cut in tasks.
+static int enqueue_ring(pspin_state* s, SweepParams& p, int pt_slots) {
+    TRY(current_plan(s, pt_slots));
+    const RingPlan& plan = s->plan[pt_slots > 0];
+    const int n_units = n_units_of(s, s->rpl);
+    p.units = units_dev(s, s->rpl);
+    p.n_units = n_units;
+    // two sweeps (PT steps) per task: units of uneven N pack without a common
+    // end of every sweep, and a task is long against its start (some 10 us)
+    p.chunk = 2 * std::max(1, p.pt_freq);
+    if (n_units > plan.resident && p.nsweeps > p.chunk) {
+        p.queue = s->d_queue;
+        p.done = s->d_queue + 1;
+        CK(cudaMemsetAsync(s->d_queue, 0, (size_t)(n_units + 1) * sizeof(int), s->st));
     }
-    if (e1) CK(cudaEventRecord(e1, s->st));
+    CK(launch_sweep_ring(p, plan, n_units, s->variant, s->max_N, s->rpl, pt_slots, s->st));
+    return PSPIN_OK;
+}
+
+static int enqueue_counter(pspin_state* s, int nsweeps, bool exchange) {
     ExchangeParams x{};
     x.n_samples = s->S;
     x.NT = s->pt_NT;
@@ -1196,6 +1204,30 @@ static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t 
     x.nsweeps_done = nsweeps;
     x.do_exchange = exchange ? 1 : 0;
     CK(launch_exchange(x, s->st));
+    return PSPIN_OK;
+}
+
+static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t e0, cudaEvent_t e1) {
+    SweepParams p = sweep_params(s, nsweeps);
+    if (e0) CK(cudaEventRecord(e0, s->st));
+    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0) {
+        CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, s->st));
+    } else if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
+        TRY(enqueue_ring(s, p, 0));
+    } else {
+        if (!s->d_site_chunks_g || !s->d_pair_chunks)
+            return fail(PSPIN_ERR_STATE, "two-pass sweep without its group-format lists (pspin_set_proposal builds them)");
+        LearnParams lp{};
+        lp.mode = s->proposal;
+        lp.w = s->d_wbf;
+        lp.records = s->d_records;
+        lp.rec_count = s->d_rec_count;
+        lp.rec_cap = s->rec_cap;
+        lp.rec_prob = s->rec_prob;
+        CK(launch_learned_sweep(p, lp, (int)s->units.size(), s->max_N, s->st, nullptr));
+    }
+    if (e1) CK(cudaEventRecord(e1, s->st));
+    TRY(enqueue_counter(s, nsweeps, exchange));
     if (exchange && s->obs_cap > 0) {
         ObserveParams o{};
         o.n_samples = s->S;
@@ -1219,17 +1251,47 @@ static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t 
 
 static int do_resync(pspin_state* s);
 
-// host counters after `steps` steps of nsweeps sweeps each; the resync when due
-static int account_steps(pspin_state* s, int steps, int nsweeps, bool exchange) {
-    s->sweep_launches += steps;
-    s->kernel_launches += (long long)steps * (2 + ((exchange && s->obs_cap > 0) ? 1 : 0));
-    s->sweeps_done += (long long)steps * nsweeps;
-    s->since_resync += (long long)steps * nsweeps;
+// host counters after `sweeps` more sweeps; the resync when due
+static int account_sweeps(pspin_state* s, long long sweeps) {
+    s->sweeps_done += sweeps;
+    s->since_resync += sweeps;
     if (s->opt.resync_every > 0 && s->since_resync >= s->opt.resync_every) {
         TRY(do_resync(s));
         s->since_resync = 0;
     }
     return PSPIN_OK;
+}
+
+// after `steps` steps of nsweeps sweeps each, one sweep launch a step
+static int account_steps(pspin_state* s, int steps, int nsweeps, bool exchange) {
+    s->sweep_launches += steps;
+    s->kernel_launches += (long long)steps * (2 + ((exchange && s->obs_cap > 0) ? 1 : 0));
+    return account_sweeps(s, (long long)steps * nsweeps);
+}
+
+// Whether PT steps run inside one sweep launch: the plain ring-fed sweep with
+// every sample one replica block, and nothing recorded between steps.
+static bool steps_in_launch(const pspin_state* s) {
+    return s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0 && s->obs_cap == 0 && !s->profiling &&
+           n_units_of(s, s->rpl) == s->S;
+}
+
+static int launch_steps(pspin_state* s, int steps) {
+    SweepParams p = sweep_params(s, steps * s->pt_freq);
+    p.pt_freq = s->pt_freq;
+    p.NT = s->pt_NT;
+    p.nrep = s->pt_nrep;
+    p.beta_sched = s->d_beta_sched;
+    p.beta_out = s->d_beta;
+    p.perm = s->d_perm;
+    p.drand_state = s->d_drand;
+    p.ex_acc = s->d_ex_acc;
+    p.ex_prop = s->d_ex_prop;
+    TRY(enqueue_ring(s, p, s->pt_NT * s->pt_nrep));
+    TRY(enqueue_counter(s, steps * s->pt_freq, false));
+    s->sweep_launches++;
+    s->kernel_launches += 2;
+    return account_sweeps(s, (long long)steps * s->pt_freq);
 }
 
 static int launch_chunk(pspin_state* s, int nsweeps, bool exchange) {
@@ -1265,7 +1327,7 @@ static int graph_steps(const pspin_state* s) {
 // same move and pair streams as direct launches would.
 static int capture_graph(pspin_state* s, int G) {
     drop_graph(s);
-    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0) TRY(current_plan(s));
+    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0) TRY(current_plan(s, 0));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
     int rc = PSPIN_OK;
@@ -1293,6 +1355,8 @@ static int timeout_error(int status) {
                 status, (status & kStatusDrain) ? ", and the drain of its copies ran out too" : "");
 }
 
+constexpr int kStepsPerLaunch = 256;     // bounds a launch's length
+
 static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
     if (!s) return fail(PSPIN_ERR_ARG, "null handle");
     if (nsweeps < 0) return fail(PSPIN_ERR_ARG, "nsweeps < 0");
@@ -1304,6 +1368,12 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
         if (G > 0 && s->sweeps_done % s->pt_freq == 0) {
             long long room = left;
             if (s->opt.resync_every > 0) room = std::min<long long>(room, s->opt.resync_every - s->since_resync);
+            if (room >= s->pt_freq && steps_in_launch(s)) {
+                const int steps = (int)std::min<long long>(room / s->pt_freq, kStepsPerLaunch);
+                TRY(launch_steps(s, steps));
+                left -= steps * s->pt_freq;
+                continue;
+            }
             const long long reps = room / ((long long)G * s->pt_freq);
             if (reps > 0) {
                 if (!s->graph_exec || s->graph_G != G) TRY(capture_graph(s, G));
@@ -1346,7 +1416,7 @@ static bool shape_fits(pspin_state* s, int warps, int cluster, int K = 1) {
     if (cluster * warps > kSplit) return false;
     if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
         RingPlan r;
-        return plan_sweep_ring(r, warps, cluster, n_units_of(s, K), s->variant, s->max_N, K);
+        return plan_sweep_ring(r, warps, cluster, n_units_of(s, K), s->variant, s->max_N, K, 0);
     }
     if (K > 1) return false;
     if (learned_smem_bytes_host(s->max_N, warps, cluster) > 227 * 1024) return false;

@@ -118,7 +118,7 @@ struct SweepParams {
     int nsweeps;
     int warps;                        // block shape: warps per CTA (divides 32) ...
     int cluster;                      //   ... and CTAs per unit, which fix the summation order of the fields
-    int exec, chains, stages;         // sweep_ring_kernel: the RingPlan the launch runs with
+    int exec, chains, stages, max_N;  // sweep_ring_kernel: the RingPlan the launch runs with, its largest N
     // trace
     int trace_sample, trace_rep, trace_cap;
     long long trace_sweep0;
@@ -126,6 +126,21 @@ struct SweepParams {
     int* status;                      // error word (kStatus* bits)
     long long wait_clocks;            // ring-wait limit in SM clocks
     int stall_move;                   // tests: move index of the stall wait (-1: none)
+    // sweep_ring_kernel, launches of more than one task per unit: tasks of `chunk`
+    // sweeps (the last one the rest of nsweeps), taken in order from *queue; done[u]:
+    // tasks of unit u that are finished (-1: it aborted)
+    int n_units, chunk;
+    int* queue;                       // null: one task, block b runs unit b / exec
+    int* done;
+    // PT steps inside the launch (pt_freq > 0; every unit a whole sample):
+    // exchange after every pt_freq sweeps
+    int pt_freq, NT, nrep;
+    const double* beta_sched;         // [NT]
+    double* beta_out;                 // = beta
+    int* perm;                        // [S][NT*nrep]
+    unsigned long long* drand_state;  // [S]
+    long long* ex_acc;                // [S][NT-1]
+    long long* ex_prop;
 };
 
 // Shared memory that one replica block of a sample needs at least: the limit
@@ -137,17 +152,18 @@ inline size_t sweep_smem_bytes(int N, int warps) {
 
 // How sweep_ring_kernel spreads a unit's chains: over exec CTAs of `chains`
 // chain warps, each with a ring of `stages` chunks; lat: the form for few
-// units.
+// units; resident: units that run at once.
 struct RingPlan {
-    int exec, chains, stages, lat;
+    int exec, chains, stages, lat, resident;
 };
 constexpr size_t kRingSmemMax = 227 * 1024 - 64;   // (the kernel's static shared memory)
-bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int variant, int max_N, int K);
+// pt_slots: replicas per unit that exchange inside the launch (0: none)
+bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int variant, int max_N, int K, int pt_slots);
 
 // kernels (launchers are host functions in the .cu files)
 // units of up to 32K replicas, K = 1, 2, 3 replicas per lane
 cudaError_t launch_sweep_ring(const SweepParams& p, const RingPlan& r, int n_units, int variant, int max_N, int K,
-                              cudaStream_t st);
+                              int pt_slots, cudaStream_t st);
 // the list-resident kernel; warps > 1 runs batches of consecutive moves that
 // commute (no site of one in the other's quartet neighbourhood) on separate
 // warps, with the neighbour masks `nbmask`

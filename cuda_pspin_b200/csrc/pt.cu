@@ -1,6 +1,6 @@
 // pt.cu -- FP64 energies (resync, split) and the device-side replica exchange.
+#include "exchange.cuh"
 #include "internal.h"
-#include "rng.cuh"
 
 namespace pspin {
 
@@ -239,20 +239,13 @@ cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStr
 }
 
 // ---------------------------------------------------------------------
-// Replica exchange, parallel_tempering.cu:316-352, one warp per sample.
-// t runs from the hottest pair upwards and a swap is applied before the
-// next t is tried, so a replica may climb several rungs in one pass; the
-// uniform is drawn only when delta < 0 (:333-334).  Then betas are
-// rebuilt from perm (:347-351).  Thread 0 of block 0 advances the global
-// sweep counter.
-//
-// The nrep columns of one t touch different replicas, so the lanes take one
-// column each; the draws keep the column order: the lane whose column is the
-// k-th with delta < 0 steps the drand48 state k + 1 times on its own.  With
-// the permutation and the energies staged in shared memory in slot order a t
-// costs a few shared-memory latencies instead of nrep chains of dependent
-// global reads: 256 samples of 24 x 4 replicas 116 -> 23 us before the schedule
-// and the counters were staged too, one sample 46 -> 25 us (32 x 4).
+// Replica exchange of every sample (exchange.cuh), one warp per sample; then
+// betas are rebuilt from perm (:347-351).  Thread 0 of block 0 advances the
+// global sweep counter.  With the permutation and the energies staged in shared
+// memory in slot order a temperature costs a few shared-memory latencies instead
+// of nrep chains of dependent global reads: 256 samples of 24 x 4 replicas took
+// 116 us with one thread each, 23 us before the schedule and the counters were
+// staged too; one sample of 32 x 4 46 and 25 us.
 // ---------------------------------------------------------------------
 // Staged per sample: [RT] energies, [NT] betas, [RT] replicas, [NT] swap counts.
 constexpr size_t kExchangeSmem = 48 * 1024;
@@ -287,54 +280,19 @@ __global__ void __launch_bounds__(32) exchange_kernel(const ExchangeParams P) {
         }
         __syncwarp();
     }
-    for (int t = 0; t < NT - 1; t++) {
-        const double db = sched[t] - sched[t + 1];
-        int n_swap = 0;
-        for (int r0 = 0; r0 < nr; r0 += 32) {
-            const int r = r0 + lane, ia = t * nr + r, ib = ia + nr;
-            const bool on = r < nr;
-            int a = 0, b = 0;
-            double Ea = 0.0, Eb = 0.0;
-            if (on) {
-                a = slot[ia];
-                b = slot[ib];
-                Ea = staged ? Es[ia] : E[a];
-                Eb = staged ? Es[ib] : E[b];
-            }
-            const double delta = db * (Ea - Eb);
-            bool ok = on && delta >= 0.0;
-            const bool draw = on && !ok;
-            const unsigned draws = __ballot_sync(0xffffffffu, draw);
-            if (draws) {
-                uint64_t mine = st;
-                if (draw) {
-                    const double w = exp(delta);
-                    double u = 0.0;
-                    for (int q = __popc(draws & ((1u << lane) - 1u)); q >= 0; q--) u = drand48_next(mine);
-                    ok = u < w;
-                }
-                st = __shfl_sync(0xffffffffu, mine, 31 - __clz(draws));
-            }
-            if (ok) {
-                slot[ia] = b;
-                slot[ib] = a;
-                if (staged) {
-                    Es[ia] = Eb;
-                    Es[ib] = Ea;
-                }
-            }
-            n_swap += __popc(__ballot_sync(0xffffffffu, ok));
-        }
-        if (lane == 0) {
-            if (staged) {
-                swaps[t] = n_swap;
-            } else {
-                acc[t] += n_swap;
-                prop[t] += nr;
-            }
-        }
-        __syncwarp();
-    }
+    if (staged)
+        exchange_pass(slot, sched, NT, nr, st, [&](int i, int) { return Es[i]; },
+                      [&](int i, int j, double Ei, double Ej) {
+                          Es[i] = Ej;
+                          Es[j] = Ei;
+                      },
+                      [&](int t, int n) { swaps[t] = n; });
+    else
+        exchange_pass(slot, sched, NT, nr, st, [&](int, int r) { return E[r]; }, [](int, int, double, double) {},
+                      [&](int t, int n) {
+                          acc[t] += n;
+                          prop[t] += nr;
+                      });
     if (lane == 0) P.drand_state[s] = st;
     double* beta = P.beta + S.rep_off;
     for (int i = lane; i < RT; i += 32) {

@@ -86,7 +86,7 @@ __device__ __forceinline__ void load_block_amplitudes(float2* sp, const float2* 
             const int idx = i0 + u * step;
             const int site = idx / kb, col = idx - site * kb;
             v[u] = make_float2(1.f, 0.f);
-            if (idx < total && col < rep_count) v[u] = src[site * R + col];
+            if (idx < total && col < rep_count) v[u] = __ldcg(src + site * R + col);
         }
 #pragma unroll
         for (int u = 0; u < kInFlight; u++) {

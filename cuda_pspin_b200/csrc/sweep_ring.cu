@@ -45,10 +45,19 @@
 //    With every warp deciding for itself and fetching its own chunks (8 warps
 //    reading list i, then list j), the benchmark's launch ran the FMA pipe at
 //    37 % and a move of a one-sample run cost 8 us of waiting.
+//  * A launch may hold several tasks per unit (chunks of sweeps, taken in order
+//    from a queue, so that units of uneven size pack onto the SMs without a
+//    barrier per sweep) and, where every unit is a whole sample, the replica
+//    exchange after every pt_freq sweeps: every CTA's deciders exchange on their
+//    own copy of the energies and the permutation, behind the chains' pass of the
+//    next move.  __FUSED__
 //  * All waits are bounded; a chain whose copy does not arrive sends a marked
 //    partial, so every CTA of the unit leaves at the same move, and nothing is
 //    written back.
 //  * FP32 amplitudes and fields; the running energy is FP64.
+#include <algorithm>
+
+#include "exchange.cuh"
 #include "sweep_common.cuh"
 #include "../../include/pspin.h"
 
@@ -64,17 +73,21 @@ __device__ __forceinline__ bool is_marked(const float2 v) { return __float_as_ui
 // Shared memory of one CTA: amplitudes [N+1][K][32] float2; rings
 // [chains][stages][kStage] int2; the chains' partials [chains][K][32] float2;
 // exchange buffer [2][messages][K][32] float2 (messages: see ring_messages);
-// mbarriers full, empty [chains][stages], chains' arrival, messages [2][K]; ring
-// tags [chains][stages] int2.
+// mbarriers full, empty [chains][stages], chains' arrival, messages [2][K],
+// deciders' meeting; ring
+// tags [chains][stages] int2; with exchanges in the launch (pt_slots replicas),
+// energies by replica, energies by slot, betas by replica, schedule [pt_slots]
+// double each, replicas by slot, swap counts [pt_slots] int each.
 struct RingLayout {
-    size_t ring, part, xbuf, bars, tags, total;
+    size_t ring, part, xbuf, bars, tags, pt, total;
 };
 // What a unit's CTAs exchange per move: the sums of the tree's 2*C groups of W
 // chains where a CTA holds whole groups, else the 2*C*W chains.
 __host__ __device__ inline int ring_messages(int warps, int cluster, int chains) {
     return chains % warps == 0 ? 2 * cluster : 2 * cluster * warps;
 }
-__host__ __device__ inline RingLayout ring_layout(int N, int warps, int cluster, int chains, int stages, int K) {
+__host__ __device__ inline RingLayout ring_layout(int N, int warps, int cluster, int chains, int stages, int K,
+                                                  int pt_slots) {
     RingLayout L;
     const size_t row = (size_t)K * kRepBlock * sizeof(float2);
     L.ring = (size_t)(N + 1) * row;
@@ -83,8 +96,9 @@ __host__ __device__ inline RingLayout ring_layout(int N, int warps, int cluster,
     // one CTA holds every group: nothing is exchanged
     const bool alone = chains == 2 * cluster * warps;
     L.bars = L.xbuf + (alone ? 0 : (size_t)2 * ring_messages(warps, cluster, chains) * row);
-    L.tags = L.bars + (size_t)(2 * chains * stages + 1 + 2 * K) * sizeof(uint64_t);
-    L.total = L.tags + (size_t)chains * stages * sizeof(int2);
+    L.tags = L.bars + (size_t)(2 * chains * stages + 2 + 2 * K) * sizeof(uint64_t);
+    L.pt = L.tags + (size_t)chains * stages * sizeof(int2);
+    L.total = L.pt + (size_t)pt_slots * (4 * sizeof(double) + 2 * sizeof(int));
     return L;
 }
 
@@ -171,13 +185,11 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int X = P.exec, c = P.chains, stages = P.stages;
     const uint32_t rank = X > 1 ? cluster_rank() : 0u;
-    const Unit U = P.units[blockIdx.x / X];
-    const SampleDev S = P.samples[U.sample];
-    const int N = S.N, R = S.R;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int CW = P.cluster * P.warps;
     constexpr int KB = K * kRepBlock;
-    const RingLayout Lo = ring_layout(N, P.warps, P.cluster, c, stages, K);
+    // one layout for every unit of the launch (the barriers live through it)
+    const RingLayout Lo = ring_layout(P.max_N, P.warps, P.cluster, c, stages, K, P.pt_freq > 0 ? P.NT * P.nrep : 0);
     float2* sp = reinterpret_cast<float2*>(smem_raw);
     float2* part = reinterpret_cast<float2*>(smem_raw + Lo.part);
     float2* xbuf = reinterpret_cast<float2*>(smem_raw + Lo.xbuf);
@@ -185,28 +197,81 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     uint64_t* empty = full + c * stages;
     uint64_t* cbar = empty + c * stages;
     uint64_t* xbar = cbar + 1;
+    uint64_t* dbar = xbar + 2 * K;
     int2* tags = reinterpret_cast<int2*>(smem_raw + Lo.tags);
+    const int RT = P.pt_freq > 0 ? P.NT * P.nrep : 0;
+    double* pt_E = reinterpret_cast<double*>(smem_raw + Lo.pt);      // [RT] by replica
+    double* pt_Es = pt_E + RT;                                        // [RT] by slot
+    double* pt_beta = pt_Es + RT;                                     // [RT] by replica
+    double* pt_sched = pt_beta + RT;                                  // [NT]
+    int* pt_slot = reinterpret_cast<int*>(pt_sched + RT);             // [RT]
+    int* pt_swaps = pt_slot + RT;                                     // [NT]
     __shared__ volatile int stop, gave_up;           // the unit aborts; a chain of this CTA gave up
+    __shared__ volatile int task_s;
     __shared__ __align__(8) uint64_t stall_bar;      // test hook: nothing arrives on it
 
     if (threadIdx.x == 0) {
         for (int q = 0; q < 2 * c * stages; q++) mbar_init(full + q, 1);
         mbar_init(cbar, (uint32_t)c);                // every chain of the CTA
         for (int q = 0; q < 2 * K; q++) mbar_init(xbar + q, 1);   // bytes, armed by the decider
+        mbar_init(dbar, (uint32_t)K);
         mbar_init(&stall_bar, 1);
         stop = gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_shared();
     }
-    load_block_amplitudes(sp, P.spins + S.spin_off + U.rep_begin, R, N, KB, U.rep_count);   // column k*32 + lane
-    for (int idx = threadIdx.x; idx < KB; idx += blockDim.x) sp[(size_t)N * KB + idx] = make_float2(1.f, 0.f);
-
-    const long long sweep0 = *P.sweep_counter;
-    const int steps = N / 2, total = P.nsweeps * steps;
+    const long long sweep_base = *P.sweep_counter;
     const int state_threads = (c + K) * 32;
     const bool decider = warp >= c && warp < c + K;
     const int k = warp - c;                          // decider's replica group
     const int rr = k * kRepBlock + lane;
+    const long long limit = 2 * P.wait_clocks + kDrainClocks;   // beyond any chain's own bounded wait
+    const int n_tasks = P.queue ? P.n_units * ((P.nsweeps + P.chunk - 1) / P.chunk) : 1;
+    // over all tasks: ring position, moves and deciders' meetings so far
+    uint32_t slot = 0, phase = 0, issued = 0, moves = 0, meetings = 0;
+    if (X > 1) cluster_sync();                       // every CTA of the cluster runs before the first remote store
+
+    for (;;) {
+    // ---- the next task: unit, first sweep, sweeps
+    int unit = (int)blockIdx.x / X, first = 0, nsweeps = P.nsweeps, task = 0;
+    if (P.queue) {
+        if (rank == 0 && threadIdx.x == 0) {
+            int t;
+            for (;;) {
+                t = atomicAdd(P.queue, 1);
+                if (t >= n_tasks) break;
+                // the unit's earlier tasks were taken earlier, by clusters that run
+                const volatile int* done = P.done + t % P.n_units;
+                const long long t0 = clock64(), most = limit * P.chunk * (P.max_N / 2);   // every move of a task bounded
+                int d;
+                while ((d = *done) >= 0 && d < t / P.n_units && clock64() - t0 < most) __nanosleep(200);
+                if (d >= t / P.n_units) break;
+                if (d >= 0) atomicOr(P.status, kStatusTimeout);
+                // the unit has aborted: its later tasks are dropped
+            }
+            __threadfence();
+            for (int q = 0; q < X; q++) {
+                if (X > 1) st_cluster_u32((const void*)&task_s, (uint32_t)q, (uint32_t)t);
+                else task_s = t;
+            }
+        }
+        if (X > 1) cluster_sync();
+        else __syncthreads();
+        task = task_s;
+        if (task >= n_tasks) break;
+        unit = task % P.n_units;
+        first = task / P.n_units * P.chunk;
+        nsweeps = min(P.chunk, P.nsweeps - first);
+    }
+    const Unit U = P.units[unit];
+    const SampleDev S = P.samples[U.sample];
+    const int N = S.N, R = S.R;
+    // amplitudes, energies and betas may have been written by another SM earlier in this launch: read past L1
+    load_block_amplitudes(sp, P.spins + S.spin_off + U.rep_begin, R, N, KB, U.rep_count);   // column k*32 + lane
+    for (int idx = threadIdx.x; idx < KB; idx += blockDim.x) sp[(size_t)N * KB + idx] = make_float2(1.f, 0.f);
+    const long long sweep0 = sweep_base + first;
+    const int steps = N / 2, total = nsweeps * steps;
+    const int per_exchange = P.pt_freq * steps;      // moves between exchanges (0: none)
     const bool active = decider && rr < U.rep_count;
     const int64_t gr = S.rep_off + U.rep_begin + rr;
 
@@ -224,13 +289,23 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         move_trig<VARIANT>(move_words(k0, k1, (uint64_t)(sweep0 + m / steps), (uint32_t)(m % steps)), tt);
     };
     auto amp = [&](int site) -> float2& { return sp[(site * K + k) * kRepBlock + lane]; };
+    uint64_t drand = 0;
     if (active) {
-        beta_d = P.beta[gr];
+        beta_d = __ldcg(P.beta + gr);
         beta = (float)beta_d;
         const uint64_t key = P.key[gr];
         k0 = (uint32_t)key;
         k1 = (uint32_t)(key >> 32);
-        E = P.energy[gr];
+        E = __ldcg(P.energy + gr);
+    }
+    if (decider && k == 0 && per_exchange > 0) {
+        const int* perm = P.perm + (int64_t)U.sample * RT;
+        for (int i = lane; i < RT; i += 32) pt_slot[i] = __ldcg(perm + i);
+        for (int t = lane; t < P.NT; t += 32) {
+            pt_sched[t] = P.beta_sched[t];
+            pt_swaps[t] = 0;
+        }
+        drand = __ldcg(P.drand_state + U.sample);
     }
     __syncthreads();
     if (decider && total > 0) {
@@ -242,8 +317,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         cu = tt[6];
         amp(cj0) = cajn;                             // h_i is evaluated at the proposed a_j
     }
-    if (X > 1) cluster_sync();                       // every CTA's barriers and state are in place
-    else __syncthreads();
+    __syncthreads();
 
     if (warp < c) {
         // ------------------------------------------------------------ chain warp
@@ -252,7 +326,6 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         uint64_t* eb = empty + warp * stages;
         const int2* tg = tags + warp * stages;
         const int2* ring = reinterpret_cast<const int2*>(smem_raw + Lo.ring) + (size_t)warp * stages * kStage;
-        uint32_t slot = 0, phase = 0;
         for (int m = 0; m < total; m++) {
             if (m > 0) {
                 __syncwarp();
@@ -293,12 +366,12 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         }
     } else if (decider) {
         // ------------------------------------------------------------ decider
-        const long long limit = 2 * P.wait_clocks + kDrainClocks;   // beyond any chain's own bounded wait
         const int W = P.warps, C = P.cluster;
         const bool grouped = c % W == 0;
         const int msgs = ring_messages(W, C, c), local = grouped ? c / W : c;
-        for (int m = 0; m < total; m++) {
-            const uint32_t par = (uint32_t)(m & 1);
+        int to_exchange = per_exchange;
+        for (int m = 0; m < total; m++, moves++) {
+            const uint32_t par = moves & 1u;
             uint64_t* bar = xbar + par * K + k;
             if (X > 1 && lane == 0) mbar_expect_tx(bar, (uint32_t)(msgs * kRepBlock * sizeof(float2)));
             // the next move's draw, and its sites' amplitudes in the state the
@@ -311,7 +384,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 naj = amp(nj0);
                 draw(m + 1);
             }
-            bool ok = __all_sync(0xffffffffu, mbar_wait(cbar, (uint32_t)m & 1u, P.status, limit) && gave_up == 0);
+            bool ok = __all_sync(0xffffffffu, mbar_wait(cbar, moves & 1u, P.status, limit) && gave_up == 0);
             const float2* mine = part + k * kRepBlock + lane;
             int gw = W;                              // values per group still to be summed
             if (X > 1) {
@@ -327,7 +400,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                         st_async_f2(map_rank(dx + u * (uint32_t)(KB * sizeof(float2)), (uint32_t)q), v,
                                     map_rank(db, (uint32_t)q));
                 }
-                ok = ok && __all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)(m >> 1) & 1u, P.status, limit));
+                ok = ok && __all_sync(0xffffffffu, mbar_wait(bar, (moves >> 1) & 1u, P.status, limit));
                 mine = xbuf + (par * msgs * K + k) * kRepBlock + lane;
                 if (grouped) gw = 1;
             }
@@ -388,6 +461,40 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 nacc++;
             }
             nprop++;
+            // the replica exchange, behind the chains' next pass (it changes only betas)
+            if (per_exchange > 0 && --to_exchange == 0) {
+                to_exchange = per_exchange;
+                auto meet = [&]() {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(dbar);
+                    return __all_sync(0xffffffffu, mbar_wait(dbar, meetings++ & 1u, P.status, limit));
+                };
+                if (active) pt_E[rr] = E;
+                bool met = meet();
+                if (k == 0 && met) {
+                    for (int i = lane; i < RT; i += 32) pt_Es[i] = pt_E[pt_slot[i]];
+                    __syncwarp();
+                    exchange_pass(pt_slot, pt_sched, P.NT, P.nrep, drand, [&](int i, int) { return pt_Es[i]; },
+                                  [&](int i, int j, double Ei, double Ej) {
+                                      pt_Es[i] = Ej;
+                                      pt_Es[j] = Ei;
+                                  },
+                                  [&](int t, int n) { pt_swaps[t] += n; });
+                    for (int i = lane; i < RT; i += 32) pt_beta[pt_slot[i]] = pt_sched[i / P.nrep];
+                }
+                met = meet() && met;
+                if (!met) {                          // (a wait ran out: the chains stop at the move after the next)
+                    stop = 1;
+                    __threadfence_block();
+                    __syncwarp();
+                    if (m + 2 < total) state_arrive(state_threads);
+                    break;
+                }
+                if (active) {
+                    beta_d = pt_beta[rr];
+                    beta = (float)beta_d;
+                }
+            }
         }
     } else if (warp == c + K) {
         // ------------------------------------------------------------ producer: lane = chain of this CTA
@@ -419,10 +526,9 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
             open();
             bounds();
         }
-        uint32_t issued = 0, slot = 0, phase = 1;    // phase of the slot's last release
         while (__any_sync(0xffffffffu, more) && !__any_sync(0xffffffffu, stop != 0)) {
             bool did = false;
-            if (more && (issued < (uint32_t)stages || mbar_test_wait(empty + lane * stages + slot, phase))) {
+            if (more && (issued < (uint32_t)stages || mbar_test_wait(empty + lane * stages + slot, phase ^ 1u))) {
                 uint64_t* fb = full + lane * stages + slot;
                 if (cur < end) {
                     const uint32_t bytes = (uint32_t)((e - b) * sizeof(int2));
@@ -458,19 +564,45 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         __syncwarp();
     }
 
-    __syncthreads();                                 // every final write before the write-back
-    if (rank == 0 && !stop) {
-        for (int idx = threadIdx.x; idx < N * KB; idx += blockDim.x) {
-            const int site = idx / KB, r = idx % KB;
-            if (r < U.rep_count) P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + r] = sp[idx];
+    if (X > 1 && stop && threadIdx.x == 0)           // a CTA that gave up takes its cluster with it
+        for (int q = 0; q < X; q++) st_cluster_u32((const void*)&stop, (uint32_t)q, 1u);
+    if (X > 1) cluster_sync();                       // every final write; no store may still target a CTA
+    else __syncthreads();
+    const bool good = stop == 0;
+    if (rank == 0) {
+        if (good) {
+            for (int idx = threadIdx.x; idx < N * KB; idx += blockDim.x) {
+                const int site = idx / KB, r = idx % KB;
+                if (r < U.rep_count) P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + r] = sp[idx];
+            }
+            if (active) {
+                P.energy[gr] = E;
+                __stcg(P.accepted + gr, __ldcg(P.accepted + gr) + nacc);
+                __stcg(P.proposed + gr, __ldcg(P.proposed + gr) + nprop);
+                if (per_exchange > 0) P.beta_out[gr] = beta_d;
+            }
+            if (decider && k == 0 && per_exchange > 0) {
+                int* perm = P.perm + (int64_t)U.sample * RT;
+                for (int i = lane; i < RT; i += 32) perm[i] = pt_slot[i];
+                long long* acc = P.ex_acc + (int64_t)U.sample * (P.NT - 1);
+                long long* prop = P.ex_prop + (int64_t)U.sample * (P.NT - 1);
+                for (int t = lane; t < P.NT - 1; t += 32) {
+                    __stcg(acc + t, __ldcg(acc + t) + pt_swaps[t]);
+                    __stcg(prop + t, __ldcg(prop + t) + (long long)(total / per_exchange) * P.nrep);
+                }
+                if (lane == 0) P.drand_state[U.sample] = drand;
+            }
         }
-        if (active) {
-            P.energy[gr] = E;
-            P.accepted[gr] += nacc;
-            P.proposed[gr] += nprop;
+        if (P.queue) {
+            __threadfence();
+            __syncthreads();
+            if (threadIdx.x == 0) atomicExch(P.done + unit, good ? task / P.n_units + 1 : -1);
         }
     }
-    if (X > 1) cluster_sync();                       // no CTA leaves while a store may still target it
+    if (!P.queue || !good) break;
+    __syncthreads();                                 // the write-back has read the amplitudes
+    }   // tasks
+    if (X > 1) cluster_sync();
 }
 
 template <int VARIANT, int K, bool kLat>
@@ -480,7 +612,7 @@ static cudaError_t ring_launch(const SweepParams& p, int n_units, size_t smem, c
     if (e == cudaSuccess && p.exec > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(n_units * p.exec));
+    cfg.gridDim = dim3((unsigned)(n_units * p.exec));          // (with a queue: the units that run at once)
     cfg.blockDim = dim3((unsigned)(32 * (p.chains + K + 1)));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
@@ -506,11 +638,12 @@ static cudaError_t ring_launch(const SweepParams& p, int n_units, size_t smem, c
 }
 
 static cudaError_t ring_dispatch(SweepParams p, const RingPlan& r, int n_units, int variant, int max_N, int K,
-                                 cudaStream_t st, int* max_clusters) {
+                                 int pt_slots, cudaStream_t st, int* max_clusters) {
+    p.max_N = max_N;
     p.exec = r.exec;
     p.chains = r.chains;
     p.stages = r.stages;
-    const size_t smem = ring_layout(max_N, p.warps, p.cluster, p.chains, p.stages, K).total;
+    const size_t smem = ring_layout(max_N, p.warps, p.cluster, p.chains, p.stages, K, pt_slots).total;
     const bool lat = r.lat != 0;
 #define PSPIN_RING(V, KK) (lat ? ring_launch<V, KK, true>(p, n_units, smem, st, max_clusters) \
                                : ring_launch<V, KK, false>(p, n_units, smem, st, max_clusters))
@@ -524,7 +657,7 @@ static cudaError_t ring_dispatch(SweepParams p, const RingPlan& r, int n_units, 
 // one chain per sub-partition, as long as all clusters are resident at once: a
 // launch that leaves SMs idle is bound by the time of one chain.  Three ring
 // slots per chain where they fit, else two, else more CTAs.
-bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int variant, int max_N, int K) {
+bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int variant, int max_N, int K, int pt_slots) {
     if (warps < 1 || cluster < 1 || cluster > 16 || kSplit % (cluster * warps) != 0 || K < 1 || K > 3) return false;
     const int T = 2 * cluster * warps;
     SweepParams p{};
@@ -532,10 +665,10 @@ bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int varia
     p.cluster = cluster;
     auto resident = [&](int X, int stages, int lat) {
         if (X > 16 || X > T || T / X > kMaxChains || (lat && T / X > kLatChains)) return 0;
-        if (ring_layout(max_N, warps, cluster, T / X, stages, K).total > kRingSmemMax) return 0;
-        const RingPlan q{X, T / X, stages, lat};
+        if (ring_layout(max_N, warps, cluster, T / X, stages, K, pt_slots).total > kRingSmemMax) return 0;
+        const RingPlan q{X, T / X, stages, lat, 0};
         int n = 0;
-        if (ring_dispatch(p, q, n_units, variant, max_N, K, nullptr, &n) != cudaSuccess) {
+        if (ring_dispatch(p, q, n_units, variant, max_N, K, pt_slots, nullptr, &n) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
@@ -546,22 +679,23 @@ bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int varia
         for (int X = 16; X >= 1; X /= 2)
             for (int lat = 1; lat >= 0; lat--)
                 if (X <= T && (X <= T / kLatChains || X == x_fill) && resident(X, stages, lat) >= n_units) {
-                    r = RingPlan{X, T / X, stages, lat};
+                    r = RingPlan{X, T / X, stages, lat, n_units};
                     return true;
                 }
     for (int X = x_fill; X <= 16 && X <= T; X *= 2)
         for (int stages = 3; stages >= 2; stages--)
-            if (resident(X, stages, 0) > 0) {
-                r = RingPlan{X, T / X, stages, 0};
+            if (const int n = resident(X, stages, 0)) {
+                r = RingPlan{X, T / X, stages, 0, n};
                 return true;
             }
     return false;
 }
 
 cudaError_t launch_sweep_ring(const SweepParams& p, const RingPlan& r, int n_units, int variant, int max_N, int K,
-                              cudaStream_t st) {
+                              int pt_slots, cudaStream_t st) {
     if (n_units <= 0) return cudaSuccess;
-    return ring_dispatch(p, r, n_units, variant, max_N, K, st, nullptr);
+    return ring_dispatch(p, r, p.queue ? std::min(n_units, r.resident) : n_units, variant, max_N, K, pt_slots, st,
+                         nullptr);
 }
 
 }  // namespace pspin

@@ -54,3 +54,33 @@ def test_tiles_equal_records(kw, warps, cluster, lanes):
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
     assert out[0][2].sum() > 0
+
+
+@pytest.mark.parametrize("samples,Ns,NT,nrep,freq,warps,cluster,lanes", [
+    (1, (12,), 4, 8, 1, 2, 1, 1),              # one block, one replica per lane
+    (3, (8, 17, 12), 6, 5, 2, 8, 1, 2),        # ragged blocks, exchange every second sweep
+    (200, (8, 11, 20, 9), 3, 4, 1, 8, 2, 3),   # more blocks than run at once: tasks from the queue
+    (170, (6, 14), 2, 40, 3, 8, 4, 3),         # the same with 40 columns, a cluster of many CTAs
+])
+def test_steps_in_one_launch_equal_single_steps(samples, Ns, NT, nrep, freq, warps, cluster, lanes):
+    """PT steps inside one launch (exchange by the sweep kernel's deciders,
+    units in tasks) equal one launch per step with the exchange kernel: states,
+    counters, betas by their effect, permutations; across resyncs and partial
+    steps."""
+    import cuda_pspin_b200 as ps
+    out = []
+    for graph_steps in (0, -1):
+        cfgs = [ps.default_config(N=Ns[k % len(Ns)], nrep=NT * nrep, seed=80 + k) for k in range(samples)]
+        opts = ps.make_options(warps_per_unit=warps, cluster_size=cluster, replicas_per_lane=lanes,
+                               graph_steps=graph_steps, resync_every=11)
+        with ps.Engine(cfgs, ps.PSPIN_DENSE, opts) as eng:
+            _, betas = ps.temperature_schedule(NT, 0.3, 1.5, True)
+            eng.pt_init(NT, nrep, betas, freq)
+            for n in (1, 7, 9):
+                eng.pt_run(n)
+            pt = [eng.pt_get(k) for k in range(samples)]
+            out.append([np.concatenate([a.ravel() for a in eng.get_spins()]), *eng.get_results(),
+                        np.stack([p[0] for p in pt]), np.stack([p[1] for p in pt]), np.stack([p[2] for p in pt])])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][5].sum() > 0
