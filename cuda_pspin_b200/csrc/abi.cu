@@ -159,6 +159,8 @@ struct pspin_state {
     // (plan_key: warps, cluster, rpl, exchanging replicas it was made for)
     RingPlan plan[2] = {};
     int plan_key[2][4] = {};
+    int4* d_prep_moves = nullptr;       // the list-resident kernel's prepared moves (workspace)
+    float* d_prep_trig = nullptr;
     int* d_queue = nullptr;             // task counter, then tasks finished per replica block
     int64_t spin_total = 0;
     cudaStream_t st = nullptr;
@@ -249,7 +251,7 @@ static void free_state(pspin_state* s) {
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     void* ptrs[] = {s->d_samples, s->d_units, s->d_spins, s->d_E, s->d_beta, s->d_target, s->d_drift,
                     s->d_e2, s->d_e4, s->d_epart, s->d_acc, s->d_prop, s->d_key, s->d_entries, s->d_chunk_start, s->d_site_chunks,
-                    s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status, s->d_queue,
+                    s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status, s->d_queue, s->d_prep_moves, s->d_prep_trig,
                     s->d_beta_sched, s->d_perm, s->d_drand, s->d_ex_acc, s->d_ex_prop, s->d_trace,
                     s->d_tc_w, s->d_tc_x, s->d_tc_f, s->d_tc_ws, s->d_tc_h, s->d_f64_h, s->d_tc_e,
                     s->d_w32, s->d_adam_m, s->d_adam_v, s->d_grad, s->d_wbf, s->d_records, s->d_rec_count,
@@ -264,6 +266,8 @@ static void free_state(pspin_state* s) {
     if (s->st) cudaStreamDestroy(s->st);
     delete s;
 }
+
+constexpr size_t kPrepBytes = (size_t)64 << 20;      // workspace of the list-resident kernel's prepared moves
 
 // ------------------------------------------------------------------ config
 extern "C" void pspin_default_config(pspin_config* c) {
@@ -1008,7 +1012,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         s->warps2 = s->warps;
         if (c == -1) {
             const int rw = s->opt.warps_per_unit > 0 ? s->opt.warps_per_unit : 1;
-            if (resident_smem_bytes_host(s->max_N, s->max_site_entries, rw) > 227 * 1024)
+            if (resident_smem_bytes_host(s->max_N, s->max_site_entries, rw, 0) > 227 * 1024 - 64)
                 return bail(fail(PSPIN_ERR_ARG, "the site lists do not fit in shared memory (cluster_size -1)"));
             s->cluster = 0;
             s->warps = rw;
@@ -1187,6 +1191,32 @@ static int enqueue_ring(pspin_state* s, SweepParams& p, int pt_slots) {
     return PSPIN_OK;
 }
 
+// sweeps whose prepared moves fit the list-resident kernel's workspace
+static int resident_chunk(const pspin_state* s) {
+    const size_t per = (size_t)(s->max_N / 2) * (s->units.size() * 7 * kRepBlock * sizeof(float) + s->S * sizeof(int4));
+    return (int)std::max<size_t>(1, std::min<size_t>(kPrepBytes / std::max<size_t>(per, 1), 256));
+}
+
+static int ensure_prep(pspin_state* s) {
+    if (s->d_prep_trig) return PSPIN_OK;
+    const size_t moves = (size_t)resident_chunk(s) * (s->max_N / 2);
+    TRY(dalloc(&s->d_prep_moves, (size_t)s->S * moves));
+    return dalloc(&s->d_prep_trig, s->units.size() * moves * 7 * kRepBlock);
+}
+
+// The list-resident kernel (nsweeps <= resident_chunk unless it runs on one warp).
+static int enqueue_resident(pspin_state* s, SweepParams& p, int pt_slots) {
+    if (s->warps > 1) {
+        TRY(ensure_prep(s));
+        p.prep_moves = s->d_prep_moves;
+        p.prep_trig = s->d_prep_trig;
+        p.prep_stride = resident_chunk(s) * (s->max_N / 2);
+    }
+    p.exec = pt_slots > 0 ? (pt_slots + kRepBlock - 1) / kRepBlock : 1;
+    CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, pt_slots, s->st));
+    return PSPIN_OK;
+}
+
 static int enqueue_counter(pspin_state* s, int nsweeps, bool exchange) {
     ExchangeParams x{};
     x.n_samples = s->S;
@@ -1211,7 +1241,7 @@ static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t 
     SweepParams p = sweep_params(s, nsweeps);
     if (e0) CK(cudaEventRecord(e0, s->st));
     if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0) {
-        CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, s->st));
+        TRY(enqueue_resident(s, p, 0));
     } else if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
         TRY(enqueue_ring(s, p, 0));
     } else {
@@ -1269,11 +1299,16 @@ static int account_steps(pspin_state* s, int steps, int nsweeps, bool exchange) 
     return account_sweeps(s, (long long)steps * nsweeps);
 }
 
-// Whether PT steps run inside one sweep launch: the plain ring-fed sweep with
-// every sample one replica block, and nothing recorded between steps.
+// Whether PT steps run inside one sweep launch: the plain sweep, with every sample
+// one replica block (ring-fed) or one cluster of blocks (list-resident), and
+// nothing recorded between steps.
 static bool steps_in_launch(const pspin_state* s) {
-    return s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0 && s->obs_cap == 0 && !s->profiling &&
-           n_units_of(s, s->rpl) == s->S;
+    if (s->proposal != PSPIN_PROPOSAL_PLAIN || s->obs_cap != 0 || s->profiling) return false;
+    if (s->cluster > 0) return n_units_of(s, s->rpl) == s->S;
+    // list-resident: the blocks of a sample as one cluster (every sample has NT*nrep replicas)
+    const int slots = s->pt_NT * s->pt_nrep;
+    return s->warps > 1 && slots <= 8 * kRepBlock && resident_chunk(s) >= s->pt_freq &&
+           resident_smem_bytes_host(s->max_N, s->max_site_entries, s->warps, slots) <= 227 * 1024 - 64;
 }
 
 static int launch_steps(pspin_state* s, int steps) {
@@ -1287,7 +1322,8 @@ static int launch_steps(pspin_state* s, int steps) {
     p.drand_state = s->d_drand;
     p.ex_acc = s->d_ex_acc;
     p.ex_prop = s->d_ex_prop;
-    TRY(enqueue_ring(s, p, s->pt_NT * s->pt_nrep));
+    if (s->cluster > 0) TRY(enqueue_ring(s, p, s->pt_NT * s->pt_nrep));
+    else TRY(enqueue_resident(s, p, s->pt_NT * s->pt_nrep));
     TRY(enqueue_counter(s, steps * s->pt_freq, false));
     s->sweep_launches++;
     s->kernel_launches += 2;
@@ -1328,6 +1364,7 @@ static int graph_steps(const pspin_state* s) {
 static int capture_graph(pspin_state* s, int G) {
     drop_graph(s);
     if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0) TRY(current_plan(s, 0));
+    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1) TRY(ensure_prep(s));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
     int rc = PSPIN_OK;
@@ -1360,7 +1397,9 @@ constexpr int kStepsPerLaunch = 256;     // bounds a launch's length
 static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
     if (!s) return fail(PSPIN_ERR_ARG, "null handle");
     if (nsweeps < 0) return fail(PSPIN_ERR_ARG, "nsweeps < 0");
-    const int G = (pt && !s->profiling) ? graph_steps(s) : 0;
+    int G = (pt && !s->profiling) ? graph_steps(s) : 0;
+    const bool prepared = s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1;
+    if (prepared && pt && s->pt_freq > resident_chunk(s)) G = 0;
     CK(cudaMemsetAsync(s->d_status, 0, sizeof(int), s->st));   // a time-out is reported by the call it happens in
     int left = nsweeps;
     while (left > 0) {
@@ -1369,7 +1408,8 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
             long long room = left;
             if (s->opt.resync_every > 0) room = std::min<long long>(room, s->opt.resync_every - s->since_resync);
             if (room >= s->pt_freq && steps_in_launch(s)) {
-                const int steps = (int)std::min<long long>(room / s->pt_freq, kStepsPerLaunch);
+                int steps = (int)std::min<long long>(room / s->pt_freq, kStepsPerLaunch);
+                if (s->cluster == 0) steps = std::min(steps, resident_chunk(s) / s->pt_freq);
                 TRY(launch_steps(s, steps));
                 left -= steps * s->pt_freq;
                 continue;
@@ -1396,6 +1436,10 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
                 ex = true;
             }
         }
+        if (prepared && chunk > resident_chunk(s)) {
+            chunk = resident_chunk(s);
+            ex = false;
+        }
         if (chunk <= 0) chunk = 1;
         TRY(launch_chunk(s, chunk, ex));
         left -= chunk;
@@ -1412,7 +1456,7 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
 static bool shape_fits(pspin_state* s, int warps, int cluster, int K = 1) {
     if (cluster == 0)
         return K == 1 && s->proposal == PSPIN_PROPOSAL_PLAIN &&
-               resident_smem_bytes_host(s->max_N, s->max_site_entries, warps) <= 227 * 1024;
+               resident_smem_bytes_host(s->max_N, s->max_site_entries, warps, 0) <= 227 * 1024 - 64;
     if (cluster * warps > kSplit) return false;
     if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
         RingPlan r;

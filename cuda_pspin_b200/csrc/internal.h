@@ -141,6 +141,10 @@ struct SweepParams {
     unsigned long long* drand_state;  // [S]
     long long* ex_acc;                // [S][NT-1]
     long long* ex_prop;
+    // sweep_resident_kernel: the prepared parts of a launch's moves
+    int prep_stride;                  // moves per sample and unit
+    int4* prep_moves;                 // [S][prep_stride]
+    float* prep_trig;                 // [units][prep_stride][7][32]
 };
 
 // Shared memory that one replica block of a sample needs at least: the limit
@@ -164,12 +168,12 @@ bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int varia
 // units of up to 32K replicas, K = 1, 2, 3 replicas per lane
 cudaError_t launch_sweep_ring(const SweepParams& p, const RingPlan& r, int n_units, int variant, int max_N, int K,
                               int pt_slots, cudaStream_t st);
-// the list-resident kernel; warps > 1 runs batches of consecutive moves that
-// commute (no site of one in the other's quartet neighbourhood) on separate
-// warps, with the neighbour masks `nbmask`
+// the list-resident kernel; warps > 1 runs moves that commute (no site of one in
+// the other's quartet neighbourhood, by the neighbour masks `nbmask`) at once, on
+// clusters of p.exec units; pt_slots: replicas that exchange inside the launch
 cudaError_t launch_sweep_resident(const SweepParams& p, int n_units, int variant, int max_N, int64_t max_entries,
-                                  cudaStream_t st);
-size_t resident_smem_bytes_host(int N, int64_t entries, int warps);
+                                  int pt_slots, cudaStream_t st);
+size_t resident_smem_bytes_host(int N, int64_t entries, int warps, int pt_slots);
 
 struct EnergyParams {
     const SampleDev* samples;

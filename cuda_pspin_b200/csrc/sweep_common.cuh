@@ -548,6 +548,24 @@ __device__ __forceinline__ void cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
+// the same shared-memory location in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
+    uint32_t ra;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
+    return ra;
+}
+// 8 bytes into a CTA of the cluster, counted on that CTA's mbarrier (cluster
+// launches only)
+__device__ __forceinline__ void st_async_f2(uint32_t addr, float2 v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr),
+                 "f"(v.x), "f"(v.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void st_async_f64(uint32_t addr, double v, uint32_t bar) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(addr), "d"(v), "r"(bar)
+                 : "memory");
+}
+
 // store v into the same shared-memory location of CTA `rank` of the cluster
 __device__ __forceinline__ void st_cluster_f4(const void* local, uint32_t rank, float4 v) {
     const uint32_t la = (uint32_t)__cvta_generic_to_shared(local);

@@ -50,7 +50,7 @@
 //    barrier per sweep) and, where every unit is a whole sample, the replica
 //    exchange after every pt_freq sweeps: every CTA's deciders exchange on their
 //    own copy of the energies and the permutation, behind the chains' pass of the
-//    next move.  __FUSED__
+//    next move.
 //  * All waits are bounded; a chain whose copy does not arrive sends a marked
 //    partial, so every CTA of the unit leaves at the same move, and nothing is
 //    written back.
@@ -113,17 +113,6 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
         : "r"(smem_u32(bar)), "r"(parity)
         : "memory");
     return ok != 0;
-}
-__device__ __forceinline__ uint32_t map_rank(uint32_t addr, uint32_t rank) {
-    uint32_t ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(addr), "r"(rank));
-    return ra;
-}
-// 8 bytes into a CTA of the cluster, counted on that CTA's mbarrier
-__device__ __forceinline__ void st_async_f2(uint32_t addr, float2 v, uint32_t bar) {
-    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(addr),
-                 "f"(v.x), "f"(v.y), "r"(bar)
-                 : "memory");
 }
 // named barrier 1: deciders arrive, chain warps wait ("the state of the next move is in place")
 __device__ __forceinline__ void state_arrive(int threads) {

@@ -84,3 +84,31 @@ def test_steps_in_one_launch_equal_single_steps(samples, Ns, NT, nrep, freq, war
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
     assert out[0][5].sum() > 0
+
+
+@pytest.mark.parametrize("samples,N,NT,nrep,freq,fmc", [(1, 96, 2, 3, 1, 1), (3, 64, 8, 8, 2, 0), (2, 48, 5, 17, 1, 1)])
+@pytest.mark.parametrize("warps", [2, 8])
+def test_resident_steps_in_one_launch_equal_single_steps(samples, N, NT, nrep, freq, fmc, warps):
+    """List-resident blocks of one sample as a cluster that exchanges inside the
+    launch (one block, two, three with a ragged last) equal one launch and one
+    exchange kernel per step, and one-warp blocks."""
+    import cuda_pspin_b200 as ps
+    out = []
+    for graph_steps, w in ((0, warps), (-1, warps), (-1, 1)):
+        cfgs = [ps.default_config(N=N, nrep=NT * nrep, seed=60 + k, fmc_mode=fmc) for k in range(samples)]
+        for c in cfgs:
+            c.gamma = 1.0 if fmc == 1 else 0.0
+        opts = ps.make_options(warps_per_unit=w, cluster_size=-1, graph_steps=graph_steps, resync_every=11,
+                               disorder_stream=True)
+        with ps.Engine(cfgs, ps.PSPIN_SPARSE, opts) as eng:
+            _, betas = ps.temperature_schedule(NT, 0.3, 1.5, True)
+            eng.pt_init(NT, nrep, betas, freq)
+            for n in (1, 7, 9):
+                eng.pt_run(n)
+            pt = [eng.pt_get(k) for k in range(samples)]
+            out.append([np.concatenate([a.ravel() for a in eng.get_spins()]), *eng.get_results(),
+                        np.stack([p[0] for p in pt]), np.stack([p[1] for p in pt]), np.stack([p[2] for p in pt])])
+    for other in out[1:]:
+        for a, b in zip(out[0], other):
+            np.testing.assert_array_equal(a, b)
+    assert out[0][5].sum() > 0
