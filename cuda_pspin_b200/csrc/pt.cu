@@ -245,12 +245,13 @@ cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStr
 // memory in slot order a temperature costs a few shared-memory latencies instead
 // of nrep chains of dependent global reads: 256 samples of 24 x 4 replicas took
 // 116 us with one thread each, 23 us before the schedule and the counters were
-// staged too; one sample of 32 x 4 46 and 25 us.
+// staged too, 12 now; one sample of 32 x 4 46, 25 and 9 us.
 // ---------------------------------------------------------------------
-// Staged per sample: [RT] energies, [NT] betas, [RT] replicas, [NT] swap counts.
+// Staged per sample: [RT] energies, [RT] drand48 states, [NT] betas, [RT] replicas,
+// [NT] swap counts.
 constexpr size_t kExchangeSmem = 48 * 1024;
 __host__ __device__ inline size_t exchange_smem_bytes(int NT, int nr) {
-    return (size_t)(NT * nr + NT) * (sizeof(double) + sizeof(int));
+    return (size_t)(NT * nr + NT) * (sizeof(double) + sizeof(int)) + (size_t)NT * nr * sizeof(uint64_t);
 }
 
 __global__ void __launch_bounds__(32) exchange_kernel(const ExchangeParams P) {
@@ -267,7 +268,8 @@ __global__ void __launch_bounds__(32) exchange_kernel(const ExchangeParams P) {
     uint64_t st = P.drand_state[s];
     const bool staged = exchange_smem_bytes(NT, nr) <= kExchangeSmem;
     double* Es = reinterpret_cast<double*>(xsm);               // in slot order
-    double* Bs = Es + RT;
+    uint64_t* seq = reinterpret_cast<uint64_t*>(Es + RT);      // the next drand48 states
+    double* Bs = reinterpret_cast<double*>(seq + RT);
     int* slot = staged ? reinterpret_cast<int*>(Bs + NT) : perm;
     int* swaps = slot + RT;                                    // (staged)
     const double* sched = staged ? Bs : P.beta_sched;
@@ -278,9 +280,12 @@ __global__ void __launch_bounds__(32) exchange_kernel(const ExchangeParams P) {
             slot[i] = r;
             Es[i] = E[r];
         }
+        if (nr <= 32) drand_ahead(seq, (NT - 1) * nr, st);
         __syncwarp();
     }
-    if (staged)
+    if (staged && nr <= 32)
+        exchange_columns(slot, Es, sched, seq, NT, nr, st, [&](int t, int n) { swaps[t] = n; });
+    else if (staged)
         exchange_pass(slot, sched, NT, nr, st, [&](int i, int) { return Es[i]; },
                       [&](int i, int j, double Ei, double Ej) {
                           Es[i] = Ej;

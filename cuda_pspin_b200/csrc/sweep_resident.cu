@@ -46,13 +46,13 @@ constexpr int kRing = 32;     // move slots
 // pairs and (sweep, step) [32] int2 each and proposal parts [32][7][32] float; with
 // more, the slots' dE [32][32] float, decisions and finished moves [32] int each,
 // betas [32] double; with exchanges in the launch (R replicas), energies by replica
-// of two exchanges, by slot, betas by replica, schedule [R] double each, replicas by
-// slot, swap counts [R] int each.
+// of two exchanges, by slot, betas by replica, schedule, drand48 states [R] of 8
+// bytes each, replicas by slot, swap counts [R] int each.
 inline size_t resident_smem_bytes(int N, int64_t entries, int K, int R = 0) {
     size_t b = (size_t)(N + 1) * kRepBlock * sizeof(float2) + (size_t)entries * sizeof(int2) + (size_t)N * sizeof(int2);
     if (K == 1) return b + 2 * kRing * sizeof(int2) + (size_t)kRing * 7 * kRepBlock * sizeof(float);
     return b + (size_t)kRing * kRepBlock * sizeof(float) + 2 * kRing * sizeof(int) + kRepBlock * sizeof(double) +
-           (size_t)R * (5 * sizeof(double) + 2 * sizeof(int));
+           (size_t)R * (6 * sizeof(double) + 2 * sizeof(int));
 }
 
 // A finished move or block: its writes, then the flag; a reader polls the flag
@@ -315,7 +315,8 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
     double* pt_Es = pt_E + 2 * RT;                                            // [RT] by slot
     double* pt_beta = pt_Es + RT;                                             // [RT] by replica
     double* pt_sched = pt_beta + RT;                                          // [RT]
-    int* pt_slot = reinterpret_cast<int*>(pt_sched + RT);                     // [RT]
+    uint64_t* pt_seq = reinterpret_cast<uint64_t*>(pt_sched + RT);            // [RT]
+    int* pt_slot = reinterpret_cast<int*>(pt_seq + RT);                       // [RT]
     int* pt_swaps = pt_slot + RT;                                             // [RT]
     __shared__ int counted, exchanged;                         // moves accounted for; exchanges made
     __shared__ volatile int stop;                              // a wait ran out
@@ -381,9 +382,13 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
         float ntt[7] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         auto fetch = [&](int m) {
             if (m >= total) return;
-            nmv = __ldg(moves + m);
+            // (volatile: issued here, a move ahead of their use)
+            asm volatile("ld.global.nc.v4.s32 {%0, %1, %2, %3}, [%4];"
+                         : "=r"(nmv.x), "=r"(nmv.y), "=r"(nmv.z), "=r"(nmv.w)
+                         : "l"(moves + m));
 #pragma unroll
-            for (int q = 0; q < 7; q++) ntt[q] = __ldg(trig + ((size_t)m * 7 + q) * kRepBlock);
+            for (int q = 0; q < 7; q++)
+                asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(ntt[q]) : "l"(trig + ((size_t)m * 7 + q) * kRepBlock));
         };
         fetch(warp);
         int version = 0;                       // exchanges in this warp's betas
@@ -398,9 +403,9 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
             const int4* A = reinterpret_cast<const int4*>(L + ri.x);
             const int4* B = reinterpret_cast<const int4*>(L + rj.x);
             const int na = (ri.y - ri.x) >> 1, nb = (rj.y - rj.x) >> 1;
-            // short record lists whose terms do not hold the partner site: the
-            // proposed a_j is in none of them
-            const bool quick = S.single_groups && na <= kHeld && nb <= kHeld && mv.z == 0;
+            // record lists whose terms do not hold the partner site: the proposed
+            // a_j is in none of them
+            const bool quick = S.single_groups && mv.z == 0;
             int4 q[2 * kHeld];
             if (quick) {
 #pragma unroll
@@ -434,6 +439,9 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
                     if (u < na) record_step<true>(q[u], a[u], ap[u], ao[u], yx, yy, hix, hiy);
                     if (u < nb) record_step<true>(q[kHeld + u], a[kHeld + u], ap[kHeld + u], ao[kHeld + u], yx, yy, hjx, hjy);
                 }
+                if (max(na, nb) > kHeld)
+                    accumulate_two<true>(A + kHeld, max(na - kHeld, 0), B + kHeld, max(nb - kHeld, 0), sp, lane, hix, hiy,
+                                         hjx, hjy);
             } else {
                 propose_with<VARIANT>(ai, aj, tt, ain, ajn);
                 sp[j0 * kRepBlock + lane] = ajn;       // h_i is evaluated at the proposed a_j
@@ -497,6 +505,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
                 pt_swaps[t] = 0;
             }
             drand = P.drand_state[U.sample];
+            if (P.nrep <= 32) drand_ahead(pt_seq, (P.NT - 1) * P.nrep, drand);
             __syncwarp();
         }
         int to_exchange = per_exchange, n_ex = 0;
@@ -531,18 +540,24 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
             }
             for (int i = lane; i < RT; i += 32) pt_Es[i] = Ex[pt_slot[i]];
             __syncwarp();
-            exchange_pass(pt_slot, pt_sched, P.NT, P.nrep, drand, [&](int i, int) { return pt_Es[i]; },
-                          [&](int i, int j, double Ei, double Ej) {
-                              pt_Es[i] = Ej;
-                              pt_Es[j] = Ei;
-                          },
-                          [&](int t2, int n) { pt_swaps[t2] += n; });
+            if (P.nrep <= 32)
+                exchange_columns(pt_slot, pt_Es, pt_sched, pt_seq, P.NT, P.nrep, drand,
+                                 [&](int t2, int n) { pt_swaps[t2] += n; });
+            else
+                exchange_pass(pt_slot, pt_sched, P.NT, P.nrep, drand, [&](int i, int) { return pt_Es[i]; },
+                              [&](int i, int j, double Ei, double Ej) {
+                                  pt_Es[i] = Ej;
+                                  pt_Es[j] = Ei;
+                              },
+                              [&](int t2, int n) { pt_swaps[t2] += n; });
             for (int i = lane; i < RT; i += 32) pt_beta[pt_slot[i]] = pt_sched[i / P.nrep];
             __syncwarp();
             if (active) beta_s[lane] = beta_d = pt_beta[U.rep_begin + lane];
             __syncwarp();
             n_ex++;
             if (lane == 0) publish(&exchanged, n_ex);
+            if (P.nrep <= 32) drand_ahead(pt_seq, (P.NT - 1) * P.nrep, drand);   // for the next one
+            __syncwarp();
         }
     }
     __syncthreads();

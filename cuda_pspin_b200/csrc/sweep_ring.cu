@@ -76,8 +76,9 @@ __device__ __forceinline__ bool is_marked(const float2 v) { return __float_as_ui
 // mbarriers full, empty [chains][stages], chains' arrival, messages [2][K],
 // deciders' meeting; ring
 // tags [chains][stages] int2; with exchanges in the launch (pt_slots replicas),
-// energies by replica, energies by slot, betas by replica, schedule [pt_slots]
-// double each, replicas by slot, swap counts [pt_slots] int each.
+// energies by replica, energies by slot, betas by replica, schedule, drand48
+// states [pt_slots] of 8 bytes each, replicas by slot, swap counts [pt_slots] int
+// each.
 struct RingLayout {
     size_t ring, part, xbuf, bars, tags, pt, total;
 };
@@ -98,7 +99,7 @@ __host__ __device__ inline RingLayout ring_layout(int N, int warps, int cluster,
     L.bars = L.xbuf + (alone ? 0 : (size_t)2 * ring_messages(warps, cluster, chains) * row);
     L.tags = L.bars + (size_t)(2 * chains * stages + 2 + 2 * K) * sizeof(uint64_t);
     L.pt = L.tags + (size_t)chains * stages * sizeof(int2);
-    L.total = L.pt + (size_t)pt_slots * (4 * sizeof(double) + 2 * sizeof(int));
+    L.total = L.pt + (size_t)pt_slots * (5 * sizeof(double) + 2 * sizeof(int));
     return L;
 }
 
@@ -165,6 +166,30 @@ __device__ __forceinline__ float2 tree_sum(const float2* __restrict__ buf, int C
     }
 }
 
+// One exchange by a warp, on the arrays that start at pt_E (RingLayout): energies by
+// replica in, betas by replica out; returns the drand48 state.  Not inlined: its
+// registers are not the sweep's.
+__device__ __noinline__ uint64_t ring_exchange(double* pt_E, int RT, int NT, int nrep, uint64_t drand) {
+    const int lane = threadIdx.x & 31;
+    double *Es = pt_E + RT, *beta = Es + RT, *sched = beta + RT;
+    uint64_t* seq = reinterpret_cast<uint64_t*>(sched + RT);
+    int *slot = reinterpret_cast<int*>(seq + RT), *swaps = slot + RT;
+    for (int i = lane; i < RT; i += 32) Es[i] = pt_E[slot[i]];
+    __syncwarp();
+    if (nrep <= 32)
+        exchange_columns(slot, Es, sched, seq, NT, nrep, drand, [&](int t, int n) { swaps[t] += n; });
+    else
+        exchange_pass(slot, sched, NT, nrep, drand, [&](int i, int) { return Es[i]; },
+                      [&](int i, int j, double Ei, double Ej) {
+                          Es[i] = Ej;
+                          Es[j] = Ei;
+                      },
+                      [&](int t, int n) { swaps[t] += n; });
+    for (int i = lane; i < RT; i += 32) beta[slot[i]] = sched[i / nrep];
+    if (nrep <= 32) drand_ahead(seq, (NT - 1) * nrep, drand);        // for the next one
+    return drand;
+}
+
 // kLat: few blocks, at most kLatChains chain warps a CTA, so a warp has its
 // sub-partition's issue slots and registers to itself and deep batches of
 // loads in flight carry it; otherwise 16 chain warps share the SM.
@@ -190,10 +215,10 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     int2* tags = reinterpret_cast<int2*>(smem_raw + Lo.tags);
     const int RT = P.pt_freq > 0 ? P.NT * P.nrep : 0;
     double* pt_E = reinterpret_cast<double*>(smem_raw + Lo.pt);      // [RT] by replica
-    double* pt_Es = pt_E + RT;                                        // [RT] by slot
-    double* pt_beta = pt_Es + RT;                                     // [RT] by replica
+    double* pt_beta = pt_E + 2 * RT;                                  // [RT] by replica (between: by slot)
     double* pt_sched = pt_beta + RT;                                  // [NT]
-    int* pt_slot = reinterpret_cast<int*>(pt_sched + RT);             // [RT]
+    uint64_t* pt_seq = reinterpret_cast<uint64_t*>(pt_sched + RT);    // [RT]
+    int* pt_slot = reinterpret_cast<int*>(pt_seq + RT);               // [RT]
     int* pt_swaps = pt_slot + RT;                                     // [NT]
     __shared__ volatile int stop, gave_up;           // the unit aborts; a chain of this CTA gave up
     __shared__ volatile int task_s;
@@ -295,6 +320,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
             pt_swaps[t] = 0;
         }
         drand = __ldcg(P.drand_state + U.sample);
+        if (P.nrep <= 32) drand_ahead(pt_seq, (P.NT - 1) * P.nrep, drand);
     }
     __syncthreads();
     if (decider && total > 0) {
@@ -460,17 +486,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 };
                 if (active) pt_E[rr] = E;
                 bool met = meet();
-                if (k == 0 && met) {
-                    for (int i = lane; i < RT; i += 32) pt_Es[i] = pt_E[pt_slot[i]];
-                    __syncwarp();
-                    exchange_pass(pt_slot, pt_sched, P.NT, P.nrep, drand, [&](int i, int) { return pt_Es[i]; },
-                                  [&](int i, int j, double Ei, double Ej) {
-                                      pt_Es[i] = Ej;
-                                      pt_Es[j] = Ei;
-                                  },
-                                  [&](int t, int n) { pt_swaps[t] += n; });
-                    for (int i = lane; i < RT; i += 32) pt_beta[pt_slot[i]] = pt_sched[i / P.nrep];
-                }
+                if (k == 0 && met) drand = ring_exchange(pt_E, RT, P.NT, P.nrep, drand);
                 met = meet() && met;
                 if (!met) {                          // (a wait ran out: the chains stop at the move after the next)
                     stop = 1;
