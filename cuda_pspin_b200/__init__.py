@@ -291,12 +291,11 @@ class Engine:
     def get_spins(self) -> list[np.ndarray]:
         """Per sample, complex128 [nrep, N] (physical replica order)."""
         tot = sum(N * R for N, R in zip(self.Ns, self.Rs))
-        buf = np.empty(2 * tot, np.float64)
+        buf = np.empty(tot, np.complex128)
         _check(self._lib.pspin_get_spins(self._h, _ptr(buf)))
         out, off = [], 0
         for N, R in zip(self.Ns, self.Rs):
-            v = buf[2 * off:2 * (off + N * R)].reshape(R, N, 2)
-            out.append(v[..., 0] + 1j * v[..., 1])
+            out.append(buf[off:off + N * R].reshape(R, N))
             off += N * R
         return out
 

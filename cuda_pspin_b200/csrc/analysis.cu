@@ -16,10 +16,14 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <random>
 #include <vector>
 
 namespace pspin {
+
+unsigned long long current_context_id();     // noalloc.cu
 
 __global__ void overlap_count_kernel(const double* __restrict__ cfg, int N, int NT, int nrep, int nsnap, int nbins,
                                      double qmin, double dq, unsigned long long* __restrict__ counts) {
@@ -335,6 +339,75 @@ __global__ void multi_pair_kernel(const double* __restrict__ cfg, const double* 
 }
 }  // namespace pspin
 
+// ---- device scratch of one call ---------------------------------------------
+// cudaMalloc and cudaFree of a few buffers took most of a call on a few MB of
+// configurations: the overlaps of 64 snapshots of 24 x 4 replicas at N = 64 (6 MB)
+// took 1.91 ms and the IFO 2.10, 0.43 and 0.57 with the buffers from a
+// stream-ordered pool on the calling thread's own stream (0.36 is the copy).  It
+// keeps at most kPoolKeep bytes between calls and gives the rest back to the
+// device as a call ends; one pool per device and context, shared by all threads.
+constexpr uint64_t kPoolKeep = (uint64_t)32 << 20;
+
+static cudaError_t scratch_pool(cudaMemPool_t* pool) {
+    struct Made { unsigned long long ctx; cudaMemPool_t pool; };
+    static std::mutex lock;
+    static std::map<int, Made> pools;                // by device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> hold(lock);
+    unsigned long long ctx = pspin::current_context_id();
+    if (ctx == 0) {                                  // no context yet on this thread
+        if ((e = cudaFree(nullptr)) != cudaSuccess) return e;
+        ctx = pspin::current_context_id();
+    }
+    auto it = pools.find(dev);
+    if (it == pools.end() || it->second.ctx != ctx) {    // a reset device lost its pool
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        Made made{ctx, nullptr};
+        if ((e = cudaMemPoolCreate(&made.pool, &props)) != cudaSuccess) return e;
+        uint64_t keep = kPoolKeep;
+        if ((e = cudaMemPoolSetAttribute(made.pool, cudaMemPoolAttrReleaseThreshold, &keep)) != cudaSuccess) {
+            cudaMemPoolDestroy(made.pool);
+            return e;
+        }
+        it = pools.insert_or_assign(dev, made).first;
+    }
+    *pool = it->second.pool;
+    return cudaSuccess;
+}
+
+struct Scratch {
+    cudaStream_t st = cudaStreamPerThread;
+    std::vector<void*> held;
+    template <class T>
+    cudaError_t get(T** p, size_t n) {
+        *p = nullptr;
+        cudaMemPool_t pool = nullptr;
+        cudaError_t e = scratch_pool(&pool);
+        void* q = nullptr;
+        if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&q, std::max<size_t>(n, 1) * sizeof(T), pool, st);
+        if (e != cudaSuccess) return e;
+        held.push_back(q);
+        *p = static_cast<T*>(q);
+        return cudaSuccess;
+    }
+    cudaError_t upload(void* dst, const void* src, size_t bytes) {
+        return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    }
+    cudaError_t download(void* dst, const void* src, size_t bytes) {
+        const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+        return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+    }
+    ~Scratch() {
+        for (void* p : held) cudaFreeAsync(p, st);
+        cudaStreamSynchronize(st);
+    }
+};
+
 // IFO and experimental-IFO counts of one sample (no reference counterpart as
 // a library call): counts [NT][nbins] and valid overlaps [NT] of each; either
 // pair of outputs may be NULL.
@@ -355,34 +428,31 @@ extern "C" int pspin_ifo_counts_impl(int N, int NT, int nrep, int nsnap, const d
     const size_t nm = (size_t)NT * nrep * N, nn = (size_t)nsnap * NT * nrep;
     double *d_cfg = nullptr, *d_mean = nullptr, *d_norm = nullptr;
     unsigned long long* d_cnt = nullptr;            // [2][NT][nbins] then [2][NT]
-    cudaError_t e = cudaMalloc(&d_cfg, n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&d_mean, nm * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&d_norm, nn * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&d_cnt, (2 * cnt + 2 * NT) * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMemcpy(d_cfg, configs, n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(d_cnt, 0, (2 * cnt + 2 * NT) * sizeof(unsigned long long));
+    Scratch mem;
+    cudaError_t e = mem.get(&d_cfg, n);
+    if (e == cudaSuccess) e = mem.get(&d_mean, nm);
+    if (e == cudaSuccess) e = mem.get(&d_norm, nn);
+    if (e == cudaSuccess) e = mem.get(&d_cnt, (2 * cnt + 2 * NT));
+    if (e == cudaSuccess) e = mem.upload(d_cfg, configs, n * sizeof(double));
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, (2 * cnt + 2 * NT) * sizeof(unsigned long long), mem.st);
     if (e == cudaSuccess) {
         const double dc = (cmax - cmin) / nbins;
         const int threads = 256;
         auto blocks = [&](long long total) { return (int)std::min<long long>((total + threads - 1) / threads, 148LL * 16); };
         const long long npairs = nrep * (nrep - 1) / 2;
-        pspin::intensity_mean_kernel<<<blocks((long long)nm), threads>>>(d_cfg, N, NT, nrep, nsnap, d_mean);
+        pspin::intensity_mean_kernel<<<blocks((long long)nm), threads, 0, mem.st>>>(d_cfg, N, NT, nrep, nsnap, d_mean);
         if (ifo_counts) {
-            pspin::ifo_norm_kernel<<<blocks((long long)nn), threads>>>(d_cfg, d_mean, N, NT, nrep, nsnap, d_norm);
-            pspin::ifo_count_kernel<<<blocks((long long)nsnap * NT * npairs), threads>>>(
+            pspin::ifo_norm_kernel<<<blocks((long long)nn), threads, 0, mem.st>>>(d_cfg, d_mean, N, NT, nrep, nsnap, d_norm);
+            pspin::ifo_count_kernel<<<blocks((long long)nsnap * NT * npairs), threads, 0, mem.st>>>(
                 d_cfg, d_mean, d_norm, N, NT, nrep, nsnap, nbins, cmin, dc, d_cnt, d_cnt + 2 * cnt);
         }
         if (exp_counts)
-            pspin::exp_ifo_count_kernel<<<blocks((long long)NT * npairs), threads>>>(
+            pspin::exp_ifo_count_kernel<<<blocks((long long)NT * npairs), threads, 0, mem.st>>>(
                 d_mean, N, NT, nrep, nbins, cmin, dc, d_cnt + cnt, d_cnt + 2 * cnt + NT);
         e = cudaGetLastError();
     }
     std::vector<unsigned long long> h(2 * cnt + 2 * NT);
-    if (e == cudaSuccess) e = cudaMemcpy(h.data(), d_cnt, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
-    cudaFree(d_cfg);
-    cudaFree(d_mean);
-    cudaFree(d_norm);
-    cudaFree(d_cnt);
+    if (e == cudaSuccess) e = mem.download(h.data(), d_cnt, h.size() * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         *err = cudaGetErrorString(e);
         return 2;
@@ -410,22 +480,21 @@ extern "C" int pspin_overlap_counts_impl(int N, int NT, int nrep, int nsnap, con
     const size_t n = (size_t)nsnap * NT * nrep * 2 * N;
     double* d_cfg = nullptr;
     unsigned long long* d_cnt = nullptr;
-    cudaError_t e = cudaMalloc(&d_cfg, n * sizeof(double) + 8);
-    if (e == cudaSuccess) e = cudaMalloc(&d_cnt, (size_t)NT * nbins * sizeof(unsigned long long));
-    if (e == cudaSuccess && n) e = cudaMemcpy(d_cfg, configs, n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(d_cnt, 0, (size_t)NT * nbins * sizeof(unsigned long long));
+    Scratch mem;
+    cudaError_t e = mem.get(&d_cfg, n);
+    if (e == cudaSuccess) e = mem.get(&d_cnt, (size_t)NT * nbins);
+    if (e == cudaSuccess && n) e = mem.upload(d_cfg, configs, n * sizeof(double));
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, (size_t)NT * nbins * sizeof(unsigned long long), mem.st);
     if (e == cudaSuccess) {
         const double dq = (qmax - qmin) / nbins;
         const long long total = (long long)nsnap * NT * (nrep * (nrep - 1) / 2);
         const int threads = 256;
         const int blocks = (int)std::min<long long>((total + threads - 1) / threads, 148LL * 16);
-        if (total > 0) pspin::overlap_count_kernel<<<blocks, threads>>>(d_cfg, N, NT, nrep, nsnap, nbins, qmin, dq, d_cnt);
+        if (total > 0) pspin::overlap_count_kernel<<<blocks, threads, 0, mem.st>>>(d_cfg, N, NT, nrep, nsnap, nbins, qmin, dq, d_cnt);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess)
-        e = cudaMemcpy(counts, d_cnt, (size_t)NT * nbins * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
-    cudaFree(d_cfg);
-    cudaFree(d_cnt);
+        e = mem.download(counts, d_cnt, (size_t)NT * nbins * sizeof(unsigned long long));
     if (e != cudaSuccess) {
         *err = cudaGetErrorString(e);
         return 2;
@@ -464,33 +533,29 @@ extern "C" int pspin_deeper_counts_impl(int N, int NT, int nrep, int nsnap, cons
     double *d_cfg = nullptr, *d_y = nullptr, *d_sc = nullptr;
     int* d_q = nullptr;
     unsigned long long* d_cnt = nullptr;
-    cudaError_t e = cudaMalloc(&d_cfg, n * sizeof(double) + 8);
-    if (e == cudaSuccess) e = cudaMalloc(&d_y, ny * sizeof(double) + 8);
-    if (e == cudaSuccess) e = cudaMalloc(&d_sc, ns * sizeof(double) + 8);
-    if (e == cudaSuccess) e = cudaMalloc(&d_q, (size_t)5 * M * sizeof(int) + 8);
-    if (e == cudaSuccess) e = cudaMalloc(&d_cnt, nc * sizeof(unsigned long long));
-    if (e == cudaSuccess && n) e = cudaMemcpy(d_cfg, configs, n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && M) e = cudaMemcpy(d_q, quartets, (size_t)5 * M * sizeof(int), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(d_cnt, 0, nc * sizeof(unsigned long long));
+    Scratch mem;
+    cudaError_t e = mem.get(&d_cfg, n);
+    if (e == cudaSuccess) e = mem.get(&d_y, ny);
+    if (e == cudaSuccess) e = mem.get(&d_sc, ns);
+    if (e == cudaSuccess) e = mem.get(&d_q, (size_t)5 * M);
+    if (e == cudaSuccess) e = mem.get(&d_cnt, nc);
+    if (e == cudaSuccess && n) e = mem.upload(d_cfg, configs, n * sizeof(double));
+    if (e == cudaSuccess && M) e = mem.upload(d_q, quartets, (size_t)5 * M * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_cnt, 0, nc * sizeof(unsigned long long), mem.st);
     if (e == cudaSuccess && nsnap > 0) {
         unsigned long long* d_marg = d_cnt;
         unsigned long long* d_phase = d_cnt + (size_t)NT * nbins_a2;
         unsigned long long* d_link = d_phase + (size_t)NT * nbins;
-        pspin::deep_site_kernel<<<launch_blocks((long long)nsnap * NT * nrep), 256>>>(d_cfg, N, NT, nrep, nsnap,
+        pspin::deep_site_kernel<<<launch_blocks((long long)nsnap * NT * nrep), 256, 0, mem.st>>>(d_cfg, N, NT, nrep, nsnap,
                                                                                       nbins_a2, da2, d_marg, d_y);
-        pspin::deep_pair_kernel<<<launch_blocks((long long)nsnap * NT * npairs), 256>>>(
+        pspin::deep_pair_kernel<<<launch_blocks((long long)nsnap * NT * npairs), 256, 0, mem.st>>>(
             d_cfg, N, NT, nrep, nsnap, nbins, 2.0 / nbins, d_q, M, d_phase, d_link, d_sc);
         e = cudaGetLastError();
     }
     std::vector<unsigned long long> h(nc);
-    if (e == cudaSuccess) e = cudaMemcpy(h.data(), d_cnt, nc * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && ny) e = cudaMemcpy(y, d_y, ny * sizeof(double), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && ns) e = cudaMemcpy(scatter, d_sc, ns * sizeof(double), cudaMemcpyDeviceToHost);
-    cudaFree(d_cfg);
-    cudaFree(d_y);
-    cudaFree(d_sc);
-    cudaFree(d_q);
-    cudaFree(d_cnt);
+    if (e == cudaSuccess) e = mem.download(h.data(), d_cnt, nc * sizeof(unsigned long long));
+    if (e == cudaSuccess && ny) e = mem.download(y, d_y, ny * sizeof(double));
+    if (e == cudaSuccess && ns) e = mem.download(scatter, d_sc, ns * sizeof(double));
     if (e != cudaSuccess) {
         *err = cudaGetErrorString(e);
         return 2;
@@ -521,23 +586,20 @@ extern "C" int pspin_multi_overlap_impl(int N, int NT, int nrep, int nsnap, cons
     if (no == 0) return 0;
     double *d_cfg = nullptr, *d_mean = nullptr, *d_out = nullptr;
     int* d_s = nullptr;
-    cudaError_t e = cudaMalloc(&d_cfg, n * sizeof(double) + 8);
-    if (e == cudaSuccess) e = cudaMalloc(&d_mean, (size_t)NT * nrep * N * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&d_out, no * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&d_s, (size_t)NT * nit * sizeof(int));
-    if (e == cudaSuccess && n) e = cudaMemcpy(d_cfg, configs, n * sizeof(double), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(d_s, snaps, (size_t)NT * nit * sizeof(int), cudaMemcpyHostToDevice);
+    Scratch mem;
+    cudaError_t e = mem.get(&d_cfg, n);
+    if (e == cudaSuccess) e = mem.get(&d_mean, (size_t)NT * nrep * N);
+    if (e == cudaSuccess) e = mem.get(&d_out, no);
+    if (e == cudaSuccess) e = mem.get(&d_s, (size_t)NT * nit);
+    if (e == cudaSuccess && n) e = mem.upload(d_cfg, configs, n * sizeof(double));
+    if (e == cudaSuccess) e = mem.upload(d_s, snaps, (size_t)NT * nit * sizeof(int));
     if (e == cudaSuccess) {
-        pspin::multi_mean_kernel<<<launch_blocks((long long)NT * nrep * N), 256>>>(d_cfg, N, NT, nrep, d_s, nit, d_mean);
-        pspin::multi_pair_kernel<<<launch_blocks((long long)NT * npairs * nit), 256>>>(d_cfg, d_mean, N, NT, nrep, d_s,
+        pspin::multi_mean_kernel<<<launch_blocks((long long)NT * nrep * N), 256, 0, mem.st>>>(d_cfg, N, NT, nrep, d_s, nit, d_mean);
+        pspin::multi_pair_kernel<<<launch_blocks((long long)NT * npairs * nit), 256, 0, mem.st>>>(d_cfg, d_mean, N, NT, nrep, d_s,
                                                                                        nit, d_out);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpy(out, d_out, no * sizeof(double), cudaMemcpyDeviceToHost);
-    cudaFree(d_cfg);
-    cudaFree(d_mean);
-    cudaFree(d_out);
-    cudaFree(d_s);
+    if (e == cudaSuccess) e = mem.download(out, d_out, no * sizeof(double));
     if (e != cudaSuccess) {
         *err = cudaGetErrorString(e);
         return 2;

@@ -113,28 +113,30 @@ static unsigned long long g_ctx_id[kMaxDevices] = {};   // context the cached ad
 // Unique id of the calling thread's current CUDA context (ids are never
 // reused within a process), through driver entry points the runtime hands
 // out; 0 when there is no current context or the entry points are missing.
-static unsigned long long current_context_id() {
+unsigned long long current_context_id() {
     using GetCurrent = int (*)(void**);
     using GetId = int (*)(void*, unsigned long long*);
-    static GetCurrent get_current = nullptr;
-    static GetId get_id = nullptr;
-    static bool looked_up = false;
-    if (!looked_up) {
-        looked_up = true;
-        cudaDriverEntryPointQueryResult q1, q2;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", (void**)&get_current, cudaEnableDefault, &q1) != cudaSuccess ||
-            q1 != cudaDriverEntryPointSuccess)
-            get_current = nullptr;
-        if (cudaGetDriverEntryPoint("cuCtxGetId", (void**)&get_id, cudaEnableDefault, &q2) != cudaSuccess ||
-            q2 != cudaDriverEntryPointSuccess)
-            get_id = nullptr;
-        cudaGetLastError();
-    }
-    if (!get_current || !get_id) return 0;
+    struct Entries {
+        GetCurrent get_current = nullptr;
+        GetId get_id = nullptr;
+        Entries() {
+            cudaDriverEntryPointQueryResult q1, q2;
+            if (cudaGetDriverEntryPoint("cuCtxGetCurrent", (void**)&get_current, cudaEnableDefault, &q1) !=
+                    cudaSuccess ||
+                q1 != cudaDriverEntryPointSuccess)
+                get_current = nullptr;
+            if (cudaGetDriverEntryPoint("cuCtxGetId", (void**)&get_id, cudaEnableDefault, &q2) != cudaSuccess ||
+                q2 != cudaDriverEntryPointSuccess)
+                get_id = nullptr;
+            cudaGetLastError();
+        }
+    };
+    static const Entries at;                         // looked up once, by whichever thread is first
+    if (!at.get_current || !at.get_id) return 0;
     void* ctx = nullptr;
     unsigned long long id = 0;
-    if (get_current(&ctx) != 0 || !ctx) return 0;
-    if (get_id(ctx, &id) != 0) return 0;
+    if (at.get_current(&ctx) != 0 || !ctx) return 0;
+    if (at.get_id(ctx, &id) != 0) return 0;
     return id;
 }
 
