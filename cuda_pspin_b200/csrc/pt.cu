@@ -245,7 +245,7 @@ cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStr
 // memory in slot order a temperature costs a few shared-memory latencies instead
 // of nrep chains of dependent global reads: 256 samples of 24 x 4 replicas took
 // 116 us with one thread each, 23 us before the schedule and the counters were
-// staged too, 12 now; one sample of 32 x 4 46, 25 and 9 us.
+// staged too, 12 now; one sample of 32 x 4 46, 25 and 11 us.
 // ---------------------------------------------------------------------
 // Staged per sample: [RT] energies, [RT] drand48 states, [NT] betas, [RT] replicas,
 // [NT] swap counts.
