@@ -921,6 +921,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         d.variant = variant;
         d.tiles = h.tiles;
         d.tiles_g = h.tiles;
+        d.tiles_p = 0;
         d.single_groups = h.single_groups;
         d.spin_off = spin_off;
         d.rep_off = rep_off;
@@ -2163,7 +2164,7 @@ static int ensure_pair_lists(pspin_state* s) {
             recs[t] = QuartetRec{e.i, e.j, e.k, e.lch & 0x3fff, e.lch >> 14, e.g};
         }
         std::vector<Q64>().swap(q[k]);
-        build_pair_lists(s->hs[k].N, s->hs[k].g2re.data(), s->hs[k].h2_active, recs, pl[k]);
+        build_pair_lists(s->hs[k].N, s->hs[k].g2re.data(), s->hs[k].h2_active, recs, pl[k], s->hs[k].tiles != 0);
         // a fully connected sample keeps its tiles (their parts are the same here)
         if (!(s->hs[k].tiles && s->hs[k].fc))
             build_site_lists(s->hs[k].N, s->hs[k].g2re.data(), s->hs[k].h2_active, recs, gl[k], kGroups,
@@ -2185,7 +2186,7 @@ static int ensure_pair_lists(pspin_state* s) {
     std::vector<int64_t> cs((size_t)chunk_new + 1);
     std::vector<int> pc((size_t)idx_total);
     std::vector<int64_t> pair_off(n);
-    std::vector<int> tiles_g(n);
+    std::vector<int> tiles_g(n), tiles_p(n);
     int64_t eoff = 0, coff = 0, ioff = 0;
     for (int k = 0; k < n; k++) {
         std::copy(pl[k].entries.begin(), pl[k].entries.end(), ent.begin() + eoff);
@@ -2196,6 +2197,7 @@ static int ensure_pair_lists(pspin_state* s) {
         eoff += (int64_t)pl[k].entries.size();
         coff += (int64_t)pl[k].chunk_start.size();
         ioff += (int64_t)pl[k].site_chunks.size();
+        tiles_p[k] = (int)pl[k].tiles;
         pl[k] = SiteLists();
         if (!gl[k].entries.empty()) {
             std::copy(gl[k].entries.begin(), gl[k].entries.end(), ent.begin() + eoff);
@@ -2224,6 +2226,7 @@ static int ensure_pair_lists(pspin_state* s) {
     for (int k = 0; k < n; k++) {
         sd[k].pair_off = pair_off[k];
         sd[k].tiles_g = tiles_g[k];
+        sd[k].tiles_p = tiles_p[k];
     }
     cudaError_t e = cudaMemcpyAsync(d_ent, s->d_entries, s->ent_total * sizeof(int2), cudaMemcpyDeviceToDevice, s->st);
     if (e == cudaSuccess)

@@ -74,6 +74,7 @@ struct SampleDev {
     int variant;           // 0 sphere (dense), 1 smoothed cube (sparse)
     int tiles;             // 1: site lists are dense tiles (layout.cpp), 0: group records
     int tiles_g;           // the same of the two-pass sweep's site lists (else groups)
+    int tiles_p;           // the same of its pair sub-lists (else groups)
     int single_groups;     // group records only, every group of one entry (each record ends its group)
     int64_t spin_off;      // float2 index of site 0, replica 0
     int64_t rep_off;       // index into the per-replica arrays

@@ -232,7 +232,7 @@ static void pack_list(const std::vector<Group>& g, const std::vector<int64_t>& e
 }
 
 void build_pair_lists(int N, const double* g2re, int h2_active, const std::vector<QuartetRec>& qs,
-                      SiteLists& out) {
+                      SiteLists& out, bool tile) {
     const int npairs = N * (N - 1) / 2;
     auto list_id = [](int m, int x) {   // m's terms that contain x
         return m < x ? 2 * (x * (x - 1) / 2 + m) : 2 * (m * (m - 1) / 2 + x) + 1;
@@ -264,9 +264,33 @@ void build_pair_lists(int N, const double* g2re, int h2_active, const std::vecto
     std::vector<int64_t> end;
     std::vector<Span> items;
     std::vector<int2> site;
+    constexpr int kStride = 4;                  // 8 pieces: one chunk per warp at 8 warps
+    if (tile) {
+        int64_t tiles = 0, groups = 0, words = 0, tile_words = 0;
+        for (int id = 0; id < 2 * npairs && tile; id++) {
+            make_groups(per[id], kGroups, g, end);
+            size_t first[kSplit + 1];
+            part_bounds(end, kStride, first);
+            for (int part = 0; part < kSplit && tile; part++) {
+                const size_t b = first[part], e = std::max(first[part], first[part + 1]);
+                if (b == e) continue;
+                site.clear();
+                items.clear();
+                const int64_t c = tile_part(g, b, e, N, &site, &items);
+                if (c == INT64_MAX) tile = false;
+                tiles += c;
+                tile_words += (int64_t)site.size();
+            }
+            for (size_t t = 0; t < g.size(); t++)
+                groups += record_cost((int)(end[t] - (t ? end[t - 1] : 0) - 1));
+            words += end.empty() ? 0 : end.back();
+        }
+        tile = tile && tiles < groups && tile_words <= words + words / 4;
+    }
+    out.tiles = tile;
     for (int id = 0; id < 2 * npairs; id++) {
         make_groups(per[id], kGroups, g, end);
-        pack_list(g, end, kGroups, false, N, id, 4, out, site, items);      // 8 pieces: one chunk per warp at 8 warps
+        pack_list(g, end, kGroups, tile, N, id, kStride, out, site, items);
         std::vector<Rec>().swap(per[id]);
     }
 }

@@ -33,12 +33,13 @@ enum GroupSize { kGroups, kRecords };
 // and the same order of additions; otherwise in the format of `size`.
 void build_site_lists(int N, const double* g2re, int h2_active, const std::vector<QuartetRec>& qs, SiteLists& out,
                       GroupSize size, bool tile);
-// Sub-lists of the terms that couple the two sites of a pair (group format):
+// Sub-lists of the terms that couple the two sites of a pair (as groups, or with
+// `tile` as dense tiles where those are cheaper to read):
 // for i < j and P = j(j-1)/2 + i, list 2P holds site i's terms that contain
 // a_j, list 2P+1 site j's terms that contain a_i.  Each term of a site list
 // is in 3 of them (one per other site of its quartet).
 void build_pair_lists(int N, const double* g2re, int h2_active, const std::vector<QuartetRec>& qs,
-                      SiteLists& out);
+                      SiteLists& out, bool tile);
 // fully connected lists as dense tiles, from the dense g4 (channel 0
 // everywhere) and g2
 void build_site_tiles_fc(int N, const double* g2re, int h2_active, const double* g4re, SiteLists& out);

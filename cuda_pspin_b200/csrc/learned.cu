@@ -3,6 +3,14 @@
 // the learned proposal with the exact Metropolis-Hastings correction; and
 // the network's training kernels (forward, backward, Adam).
 //
+// What bounds it: at a replica block per few SMs, latency (of a move's 76k cycles
+// with one block alone the field passes take 29k and 13k, the network, the samplers
+// and the densities on their critical path 34k); with every SM full, issue of the
+// field passes.  The chains of both lists run on warps of their own, spread over as
+// many SMs as the blocks leave free, and the pair's sub-lists are dense tiles: as
+// groups of mostly one term a chunk's dependent loads had taken 36k cycles a pass
+// however few terms it held.
+//
 // Two field passes per move.  Pass 1 reads site i's and site j's lists at
 // the current state x: h_i(x), h_j(x) (the proposal's features).  Pass 2
 // reads only the pair's sub-lists (the terms of h_i that contain a_j and of
@@ -12,6 +20,8 @@
 //     dE = -Re[da_i h_i(x')] - Re[da_j h_j(x)]
 // exactly (h_i(x') is h_i with a_j' in place, h_j(x) is h_j with a_i).
 #include <cuda_bf16.h>
+
+#include <algorithm>
 
 #include "../../include/pspin.h"
 #include "mlp.cuh"
@@ -143,57 +153,121 @@ constexpr int kLStages = 2;
 constexpr int kMlpBufWords = (kMlpHidden / 2) * kActStride;
 static_assert(kMlpOut * kOutStride <= kMlpBufWords, "output rows fit a network buffer");
 
-// amplitudes [N+1][32] float2, partial fields [W][32] float4, TMA rings
-// [W][kLStages][kStage] int2, their barriers [W][kLStages], the two network
-// buffers, then the roles' exchange rows [kXchRows][32] float
-__host__ __device__ inline size_t learned_base_bytes(int N, int warps) {
-    return (size_t)(N + 1) * kRepBlock * sizeof(float2) + (size_t)warps * kRepBlock * sizeof(float4) +
-           (size_t)warps * kLStages * kStage * sizeof(int2) + (size_t)warps * kLStages * sizeof(uint64_t) +
-           (size_t)2 * kMlpBufWords * sizeof(uint32_t) + (size_t)kXchRows * kRepBlock * sizeof(float);
-}
+// The sums of a move's two lists are taken by 2 C W chains (list, warp of the
+// block shape); a CTA of kLWarps warps reads `chains` of them, chain x * chains + q
+// on warp q % kLWarps of CTA x of the P.exec CTAs that run a replica block.
+constexpr int kLWarps = 8;
+struct LearnLayout {
+    int rings;                                  // warps that read lists
+    size_t ring, bars, buf, xch, parts, flag, total;
+    __host__ __device__ LearnLayout(int N, int all_chains, int exec, int chains) {
+        rings = chains < kLWarps ? chains : kLWarps;
+        size_t at = (size_t)(N + 1) * kRepBlock * sizeof(float2);           // amplitudes
+        ring = at;
+        at += (size_t)rings * kLStages * kStage * sizeof(int2);
+        bars = at;
+        at += (size_t)rings * kLStages * sizeof(uint64_t);
+        buf = at;                               // two network buffers
+        at += (size_t)2 * kMlpBufWords * sizeof(uint32_t);
+        xch = at;                               // the roles' exchange rows
+        at += (size_t)kXchRows * kRepBlock * sizeof(float);
+        parts = (at + 15) & ~(size_t)15;        // partial fields, double-buffered across CTAs
+        at = parts + (size_t)(exec > 1 ? 2 : 1) * all_chains * kRepBlock * sizeof(float2);
+        flag = at;                              // the cluster's abort flag
+        total = at + 16;
+    }
+};
 
-// cluster variant: the partial-field exchange buffer [2][C][32] float4 after
-// the network buffers, at a 16-byte boundary
-__host__ __device__ inline size_t learned_cluster_buffer_offset(int N, int warps) {
-    return (learned_base_bytes(N, warps) + 15) & ~(size_t)15;
-}
-
-// cluster variant: the exchange buffer, then the cluster's abort flag (one word)
+// shared memory of the block shape as one CTA (cluster of CTAs) per replica block
+// had it; which shapes are accepted goes by this
 inline size_t learned_smem_bytes(int N, int warps, int C = 1) {
-    if (C > 1) return learned_cluster_buffer_offset(N, warps) + (size_t)2 * C * kRepBlock * sizeof(float4) + 16;
-    return learned_base_bytes(N, warps);
+    const size_t base = (size_t)(N + 1) * kRepBlock * sizeof(float2) + (size_t)warps * kRepBlock * sizeof(float4) +
+                        (size_t)warps * kLStages * kStage * sizeof(int2) + (size_t)warps * kLStages * sizeof(uint64_t) +
+                        (size_t)2 * kMlpBufWords * sizeof(uint32_t) + (size_t)kXchRows * kRepBlock * sizeof(float);
+    if (C > 1) return ((base + 15) & ~(size_t)15) + (size_t)2 * C * kRepBlock * sizeof(float4) + 16;
+    return base;
 }
 
-// CL: one replica block over a thread-block cluster of P.cluster CTAs.  Each
-// CTA reads 1/C of every list; the partial fields of both passes meet in every
-// CTA's exchange buffer (distributed shared memory, one cluster barrier per
-// exchange, double-buffered by exchange parity); every CTA then evaluates the
-// network and takes the same decision on the same numbers, so the amplitude
-// copies stay identical; rank 0 writes records, trace and results.
-template <bool CL>
-__global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams P, const LearnParams L) {
+// A warp's stream of chunks: per move its share of the sites' lists (pass 0), then of
+// the pair's sub-lists (pass 1); in each, its one or two chains (list, part range).
+struct LearnStream {
+    uint32_t key0, key1;
+    int N;
+    const int* site_chunks;   // this sample's N*(kSplit+1) absolute chunk indices
+    const int* pair_chunks;   // this sample's N(N-1)*(kSplit+1) pair sub-list chunk indices
+    long long sweep0;
+    int steps, total, n;      // n chains of this warp (0..2)
+    int list[2], part0[2], part1[2];
+    // the last pair pick of the consumer (slot 0) and of the prefetch cursor
+    // (slot 1): each list lookup of a move reuses it instead of another Philox
+    int cm[2] = {-1, -1}, ci[2] = {0, 0}, cj[2] = {0, 0};
+
+    __device__ __forceinline__ void range(int m, int pass, int q, int& c, int& c_end, int slot) {
+        if (m != cm[slot]) {
+            const long long sw = sweep0 + m / steps;
+            pair_pick(key0, key1, (uint64_t)sw, (uint32_t)(m % steps), N, ci[slot], cj[slot]);
+            cm[slot] = m;
+        }
+        const int i0 = ci[slot], j0 = cj[slot];
+        const int li = q ? list[1] : list[0];
+        const int* sc = pass == 0 ? site_chunks + (li ? j0 : i0) * (kSplit + 1)
+                                  : pair_chunks + (2 * (j0 * (j0 - 1) / 2 + i0) + li) * (kSplit + 1);
+        c = __ldg(sc + (q ? part0[1] : part0[0]));
+        c_end = __ldg(sc + (q ? part1[1] : part1[0]));
+    }
+    // cursor of the copies: at move m, pass and chain `at`, chunk c of [c, c_end)
+    int m = 0, at = 0, c = 0, c_end = 0;
+    __device__ __forceinline__ void next() {    // m == total at the end
+        c++;
+        while (c >= c_end) {
+            if (++at == 2 * n) {
+                at = 0;
+                if (++m >= total) return;
+            }
+            range(m, at >= n, at >= n ? at - n : at, c, c_end, 1);
+        }
+    }
+    __device__ __forceinline__ void first() {
+        if (n == 0) m = total;
+        if (m >= total) return;
+        range(0, 0, 0, c, c_end, 1);
+        c--;
+        next();
+    }
+};
+
+// One replica block on P.exec CTAs (CL: a thread-block cluster of more than one):
+// each reads its chains' share of the lists, the chains' partial fields of both
+// passes meet in every CTA's buffer (distributed shared memory, one cluster barrier
+// per exchange, double-buffered by exchange parity) and are added there in the order
+// of the block shape (the warps of a CTA of the shape, then its CTAs); every CTA then
+// evaluates the network and takes the same decision on the same numbers, so the
+// amplitude copies stay identical; rank 0 writes records, trace and results.
+// kOne: one CTA has the SM (256 registers; loads of a tile ahead), else three share it.
+template <bool CL, bool kOne>
+__global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
+    learned_sweep_kernel(const SweepParams P, const LearnParams L) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int C = CL ? P.cluster : 1;
+    const int X = CL ? P.exec : 1, CW = P.cluster * P.warps;
     const uint32_t rank = CL ? cluster_rank() : 0u;
     const bool writer = rank == 0;
-    const Unit U = P.units[blockIdx.x / C];
+    const Unit U = P.units[blockIdx.x / X];
     const SampleDev S = P.samples[U.sample];
     const int N = S.N, R = S.R;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = P.warps;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int W = kLWarps;
     const bool learned = L.mode == 2;
     float2* sp = reinterpret_cast<float2*>(smem_raw);
-    float4* red = reinterpret_cast<float4*>(sp + (size_t)(N + 1) * kRepBlock);
-    int2* ring_all = reinterpret_cast<int2*>(red + (size_t)W * kRepBlock);
-    int2* ring = ring_all + (size_t)warp * kLStages * kStage;
-    uint64_t* bars_all = reinterpret_cast<uint64_t*>(ring_all + (size_t)W * kLStages * kStage);
-    uint64_t* bars = bars_all + warp * kLStages;
-    uint32_t* bufA = reinterpret_cast<uint32_t*>(bars_all + W * kLStages);
+    const LearnLayout Lo(N, 2 * CW, X, P.chains);
+    int2* ring = reinterpret_cast<int2*>(smem_raw + Lo.ring) + (size_t)warp * kLStages * kStage;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + Lo.bars) + warp * kLStages;
+    uint32_t* bufA = reinterpret_cast<uint32_t*>(smem_raw + Lo.buf);
     uint32_t* bufB = bufA + kMlpBufWords;
     const float* outs = reinterpret_cast<const float*>(bufB);
-    float* xch = reinterpret_cast<float*>(bufB + kMlpBufWords);
+    float* xch = reinterpret_cast<float*>(smem_raw + Lo.xch);
     auto out_of = [&](int o) { return outs[o * kOutStride + lane]; };
-    float4* cred = CL ? reinterpret_cast<float4*>(smem_raw + learned_cluster_buffer_offset(N, W)) : nullptr;
-    int* cflag = CL ? reinterpret_cast<int*>(cred + (size_t)2 * C * kRepBlock) : nullptr;   // cluster abort flag
+    float2* parts = reinterpret_cast<float2*>(smem_raw + Lo.parts);      // [parity][2 C W][32]
+    int* cflag = reinterpret_cast<int*>(smem_raw + Lo.flag);             // cluster abort flags, by parity
 
     const bool active = lane < U.rep_count;
     const int64_t gr = S.rep_off + U.rep_begin + lane;
@@ -204,7 +278,7 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
         sp[idx] = v;
     }
     if (threadIdx.x < kRepBlock) sp[N * kRepBlock + threadIdx.x] = make_float2(1.f, 0.f);
-    if (CL && threadIdx.x == 0) *cflag = 0;
+    if (CL && threadIdx.x < 2) cflag[threadIdx.x] = 0;
 
     double E = 0.0, beta_d = 0.0;
     float beta = 0.f;
@@ -222,7 +296,7 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
     }
     const long long sweep0 = *P.sweep_counter;
     const int steps = N / 2, total = P.nsweeps * steps;
-    Stream<4> st;
+    LearnStream st;
     st.key0 = S.pair_key0;
     st.key1 = S.pair_key1;
     st.N = N;
@@ -231,29 +305,36 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
     st.sweep0 = sweep0;
     st.steps = steps;
     st.total = total;
-    const int TW = C * W, gw = (int)rank * W + warp;
-    st.part0 = gw * (kSplit / TW);
-    st.part1 = (gw + 1) * (kSplit / TW);
-    if (lane == 0) {
+    const int chain0 = (int)rank * P.chains + warp;   // this warp's chains: chain0, chain0 + kLWarps
+    st.n = 0;
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+        const int ch = chain0 + q * kLWarps, g = ch % CW;
+        if (warp + q * kLWarps < P.chains && ch < 2 * CW) st.n = q + 1;
+        st.list[q] = ch / CW;
+        st.part0[q] = g * (kSplit / CW);
+        st.part1[q] = (g + 1) * (kSplit / CW);
+    }
+    if (lane == 0 && warp < Lo.rings) {
         for (int s = 0; s < kLStages; s++) mbar_init(bars + s, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_async_shared();
     }
     __syncwarp();
-    Cursor pc = st.first();
+    st.first();
     uint32_t issued = 0, consumed = 0;
     bool ok_wait = true;
     auto issue = [&]() {
-        if (pc.m >= total) return;
+        if (st.m >= total) return;
         const uint32_t slot = issued % kLStages;
         if (lane == 0) {
-            const int64_t b = __ldg(P.chunk_start + pc.c), e = __ldg(P.chunk_start + pc.c + 1);
+            const int64_t b = __ldg(P.chunk_start + st.c), e = __ldg(P.chunk_start + st.c + 1);
             const uint32_t bytes = (uint32_t)((e - b) * sizeof(int2));
             mbar_expect_tx(bars + slot, bytes);
             bulk_g2s(ring + slot * kStage, P.entries + b, bytes, bars + slot);
         }
         issued++;
-        st.next(pc);
+        st.next();
     };
     for (int s = 0; s < kLStages; s++) issue();
     __shared__ __align__(8) uint64_t stall_bar;      // test hook: nothing arrives on it
@@ -266,22 +347,24 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
     uint32_t xchg = 0;                         // exchanges so far (buffer parity)
     bool aborted = false;                      // set uniformly over the CTA (cluster) by reduce()
 
-    // one pass over this warp's share of two lists: the sites' lists (base 0;
-    // tiles, or the group format built with the pair sub-lists) or the pair's
-    // sub-lists (base 2, group format)
-    auto pass = [&](int m, int base, float* h) {
-        for (int which = base; which < base + 2 && ok_wait; which++) {
+    // this warp's chains over the sites' lists (second 0) or the pair's sub-lists (1);
+    // tiles or groups
+    auto pass = [&](int m, int second, float (&h)[2][2]) {
+        const int tiles = second ? S.tiles_p : S.tiles_g;
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            h[q][0] = h[q][1] = 0.f;
+            if (q >= st.n || !ok_wait) continue;
             int c, c_end;
-            st.range(m, which, c, c_end);
+            st.range(m, second, q, c, c_end, 0);
             for (; c < c_end; c++) {
                 const uint32_t slot = consumed % kLStages;
                 ok_wait = ring_wait(bars + slot, (consumed / kLStages) & 1u, P.status, P.wait_clocks);
                 if (!ok_wait) break;               // stop consuming and issuing; abort in reduce()
                 const int n = (int)(__ldg(P.chunk_start + c + 1) - __ldg(P.chunk_start + c));
-                const int k2 = 2 * (which & 1);
-                if (which < 2 && S.tiles_g)       // small unrolls: the kernel is held to 80 registers
-                    accumulate_tiles_1<2, 2, false>(ring + slot * kStage, n, sp, lane, h[k2], h[k2 + 1]);
-                else accumulate_chunk(ring + slot * kStage, n, sp, lane, h[k2], h[k2 + 1]);
+                if (!tiles) accumulate_chunk(ring + slot * kStage, n, sp, lane, h[q][0], h[q][1]);
+                else if (kOne) accumulate_tiles_1<8, 4, true>(ring + slot * kStage, n, sp, lane, h[q][0], h[q][1]);
+                else accumulate_tiles_1<2, 2, false>(ring + slot * kStage, n, sp, lane, h[q][0], h[q][1]);
                 consumed++;
                 __syncwarp();
                 if (lane == 0) fence_async_shared();
@@ -289,42 +372,39 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
             }
         }
     };
-    // partial sums of all warps (and all CTAs of the cluster) -> warp 0.
-    // Also agrees on an abort: a warp whose wait ran out makes the whole CTA
-    // (and, through the flag, the whole cluster) set `aborted` here.
-    auto reduce = [&](const float* h) {
-        red[warp * kRepBlock + lane] = make_float4(h[0], h[1], h[2], h[3]);
-        const bool bad = __syncthreads_or(!ok_wait);
-        float4 hs = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (!CL && bad) {
-            aborted = true;
-            return hs;
+    // partial sums of all chains -> warp 0 of every CTA.  Also agrees on an abort:
+    // a warp whose wait ran out makes the whole CTA (and, through the flag, the
+    // whole cluster) set `aborted` here.
+    auto reduce = [&](const float (&h)[2][2]) {
+        float2* buf = parts + (CL ? (size_t)(xchg & 1u) * 2 * CW * kRepBlock : 0);
+#pragma unroll
+        for (int q = 0; q < 2; q++) {
+            if (q >= st.n) continue;
+            float2* to = buf + (size_t)(chain0 + q * kLWarps) * kRepBlock + lane;
+            const float2 v = make_float2(h[q][0], h[q][1]);
+            if (!CL) *to = v;
+            else
+                for (int r = 0; r < X; r++) st_cluster_f2(to, (uint32_t)r, v);
         }
-        if (warp == 0)
-            for (int w = 0; w < W; w++) {
-                const float4 v = red[w * kRepBlock + lane];
-                hs.x += v.x; hs.y += v.y; hs.z += v.z; hs.w += v.w;
-            }
+        float4 hs = make_float4(0.f, 0.f, 0.f, 0.f);
         if (CL) {
-            float4* buf = cred + (size_t)(xchg & 1u) * C * kRepBlock;
-            if (warp == 0) {
-                for (int q = 0; q < C; q++) st_cluster_f4(buf + rank * kRepBlock + lane, (uint32_t)q, hs);
-                if (bad && lane == 0)
-                    for (int q = 0; q < C; q++) st_cluster_u32(cflag, (uint32_t)q, 1u);
-            }
+            if (!ok_wait && lane == 0)
+                for (int r = 0; r < X; r++) st_cluster_u32(cflag + (xchg & 1u), (uint32_t)r, 1u);
             cluster_sync();
-            if (*(volatile int*)cflag) {
-                aborted = true;
-                return hs;
-            }
-            if (warp == 0) {
-                hs = buf[lane];
-                for (int q = 1; q < C; q++) {
-                    const float4 v = buf[q * kRepBlock + lane];
-                    hs.x += v.x; hs.y += v.y; hs.z += v.z; hs.w += v.w;
-                }
-            }
+            aborted = ((volatile int*)cflag)[xchg & 1u] != 0;
             xchg++;
+        } else {
+            aborted = __syncthreads_or(!ok_wait) != 0;
+        }
+        if (aborted || warp != 0) return hs;
+        for (int c = 0; c < P.cluster; c++) {
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int w = c * P.warps; w < (c + 1) * P.warps; w++) {
+                const float2 a = buf[w * kRepBlock + lane], b = buf[(CW + w) * kRepBlock + lane];
+                s.x += a.x; s.y += a.y; s.z += b.x; s.w += b.y;
+            }
+            if (c == 0) hs = s;
+            else { hs.x += s.x; hs.y += s.y; hs.z += s.z; hs.w += s.w; }
         }
         return hs;
     };
@@ -336,7 +416,7 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
         pair_pick(S.pair_key0, S.pair_key1, (uint64_t)sw, (uint32_t)k, N, i0, j0);
 
         // ---- fields at x: h_i (with a_j), h_j (with a_i) ---------------------------
-        float h[4] = {0.f, 0.f, 0.f, 0.f};
+        float h[2][2];
         if (m == P.stall_move) ok_wait = stall_wait(&stall_bar, P.status, P.wait_clocks);
         pass(m, 0, h);
         const float4 hs1 = reduce(h);
@@ -409,8 +489,7 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
         __syncthreads();
 
         // ---- field changes from the pair's sub-lists --------------------------------
-        h[0] = h[1] = h[2] = h[3] = 0.f;
-        pass(m, 2, h);
+        pass(m, 1, h);
         const float4 dh = reduce(h);
         if (aborted) break;
         float dE = 0.f;
@@ -492,7 +571,7 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
         }
         __syncthreads();
     }
-    if (aborted) drain_ring(bars, kLStages, consumed, issued, P.status);   // state stays as before the launch
+    if (aborted && warp < Lo.rings) drain_ring(bars, kLStages, consumed, issued, P.status);   // state stays as before the launch
     if (writer && !aborted) {
         for (int idx = threadIdx.x; idx < N * kRepBlock; idx += blockDim.x) {
             const int site = idx >> 5, l = idx & 31;
@@ -509,40 +588,70 @@ __global__ void __launch_bounds__(256, 3) learned_sweep_kernel(const SweepParams
 
 size_t learned_smem_bytes_host(int N, int warps, int C) { return learned_smem_bytes(N, warps, C); }
 
-// max_clusters != null (clusters only): reports how many clusters of this
-// shape can be resident instead of launching (0: the shape does not fit)
+// max_clusters != null: reports how many replica blocks of this shape can be
+// resident instead of launching (0: the shape does not fit)
 cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, int n_units, int max_N,
                                  cudaStream_t st, int* max_clusters) {
     if (n_units <= 0) return cudaSuccess;
     if (p.pair_chunks == nullptr && max_clusters == nullptr) return cudaErrorInvalidValue;
-    const int C = p.cluster > 1 ? p.cluster : 1;
+    const int C = p.cluster > 1 ? p.cluster : 1, all = 2 * C * p.warps;
     if (C > 16 || (kSplit % (C * p.warps)) != 0) return cudaErrorInvalidValue;
-    const size_t smem = learned_smem_bytes(max_N, p.warps, C);
-    if (C == 1) {
-        cudaError_t e = cudaFuncSetAttribute(learned_sweep_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-        learned_sweep_kernel<false><<<n_units, 32 * p.warps, smem, st>>>(p, l);
-        return cudaGetLastError();
-    }
-    auto kern = learned_sweep_kernel<true>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e == cudaSuccess && C > 8) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(n_units * C));
-    cfg.blockDim = dim3((unsigned)(32 * p.warps));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
+    SweepParams q = p;
+    q.cluster = C;
+    void (*kern)(const SweepParams, const LearnParams) = nullptr;
+    // As many CTAs per replica block as the blocks can all have at once with an SM
+    // for each CTA (8 at most, no more than there are chains), and no fewer than the
+    // shape has: chains on more SMs finish sooner, a second wave costs twice.  A move
+    // of 24 blocks at N = 64 (gamma = 0.1, 8 warps x 2 CTAs) took 128 us on 2 CTAs
+    // each, 84 on 6 (144 CTAs, but clusters of 6 do not tile the chip: two waves), 46
+    // on the most that run at once; of 3 blocks 117 and 41 (8 CTAs); of 12 fully
+    // connected blocks at N = 48 (one CTA's shape) 113 and 53.
+    auto prepare = [&](int X, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int* clusters) -> cudaError_t {
+        q.exec = X;
+        q.chains = (all + X - 1) / X;
+        const size_t smem = LearnLayout(max_N, all, X, q.chains).total;
+        const bool one = (long long)n_units * X <= sms;
+        kern = X > 1 ? (one ? learned_sweep_kernel<true, true> : learned_sweep_kernel<true, false>)
+                     : (one ? learned_sweep_kernel<false, true> : learned_sweep_kernel<false, false>);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess && X > 8)
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+        cfg = cudaLaunchConfig_t{};
+        cfg.gridDim = dim3((unsigned)(n_units * X));
+        cfg.blockDim = dim3((unsigned)(32 * kLWarps));
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        attr->id = cudaLaunchAttributeClusterDimension;
+        attr->val.clusterDim.x = (unsigned)X;
+        attr->val.clusterDim.y = 1;
+        attr->val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = X > 1 ? 1 : 0;
+        if (clusters && X > 1) return cudaOccupancyMaxActiveClusters(clusters, kern, &cfg);
+        return cudaSuccess;
+    };
+    cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)C;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (max_clusters) return cudaOccupancyMaxActiveClusters(max_clusters, kern, &cfg);
-    e = cudaLaunchKernelEx(&cfg, kern, p, l);
+    int X = std::max(C, std::min({8, sms / n_units, all})), fit = 0;
+    for (; X > C; X--) {
+        if ((all + X - 1) / X * (X - 1) >= all) continue;            // a CTA without a chain
+        if (LearnLayout(max_N, all, X, (all + X - 1) / X).total > 227 * 1024) continue;
+        e = prepare(X, cfg, attr, &fit);
+        if (e != cudaSuccess) return e;
+        if (fit >= n_units) break;
+    }
+    if (X == C) e = prepare(C, cfg, attr, max_clusters ? &fit : nullptr);
+    if (e != cudaSuccess) return e;
+    if (max_clusters) {
+        *max_clusters = X > 1 ? fit : 1;
+        return cudaSuccess;
+    }
+    e = cudaLaunchKernelEx(&cfg, kern, q, l);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }

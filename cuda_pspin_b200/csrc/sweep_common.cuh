@@ -195,69 +195,6 @@ __device__ __forceinline__ bool stall_wait(uint64_t* bar, int* status, long long
     return ring_wait(bar, 0u, status, limit);
 }
 
-// Position in a warp's chunk stream: move m, list (0: site i0, 1: site j0),
-// chunk c of [c, c_end).
-struct Cursor {
-    int m, which, c, c_end;
-};
-
-// kLists: lists visited per move -- sites i0, j0 (2); then, for the two-pass
-// sweep, the pair's two sub-lists (4).  kCache: keep the last pair pick of the
-// consumer and of the cursor (fewer Philox evaluations, two more live
-// registers; measured faster for sweep_kernel and the two-pass sweep, slower
-// for the cluster sweep)
-template <int kLists, bool kCache = true>
-struct Stream {
-    uint32_t key0, key1;
-    int N;
-    const int* site_chunks;   // this sample's N*(kSplit+1) absolute chunk indices
-    const int* pair_chunks;   // this sample's N(N-1)*(kSplit+1) pair sub-list chunk indices
-    long long sweep0;
-    int steps, total, part0, part1;
-    // the last pair pick of the consumer (slot 0) and of the prefetch cursor
-    // (slot 1): each list lookup of a move reuses it instead of another Philox
-    int cm[2] = {-1, -1}, ci[2] = {0, 0}, cj[2] = {0, 0};
-
-    __device__ __forceinline__ void range(int m, int which, int& c, int& c_end, int slot = 0) {
-        int i0, j0;
-        if (kCache) {
-            if (m != cm[slot]) {
-                const long long sw = sweep0 + m / steps;
-                pair_pick(key0, key1, (uint64_t)sw, (uint32_t)(m % steps), N, ci[slot], cj[slot]);
-                cm[slot] = m;
-            }
-            i0 = ci[slot];
-            j0 = cj[slot];
-        } else {
-            const long long sw = sweep0 + m / steps;
-            pair_pick(key0, key1, (uint64_t)sw, (uint32_t)(m % steps), N, i0, j0);
-        }
-        const int* sc = (kLists == 2 || which < 2) ? site_chunks + ((which & 1) ? j0 : i0) * (kSplit + 1)
-                                                   : pair_chunks + (2 * (j0 * (j0 - 1) / 2 + i0) + (which & 1)) * (kSplit + 1);
-        c = __ldg(sc + part0);
-        c_end = __ldg(sc + part1);
-    }
-    // move to the next chunk (skipping empty ranges); m == total at the end
-    __device__ __forceinline__ void next(Cursor& k) {
-        k.c++;
-        while (k.c >= k.c_end) {
-            if (++k.which == kLists) {
-                k.which = 0;
-                if (++k.m >= total) return;
-            }
-            range(k.m, k.which, k.c, k.c_end, 1);
-        }
-    }
-    __device__ __forceinline__ Cursor first() {
-        Cursor k{0, 0, 0, 0};
-        if (total <= 0) return k;
-        range(0, 0, k.c, k.c_end, 1);
-        k.c--;
-        next(k);
-        return k;
-    }
-};
-
 // Field contribution of the groups in one staged chunk for this lane's replica.
 __device__ __forceinline__ void accumulate_chunk(const int2* __restrict__ R, int n,
                                                  const float2* __restrict__ sp, int lane,
@@ -567,13 +504,11 @@ __device__ __forceinline__ void st_async_f64(uint32_t addr, double v, uint32_t b
 }
 
 // store v into the same shared-memory location of CTA `rank` of the cluster
-__device__ __forceinline__ void st_cluster_f4(const void* local, uint32_t rank, float4 v) {
+__device__ __forceinline__ void st_cluster_f2(const void* local, uint32_t rank, float2 v) {
     const uint32_t la = (uint32_t)__cvta_generic_to_shared(local);
     uint32_t ra;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(la), "r"(rank));
-    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(ra), "f"(v.x), "f"(v.y), "f"(v.z),
-                 "f"(v.w)
-                 : "memory");
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ra), "f"(v.x), "f"(v.y) : "memory");
 }
 
 __device__ __forceinline__ void st_cluster_u32(const void* local, uint32_t rank, uint32_t v) {
