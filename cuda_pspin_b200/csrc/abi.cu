@@ -16,11 +16,13 @@
 #include <string>
 #include <chrono>
 #include <unordered_map>
+#include <memory>
 #include <vector>
 
 #include "../../include/pspin.h"
 #include "internal.h"
 #include "layout.h"
+#include "lists.h"
 #include "rng.cuh"
 
 #include <cuda_bf16.h>
@@ -660,9 +662,26 @@ static int setup_sparse_quartets(pspin_state* s, SampleHost& h, std::vector<Quar
     return PSPIN_OK;
 }
 
+// Device list builders of a create call hold at most this much at once (7 MB a
+// sample at N = 64); samples beyond it are laid out on the host.
+constexpr size_t kListBuilderBytes = (size_t)1 << 30;
+constexpr int kListBuilderMaxN = 256;
+
+// a masked dense sample's lists, on the device when they are tiles
+static bool device_lists(pspin_state* s, const SampleHost& h, size_t held, std::unique_ptr<DeviceLists>& out) {
+    if (s->opt.generic_lists || h.cfg.fmc_mode == 0 || h.N > kListBuilderMaxN || held >= kListBuilderBytes) return false;
+    out = std::make_unique<DeviceLists>();
+    const cudaError_t e = out->plan(h.N, s->d_g4re + h.g4_off, s->d_mask + h.g4_off,
+                                    h.h2_active ? h.g2re.data() : nullptr, s->st);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+    if (e == cudaSuccess && out->tiles) return true;
+    out.reset();
+    return false;
+}
+
 // dense g4: generation, FMC mask, popcount, rescale, shift, all on the
 // device (mc.cu:445-446, 480-483, 492, 499-502)
-static int setup_dense_g4(pspin_state* s, SampleHost& h, std::vector<double>& g4re, std::vector<uint8_t>& mask) {
+static int setup_dense_g4(pspin_state* s, SampleHost& h) {
     const pspin_config& c = h.cfg;
     const int N = c.N;
     const int64_t nq = C4(N);
@@ -695,13 +714,7 @@ static int setup_dense_g4(pspin_state* s, SampleHost& h, std::vector<double>& g4
             const double mean = (J40 != 0.0 && a > 0) ? J40 * (double)N / (double)a : 0.0;
             e = dev_g4_real(d_nrm, g4, nq, sigma, mean, s->st);
         }
-        if (e == cudaSuccess) {
-            g4re.resize(nq);
-            mask.resize(nq);
-            e = cudaMemcpyAsync(g4re.data(), g4, nq * sizeof(double), cudaMemcpyDeviceToHost, s->st);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(mask.data(), m, nq, cudaMemcpyDeviceToHost, s->st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
-        }
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
         if (e != cudaSuccess) rc = fail(PSPIN_ERR_CUDA, "dense g4 set-up: %s", cudaGetErrorString(e));
     }
     cudaFree(d_nrm);
@@ -831,6 +844,8 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
     std::vector<std::vector<QuartetRec>> qsv(n);
     std::vector<std::vector<double>> g4h(n);
     std::vector<std::vector<uint8_t>> maskh(n);
+    std::vector<std::unique_ptr<DeviceLists>> built(n);
+    size_t held = 0;
     // each sample's replica normals stay on the device until the normalisation
     // kernel writes them, scaled, into the amplitude array
     struct DevNormals {
@@ -846,8 +861,21 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         rc = setup_g2(h, s->st);
         if (rc != PSPIN_OK) return bail(rc);
         if (variant == PSPIN_DENSE) {
-            rc = setup_dense_g4(s, h, g4h[k], maskh[k]);
+            rc = setup_dense_g4(s, h);
             if (rc != PSPIN_OK) return bail(rc);
+            if (device_lists(s, h, held, built[k])) {
+                held += built[k]->held;
+            } else {
+                g4h[k].resize((size_t)h.nq_dense);
+                maskh[k].resize((size_t)h.nq_dense);
+                cudaError_t e = cudaMemcpyAsync(g4h[k].data(), s->d_g4re + h.g4_off, h.nq_dense * sizeof(double),
+                                                cudaMemcpyDeviceToHost, s->st);
+                if (e == cudaSuccess)
+                    e = cudaMemcpyAsync(maskh[k].data(), s->d_mask + h.g4_off, h.nq_dense, cudaMemcpyDeviceToHost, s->st);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(s->st);
+                if (e != cudaSuccess)
+                    return bail(fail(PSPIN_ERR_CUDA, "dense g4 set-up: %s", cudaGetErrorString(e)));
+            }
         } else {
             rc = setup_sparse_quartets(s, h, qsv[k]);
             if (rc != PSPIN_OK) return bail(rc);
@@ -883,6 +911,15 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
     for (int k = 0; k < n; k++) {
         SampleHost& h = s->hs[k];
         const int N = h.N;
+        if (built[k]) {
+            h.fc = 0;
+            h.tiles = 1;
+            h.single_groups = 0;
+            h.site_entries = built[k]->nominal;
+            h.stored_entries = built[k]->entries;
+            h.exec_flops_lists = built[k]->flops;
+            continue;
+        }
         bool fc = false;
         if (variant == PSPIN_DENSE) {
             dense_quartets(N, g4h[k].data(), maskh[k].data(), qsv[k]);
@@ -911,6 +948,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
     // ---- concatenate and upload
     int64_t ent_total = 0, split_total = 0, q_total = 0, g2_total = 0, spin_off = 0, rep_off = 0, chunk_total = 0;
     int64_t nb_total = 0;
+    bool all_built = true;
     s->sd.resize(n);
     for (int k = 0; k < n; k++) {
         SampleHost& h = s->hs[k];
@@ -927,7 +965,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         d.rep_off = rep_off;
         d.split_off = split_total;
         d.q_off = q_total;
-        d.nq = (int64_t)q64[k].size();
+        d.nq = built[k] ? built[k]->quartets : (int64_t)q64[k].size();
         d.g2_off = g2_total;
         d.pair_off = -1;
         d.nb_off = nb_total;
@@ -942,14 +980,17 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         q_total += d.nq;
         g2_total += (int64_t)h.N * h.N;
         ent_total += h.stored_entries;
-        chunk_total += (int64_t)lists[k].chunk_start.size();
+        chunk_total += built[k] ? built[k]->chunks : (int64_t)lists[k].chunk_start.size();
+        if (!built[k]) all_built = false;
     }
     if (chunk_total >= (1ll << 31)) return bail(fail(PSPIN_ERR_ARG, "too many list chunks"));
-    std::vector<int2> ent(ent_total);
-    std::vector<int> site_chunks(split_total);
-    std::vector<int64_t> chunk_start(chunk_total + 1);
-    std::vector<Q64> qall(q_total);
-    std::vector<uint32_t> nball(nb_total, 0u);
+    // host-made parts (all empty when the device makes every sample's)
+    std::vector<int2> ent(all_built ? 0 : ent_total);
+    std::vector<int> site_chunks(all_built ? 0 : split_total);
+    std::vector<int64_t> chunk_start(all_built ? 0 : chunk_total);
+    std::vector<Q64> qall(all_built ? 0 : q_total);
+    std::vector<uint32_t> nball(all_built ? 0 : nb_total, 0u);
+    std::vector<int64_t> entry0(n), chunk0(n);
     std::vector<double> g2all(g2_total);
     std::vector<double> Eall(s->R_tot, 0.0);
     std::vector<uint64_t> kall(s->R_tot);
@@ -957,6 +998,15 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         int64_t eoff = 0, coff = 0;
         for (int k = 0; k < n; k++) {
             const SampleDev& d = s->sd[k];
+            entry0[k] = eoff;
+            chunk0[k] = coff;
+            std::copy(s->hs[k].g2re.begin(), s->hs[k].g2re.end(), g2all.begin() + d.g2_off);
+            std::copy(keys[k].begin(), keys[k].end(), kall.begin() + d.rep_off);
+            if (built[k]) {
+                eoff += built[k]->entries;
+                coff += built[k]->chunks;
+                continue;
+            }
             std::copy(lists[k].entries.begin(), lists[k].entries.end(), ent.begin() + eoff);
             for (size_t t = 0; t < lists[k].chunk_start.size(); t++) chunk_start[coff + t] = lists[k].chunk_start[t] + eoff;
             for (size_t t = 0; t < lists[k].site_chunks.size(); t++)
@@ -979,12 +1029,9 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
                         for (int b = 0; b < Nk; b++)
                             if (a != b) set(a, b);
             }
-            std::copy(s->hs[k].g2re.begin(), s->hs[k].g2re.end(), g2all.begin() + d.g2_off);
-            std::copy(keys[k].begin(), keys[k].end(), kall.begin() + d.rep_off);
             lists[k] = SiteLists();
             q64[k].clear();
         }
-        chunk_start[chunk_total] = eoff;
     }
     s->ent_total = ent_total;
     s->chunk_total = chunk_total;
@@ -1064,11 +1111,20 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         (rc = up(s->d_entries, ent.data(), ent.size() * sizeof(int2))) ||
         (rc = up(s->d_site_chunks, site_chunks.data(), site_chunks.size() * sizeof(int))) ||
         (rc = up(s->d_chunk_start, chunk_start.data(), chunk_start.size() * sizeof(int64_t))) ||
+        (rc = up(s->d_chunk_start + chunk_total, &ent_total, sizeof(int64_t))) ||
         (rc = up(s->d_q64, qall.data(), qall.size() * sizeof(Q64))) ||
         (rc = up(s->d_g2, g2all.data(), g2all.size() * sizeof(double))) ||
         (rc = up(s->d_nbmask, nball.data(), nball.size() * sizeof(uint32_t))) ||
         (rc = up(s->d_beta, ones.data(), ones.size() * sizeof(double))))
         return bail(rc);
+    for (int k = 0; k < n; k++) {
+        if (!built[k]) continue;
+        const SampleDev& d = s->sd[k];
+        const cudaError_t e = built[k]->write(entry0[k], chunk0[k], s->d_entries + entry0[k], s->d_chunk_start + chunk0[k],
+                                              s->d_site_chunks + d.split_off, s->d_q64 + d.q_off, s->d_nbmask + d.nb_off,
+                                              s->st);
+        if (e != cudaSuccess) return bail(fail(PSPIN_ERR_CUDA, "site lists: %s", cudaGetErrorString(e)));
+    }
     {
         cudaError_t e = cudaMemsetAsync(s->d_acc, 0, s->R_tot * sizeof(long long), s->st);
         if (e == cudaSuccess) e = cudaMemsetAsync(s->d_prop, 0, s->R_tot * sizeof(long long), s->st);
