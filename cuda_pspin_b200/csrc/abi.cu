@@ -667,12 +667,13 @@ static int setup_sparse_quartets(pspin_state* s, SampleHost& h, std::vector<Quar
 constexpr size_t kListBuilderBytes = (size_t)1 << 30;
 constexpr int kListBuilderMaxN = 256;
 
-// a masked dense sample's lists, on the device when they are tiles
+// a dense sample's lists, on the device when they are tiles
 static bool device_lists(pspin_state* s, const SampleHost& h, size_t held, std::unique_ptr<DeviceLists>& out) {
-    if (s->opt.generic_lists || h.cfg.fmc_mode == 0 || h.N > kListBuilderMaxN || held >= kListBuilderBytes) return false;
+    if (s->opt.generic_lists || h.N > kListBuilderMaxN || held >= kListBuilderBytes) return false;
     out = std::make_unique<DeviceLists>();
-    const cudaError_t e = out->plan(h.N, s->d_g4re + h.g4_off, s->d_mask + h.g4_off,
-                                    h.h2_active ? h.g2re.data() : nullptr, s->st);
+    auto plan = h.cfg.fmc_mode == 0 ? &DeviceLists::plan_fc : &DeviceLists::plan;
+    const cudaError_t e = ((*out).*plan)(h.N, s->d_g4re + h.g4_off, s->d_mask + h.g4_off,
+                                         h.h2_active ? h.g2re.data() : nullptr, s->st);
     if (e == cudaErrorMemoryAllocation) cudaGetLastError();
     if (e == cudaSuccess && out->tiles) return true;
     out.reset();
@@ -912,7 +913,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         SampleHost& h = s->hs[k];
         const int N = h.N;
         if (built[k]) {
-            h.fc = 0;
+            h.fc = h.cfg.fmc_mode == 0 ? 1 : 0;
             h.tiles = 1;
             h.single_groups = 0;
             h.site_entries = built[k]->nominal;

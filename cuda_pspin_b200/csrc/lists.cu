@@ -1,8 +1,8 @@
-// lists.cu -- site lists, FP64 quartet table and neighbour masks of one masked
-// dense sample, built on the device from its couplings and channel mask: the
-// same entries, chunks and quartets, in the same order, as layout.cpp's
-// dense_quartets, build_site_lists(kRecords, tile) and build_q64 make on the host
-// (where the formats are described).
+// lists.cu -- site lists, FP64 quartet table and neighbour masks of one dense
+// sample, built on the device from its couplings and channel mask: the same
+// entries, chunks and quartets, in the same order, as layout.cpp's dense_quartets,
+// build_site_lists(kRecords, tile) or build_site_tiles_fc, and build_q64 make on the
+// host (where the formats are described).
 //
 // A site's terms need no sorting here: (site, p, o1) enumerates its groups in
 // list order, a thread each, and the inner sites o2 their terms; a term's coupling
@@ -12,8 +12,9 @@
 // parts' paths.  A whole set-up with the lists made on the host (one thread a sample;
 // sorts and shortest paths) and here, gamma = 0.1: N = 16 4.0 and 4.0 ms, N = 32 8.4
 // and 3.8, N = 48 28 and 7.5, N = 64 87 and 9.7, N = 96 480 and 13, 16 samples of
-// N = 64 (16 host threads) 315 and 105 (the rest is the generator calls): no size is
-// left to the host's builder for its speed.
+// N = 64 (16 host threads) 315 and 105 (the rest is the generator calls); fully
+// connected N = 24 5.5 and 3.5, N = 48 27 and 7, N = 64 87 and 8, N = 96 490 and 9:
+// no size is left to the host's builder for its speed.
 #include <algorithm>
 #include <cstdint>
 
@@ -324,6 +325,162 @@ __global__ void emit_kernel(const In in, const int4* __restrict__ groups, const 
     }
 }
 
+// ---- fully connected samples: layout.cpp's build_site_tiles_fc
+// Key x of site m: 0 the two-body terms; 1 .. N-1-m the outer sites above m (m among
+// a quartet's two smallest); the rest those below m.  A key holds, four partners at a
+// time, its inner range in steps of kGroupMax ("fours").
+struct FcKey {
+    int outer, lo, hi, partners;
+    bool above;
+};
+__device__ __forceinline__ FcKey fc_key(const In& in, int m, int x) {
+    const int N = in.N;
+    FcKey k;
+    k.above = x <= N - 1 - m;
+    if (x == 0) return FcKey{N, 0, in.g2 ? N : 0, 1, false};
+    k.outer = k.above ? m + x : x - (N - m);
+    k.lo = k.above ? k.outer + 1 : 0;
+    k.hi = k.above ? N : k.outer;
+    k.partners = k.lo >= k.hi ? 0 : k.above ? k.outer - 1 : N - 2 - k.outer;
+    return k;
+}
+
+// int4 {outer | first partner << 16, lo | hi << 16, end (entries, cumulative), partners
+// | above << 16} per four; scanned with one block per site.
+__global__ void __launch_bounds__(kScan) fc_fours_kernel(const In in, const int* __restrict__ gbase, int4* __restrict__ fours,
+                                                         int2* __restrict__ totals) {
+    const int m = blockIdx.x, N = in.N;
+    int2 run = make_int2(0, 0), total;
+    for (int x0 = 0; x0 < N; x0 += kScan) {
+        const int x = x0 + threadIdx.x;
+        FcKey k{0, 0, 0, 0, false};
+        int2 v = make_int2(0, 0);
+        if (x < N) {
+            k = fc_key(in, m, x);
+            const int blocks = (k.partners + 3) / 4, len = max(k.hi - k.lo, 0), steps = (len + kGroupMax - 1) / kGroupMax;
+            v = make_int2(blocks * steps, 2 * blocks * (len + steps));
+        }
+        const int2 b = block_scan(v, total);
+        if (fours != nullptr && v.x > 0) {
+            int4* out = fours + gbase[m] + run.x + b.x;
+            int end = run.y + b.y;
+            for (int p = 0; p < k.partners; p += 4)
+                for (int lo = k.lo; lo < k.hi; lo += kGroupMax) {
+                    const int hi = min(k.hi, lo + kGroupMax);
+                    end += 2 * (1 + hi - lo);
+                    *out++ = make_int4(k.outer | (p << 16), lo | (hi << 16), end, min(4, k.partners - p) | (k.above << 16));
+                }
+        }
+        run.x += total.x;
+        run.y += total.y;
+    }
+    if (threadIdx.x == 0) totals[m] = run;
+}
+
+// the tile at four t of [.., e): one four, or two over the same inner range
+__device__ __forceinline__ bool fc_two(const int4* __restrict__ f, int t, int e, int N) {
+    return t + 1 < e && (f[t].w & 0xFFFF) == 4 && (f[t].x & 0xFFFF) < N && (f[t + 1].x & 0xFFFF) == (f[t].x & 0xFFFF) &&
+           f[t + 1].y == f[t].y;
+}
+
+__global__ void fc_cut_kernel(const int4* __restrict__ fours, const int* __restrict__ gbase, const int2* __restrict__ totals,
+                              int N, int2* __restrict__ sizes, unsigned long long* __restrict__ sums) {
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= N * kSplit) return;
+    const int m = id / kSplit, part = id % kSplit, n = totals[m].x;
+    const int4* f = fours + gbase[m];
+    const int b = part_begin(f, n, part), e = max(b, part_begin(f, n, part + 1));
+    int2 size = make_int2(0, 0);
+    int len = 0;
+    unsigned long long ops = 0;
+    for (int t = b; t < e;) {
+        const bool two = fc_two(f, t, e, N);
+        const int w = two ? 8 : 4, rows = (f[t].y >> 16) - (f[t].y & 0xFFFF), words = w / 2 * (1 + rows);
+        const int c = two ? 4 + (f[t + 1].w & 0xFFFF) : f[t].w & 0xFFFF;
+        if (len == 0 || len + words > kStage) {
+            size.x++;
+            len = 0;
+        }
+        len += words;
+        size.y += words;
+        ops += 14 * c + 4 * w * rows;
+        t += two ? 2 : 1;
+    }
+    if (ops) atomicAdd(sums + 2, ops);
+    sizes[id] = size;
+}
+
+__global__ void fc_emit_kernel(const In in, const int4* __restrict__ fours, const int* __restrict__ gbase,
+                               const int2* __restrict__ totals, const int2* __restrict__ sizes, int chunks, int64_t entry0,
+                               int chunk0, int2* __restrict__ entries, int64_t* __restrict__ chunk_start,
+                               int* __restrict__ site_chunks) {
+    const int id = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31, N = in.N;
+    if (id >= N * kSplit) return;
+    const int m = id / kSplit, part = id % kSplit, n = totals[m].x;
+    const int4* f = fours + gbase[m];
+    const int b = part_begin(f, n, part), e = max(b, part_begin(f, n, part + 1));
+    int chunk = sizes[id].x, len = 0;
+    int64_t at = sizes[id].y;
+    if (lane == 0) {
+        site_chunks[m * (kSplit + 1) + part] = chunk0 + chunk;
+        if (part == kSplit - 1) site_chunks[m * (kSplit + 1) + kSplit] = chunk0 + (id + 1 < N * kSplit ? sizes[id + 1].x : chunks);
+    }
+    for (int t = b; t < e;) {
+        const bool two = fc_two(f, t, e, N);
+        const int4 f0 = f[t], f1 = f[two ? t + 1 : t];
+        const int outer = f0.x & 0xFFFF, lo = f0.y & 0xFFFF, rows = (f0.y >> 16) - lo, w = two ? 8 : 4;
+        const int c = two ? 4 + (f1.w & 0xFFFF) : f0.w & 0xFFFF, words = w / 2 * (1 + rows);
+        const bool above = (f0.w >> 16) != 0;
+        auto v = [&](int q) {                       // column q's partner: the sites but m, from 0 or after outer
+            if (q >= c || outer == N) return N;
+            const int p = (q < 4 ? f0.x >> 16 : f1.x >> 16) + (q & 3) + (above ? 0 : outer + 1);
+            return p < m ? p : p + 1;
+        };
+        if (len == 0 || len + words > kStage) {
+            if (lane == 0) chunk_start[chunk] = entry0 + at;
+            chunk++;
+            len = 0;
+        }
+        len += words;
+        int2* out = entries + at;
+        if (lane == 0) {
+            out[0] = make_int2(outer | ((two ? 1 : 0) << 16), lo | (rows << 16) | (c << 24));
+            out[1] = make_int2(v(0) | (v(1) << 16), v(2) | (v(3) << 16));
+            if (two) {
+                out[2] = make_int2(v(4) | (v(5) << 16), v(6) | (v(7) << 16));
+                out[3] = make_int2(0, 0);
+            }
+        }
+        float* couplings = reinterpret_cast<float*>(out + w / 2);
+        for (int u = lane; u < rows * w; u += 32) {
+            const int q = u % w, r = lo + u / w;
+            float g = 0.f;
+            if (q < c) {
+                if (outer == N) {
+                    if (r != m) g = (float)in.g2[(size_t)m * N + r];
+                } else {
+                    // sorted {m, p, outer, r}: above, m and p below outer below r; else r below outer below m and p
+                    const int p = v(q), a = min(m, p), z = max(m, p);
+                    const int64_t quartet = above ? b4(r) + b3(outer) + b2(z) + a : b4(z) + b3(a) + b2(outer) + r;
+                    g = (float)in.g4[quartet];
+                }
+            }
+            couplings[u] = g;
+        }
+        at += words;
+        t += two ? 2 : 1;
+    }
+}
+
+__global__ void fc_neighbours_kernel(int N, bool all, uint32_t* __restrict__ nb) {
+    const int wpr = (N + 31) / 32, id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= N * wpr) return;
+    const int m = id / wpr, first = 32 * (id % wpr), n = min(32, N - first);
+    uint32_t w = !all ? 0u : n == 32 ? 0xffffffffu : (1u << n) - 1u;
+    if (m / 32 == id % wpr) w &= ~(1u << (m % 32));
+    nb[id] = w;
+}
+
 // ---- FP64 quartet table: block (l, k) holds quartets b4(l) + b3(k) + [0, b2(k))
 __global__ void count_quartets_kernel(const In in, int* __restrict__ counts) {
     const int l = blockIdx.x, k = blockIdx.y;
@@ -386,7 +543,6 @@ __global__ void __launch_bounds__(kScan) quartets_kernel(const In in, const int6
 DeviceLists::~DeviceLists() {
     cudaFree(slab);
     cudaFree(groups_slab);
-    cudaFree(d_g2);
 }
 
 // 16-byte-aligned pieces of one allocation
@@ -403,13 +559,6 @@ cudaError_t DeviceLists::plan(int N_, const double* g4, const uint8_t* mask, con
     d_g4 = g4;
     d_mask = mask;
     cudaError_t e = cudaSuccess;
-    if (g2_host) {
-        e = cudaMalloc(&d_g2, (size_t)N * N * sizeof(double));
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(d_g2, g2_host, (size_t)N * N * sizeof(double), cudaMemcpyHostToDevice, st);
-        if (e != cudaSuccess) return e;
-    }
-    const In in{d_g4, d_mask, d_g2, N};
     const int keys = N * N + 1, wpr = (N + 31) / 32;
     uint16_t* cnt = nullptr;
     int2* off = nullptr;
@@ -426,10 +575,14 @@ cudaError_t DeviceLists::plan(int N_, const double* g4, const uint8_t* mask, con
         d_nb = piece<uint32_t>(at, base, (size_t)N * wpr);
         qcnt = piece<int>(at, base, (size_t)N * N);
         d_qoff = piece<int64_t>(at, base, (size_t)N * N);
+        if (g2_host) d_g2 = piece<double>(at, base, (size_t)N * N);
         if (pass == 0) e = cudaMalloc(&slab, at);
         held = at;
     }
+    if (e == cudaSuccess && g2_host)
+        e = cudaMemcpyAsync(d_g2, g2_host, (size_t)N * N * sizeof(double), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;
+    const In in{d_g4, d_mask, d_g2, N};
     const dim3 grid((keys + 255) / 256, N);
     count_terms_kernel<<<grid, 256, 0, st>>>(in, cnt);
     scan_keys_kernel<<<N, kScan, 0, st>>>(cnt, keys, off, d_totals);
@@ -484,15 +637,84 @@ cudaError_t DeviceLists::plan(int N_, const double* g4, const uint8_t* mask, con
     return cudaSuccess;
 }
 
+cudaError_t DeviceLists::plan_fc(int N_, const double* g4, const uint8_t* mask, const double* g2_host, cudaStream_t st) {
+    N = N_;
+    fc = true;
+    d_g4 = g4;
+    d_mask = mask;
+    cudaError_t e = cudaSuccess;
+    // as fc_fours_kernel counts them
+    std::vector<int> gbase(N);
+    int64_t n_fours = 0;
+    for (int m = 0; m < N; m++) {
+        gbase[m] = (int)n_fours;
+        auto add = [&](int partners, int len) {
+            n_fours += (int64_t)((partners + 3) / 4) * ((len + kGroupMax - 1) / kGroupMax);
+        };
+        if (g2_host) add(1, N);
+        for (int o = m + 1; o < N - 1; o++) add(o - 1, N - 1 - o);
+        for (int o = 1; o < m; o++) add(N - 2 - o, o);
+    }
+    if (n_fours >= (1ll << 27)) return cudaErrorMemoryAllocation;      // counts of entries stay below 2^31
+    int* qcnt = nullptr;
+    for (int pass = 0; pass < 2 && e == cudaSuccess; pass++) {
+        size_t at = 0;
+        unsigned char* base = static_cast<unsigned char*>(slab);
+        d_totals = piece<int2>(at, base, N);
+        d_gbase = piece<int>(at, base, N);
+        d_sizes = piece<int2>(at, base, (size_t)N * kSplit);
+        d_sums = piece<unsigned long long>(at, base, 8);
+        qcnt = piece<int>(at, base, (size_t)N * N);
+        d_qoff = piece<int64_t>(at, base, (size_t)N * N);
+        d_groups = piece<int4>(at, base, (size_t)n_fours);
+        if (g2_host) d_g2 = piece<double>(at, base, (size_t)N * N);
+        if (pass == 0) e = cudaMalloc(&slab, at);
+        held = at;
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_gbase, gbase.data(), N * sizeof(int), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_sums, 0, 8 * sizeof(unsigned long long), st);
+    if (e == cudaSuccess && g2_host)
+        e = cudaMemcpyAsync(d_g2, g2_host, (size_t)N * N * sizeof(double), cudaMemcpyHostToDevice, st);
+    if (e != cudaSuccess) return e;
+    const In in{d_g4, d_mask, d_g2, N};
+    fc_fours_kernel<<<N, kScan, 0, st>>>(in, d_gbase, d_groups, d_totals);
+    fc_cut_kernel<<<(N * kSplit + 31) / 32, 32, 0, st>>>(d_groups, d_gbase, d_totals, N, d_sizes, d_sums);
+    scan_parts_kernel<<<1, kScan, 0, st>>>(d_sizes, N * kSplit, d_sums);
+    count_quartets_kernel<<<dim3(N, N), 128, 0, st>>>(in, qcnt);
+    scan_quartets_kernel<<<1, kScan, 0, st>>>(qcnt, N * N, d_qoff, d_sums);
+    unsigned long long sums[8];
+    std::vector<int2> totals(N);
+    e = cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(totals.data(), d_totals, N * sizeof(int2), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    nominal = 0;
+    for (const int2& t : totals) nominal += t.y;
+    chunks = (int64_t)sums[4];
+    entries = (int64_t)sums[5];
+    flops = (double)sums[2];
+    quartets = (int64_t)sums[6];
+    tiles = quartets == b4(N);                  // a zero coupling: not fully connected
+    return cudaSuccess;
+}
+
 cudaError_t DeviceLists::write(int64_t entry0, int64_t chunk0, int2* out, int64_t* chunk_start, int* site_chunks, Q64* q,
                                uint32_t* nb, cudaStream_t st) const {
     const In in{d_g4, d_mask, d_g2, N};
+    const int wpr = (N + 31) / 32;
+    quartets_kernel<<<dim3(N, N), kScan, 0, st>>>(in, d_qoff, q);
+    if (fc) {
+        fc_emit_kernel<<<(N * kSplit + 3) / 4, 128, 0, st>>>(in, d_groups, d_gbase, d_totals, d_sizes, (int)chunks, entry0,
+                                                             (int)chunk0, out, chunk_start, site_chunks);
+        fc_neighbours_kernel<<<(N * wpr + 127) / 128, 128, 0, st>>>(N, N >= 4 || d_g2 != nullptr, nb);
+        return cudaGetLastError();
+    }
     emit_kernel<<<(N * kSplit + 3) / 4, 128, 0, st>>>(in, d_groups, d_gbase, d_totals, d_width, d_sizes, (int)chunks, entry0,
                                                       (int)chunk0, out, chunk_start, site_chunks);
-    quartets_kernel<<<dim3(N, N), kScan, 0, st>>>(in, d_qoff, q);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(nb, d_nb, (size_t)N * ((N + 31) / 32) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
+    return cudaMemcpyAsync(nb, d_nb, (size_t)N * wpr * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
 }
 
 }  // namespace pspin

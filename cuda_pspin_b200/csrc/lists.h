@@ -1,5 +1,5 @@
-// lists.h -- device construction of a masked dense sample's site lists, quartet
-// table and neighbour masks (lists.cu).
+// lists.h -- device construction of a dense sample's site lists, quartet table and
+// neighbour masks (lists.cu).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -10,7 +10,8 @@
 
 namespace pspin {
 
-// plan() finds the sizes and whether tiles pay; write() puts everything in place:
+// plan() (masked) or plan_fc() (every quartet active in channel 0, or !tiles) finds
+// the sizes and whether tiles pay; write() puts everything in place:
 // the entries at `out` (entry `entry0` of the engine's), its chunk starts (chunk
 // `chunk0`), site-chunk table, quartets and neighbour masks.  g4 and mask stay
 // the caller's until then.
@@ -25,11 +26,13 @@ struct DeviceLists {
     DeviceLists& operator=(const DeviceLists&) = delete;
     ~DeviceLists();
     cudaError_t plan(int N, const double* g4, const uint8_t* mask, const double* g2_host, cudaStream_t st);
+    cudaError_t plan_fc(int N, const double* g4, const uint8_t* mask, const double* g2_host, cudaStream_t st);
     cudaError_t write(int64_t entry0, int64_t chunk0, int2* out, int64_t* chunk_start, int* site_chunks, Q64* q, uint32_t* nb,
                       cudaStream_t st) const;
 
 private:
     int N = 0;
+    bool fc = false;
     const double* d_g4 = nullptr;
     const uint8_t* d_mask = nullptr;
     double* d_g2 = nullptr;

@@ -2,7 +2,7 @@
 // set of site lists fits in shared memory next to the amplitudes (sparse
 // samples: ~8 list entries per site).
 //
-// Same moves, RNG streams and Metropolis rule as sweep_kernel.  The lists
+// Same moves, RNG streams and Metropolis rule as the ring sweep.  The lists
 // are copied into shared memory once per launch, so a move reads them
 // without TMA copies; site m's list is the contiguous range of its chunks
 // (groups or tiles never span chunks; the padding entry of an odd chunk is

@@ -83,20 +83,26 @@ typedef struct pspin_options {
     int trace_capacity;  /*   ... number of move records kept */
     int quiet;           /* suppress the reference's stdout lines */
     int generic_lists;   /* 1: per-entry site lists for every sample; 0 (default):
-                            fully connected dense samples use blocked tiles */
-    int graph_steps;     /* pspin_pt_run replays a CUDA graph of this many PT
-                            steps (sweeps + exchange); 0 -> 32, <0 -> direct
-                            launches.  Results are identical either way. */
+                            dense samples use dense tiles where those are
+                            cheaper to read (the same chain for masked samples) */
+    int graph_steps;     /* pspin_pt_run where PT steps do not run inside one
+                            sweep launch (see pspin_pt_run) replays a CUDA graph
+                            of this many PT steps (sweeps + exchange); 0 -> 32,
+                            <0 -> direct launches of single steps everywhere.
+                            Results are identical either way. */
     int resync_method;   /* PSPIN_RESYNC_FP64 (default) or PSPIN_RESYNC_TC:
                             periodic energies from the split-BF16 tensor-core
                             contraction (one dense sample per handle) */
     int cluster_size;    /* CTAs (a thread-block cluster) sharing one replica
                             block's lists: 1, 2, 4, 8 or 16 with
                             cluster_size * warps_per_unit <= 32; 0 -> 1;
-                            -1: one warp per block with the sample's whole
-                            lists resident in shared memory (small lists;
-                            plain move only).  Both the plain and the
-                            two-pass sweep start with this shape. */
+                            -1: the sample's whole lists resident in shared
+                            memory (small lists; plain move only),
+                            warps_per_unit moves that commute at a time.
+                            The shape fixes the order the fields are summed in;
+                            how many SMs a block runs on follows from the
+                            number of blocks.  Both the plain and the two-pass
+                            sweep start with this shape. */
     int wait_limit_clocks; /* the sweep kernels' bounded waits on their copy
                             rings give up after this many SM clocks; 0 ->
                             2^31 (about one second).  A replica block whose
@@ -117,7 +123,7 @@ typedef struct pspin_options {
                             values, with no C(N,4)-sized memory.  The FMC
                             survivors and the quartet selection are the
                             reference's either way. */
-    int replicas_per_lane; /* plain sweep on the CTA / cluster kernels
+    int replicas_per_lane; /* plain sweep with streamed lists
                             (cluster_size >= 1): 2 or 3 replicas per lane, so
                             one block is 64 or 96 replicas of a sample and
                             every staged coupling serves them all; 1: one
@@ -205,7 +211,10 @@ int  pspin_get_sparse_quartets(pspin_state* s, int sample, int32_t* ijklch /*[n]
 int  pspin_pt_init(pspin_state* s, int NT, int nrep_per_temp, const double* beta_sched,
                    int pt_freq);
 /* Runs nsweeps sweeps; after every sweep whose 1-based index is a multiple
- * of pt_freq, proposes the NT-1 adjacent exchanges per replica column. */
+ * of pt_freq, proposes the NT-1 adjacent exchanges per replica column.  With
+ * the plain move, no observer and graph_steps >= 0, up to 256 steps run inside
+ * one sweep launch where every replica block is a whole sample (NT*nrep_per_temp
+ * <= 32 replicas_per_lane) or the lists are resident. */
 int  pspin_pt_run(pspin_state* s, int nsweeps);
 /* perm[NT*nrep_per_temp] (logical t*nrep+r -> physical replica) and the
  * cumulative exchange counters [NT-1] of one sample. */

@@ -1,12 +1,17 @@
-"""Lists of masked dense samples built on the device: the chain (whose bits
-depend on every list's order and parts), the FP64 energies (the quartet table's
-order) and the list-resident sweep (the neighbour masks) equal those of an
-engine whose lists the host makes (generic_lists), bit for bit.
+"""Lists of dense samples built on the device: the chain (whose bits depend on
+every list's order and parts), the FP64 energies (the quartet table's order) and
+the list-resident sweep (the neighbour masks) equal those of an engine whose lists
+the host makes (generic_lists), bit for bit.
 """
+import hashlib
+import json
+import os
+
 import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
+GOLDEN = os.path.join(os.path.dirname(__file__), "golden", "fc_chains.json")
 
 
 def _run(ps, cfgs, generic, **opts):
@@ -33,7 +38,7 @@ def test_device_lists_equal_host_lists(kw, shape):
 
 
 def test_mixed_batch():
-    """Fully connected (host) and masked (device) samples in one engine."""
+    """Fully connected and masked samples in one engine."""
     import cuda_pspin_b200 as ps
     cfgs = [ps.default_config(N=n, nrep=4, seed=30 + n, fmc_mode=f, gamma=0.2) for n, f in ((9, 0), (21, 2), (16, 0), (34, 2))]
     opts = dict(warps_per_unit=2, cluster_size=2)
@@ -58,3 +63,18 @@ def test_neighbours_of_resident_moves(kw):
     for warps in (1, 8):
         for a, b in zip(_run(ps, cfg, False, warps_per_unit=warps, cluster_size=-1), ref):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("key", sorted(json.load(open(GOLDEN))))
+def test_fully_connected_chain_is_pinned(key):
+    """Digests of amplitudes after three sweeps and of the first energies, recorded
+    with lists made on the host (they have no generic twin of the same order)."""
+    import cuda_pspin_b200 as ps
+    N, R, warps, cluster = map(int, key.split(","))
+    cfg = ps.default_config(N=N, nrep=R, seed=40 + N, T=0.5)
+    with ps.Engine(cfg, ps.PSPIN_DENSE, ps.make_options(warps_per_unit=warps, cluster_size=cluster)) as eng:
+        eng.fill_betas(2.0)
+        E0 = eng.get_results()[0]
+        eng.sweep(3)
+        s = np.ascontiguousarray(eng.get_spins()[0])
+    assert hashlib.md5(s.tobytes() + E0.tobytes()).hexdigest() == json.load(open(GOLDEN))[key]
