@@ -1238,8 +1238,11 @@ static int enqueue_ring(pspin_state* s, SweepParams& p, int pt_slots) {
     p.units = units_dev(s, s->rpl);
     p.n_units = n_units;
     // two sweeps (PT steps) per task: units of uneven N pack without a common
-    // end of every sweep, and a task is long against its start (some 10 us)
-    p.chunk = 2 * std::max(1, p.pt_freq);
+    // end of every sweep, and a task is long against its start (some 10 us);
+    // more where all units' tasks would not be counted in 31 bits
+    const long long step = std::max(1, p.pt_freq), most = std::max(1, (1 << 30) / std::max(1, n_units));
+    const long long per_task = step * std::max(2LL, (p.nsweeps + step * most - 1) / (step * most));
+    p.chunk = (int)std::min<long long>(per_task, p.nsweeps);
     if (n_units > plan.resident && p.nsweeps > p.chunk) {
         p.queue = s->d_queue;
         p.done = s->d_queue + 1;
@@ -1450,7 +1453,7 @@ static int timeout_error(int status) {
                 status, (status & kStatusDrain) ? ", and the drain of its copies ran out too" : "");
 }
 
-constexpr int kStepsPerLaunch = 256;     // bounds a launch's length
+constexpr int kSweepsPerLaunch = 256;    // of several PT steps: bounds a launch's length and its moves' count
 
 static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
     if (!s) return fail(PSPIN_ERR_ARG, "null handle");
@@ -1466,7 +1469,7 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
             long long room = left;
             if (s->opt.resync_every > 0) room = std::min<long long>(room, s->opt.resync_every - s->since_resync);
             if (room >= s->pt_freq && steps_in_launch(s)) {
-                int steps = (int)std::min<long long>(room / s->pt_freq, kStepsPerLaunch);
+                int steps = (int)std::max<long long>(1, std::min<long long>(room, kSweepsPerLaunch) / s->pt_freq);
                 if (s->cluster == 0) steps = std::min(steps, resident_chunk(s) / s->pt_freq);
                 TRY(launch_steps(s, steps));
                 left -= steps * s->pt_freq;

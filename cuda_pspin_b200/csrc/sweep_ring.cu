@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     const int k = warp - c;                          // decider's replica group
     const int rr = k * kRepBlock + lane;
     const long long limit = 2 * P.wait_clocks + kDrainClocks;   // beyond any chain's own bounded wait
-    const int n_tasks = P.queue ? P.n_units * ((P.nsweeps + P.chunk - 1) / P.chunk) : 1;
+    const int n_tasks = P.queue ? P.n_units * ((P.nsweeps - 1) / P.chunk + 1) : 1;
     // over all tasks: ring position, moves and deciders' meetings so far
     uint32_t slot = 0, phase = 0, issued = 0, moves = 0, meetings = 0;
     if (X > 1) cluster_sync();                       // every CTA of the cluster runs before the first remote store

@@ -212,8 +212,8 @@ int  pspin_pt_init(pspin_state* s, int NT, int nrep_per_temp, const double* beta
                    int pt_freq);
 /* Runs nsweeps sweeps; after every sweep whose 1-based index is a multiple
  * of pt_freq, proposes the NT-1 adjacent exchanges per replica column.  With
- * the plain move, no observer and graph_steps >= 0, up to 256 steps run inside
- * one sweep launch where every replica block is a whole sample (NT*nrep_per_temp
+ * the plain move, no observer and graph_steps >= 0, the steps of up to 256
+ * sweeps (one step at least) run inside one sweep launch where every replica block is a whole sample (NT*nrep_per_temp
  * <= 32 replicas_per_lane) or the lists are resident. */
 int  pspin_pt_run(pspin_state* s, int nsweeps);
 /* perm[NT*nrep_per_temp] (logical t*nrep+r -> physical replica) and the
