@@ -174,8 +174,8 @@ struct pspin_state {
     float2* d_spins = nullptr;
     double *d_E = nullptr, *d_beta = nullptr, *d_target = nullptr, *d_drift = nullptr, *d_e2 = nullptr,
            *d_e4 = nullptr;
-    double* d_epart = nullptr;          // per-CTA partial energies
-    int energy_splits = 1;
+    double* d_epart = nullptr;          // partial energies, by piece of a sample's table
+    int energy_pieces = 1;
     long long *d_acc = nullptr, *d_prop = nullptr;
     uint64_t* d_key = nullptr;
     int2* d_entries = nullptr;
@@ -751,7 +751,7 @@ static int run_energy(pspin_state* s, double* e2, double* e4, bool overwrite, bo
     p.drift = overwrite ? s->d_drift : nullptr;
     p.target = renorm ? s->d_target : nullptr;
     p.partial = s->d_epart;
-    p.max_splits = s->energy_splits;
+    p.max_pieces = s->energy_pieces;
     CK(launch_energy(p, (int)s->units.size(), s->max_N, s->st));
     s->kernel_launches += renorm ? 3 : 2;
     return PSPIN_OK;
@@ -1079,13 +1079,13 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         return bail(fail(PSPIN_ERR_ARG, "N=%d with %d replicas per lane needs more shared memory than a CTA has",
                          s->max_N, s->rpl));
 
-    s->energy_splits = energy_max_splits((int)s->units.size());
+    for (const SampleDev& d : s->sd) s->energy_pieces = std::max(s->energy_pieces, energy_max_pieces(d.nq));
     if ((rc = dalloc(&s->d_samples, n)) || (rc = dalloc(&s->d_units, s->units.size())) ||
         (rc = dalloc(&s->d_spins, (size_t)s->spin_total)) || (rc = dalloc(&s->d_E, s->R_tot)) ||
         (rc = dalloc(&s->d_beta, s->R_tot)) || (rc = dalloc(&s->d_target, s->R_tot)) ||
         (rc = dalloc(&s->d_drift, s->R_tot)) || (rc = dalloc(&s->d_e2, s->R_tot)) ||
         (rc = dalloc(&s->d_e4, s->R_tot)) ||
-        (rc = dalloc(&s->d_epart, energy_partial_doubles((int)s->units.size(), s->energy_splits))) || (rc = dalloc(&s->d_acc, s->R_tot)) ||
+        (rc = dalloc(&s->d_epart, energy_partial_doubles((int)s->units.size(), s->energy_pieces))) || (rc = dalloc(&s->d_acc, s->R_tot)) ||
         (rc = dalloc(&s->d_prop, s->R_tot)) || (rc = dalloc(&s->d_key, s->R_tot)) ||
         (rc = dalloc(&s->d_entries, (size_t)ent_total)) || (rc = dalloc(&s->d_site_chunks, (size_t)split_total)) ||
         (rc = dalloc(&s->d_chunk_start, (size_t)chunk_total + 1)) ||

@@ -188,11 +188,12 @@ struct EnergyParams {
     double* drift;            // |E_running - E_fp64| before the overwrite (when energy set)
     const double* target;     // constraint target per replica (renormalise when non-null)
     int renorm_only;          // 1: renormalise and return (energies come from elsewhere)
-    double* partial;          // [n_units][max_splits][32][2]: (e2, e4) of each CTA's share of the tables
-    int max_splits;           // most CTAs per unit
+    double* partial;          // [n_units][max_pieces][32][2]: (e2, e4) of each piece of the tables
+    int max_pieces;           // most pieces of a sample's table
+    int max_ctas, n_units;    // most CTAs per unit, units (set at the launch)
 };
-int energy_max_splits(int n_units);
-size_t energy_partial_doubles(int n_units, int max_splits);
+int energy_max_pieces(int64_t max_nq);
+size_t energy_partial_doubles(int n_units, int max_pieces);
 cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStream_t st);
 
 struct ExchangeParams {

@@ -66,28 +66,42 @@ __global__ void __launch_bounds__(256) renorm_kernel(const EnergyParams P) {
 // FP32 upcast at each use), so an entry is bound by its shared-memory reads
 // (16-byte broadcast + 512-byte row: 5 wavefronts a warp).
 //
-// Lanes are replicas; a unit's table is cut over `splits` CTAs of 8 warps, so
-// few units still fill the chip; each CTA writes one partial per replica and
-// energy_sum_kernel adds them in a fixed order.  768 units of a 256-sample
-// batch (N 24..64, fully connected, 96 replicas): 45 ms before, 5.5 ms now;
-// two units at N=128 (10.7 M entries): 728 ms before, 0.94 ms now.
+// Lanes are replicas; a unit's table is cut in pieces, each summed by the 8 warps
+// of a CTA into one partial per replica, and energy_sum_kernel adds the partials
+// in order.  The pieces follow from the sample alone, so its energies have the
+// same bits in any batch and on any device; how many CTAs share a unit's pieces
+// follows from the number of units, so few units still fill the chip.  The CTAs of
+// kEnergyGroup neighbouring units (of one sample, mostly) alternate, so that they
+// read a table that is larger than L2 together, and the heaviest units come first.
+// 768 units of a 256-sample batch (N 24..64, fully connected, 96 replicas): 45 ms
+// as one product per entry, 4.9 ms now; two units at N=128 (10.7 M entries): 728
+// and 0.89 ms.  (With 16 CTAs per SM and a unit's CTAs a grid apart: 5.7 and 0.89.)
 // ---------------------------------------------------------------------
 constexpr int kDoubleN = 192;      // amplitudes as double2 up to here: 96 KB of shared memory a CTA
 constexpr int kEnergyWarps = 8;
+constexpr int kMaxPieces = 256;
+constexpr int kEnergyGroup = 4;
 
-// CTAs sharing a sample's table: at least 1024 entries for each of their warps
-__host__ __device__ inline int energy_splits(int64_t nq, int max_splits) {
+// pieces of a sample's table: at least 1024 entries for each warp of a CTA
+__host__ __device__ inline int energy_pieces(int64_t nq) {
     const int64_t want = nq / (kEnergyWarps * 1024) + 1;
-    return (int)(want < max_splits ? want : max_splits);
+    return (int)(want < kMaxPieces ? want : kMaxPieces);
 }
 
-template <bool kDouble>
+// kOne: a CTA for every piece, where there are as many (with the loop's registers the
+// two units at N=128 took 0.99 ms)
+template <bool kDouble, bool kOne>
 __global__ void __launch_bounds__(32 * kEnergyWarps) energy_kernel(const EnergyParams P) {
     extern __shared__ __align__(16) unsigned char esm[];
-    const Unit U = P.units[blockIdx.x];
-    const SampleDev S = P.samples[U.sample];
-    const int splits = energy_splits(S.nq, P.max_splits), split = blockIdx.y;
-    if (split >= splits) return;
+    const int group = (int)(blockIdx.x / (kEnergyGroup * P.max_ctas)), in_group = (int)(blockIdx.x % (kEnergyGroup * P.max_ctas));
+    const int members = min(kEnergyGroup, P.n_units - group * kEnergyGroup);
+    const int unit = group * kEnergyGroup + in_group % members;
+    const Unit U = P.units[unit];
+    const SampleDev& S = P.samples[U.sample];       // (read again for every piece: few registers)
+    // this CTA's pieces: the same number for every CTA of the unit but the last
+    const int pieces = energy_pieces(S.nq), each = kOne ? 1 : (pieces + P.max_ctas - 1) / P.max_ctas;
+    const int first = in_group / members * each, end = min(pieces, first + each);
+    if (first >= end) return;
     const int N = S.N, R = S.R;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int nw = kEnergyWarps;
@@ -110,76 +124,80 @@ __global__ void __launch_bounds__(32 * kEnergyWarps) energy_kernel(const EnergyP
         return make_double2(v.x, v.y);
     };
 
-    double e2 = 0.0, e4 = 0.0;
-    if (S.h2_active) {
-        const int64_t npair = (int64_t)N * (N - 1) / 2;
-        for (int64_t pidx = split * nw + warp; pidx < npair; pidx += (int64_t)splits * nw) {
-            // pair index -> (i<j), row-major over j
-            int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)pidx)) * 0.5f);
-            while ((int64_t)j * (j - 1) / 2 > pidx) j--;
-            while ((int64_t)(j + 1) * j / 2 <= pidx) j++;
-            const int i = (int)(pidx - (int64_t)j * (j - 1) / 2);
-            const double g = __ldg(P.g2 + S.g2_off + (int64_t)i * N + j);
-            if (g == 0.0) continue;
-            const double2 ai = amp(i), aj = amp(j);
-            // -Re[g a_i conj(a_j)]
-            e2 -= g * (ai.x * aj.x + ai.y * aj.y);
-        }
-    }
-    // this warp's contiguous share of the table, 32 entries at a time: the
-    // next 32 are in flight while these are summed
-    const int64_t workers = (int64_t)splits * nw, me = (int64_t)split * nw + warp;
-    const int64_t t0 = S.nq * me / workers, t1 = S.nq * (me + 1) / workers;
-    const int4* __restrict__ Q = reinterpret_cast<const int4*>(P.quartets + S.q_off);
-    int4 mine = make_int4(0, 0, 0, 0);
-    if (t0 + lane < t1) mine = __ldg(Q + t0 + lane);
-    for (int64_t t = t0; t < t1; t += 32) {
-        const int n = (int)(t1 - t < 32 ? t1 - t : 32);
-        reinterpret_cast<int4*>(stage)[lane] = mine;
-        const int4 cur = mine;
-        if (t + 32 + lane < t1) mine = __ldg(Q + t + 32 + lane);
-        // starts of the runs of equal (j, k, l, ch)
-        const unsigned kl = (unsigned)cur.y, kj = (unsigned)cur.x >> 16;
-        const unsigned pkl = __shfl_up_sync(0xffffffffu, kl, 1), pkj = __shfl_up_sync(0xffffffffu, kj, 1);
-        unsigned starts = __ballot_sync(0xffffffffu, lane < n && (lane == 0 || kl != pkl || kj != pkj));
-        __syncwarp();
-        while (starts) {
-            const int b = __ffs(starts) - 1;
-            starts &= starts - 1;
-            const int e = starts ? __ffs(starts) - 1 : n;
-            double yx = 0.0, yy = 0.0;
-#pragma unroll 4
-            for (int u = b; u < e; u++) {
-                const Q64 q = stage[u];
-                const double2 a = amp(q.i);
-                yx = fma(q.g, a.x, yx);
-                yy = fma(q.g, a.y, yy);
+    for (int piece = first; piece < end; piece++) {
+        double e2 = 0.0, e4 = 0.0;
+        if (S.h2_active) {
+            const int64_t npair = (int64_t)N * (N - 1) / 2;
+            for (int64_t pidx = piece * nw + warp; pidx < npair; pidx += (int64_t)pieces * nw) {
+                // pair index -> (i<j), row-major over j
+                int j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)pidx)) * 0.5f);
+                while ((int64_t)j * (j - 1) / 2 > pidx) j--;
+                while ((int64_t)(j + 1) * j / 2 <= pidx) j++;
+                const int i = (int)(pidx - (int64_t)j * (j - 1) / 2);
+                const double g = __ldg(P.g2 + S.g2_off + (int64_t)i * N + j);
+                if (g == 0.0) continue;
+                const double2 ai = amp(i), aj = amp(j);
+                // -Re[g a_i conj(a_j)]
+                e2 -= g * (ai.x * aj.x + ai.y * aj.y);
             }
-            const Q64 q = stage[b];
-            const int ch = q.lch >> 14;
-            double2 aj = amp(q.j), ak = amp(q.k), al = amp(q.lch & 0x3FFF);
-            // conjugations: ch0 {k,l}, ch1 {j,k}, ch2 {j,l} (mc.cu:389-391)
-            if (ch != 0) aj.y = -aj.y;
-            if (ch != 2) ak.y = -ak.y;
-            if (ch != 1) al.y = -al.y;
-            const double bx = ak.x * al.x - ak.y * al.y, by = ak.x * al.y + ak.y * al.x;   // s2 s3
-            const double ax = yx * aj.x - yy * aj.y, ay = yx * aj.y + yy * aj.x;           // sum g s0 s1
-            e4 -= ax * bx - ay * by;
         }
-        __syncwarp();
-    }
-    double2* red = reinterpret_cast<double2*>(&stage_all[0][0]);          // [nw][32], each warp its own staging rows
-    red[warp * kRepBlock + lane] = make_double2(e2, e4);
-    __syncthreads();
-    if (warp == 0) {
-        double s2 = 0.0, s4 = 0.0;
-        for (int w = 0; w < nw; w++) {
-            const double2 v = red[w * kRepBlock + lane];
-            s2 += v.x;
-            s4 += v.y;
+        // this warp's contiguous share of the table, 32 entries at a time: the
+        // next 32 are in flight while these are summed
+        const int64_t workers = (int64_t)pieces * nw, me = (int64_t)piece * nw + warp;
+        const int64_t t0 = S.nq * me / workers, t1 = S.nq * (me + 1) / workers;
+        const int4* __restrict__ Q = reinterpret_cast<const int4*>(P.quartets + S.q_off);
+        int4 mine = make_int4(0, 0, 0, 0);
+        if (t0 + lane < t1) mine = __ldg(Q + t0 + lane);
+        for (int64_t t = t0; t < t1; t += 32) {
+            const int n = (int)(t1 - t < 32 ? t1 - t : 32);
+            reinterpret_cast<int4*>(stage)[lane] = mine;
+            const int4 cur = mine;
+            if (t + 32 + lane < t1) mine = __ldg(Q + t + 32 + lane);
+            // starts of the runs of equal (j, k, l, ch)
+            const unsigned kl = (unsigned)cur.y, kj = (unsigned)cur.x >> 16;
+            const unsigned pkl = __shfl_up_sync(0xffffffffu, kl, 1), pkj = __shfl_up_sync(0xffffffffu, kj, 1);
+            unsigned starts = __ballot_sync(0xffffffffu, lane < n && (lane == 0 || kl != pkl || kj != pkj));
+            __syncwarp();
+            while (starts) {
+                const int b = __ffs(starts) - 1;
+                starts &= starts - 1;
+                const int e = starts ? __ffs(starts) - 1 : n;
+                double yx = 0.0, yy = 0.0;
+#pragma unroll 4
+                for (int u = b; u < e; u++) {
+                    const Q64 q = stage[u];
+                    const double2 a = amp(q.i);
+                    yx = fma(q.g, a.x, yx);
+                    yy = fma(q.g, a.y, yy);
+                }
+                const Q64 q = stage[b];
+                const int ch = q.lch >> 14;
+                double2 aj = amp(q.j), ak = amp(q.k), al = amp(q.lch & 0x3FFF);
+                // conjugations: ch0 {k,l}, ch1 {j,k}, ch2 {j,l} (mc.cu:389-391)
+                if (ch != 0) aj.y = -aj.y;
+                if (ch != 2) ak.y = -ak.y;
+                if (ch != 1) al.y = -al.y;
+                const double bx = ak.x * al.x - ak.y * al.y, by = ak.x * al.y + ak.y * al.x;   // s2 s3
+                const double ax = yx * aj.x - yy * aj.y, ay = yx * aj.y + yy * aj.x;           // sum g s0 s1
+                e4 -= ax * bx - ay * by;
+            }
+            __syncwarp();
         }
-        double2* out = reinterpret_cast<double2*>(P.partial);             // [units][max_splits][32]
-        out[((int64_t)blockIdx.x * P.max_splits + split) * kRepBlock + lane] = make_double2(s2, s4);
+        double2* red = reinterpret_cast<double2*>(&stage_all[0][0]);          // [nw][32], each warp its own staging rows
+        red[warp * kRepBlock + lane] = make_double2(e2, e4);
+        __syncthreads();
+        if (warp == 0) {
+            double s2 = 0.0, s4 = 0.0;
+            for (int w = 0; w < nw; w++) {
+                const double2 v = red[w * kRepBlock + lane];
+                s2 += v.x;
+                s4 += v.y;
+            }
+            double2* out = reinterpret_cast<double2*>(P.partial);             // [units][max_pieces][32]
+            out[((int64_t)unit * P.max_pieces + piece) * kRepBlock + lane] = make_double2(s2, s4);
+        }
+        if (kOne) return;
+        __syncthreads();                                                       // the staging rows are the next piece's
     }
 }
 
@@ -188,11 +206,11 @@ __global__ void __launch_bounds__(kRepBlock) energy_sum_kernel(const EnergyParam
     const SampleDev S = P.samples[U.sample];
     const int lane = threadIdx.x;
     if (lane >= U.rep_count) return;
-    const int splits = energy_splits(S.nq, P.max_splits);
-    const double2* part = reinterpret_cast<const double2*>(P.partial) + (int64_t)blockIdx.x * P.max_splits * kRepBlock + lane;
+    const int pieces = energy_pieces(S.nq);
+    const double2* part = reinterpret_cast<const double2*>(P.partial) + (int64_t)blockIdx.x * P.max_pieces * kRepBlock + lane;
     double s2 = 0.0, s4 = 0.0;
 #pragma unroll 8
-    for (int q = 0; q < splits; q++) {
+    for (int q = 0; q < pieces; q++) {
         const double2 v = part[(int64_t)q * kRepBlock];
         s2 += v.x;
         s4 += v.y;
@@ -206,16 +224,17 @@ __global__ void __launch_bounds__(kRepBlock) energy_sum_kernel(const EnergyParam
     }
 }
 
-// most CTAs a unit's table is cut into: 16 CTAs per SM over all units
-int energy_max_splits(int n_units) {
+// most CTAs that share a unit's pieces: 32 CTAs per SM over all units
+static int energy_ctas(int n_units, int max_pieces) {
     int sms = 0, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         sms = 148;
-    const int want = n_units > 0 ? (16 * sms + n_units - 1) / n_units : 1;
-    return want < 1 ? 1 : (want > 256 ? 256 : want);
+    const int want = (32 * sms + n_units - 1) / n_units;
+    return want < 1 ? 1 : (want > max_pieces ? max_pieces : want);
 }
 
-size_t energy_partial_doubles(int n_units, int max_splits) { return (size_t)n_units * max_splits * kRepBlock * 2; }
+int energy_max_pieces(int64_t max_nq) { return energy_pieces(max_nq); }
+size_t energy_partial_doubles(int n_units, int max_pieces) { return (size_t)n_units * max_pieces * kRepBlock * 2; }
 
 cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStream_t st) {
     if (n_units <= 0) return cudaSuccess;
@@ -229,10 +248,15 @@ cudaError_t launch_energy(const EnergyParams& p, int n_units, int max_N, cudaStr
     }
     const bool dbl = max_N <= kDoubleN;
     const size_t smem = (size_t)max_N * kRepBlock * (dbl ? sizeof(double2) : sizeof(float2));
-    auto kern = dbl ? energy_kernel<true> : energy_kernel<false>;
+    EnergyParams q = p;
+    q.n_units = n_units;
+    q.max_ctas = energy_ctas(n_units, p.max_pieces);
+    const bool one = q.max_ctas >= p.max_pieces;
+    auto kern = one ? (dbl ? energy_kernel<true, true> : energy_kernel<false, true>)
+                    : (dbl ? energy_kernel<true, false> : energy_kernel<false, false>);
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    kern<<<dim3((unsigned)n_units, (unsigned)p.max_splits), 32 * kEnergyWarps, smem, st>>>(p);
+    kern<<<(unsigned)(n_units * q.max_ctas), 32 * kEnergyWarps, smem, st>>>(q);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     energy_sum_kernel<<<n_units, kRepBlock, 0, st>>>(p);
     return cudaGetLastError();
