@@ -164,6 +164,12 @@ struct pspin_state {
     int4* d_prep_moves = nullptr;       // the list-resident kernel's prepared moves (workspace)
     float* d_prep_trig = nullptr;
     int* d_queue = nullptr;             // task counter, then tasks finished per replica block
+    // the state that the tasks of a queued launch hand on (null: no launch is queued)
+    float2* d_mid_spins = nullptr;
+    double *d_mid_E = nullptr, *d_mid_beta = nullptr;
+    long long *d_mid_acc = nullptr, *d_mid_prop = nullptr, *d_mid_ex_acc = nullptr, *d_mid_ex_prop = nullptr;
+    int* d_mid_perm = nullptr;
+    unsigned long long* d_mid_drand = nullptr;
     int64_t spin_total = 0;
     cudaStream_t st = nullptr;
     int device = 0;
@@ -254,6 +260,7 @@ static void free_state(pspin_state* s) {
     void* ptrs[] = {s->d_samples, s->d_units, s->d_spins, s->d_E, s->d_beta, s->d_target, s->d_drift,
                     s->d_e2, s->d_e4, s->d_epart, s->d_acc, s->d_prop, s->d_key, s->d_entries, s->d_chunk_start, s->d_site_chunks,
                     s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status, s->d_queue, s->d_prep_moves, s->d_prep_trig,
+                    s->d_mid_spins, s->d_mid_perm,
                     s->d_beta_sched, s->d_perm, s->d_drand, s->d_ex_acc, s->d_ex_prop, s->d_trace,
                     s->d_tc_w, s->d_tc_x, s->d_tc_f, s->d_tc_ws, s->d_tc_h, s->d_f64_h, s->d_tc_e,
                     s->d_w32, s->d_adam_m, s->d_adam_v, s->d_grad, s->d_wbf, s->d_records, s->d_rec_count,
@@ -267,6 +274,34 @@ static void free_state(pspin_state* s) {
     }
     if (s->st) cudaStreamDestroy(s->st);
     delete s;
+}
+
+// One allocation cut in pieces: with a null base only their sizes are counted.
+struct Carve {
+    unsigned char* base;
+    size_t used = 0;
+    template <class T>
+    void take(T*& p, size_t n) {
+        p = base ? reinterpret_cast<T*>(base + used) : nullptr;
+        used += (n * sizeof(T) + 255) & ~(size_t)255;
+    }
+};
+
+// The arrays of queued launches.  More blocks than run at once are cut in tasks only
+// where these exist: fewer than this many blocks always run at once (148 SMs, clusters
+// of 16), and where the device has no room the launch goes on without tasks.
+constexpr int kQueueUnits = 8;
+template <class Lay>
+static void alloc_mid(Lay lay) {
+    Carve count{nullptr};
+    lay(count);
+    void* p = nullptr;
+    if (cudaMalloc(&p, count.used) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    Carve place{static_cast<unsigned char*>(p)};
+    lay(place);
 }
 
 constexpr size_t kPrepBytes = (size_t)64 << 20;      // workspace of the list-resident kernel's prepared moves
@@ -1095,6 +1130,13 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         (rc = dalloc(&s->d_status, 1)) || (rc = dalloc(&s->d_queue, s->units.size() + 1)) || (rc = dalloc(&s->d_units_k[0], s->units_k[0].size())) ||
         (rc = dalloc(&s->d_units_k[1], s->units_k[1].size())))
         return bail(rc);
+    if (s->units.size() > kQueueUnits)
+        alloc_mid([&](Carve& c) {
+            c.take(s->d_mid_spins, (size_t)s->spin_total);
+            c.take(s->d_mid_E, s->R_tot);
+            c.take(s->d_mid_acc, s->R_tot);
+            c.take(s->d_mid_prop, s->R_tot);
+        });
     auto up = [&](void* dst, const void* src, size_t bytes) -> int {
         if (!bytes) return PSPIN_OK;
         cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s->st);
@@ -1243,9 +1285,18 @@ static int enqueue_ring(pspin_state* s, SweepParams& p, int pt_slots) {
     const long long step = std::max(1, p.pt_freq), most = std::max(1, (1 << 30) / std::max(1, n_units));
     const long long per_task = step * std::max(2LL, (p.nsweeps + step * most - 1) / (step * most));
     p.chunk = (int)std::min<long long>(per_task, p.nsweeps);
-    if (n_units > plan.resident && p.nsweeps > p.chunk) {
+    if (n_units > plan.resident && p.nsweeps > p.chunk && s->d_mid_spins && (pt_slots == 0 || s->d_mid_perm)) {
         p.queue = s->d_queue;
         p.done = s->d_queue + 1;
+        p.mid_spins = s->d_mid_spins;
+        p.mid_energy = s->d_mid_E;
+        p.mid_accepted = s->d_mid_acc;
+        p.mid_proposed = s->d_mid_prop;
+        p.mid_beta = s->d_mid_beta;
+        p.mid_perm = s->d_mid_perm;
+        p.mid_drand = s->d_mid_drand;
+        p.mid_ex_acc = s->d_mid_ex_acc;
+        p.mid_ex_prop = s->d_mid_ex_prop;
         CK(cudaMemsetAsync(s->d_queue, 0, (size_t)(n_units + 1) * sizeof(int), s->st));
     }
     CK(launch_sweep_ring(p, plan, n_units, s->variant, s->max_N, s->rpl, pt_slots, s->st));
@@ -1835,6 +1886,8 @@ extern "C" int pspin_pt_init(pspin_state* s, int NT, int nrep, const double* bet
     cudaFree(s->d_ex_acc);
     cudaFree(s->d_ex_prop);
     s->d_beta_sched = nullptr; s->d_perm = nullptr; s->d_drand = nullptr; s->d_ex_acc = nullptr; s->d_ex_prop = nullptr;
+    cudaFree(s->d_mid_perm);
+    s->d_mid_perm = nullptr;
     s->pt_NT = NT;
     s->pt_nrep = nrep;
     s->pt_freq = pt_freq;
@@ -1843,6 +1896,14 @@ extern "C" int pspin_pt_init(pspin_state* s, int NT, int nrep, const double* bet
         (rc = dalloc(&s->d_drand, s->S)) || (rc = dalloc(&s->d_ex_acc, (size_t)s->S * (NT - 1))) ||
         (rc = dalloc(&s->d_ex_prop, (size_t)s->S * (NT - 1))))
         return rc;
+    if (s->units.size() > kQueueUnits)
+        alloc_mid([&](Carve& c) {
+            c.take(s->d_mid_perm, (size_t)s->S * NT * nrep);
+            c.take(s->d_mid_beta, s->R_tot);
+            c.take(s->d_mid_drand, s->S);
+            c.take(s->d_mid_ex_acc, (size_t)s->S * (NT - 1));
+            c.take(s->d_mid_ex_prop, (size_t)s->S * (NT - 1));
+        });
     std::vector<int> perm((size_t)s->S * NT * nrep);
     std::vector<unsigned long long> dr(s->S);
     std::vector<double> betas(s->R_tot);

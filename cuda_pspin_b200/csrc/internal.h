@@ -133,6 +133,15 @@ struct SweepParams {
     int n_units, chunk;
     int* queue;                       // null: one task, block b runs unit b / exec
     int* done;
+    // what a unit's tasks hand to its next one (null without a queue): a unit that
+    // aborts keeps the arrays below and above as they were before the launch
+    float2* mid_spins;
+    double* mid_energy;
+    long long *mid_accepted, *mid_proposed;
+    double* mid_beta;                 // ... with PT steps inside the launch
+    int* mid_perm;
+    unsigned long long* mid_drand;
+    long long *mid_ex_acc, *mid_ex_prop;
     // PT steps inside the launch (pt_freq > 0; every unit a whole sample):
     // exchange after every pt_freq sweeps
     int pt_freq, NT, nrep;

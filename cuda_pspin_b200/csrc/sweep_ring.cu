@@ -53,7 +53,8 @@
 //    next move.
 //  * All waits are bounded; a chain whose copy does not arrive sends a marked
 //    partial, so every CTA of the unit leaves at the same move, and nothing is
-//    written back.
+//    written back: a unit's tasks but the last hand their state on in arrays of
+//    their own.
 //  * FP32 amplitudes and fields; the running energy is FP64.
 #include <algorithm>
 
@@ -221,7 +222,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     int* pt_slot = reinterpret_cast<int*>(pt_seq + RT);               // [RT]
     int* pt_swaps = pt_slot + RT;                                     // [NT]
     __shared__ volatile int stop, gave_up;           // the unit aborts; a chain of this CTA gave up
-    __shared__ volatile int task_s;
+    __shared__ volatile int task_s, first_s;         // the task, its first sweep
     __shared__ __align__(8) uint64_t stall_bar;      // test hook: nothing arrives on it
 
     if (threadIdx.x == 0) {
@@ -280,8 +281,11 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     const Unit U = P.units[unit];
     const SampleDev S = P.samples[U.sample];
     const int N = S.N, R = S.R;
+    // a unit's first task reads the engine's state and its last one writes it
+    const bool head = first == 0;
+    if (threadIdx.x == 0) first_s = first;
     // amplitudes, energies and betas may have been written by another SM earlier in this launch: read past L1
-    load_block_amplitudes(sp, P.spins + S.spin_off + U.rep_begin, R, N, KB, U.rep_count);   // column k*32 + lane
+    load_block_amplitudes(sp, (head ? P.spins : P.mid_spins) + S.spin_off + U.rep_begin, R, N, KB, U.rep_count);   // column k*32 + lane
     for (int idx = threadIdx.x; idx < KB; idx += blockDim.x) sp[(size_t)N * KB + idx] = make_float2(1.f, 0.f);
     const long long sweep0 = sweep_base + first;
     const int steps = N / 2, total = nsweeps * steps;
@@ -305,21 +309,21 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     auto amp = [&](int site) -> float2& { return sp[(site * K + k) * kRepBlock + lane]; };
     uint64_t drand = 0;
     if (active) {
-        beta_d = __ldcg(P.beta + gr);
+        beta_d = __ldcg((head || per_exchange == 0 ? P.beta : P.mid_beta) + gr);
         beta = (float)beta_d;
         const uint64_t key = P.key[gr];
         k0 = (uint32_t)key;
         k1 = (uint32_t)(key >> 32);
-        E = __ldcg(P.energy + gr);
+        E = __ldcg((head ? P.energy : P.mid_energy) + gr);
     }
     if (decider && k == 0 && per_exchange > 0) {
-        const int* perm = P.perm + (int64_t)U.sample * RT;
+        const int* perm = (head ? P.perm : P.mid_perm) + (int64_t)U.sample * RT;
         for (int i = lane; i < RT; i += 32) pt_slot[i] = __ldcg(perm + i);
         for (int t = lane; t < P.NT; t += 32) {
             pt_sched[t] = P.beta_sched[t];
             pt_swaps[t] = 0;
         }
-        drand = __ldcg(P.drand_state + U.sample);
+        drand = __ldcg((head ? P.drand_state : P.mid_drand) + U.sample);
         if (P.nrep <= 32) drand_ahead(pt_seq, (P.NT - 1) * P.nrep, drand);
     }
     __syncthreads();
@@ -351,7 +355,8 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
 #pragma unroll
             for (int q = 0; q < K; q++) hx[q] = hy[q] = 0.f;
             bool ok = true;
-            if (m == P.stall_move) ok = stall_wait(&stall_bar, P.status, P.wait_clocks);
+            // test hook: the launch's move
+            if (P.stall_move >= 0 && (long long)first_s * steps + m == P.stall_move) ok = stall_wait(&stall_bar, P.status, P.wait_clocks);
             for (bool last = false; ok && !last;) {
                 ok = ring_wait(fb + slot, phase, P.status, P.wait_clocks);
                 if (!ok) break;
@@ -576,26 +581,31 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     const bool good = stop == 0;
     if (rank == 0) {
         if (good) {
+            const bool head = first_s == 0, tail = !P.queue || P.nsweeps - first_s <= P.chunk;
+            float2* spins = tail ? P.spins : P.mid_spins;
             for (int idx = threadIdx.x; idx < N * KB; idx += blockDim.x) {
                 const int site = idx / KB, r = idx % KB;
-                if (r < U.rep_count) P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + r] = sp[idx];
+                if (r < U.rep_count) spins[S.spin_off + (int64_t)site * R + U.rep_begin + r] = sp[idx];
             }
             if (active) {
-                P.energy[gr] = E;
-                __stcg(P.accepted + gr, __ldcg(P.accepted + gr) + nacc);
-                __stcg(P.proposed + gr, __ldcg(P.proposed + gr) + nprop);
-                if (per_exchange > 0) P.beta_out[gr] = beta_d;
+                (tail ? P.energy : P.mid_energy)[gr] = E;
+                const long long a = __ldcg((head ? P.accepted : P.mid_accepted) + gr);
+                const long long b = __ldcg((head ? P.proposed : P.mid_proposed) + gr);
+                __stcg((tail ? P.accepted : P.mid_accepted) + gr, a + nacc);
+                __stcg((tail ? P.proposed : P.mid_proposed) + gr, b + nprop);
+                if (per_exchange > 0) (tail ? P.beta_out : P.mid_beta)[gr] = beta_d;
             }
             if (decider && k == 0 && per_exchange > 0) {
-                int* perm = P.perm + (int64_t)U.sample * RT;
+                const int64_t at = (int64_t)U.sample * (P.NT - 1);
+                int* perm = (tail ? P.perm : P.mid_perm) + (int64_t)U.sample * RT;
                 for (int i = lane; i < RT; i += 32) perm[i] = pt_slot[i];
-                long long* acc = P.ex_acc + (int64_t)U.sample * (P.NT - 1);
-                long long* prop = P.ex_prop + (int64_t)U.sample * (P.NT - 1);
                 for (int t = lane; t < P.NT - 1; t += 32) {
-                    __stcg(acc + t, __ldcg(acc + t) + pt_swaps[t]);
-                    __stcg(prop + t, __ldcg(prop + t) + (long long)(total / per_exchange) * P.nrep);
+                    const long long a = __ldcg((head ? P.ex_acc : P.mid_ex_acc) + at + t);
+                    const long long b = __ldcg((head ? P.ex_prop : P.mid_ex_prop) + at + t);
+                    __stcg((tail ? P.ex_acc : P.mid_ex_acc) + at + t, a + pt_swaps[t]);
+                    __stcg((tail ? P.ex_prop : P.mid_ex_prop) + at + t, b + (long long)(total / per_exchange) * P.nrep);
                 }
-                if (lane == 0) P.drand_state[U.sample] = drand;
+                if (lane == 0) (tail ? P.drand_state : P.mid_drand)[U.sample] = drand;
             }
         }
         if (P.queue) {

@@ -1,0 +1,77 @@
+"""A wait that runs out in a launch whose replica blocks run as several tasks, or as
+a cluster of blocks that exchange: every block keeps its state from before the
+launch, with PT its permutation, counters and betas too.
+
+The waits are made to run out by the test option test_stall_move, within about a
+millisecond each; no GPU fault or endless wait is involved.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STALL_CLOCKS = 2_000_000        # ~1 ms at 1.9 GHz
+
+
+def _state(eng, samples, pt):
+    E, acc, prop = eng.get_results()
+    out = [np.concatenate([a.ravel() for a in eng.get_spins()]), E, acc, prop]
+    for k in range(samples if pt else 0):
+        out += [x.copy() for x in eng.pt_get(k)]
+    return out
+
+
+def _engine(ps, Ns, samples, NT, nrep, stall, pt, sparse=False, **opts):
+    cfgs = [ps.default_config(N=Ns[k % len(Ns)], nrep=NT * nrep, seed=40 + k, fmc_mode=1 if sparse else 0)
+            for k in range(samples)]
+    for c in cfgs:
+        c.gamma = 1.0 if sparse else c.gamma
+    eng = ps.Engine(cfgs, ps.PSPIN_SPARSE if sparse else ps.PSPIN_DENSE,
+                    ps.make_options(resync_every=-1, wait_limit_clocks=STALL_CLOCKS, test_stall_move=stall,
+                                    disorder_stream=sparse, **opts))
+    _, betas = ps.temperature_schedule(NT, 0.3, 1.5, True)
+    if pt:
+        eng.pt_init(NT, nrep, betas, 1)
+    else:
+        eng.set_betas(np.tile(np.repeat(betas, nrep), samples))
+    return eng
+
+
+@pytest.mark.parametrize("pt", [False, True])
+@pytest.mark.parametrize("Ns,samples,warps,cluster,lanes,stall", [
+    ((8,), 400, 8, 1, 3, 14),            # four moves a sweep, tasks of two sweeps: in the second task
+    ((8,), 400, 8, 4, 3, 21),            # in the third, on clusters
+    ((8, 20), 400, 8, 2, 3, 33),         # in the fifth of the small samples and the second of the large
+    ((8,), 400, 8, 1, 3, 24),            # at the launch's last move
+])
+def test_a_queued_launch_keeps_the_state_from_before_it(ps, Ns, samples, warps, cluster, lanes, stall, pt):
+    NT, nrep, sweeps = 24, 4, 6
+    opts = dict(warps_per_unit=warps, cluster_size=cluster, replicas_per_lane=lanes)
+    with _engine(ps, Ns, samples, NT, nrep, stall, pt, **opts) as eng:
+        run = eng.pt_run if pt else eng.sweep
+        before = _state(eng, samples, pt)
+        with pytest.raises(ps.PspinError) as ei:
+            run(sweeps)
+        assert ei.value.code == ps.PSPIN_ERR_TIMEOUT, str(ei.value)
+        after = _state(eng, samples, pt)
+        steps = np.repeat([Ns[k % len(Ns)] // 2 for k in range(samples)], NT * nrep)
+        reached = steps * sweeps >= stall                # the stall is a move of these samples' launch
+        assert np.array_equal(before[3][reached], after[3][reached])
+        if reached.all():
+            for a, b in zip(before, after):
+                np.testing.assert_array_equal(a, b)
+        e2, e4 = eng.split_energies()                    # the context works, energies and amplitudes agree
+        np.testing.assert_allclose(after[1], e2 + e4, rtol=0, atol=1e-4 * np.abs(e2 + e4).max())
+
+
+@pytest.mark.parametrize("pt", [False, True])
+def test_a_stall_beyond_the_launch_changes_nothing(ps, pt):
+    out = []
+    for stall in (0, 1000):
+        opts = dict(warps_per_unit=8, cluster_size=2, replicas_per_lane=3)
+        with _engine(ps, (8, 12), 300, 12, 4, stall, pt, **opts) as eng:
+            (eng.pt_run if pt else eng.sweep)(7)
+            out.append(_state(eng, 300, pt))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][2].sum() > 0
