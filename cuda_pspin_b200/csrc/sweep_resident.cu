@@ -32,6 +32,8 @@
 // consecutive commuting moves with a CTA barrier each, took 7500 cycles of
 // preparation a window and 8.6 batches of 1950 cycles: 118 us a sweep launch and
 // 25 us of exchange; now 91 us for both.
+#include <climits>
+
 #include "exchange.cuh"
 #include "sweep_common.cuh"
 #include "../../include/pspin.h"
@@ -62,6 +64,12 @@ __device__ __forceinline__ int peek(const int* p) { return *(const volatile int*
 __device__ __forceinline__ void publish(int* p, int v) {
     __threadfence_block();
     *(volatile int*)p = v;
+}
+
+// What a move waits for other moves and blocks (clocks): beyond any limit set for a
+// copy, but for the test hook.
+__device__ __forceinline__ long long resident_patience(const SweepParams& P) {
+    return P.stall_move >= 0 ? P.wait_clocks : 2 * P.wait_clocks + kDrainClocks;
 }
 
 // Fields of two sites from their record lists, four records of each at a time with
@@ -350,7 +358,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
     double E = 0.0;
     long long nacc = 0, nprop = 0;
     uint64_t drand = 0;
-    // until cond() holds, within the bounded wait
+    // until cond() holds, within a bound
     auto wait = [&](auto cond) {
         if (__all_sync(0xffffffffu, cond())) {
             __threadfence_block();
@@ -362,7 +370,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
                 __threadfence_block();
                 return true;
             }
-            const bool late = clock64() - t0 > P.wait_clocks;
+            const bool late = clock64() - t0 > resident_patience(P);
             if (__any_sync(0xffffffffu, late || stop != 0)) {
                 if (late) atomicOr(P.status, kStatusTimeout);
                 stop = 1;
@@ -418,7 +426,8 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
             // the earlier moves it does not commute with, and every move a ring ago;
             // this slot's last dE is accounted for
             const int last = m - 1 - ((t - 1 - lane) & (kRing - 1));
-            const int need = ((uint32_t)mv.y >> lane) & 1u ? last : last - kRing;
+            int need = ((uint32_t)mv.y >> lane) & 1u ? last : last - kRing;
+            if (m == P.stall_move && rank == (uint32_t)X - 1) need = INT_MAX;     // test hook, in one CTA of a cluster
             if (!wait([&]() { return peek(done + lane) >= need && peek(&counted) > m - kRing; })) break;
             const float2 ai = sp[i0 * kRepBlock + lane], aj = sp[j0 * kRepBlock + lane];
             float2 ain, ajn;
@@ -529,8 +538,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
                     const uint32_t dx = smem_u32(Ex + U.rep_begin + lane), db = smem_u32(ebar + par);
                     for (int q = 0; q < X; q++) st_async_f64(map_rank(dx, (uint32_t)q), E, map_rank(db, (uint32_t)q));
                 }
-                if (!__all_sync(0xffffffffu, mbar_wait(ebar + par, (uint32_t)(n_ex >> 1) & 1u, P.status,
-                                                       2 * P.wait_clocks + kDrainClocks))) {
+                if (!__all_sync(0xffffffffu, mbar_wait(ebar + par, (uint32_t)(n_ex >> 1) & 1u, P.status, resident_patience(P)))) {
                     stop = 1;
                     break;
                 }
@@ -561,7 +569,11 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
         }
     }
     __syncthreads();
-    if (X > 1) cluster_sync();                 // no store may still target a CTA that has gone
+    if (X > 1) {
+        if (stop && threadIdx.x == 0)          // a CTA that gave up takes its cluster, one PT sample, with it
+            for (int q = 0; q < X; q++) st_cluster_u32((const void*)&stop, (uint32_t)q, 1u);
+        cluster_sync();                        // no store may still target a CTA that has gone
+    }
     if (stop) return;                          // the block keeps its state from before the launch
     for (int idx = threadIdx.x; idx < N * kRepBlock; idx += blockDim.x) {
         const int site = idx >> 5, l = idx & 31;

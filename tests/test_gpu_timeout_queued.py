@@ -75,3 +75,36 @@ def test_a_stall_beyond_the_launch_changes_nothing(ps, pt):
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
     assert out[0][2].sum() > 0
+
+
+@pytest.mark.parametrize("warps", [2, 8])
+@pytest.mark.parametrize("samples,N,NT,nrep,stall,pt", [
+    (1, 96, 24, 4, 1, True), (3, 64, 24, 4, 70, True),       # three blocks a sample: one of a cluster gives up
+    (2, 48, 10, 17, 144, True),                              # six, a ragged last, at the launch's last move
+    (2, 48, 4, 8, 100, True), (3, 64, 10, 4, 33, False),     # one block; blocks of their own
+])
+def test_resident_blocks_of_a_sample_abort_together(ps, samples, N, NT, nrep, stall, pt, warps):
+    with _engine(ps, (N,), samples, NT, nrep, stall, pt, sparse=True, warps_per_unit=warps, cluster_size=-1) as eng:
+        before = _state(eng, samples, pt)
+        with pytest.raises(ps.PspinError) as ei:
+            (eng.pt_run if pt else eng.sweep)(6)
+        assert ei.value.code == ps.PSPIN_ERR_TIMEOUT, str(ei.value)
+        for a, b in zip(before, _state(eng, samples, pt)):
+            np.testing.assert_array_equal(a, b)
+
+
+def test_a_short_copy_limit_does_not_end_resident_moves(ps):
+    """Waits for earlier moves and for other blocks are not copies: a limit of a few
+    clocks leaves them alone."""
+    out = []
+    for limit in (0, 50):
+        cfgs = [ps.default_config(N=96, nrep=96, seed=3, fmc_mode=1)]
+        cfgs[0].gamma = 1.0
+        opts = ps.make_options(warps_per_unit=8, cluster_size=-1, disorder_stream=True, wait_limit_clocks=limit)
+        with ps.Engine(cfgs, ps.PSPIN_SPARSE, opts) as eng:
+            _, betas = ps.temperature_schedule(24, 0.3, 1.5, True)
+            eng.pt_init(24, 4, betas, 1)
+            eng.pt_run(20)
+            out.append(_state(eng, 1, True))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
