@@ -57,9 +57,10 @@ inline size_t resident_smem_bytes(int N, int64_t entries, int K, int R = 0) {
            (size_t)R * (6 * sizeof(double) + 2 * sizeof(int));
 }
 
-// A finished move or block: its writes, then the flag; a reader polls the flag
-// with plain loads and fences once (an acquire load per poll slowed the warps at
-// work).
+// A finished move or block: its warp's writes, a __syncwarp, then the flag by one
+// lane; a reader's lanes poll flags with plain loads, fence once (an acquire load
+// per poll slowed the warps at work) and meet in a __syncwarp, since each lane goes
+// on to read what others' flags stand for.
 __device__ __forceinline__ int peek(const int* p) { return *(const volatile int*)p; }
 __device__ __forceinline__ void publish(int* p, int v) {
     __threadfence_block();
@@ -362,12 +363,14 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
     auto wait = [&](auto cond) {
         if (__all_sync(0xffffffffu, cond())) {
             __threadfence_block();
+            __syncwarp();
             return true;
         }
         const long long t0 = clock64();
         for (;;) {
             if (__all_sync(0xffffffffu, cond())) {
                 __threadfence_block();
+                __syncwarp();
                 return true;
             }
             const bool late = clock64() - t0 > resident_patience(P);
@@ -483,6 +486,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
             }
             dEx[t * kRepBlock + lane] = dE;
             const unsigned yes = __ballot_sync(0xffffffffu, accept);
+            __syncwarp();                          // a vote orders no memory
             if (lane == 0) {
                 acx[t] = yes;
                 publish(done + t, m);
@@ -527,7 +531,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
             }
             nprop++;
             __syncwarp();
-            if (lane == 0) *(volatile int*)&counted = m + 1;   // (this slot's values have been read)
+            if (lane == 0) publish(&counted, m + 1);          // (this slot's values have been read)
             if (per_exchange == 0 || --to_exchange > 0) continue;
             to_exchange = per_exchange;
             const int par = n_ex & 1;
