@@ -390,6 +390,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         const bool grouped = c % W == 0;
         const int msgs = ring_messages(W, C, c), local = grouped ? c / W : c;
         int to_exchange = per_exchange;
+        bool lost = false;                           // a meeting with the other deciders failed
         for (int m = 0; m < total; m++, moves++) {
             const uint32_t par = moves & 1u;
             uint64_t* bar = xbar + par * K + k;
@@ -404,7 +405,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 naj = amp(nj0);
                 draw(m + 1);
             }
-            bool ok = __all_sync(0xffffffffu, mbar_wait(cbar, moves & 1u, P.status, limit) && gave_up == 0);
+            bool ok = __all_sync(0xffffffffu, mbar_wait(cbar, moves & 1u, P.status, limit) && gave_up == 0) && !lost;
             const float2* mine = part + k * kRepBlock + lane;
             int gw = W;                              // values per group still to be summed
             if (X > 1) {
@@ -420,7 +421,9 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                         st_async_f2(map_rank(dx + u * (uint32_t)(KB * sizeof(float2)), (uint32_t)q), v,
                                     map_rank(db, (uint32_t)q));
                 }
-                ok = ok && __all_sync(0xffffffffu, mbar_wait(bar, (moves >> 1) & 1u, P.status, limit));
+                // (a CTA that gives up, too, waits for what is on its way to it)
+                const bool came = __all_sync(0xffffffffu, mbar_wait(bar, (moves >> 1) & 1u, P.status, limit));
+                ok = ok && came;
                 mine = xbuf + (par * msgs * K + k) * kRepBlock + lane;
                 if (grouped) gw = 1;
             }
@@ -493,14 +496,11 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 bool met = meet();
                 if (k == 0 && met) drand = ring_exchange(pt_E, RT, P.NT, P.nrep, drand);
                 met = meet() && met;
-                if (!met) {                          // (a wait ran out: the chains stop at the move after the next)
-                    stop = 1;
-                    __threadfence_block();
-                    __syncwarp();
-                    if (m + 2 < total) state_arrive(state_threads);
-                    break;
-                }
-                if (active) {
+                if (!met) {                          // a wait ran out: the next move's messages say so
+                    lost = true;
+                    if (m + 1 < total) gave_up = 1;
+                    else stop = 1;
+                } else if (active) {
                     beta_d = pt_beta[rr];
                     beta = (float)beta_d;
                 }

@@ -108,3 +108,19 @@ def test_a_short_copy_limit_does_not_end_resident_moves(ps):
             out.append(_state(eng, 1, True))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("pt", [False, True])
+@pytest.mark.parametrize("samples,warps,cluster,lanes", [(1, 8, 1, 1), (1, 2, 16, 1), (2, 8, 4, 3), (60, 8, 1, 3)])
+@pytest.mark.parametrize("stall", [1, 7, 24])            # the first move, one between, the last
+def test_every_block_of_a_launch_gives_up_at_any_move(ps, samples, warps, cluster, lanes, stall, pt):
+    """One task a block, on one CTA and on clusters."""
+    opts = dict(warps_per_unit=warps, cluster_size=cluster, replicas_per_lane=lanes)
+    with _engine(ps, (8,), samples, 6, 4, stall, pt, **opts) as eng:
+        before = _state(eng, samples, pt)
+        for _ in range(2):
+            with pytest.raises(ps.PspinError) as ei:
+                (eng.pt_run if pt else eng.sweep)(6)
+            assert ei.value.code == ps.PSPIN_ERR_TIMEOUT, str(ei.value)
+            for a, b in zip(before, _state(eng, samples, pt)):
+                np.testing.assert_array_equal(a, b)
