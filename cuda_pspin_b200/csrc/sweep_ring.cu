@@ -124,6 +124,16 @@ __device__ __forceinline__ void state_wait(int threads) {
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
+// named barrier 2: chain warps and deciders arrive as they leave a task, the producer waits
+__device__ __forceinline__ void left_arrive(int threads) {
+    __syncwarp();
+    asm volatile("bar.arrive 2, %0;" ::"r"(threads) : "memory");
+}
+__device__ __forceinline__ void left_wait(int threads) {
+    __syncwarp();
+    asm volatile("bar.sync 2, %0;" ::"r"(threads) : "memory");
+}
+
 // Partial fields from buf[q * group + w * stride] in tree order: a CTA's W
 // chains, then the C CTAs.  Eight loads in flight before their additions.
 // `ok` is cleared where a value is marked.
@@ -384,6 +394,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
             __syncwarp();
             if (lane == 0) mbar_arrive(cbar);
         }
+        left_arrive(state_threads + 32);
     } else if (decider) {
         // ------------------------------------------------------------ decider
         const int W = P.warps, C = P.cluster;
@@ -506,6 +517,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 }
             }
         }
+        left_arrive(state_threads + 32);
     } else if (warp == c + K) {
         // ------------------------------------------------------------ producer: lane = chain of this CTA
         // chain g of the move: the groups alternate between the lists, group 2q
@@ -564,8 +576,11 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
             }
             if (!__any_sync(0xffffffffu, did)) __nanosleep(40);
         }
-        // copies still in flight after an abort (each slot's last one): none may
-        // land after the CTA has gone
+        // copies still in flight after an abort (each slot's last one): none may land
+        // after the CTA has gone.  The producer may have issued its last copies long
+        // before, so it looks once the other warps have left (an abort that another
+        // CTA makes known later still finds every copy of this one read).
+        left_wait(state_threads + 32);
         if (mine && stop)
             for (uint32_t q = 0; q < (uint32_t)stages && q < issued; q++) {
                 const uint32_t i = issued - 1 - q;
