@@ -1225,15 +1225,21 @@ static int n_units_of(const pspin_state* s, int K) {
 static const Unit* units_dev(const pspin_state* s, int K) { return K > 1 ? s->d_units_k[K - 2] : s->d_units; }
 
 // How the current block shape's chains are spread over the machine, in launches
-// without (pt_slots 0) or with exchanges inside.
-static int current_plan(pspin_state* s, int pt_slots) {
+// without (pt_slots 0) or with exchanges inside; false where it does not fit.
+static bool find_plan(pspin_state* s, int pt_slots) {
     const int w = pt_slots > 0, key[4] = {s->warps, s->cluster, s->rpl, pt_slots};
-    if (std::memcmp(key, s->plan_key[w], sizeof(key)) == 0) return PSPIN_OK;
-    if (!plan_sweep_ring(s->plan[w], s->warps, s->cluster, n_units_of(s, s->rpl), s->variant, s->max_N, s->rpl, pt_slots))
-        return fail(PSPIN_ERR_CUDA, "block shape %d warps x %d CTAs with %d replicas per lane does not fit at N=%d", s->warps,
-                    s->cluster, s->rpl, s->max_N);
-    std::memcpy(s->plan_key[w], key, sizeof(key));
-    return PSPIN_OK;
+    if (std::memcmp(key, s->plan_key[w], sizeof(key)) != 0) {
+        if (!plan_sweep_ring(s->plan[w], s->warps, s->cluster, n_units_of(s, s->rpl), s->variant, s->max_N, s->rpl, pt_slots))
+            s->plan[w] = RingPlan{};
+        std::memcpy(s->plan_key[w], key, sizeof(key));
+    }
+    return s->plan[w].exec > 0;
+}
+
+static int current_plan(pspin_state* s, int pt_slots) {
+    if (find_plan(s, pt_slots)) return PSPIN_OK;
+    return fail(PSPIN_ERR_CUDA, "block shape %d warps x %d CTAs with %d replicas per lane does not fit at N=%d", s->warps,
+                s->cluster, s->rpl, s->max_N);
 }
 
 // Enqueues one step: a sweep launch of nsweeps sweeps, the exchange launch
@@ -1412,13 +1418,13 @@ static int account_steps(pspin_state* s, int steps, int nsweeps, bool exchange) 
 }
 
 // Whether PT steps run inside one sweep launch: the plain sweep, with every sample
-// one replica block (ring-fed) or one cluster of blocks (list-resident), and
-// nothing recorded between steps.
-static bool steps_in_launch(const pspin_state* s) {
+// one replica block (ring-fed) or one cluster of blocks (list-resident), nothing
+// recorded between steps, and room for the exchange's arrays beside the sweep's.
+static bool steps_in_launch(pspin_state* s) {
     if (s->proposal != PSPIN_PROPOSAL_PLAIN || s->obs_cap != 0 || s->profiling) return false;
-    if (s->cluster > 0) return n_units_of(s, s->rpl) == s->S;
-    // list-resident: the blocks of a sample as one cluster (every sample has NT*nrep replicas)
     const int slots = s->pt_NT * s->pt_nrep;
+    if (s->cluster > 0) return n_units_of(s, s->rpl) == s->S && find_plan(s, slots);
+    // list-resident: the blocks of a sample as one cluster (every sample has NT*nrep replicas)
     return s->warps > 1 && slots <= 8 * kRepBlock && resident_chunk(s) >= s->pt_freq &&
            resident_smem_bytes_host(s->max_N, s->max_site_entries, s->warps, slots) <= 227 * 1024 - 64;
 }

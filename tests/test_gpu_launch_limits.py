@@ -1,0 +1,46 @@
+"""Limits of one sweep launch: how many sweeps pspin_pt_run puts into it, and block
+shapes near the shared-memory limit.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("freq,nsweeps,launches", [(1, 300, 2), (100, 600, 3), (300, 900, 3)])
+def test_a_launch_holds_at_most_256_sweeps_or_one_step(freq, nsweeps, launches):
+    """The length of a launch, and with it the number of its moves (31 bits), is
+    bounded by its sweeps, not by its PT steps: 256 sweeps, or one step."""
+    import cuda_pspin_b200 as ps
+    NT, nrep = 2, 3
+    c = ps.default_config(N=8, nrep=NT * nrep, seed=5)
+    with ps.Engine(c, ps.PSPIN_DENSE, ps.make_options(resync_every=-1)) as eng:
+        _, betas = ps.temperature_schedule(NT, 0.3, 1.5, True)
+        eng.pt_init(NT, nrep, betas, freq)
+        eng.get_profile()
+        eng.pt_run(nsweeps)
+        assert eng.get_profile()[1] == launches
+        perm, acc, prop = eng.pt_get(0)
+        assert np.all(prop == nsweeps // freq * nrep)
+        assert np.all(eng.get_results()[2] == nsweeps * 4)
+
+
+@pytest.mark.parametrize("N,NT,nrep,lanes", [(288, 24, 4, 3), (291, 24, 4, 3), (437, 16, 4, 2), (880, 8, 4, 1)])
+def test_steps_whose_exchange_does_not_fit_the_launch(N, NT, nrep, lanes):
+    """Block shapes that hold a sample's amplitudes but not the exchange's arrays
+    beside them run one step a launch, with the same results."""
+    import cuda_pspin_b200 as ps
+    out = []
+    for graph_steps in (0, -1):
+        c = ps.default_config(N=N, nrep=NT * nrep, seed=7, fmc_mode=1)
+        c.gamma = 1.0
+        opts = ps.make_options(warps_per_unit=1, cluster_size=1, replicas_per_lane=lanes, graph_steps=graph_steps,
+                               disorder_stream=True)
+        with ps.Engine(c, ps.PSPIN_SPARSE, opts) as eng:
+            _, betas = ps.temperature_schedule(NT, 0.3, 1.5, True)
+            eng.pt_init(NT, nrep, betas, 1)
+            eng.pt_run(3)
+            out.append([eng.get_spins()[0], *eng.get_results(), *eng.pt_get(0)])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
+    assert out[0][2].sum() > 0
