@@ -792,8 +792,6 @@ static int run_energy(pspin_state* s, double* e2, double* e4, bool overwrite, bo
     return PSPIN_OK;
 }
 
-static int current_plan(pspin_state* s, int pt_slots);
-
 extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, const pspin_options* opt,
                                   pspin_state** out) {
     if (!cfgs || n <= 0 || !out) return fail(PSPIN_ERR_ARG, "pspin_create_batch: bad arguments");
@@ -1110,7 +1108,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
     }
     if (sweep_smem_bytes(s->max_N, s->warps) > 227 * 1024)
         return bail(fail(PSPIN_ERR_ARG, "N=%d needs more shared memory than a CTA has", s->max_N));
-    if (s->rpl > 1 && s->cluster >= 1 && current_plan(s, 0) != PSPIN_OK)
+    if (s->rpl > 1 && s->cluster >= 1 && !ring_shape_fits(s->warps, s->cluster, s->max_N, s->rpl))
         return bail(fail(PSPIN_ERR_ARG, "N=%d with %d replicas per lane needs more shared memory than a CTA has",
                          s->max_N, s->rpl));
 

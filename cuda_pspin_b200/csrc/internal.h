@@ -171,6 +171,8 @@ struct RingPlan {
     int exec, chains, stages, lat, resident;
 };
 constexpr size_t kRingSmemMax = 227 * 1024 - 64;   // (the kernel's static shared memory)
+// whether any spread of the block shape's chains has the shared memory it needs
+bool ring_shape_fits(int warps, int cluster, int max_N, int K);
 // pt_slots: replicas per unit that exchange inside the launch (0: none)
 bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int variant, int max_N, int K, int pt_slots);
 

@@ -682,6 +682,18 @@ static cudaError_t ring_dispatch(SweepParams p, const RingPlan& r, int n_units, 
 #undef PSPIN_RING
 }
 
+static bool ring_fits(int max_N, int warps, int cluster, int X, int stages, int K, int pt_slots) {
+    return ring_layout(max_N, warps, cluster, 2 * cluster * warps / X, stages, K, pt_slots).total <= kRingSmemMax;
+}
+
+bool ring_shape_fits(int warps, int cluster, int max_N, int K) {
+    if (warps < 1 || cluster < 1 || cluster > 16 || kSplit % (cluster * warps) != 0 || K < 1 || K > 3) return false;
+    const int T = 2 * cluster * warps;
+    for (int X = T > kMaxChains ? T / kMaxChains : 1; X <= 16 && X <= T; X *= 2)
+        if (ring_fits(max_N, warps, cluster, X, 2, K, 0)) return true;
+    return false;
+}
+
 // Spreads the 2*C*W chains of a unit's move over X CTAs.  16 chains fill an SM
 // (four per sub-partition); with few units the chains go to more CTAs, down to
 // one chain per sub-partition, as long as all clusters are resident at once: a
@@ -695,7 +707,7 @@ bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int varia
     p.cluster = cluster;
     auto resident = [&](int X, int stages, int lat) {
         if (X > 16 || X > T || T / X > kMaxChains || (lat && T / X > kLatChains)) return 0;
-        if (ring_layout(max_N, warps, cluster, T / X, stages, K, pt_slots).total > kRingSmemMax) return 0;
+        if (!ring_fits(max_N, warps, cluster, X, stages, K, pt_slots)) return 0;
         const RingPlan q{X, T / X, stages, lat, 0};
         int n = 0;
         if (ring_dispatch(p, q, n_units, variant, max_N, K, pt_slots, nullptr, &n) != cudaSuccess) {

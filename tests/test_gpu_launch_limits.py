@@ -44,3 +44,22 @@ def test_steps_whose_exchange_does_not_fit_the_launch(N, NT, nrep, lanes):
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
     assert out[0][2].sum() > 0
+
+
+@pytest.mark.parametrize("N,warps,cluster,lanes,fits", [(291, 1, 1, 3, True), (292, 1, 1, 3, False), (439, 1, 1, 2, True),
+                                                        (440, 1, 1, 2, False), (211, 2, 16, 3, True), (212, 2, 16, 3, False),
+                                                        (234, 8, 4, 3, True), (235, 8, 4, 3, False)])
+def test_the_largest_N_of_a_block_shape_is_accepted_and_runs(N, warps, cluster, lanes, fits):
+    """What set-up accepts by the sizes alone, the sweep runs; the next N is refused."""
+    import cuda_pspin_b200 as ps
+    c = ps.default_config(N=N, nrep=8, seed=7, fmc_mode=1)
+    c.gamma = 1.0
+    opts = ps.make_options(warps_per_unit=warps, cluster_size=cluster, replicas_per_lane=lanes, disorder_stream=True)
+    if not fits:
+        with pytest.raises(ps.PspinError):
+            ps.Engine(c, ps.PSPIN_SPARSE, opts)
+        return
+    with ps.Engine(c, ps.PSPIN_SPARSE, opts) as eng:
+        eng.fill_betas(1.0)
+        eng.sweep(1)
+        assert np.all(eng.get_results()[2] == N // 2)
