@@ -45,9 +45,8 @@ struct LearnParams {
     int rec_cap;
     float rec_prob;
 };
-cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, int n_units, int max_N, cudaStream_t st,
-                                 int* max_clusters);
-size_t learned_smem_bytes_host(int N, int warps, int C);
+cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, const LearnPlan& r, int n_units, int max_N,
+                                 cudaStream_t st);
 cudaError_t launch_mlp_train(float* w, const float* records, unsigned long long filled, uint64_t key, uint32_t step,
                              int n, float* partial, float* loss, float* grad, float* m, float* v, __nv_bfloat16* wbf,
                              float lr, int adam_step, cudaStream_t st);
@@ -161,6 +160,8 @@ struct pspin_state {
     // (plan_key: warps, cluster, rpl, exchanging replicas it was made for)
     RingPlan plan[2] = {};
     int plan_key[2][4] = {};
+    LearnPlan plan2 = {};               // of warps2, cluster2 (plan2_key)
+    int plan2_key[2] = {};
     int4* d_prep_moves = nullptr;       // the list-resident kernel's prepared moves (workspace)
     float* d_prep_trig = nullptr;
     int* d_queue = nullptr;             // task counter, then tasks finished per replica block
@@ -1240,6 +1241,18 @@ static int current_plan(pspin_state* s, int pt_slots) {
                 s->cluster, s->rpl, s->max_N);
 }
 
+// the same of the two-pass sweep
+static int current_plan2(pspin_state* s) {
+    if (s->plan2_key[0] != s->warps2 || s->plan2_key[1] != s->cluster2) {
+        if (!plan_learned_sweep(s->plan2, s->warps2, s->cluster2, (int)s->units.size(), s->max_N)) s->plan2 = LearnPlan{};
+        s->plan2_key[0] = s->warps2;
+        s->plan2_key[1] = s->cluster2;
+    }
+    if (s->plan2.exec > 0) return PSPIN_OK;
+    return fail(PSPIN_ERR_CUDA, "block shape %d warps x %d CTAs of the two-pass sweep does not fit at N=%d", s->warps2,
+                s->cluster2, s->max_N);
+}
+
 // Enqueues one step: a sweep launch of nsweeps sweeps, the exchange launch
 // (which advances the device sweep counter) and, after an exchange, the
 // observable recorder.  No host bookkeeping, so a sequence of steps can be
@@ -1370,7 +1383,8 @@ static int enqueue_step(pspin_state* s, int nsweeps, bool exchange, cudaEvent_t 
         lp.rec_count = s->d_rec_count;
         lp.rec_cap = s->rec_cap;
         lp.rec_prob = s->rec_prob;
-        CK(launch_learned_sweep(p, lp, (int)s->units.size(), s->max_N, s->st, nullptr));
+        TRY(current_plan2(s));
+        CK(launch_learned_sweep(p, lp, s->plan2, (int)s->units.size(), s->max_N, s->st));
     }
     if (e1) CK(cudaEventRecord(e1, s->st));
     TRY(enqueue_counter(s, nsweeps, exchange));
@@ -1480,6 +1494,7 @@ static int graph_steps(const pspin_state* s) {
 static int capture_graph(pspin_state* s, int G) {
     drop_graph(s);
     if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0) TRY(current_plan(s, 0));
+    if (s->proposal != PSPIN_PROPOSAL_PLAIN) TRY(current_plan2(s));
     if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1) TRY(ensure_prep(s));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
@@ -1579,18 +1594,8 @@ static bool shape_fits(pspin_state* s, int warps, int cluster, int K = 1) {
         return plan_sweep_ring(r, warps, cluster, n_units_of(s, K), s->variant, s->max_N, K, 0);
     }
     if (K > 1) return false;
-    if (learned_smem_bytes_host(s->max_N, warps, cluster) > 227 * 1024) return false;
-    if (cluster == 1) return true;
-    SweepParams p{};
-    p.warps = warps;
-    p.cluster = cluster;
-    LearnParams lp{};
-    int n = 0;
-    if (launch_learned_sweep(p, lp, (int)s->units.size(), s->max_N, s->st, &n) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return n > 0;
+    LearnPlan r;
+    return plan_learned_sweep(r, warps, cluster, (int)s->units.size(), s->max_N);
 }
 
 // Times `sweeps` sweeps (no exchange) for every block shape -- CTAs per

@@ -180,6 +180,12 @@ bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int varia
 // units of up to 32K replicas, K = 1, 2, 3 replicas per lane
 cudaError_t launch_sweep_ring(const SweepParams& p, const RingPlan& r, int n_units, int variant, int max_N, int K,
                               int pt_slots, cudaStream_t st);
+// How the two-pass sweep spreads a unit's chains: `chains` of them on each of exec
+// CTAs; one: every CTA has an SM to itself.
+struct LearnPlan {
+    int exec, chains, one;
+};
+bool plan_learned_sweep(LearnPlan& r, int warps, int cluster, int n_units, int max_N);
 // the list-resident kernel; warps > 1 runs moves that commute (no site of one in
 // the other's quartet neighbourhood, by the neighbour masks `nbmask`) at once, on
 // clusters of p.exec units; pt_slots: replicas that exchange inside the launch

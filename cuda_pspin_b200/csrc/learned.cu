@@ -178,16 +178,6 @@ struct LearnLayout {
     }
 };
 
-// shared memory of the block shape as one CTA (cluster of CTAs) per replica block
-// had it; which shapes are accepted goes by this
-inline size_t learned_smem_bytes(int N, int warps, int C = 1) {
-    const size_t base = (size_t)(N + 1) * kRepBlock * sizeof(float2) + (size_t)warps * kRepBlock * sizeof(float4) +
-                        (size_t)warps * kLStages * kStage * sizeof(int2) + (size_t)warps * kLStages * sizeof(uint64_t) +
-                        (size_t)2 * kMlpBufWords * sizeof(uint32_t) + (size_t)kXchRows * kRepBlock * sizeof(float);
-    if (C > 1) return ((base + 15) & ~(size_t)15) + (size_t)2 * C * kRepBlock * sizeof(float4) + 16;
-    return base;
-}
-
 // A warp's stream of chunks: per move its share of the sites' lists (pass 0), then of
 // the pair's sub-lists (pass 1); in each, its one or two chains (list, part range).
 struct LearnStream {
@@ -586,72 +576,84 @@ __global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
     if (CL) cluster_sync();                    // no CTA leaves while a remote store may target it
 }
 
-size_t learned_smem_bytes_host(int N, int warps, int C) { return learned_smem_bytes(N, warps, C); }
+using LearnKernel = void (*)(const SweepParams, const LearnParams);
+static LearnKernel learned_kernel(const LearnPlan& r) {
+    return r.exec > 1 ? (r.one ? learned_sweep_kernel<true, true> : learned_sweep_kernel<true, false>)
+                      : (r.one ? learned_sweep_kernel<false, true> : learned_sweep_kernel<false, false>);
+}
 
-// max_clusters != null: reports how many replica blocks of this shape can be
-// resident instead of launching (0: the shape does not fit)
-cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, int n_units, int max_N,
-                                 cudaStream_t st, int* max_clusters) {
-    if (n_units <= 0) return cudaSuccess;
-    if (p.pair_chunks == nullptr && max_clusters == nullptr) return cudaErrorInvalidValue;
-    const int C = p.cluster > 1 ? p.cluster : 1, all = 2 * C * p.warps;
-    if (C > 16 || (kSplit % (C * p.warps)) != 0) return cudaErrorInvalidValue;
+// The launch of a plan; `attr` is its cluster dimension.
+static cudaError_t learned_config(const LearnPlan& r, int all, int n_units, int max_N, cudaStream_t st,
+                                  cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
+    const size_t smem = LearnLayout(max_N, all, r.exec, r.chains).total;
+    const LearnKernel kern = learned_kernel(r);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && r.exec > 8)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3((unsigned)(n_units * r.exec));
+    cfg.blockDim = dim3((unsigned)(32 * kLWarps));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    attr->id = cudaLaunchAttributeClusterDimension;
+    attr->val.clusterDim.x = (unsigned)r.exec;
+    attr->val.clusterDim.y = 1;
+    attr->val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = r.exec > 1 ? 1 : 0;
+    return e;
+}
+
+// As many CTAs per replica block as the blocks can all have at once with an SM
+// for each CTA (8 at most, no more than there are chains), and no fewer than the
+// shape has: chains on more SMs finish sooner, a second wave costs twice.  A move
+// of 24 blocks at N = 64 (gamma = 0.1, 8 warps x 2 CTAs) took 128 us on 2 CTAs
+// each, 84 on 6 (144 CTAs, but clusters of 6 do not tile the chip: two waves), 46
+// on the most that run at once; of 3 blocks 117 and 41 (8 CTAs); of 12 fully
+// connected blocks at N = 48 (one CTA's shape) 113 and 53.  Where the shape's own
+// CTAs are too few for the amplitudes beside their lists' share, the fewest that do.
+bool plan_learned_sweep(LearnPlan& r, int warps, int cluster, int n_units, int max_N) {
+    const int C = cluster > 1 ? cluster : 1, all = 2 * C * warps;
+    if (warps < 1 || n_units < 1 || C > 16 || kSplit % (C * warps) != 0) return false;
     int dev = 0, sms = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    SweepParams q = p;
-    q.cluster = C;
-    void (*kern)(const SweepParams, const LearnParams) = nullptr;
-    // As many CTAs per replica block as the blocks can all have at once with an SM
-    // for each CTA (8 at most, no more than there are chains), and no fewer than the
-    // shape has: chains on more SMs finish sooner, a second wave costs twice.  A move
-    // of 24 blocks at N = 64 (gamma = 0.1, 8 warps x 2 CTAs) took 128 us on 2 CTAs
-    // each, 84 on 6 (144 CTAs, but clusters of 6 do not tile the chip: two waves), 46
-    // on the most that run at once; of 3 blocks 117 and 41 (8 CTAs); of 12 fully
-    // connected blocks at N = 48 (one CTA's shape) 113 and 53.
-    auto prepare = [&](int X, cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int* clusters) -> cudaError_t {
-        q.exec = X;
-        q.chains = (all + X - 1) / X;
-        const size_t smem = LearnLayout(max_N, all, X, q.chains).total;
-        const bool one = (long long)n_units * X <= sms;
-        kern = X > 1 ? (one ? learned_sweep_kernel<true, true> : learned_sweep_kernel<true, false>)
-                     : (one ? learned_sweep_kernel<false, true> : learned_sweep_kernel<false, false>);
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess && X > 8)
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return e;
-        cfg = cudaLaunchConfig_t{};
-        cfg.gridDim = dim3((unsigned)(n_units * X));
-        cfg.blockDim = dim3((unsigned)(32 * kLWarps));
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        attr->id = cudaLaunchAttributeClusterDimension;
-        attr->val.clusterDim.x = (unsigned)X;
-        attr->val.clusterDim.y = 1;
-        attr->val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = X > 1 ? 1 : 0;
-        if (clusters && X > 1) return cudaOccupancyMaxActiveClusters(clusters, kern, &cfg);
-        return cudaSuccess;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    // blocks that run at once on X CTAs each (0: they do not fit)
+    auto resident = [&](int X) {
+        r = LearnPlan{X, (all + X - 1) / X, (long long)n_units * X <= sms};
+        if (r.chains * (X - 1) >= all) return 0;                     // a CTA without a chain
+        if (LearnLayout(max_N, all, X, r.chains).total > kRingSmemMax) return 0;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        int fit = 1;
+        cudaError_t e = learned_config(r, all, n_units, max_N, nullptr, cfg, attr);
+        if (e == cudaSuccess && X > 1) e = cudaOccupancyMaxActiveClusters(&fit, learned_kernel(r), &cfg);
+        if (e == cudaSuccess) return fit;
+        cudaGetLastError();
+        return 0;
     };
+    const int most = std::max(C, std::min({8, sms / n_units, all}));
+    for (int X = most; X > C; X--)
+        if (resident(X) >= n_units) return true;
+    for (int X = C; X <= 16 && X <= all; X++)
+        if (resident(X) > 0) return true;
+    return false;
+}
+
+cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, const LearnPlan& r, int n_units, int max_N,
+                                 cudaStream_t st) {
+    if (n_units <= 0) return cudaSuccess;
+    if (p.pair_chunks == nullptr) return cudaErrorInvalidValue;
+    SweepParams q = p;
+    q.cluster = p.cluster > 1 ? p.cluster : 1;
+    q.exec = r.exec;
+    q.chains = r.chains;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    int X = std::max(C, std::min({8, sms / n_units, all})), fit = 0;
-    for (; X > C; X--) {
-        if ((all + X - 1) / X * (X - 1) >= all) continue;            // a CTA without a chain
-        if (LearnLayout(max_N, all, X, (all + X - 1) / X).total > 227 * 1024) continue;
-        e = prepare(X, cfg, attr, &fit);
-        if (e != cudaSuccess) return e;
-        if (fit >= n_units) break;
-    }
-    if (X == C) e = prepare(C, cfg, attr, max_clusters ? &fit : nullptr);
-    if (e != cudaSuccess) return e;
-    if (max_clusters) {
-        *max_clusters = X > 1 ? fit : 1;
-        return cudaSuccess;
-    }
-    e = cudaLaunchKernelEx(&cfg, kern, q, l);
+    cudaError_t e = learned_config(r, 2 * q.cluster * p.warps, n_units, max_N, st, cfg, attr);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, learned_kernel(r), q, l);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
