@@ -162,8 +162,9 @@ struct pspin_state {
     int plan_key[2][4] = {};
     LearnPlan plan2 = {};               // of warps2, cluster2 (plan2_key)
     int plan2_key[2] = {};
-    int4* d_prep_moves = nullptr;       // the list-resident kernel's prepared moves (workspace)
+    int4* d_prep_moves = nullptr;       // the list-resident kernel's prepared moves (workspace), one allocation
     float* d_prep_trig = nullptr;
+    int prep_sweeps = 0;                // sweeps it holds (0: none)
     int* d_queue = nullptr;             // task counter, then tasks finished per replica block
     // the state that the tasks of a queued launch hand on (null: no launch is queued)
     float2* d_mid_spins = nullptr;
@@ -260,7 +261,7 @@ static void free_state(pspin_state* s) {
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     void* ptrs[] = {s->d_samples, s->d_units, s->d_spins, s->d_E, s->d_beta, s->d_target, s->d_drift,
                     s->d_e2, s->d_e4, s->d_epart, s->d_acc, s->d_prop, s->d_key, s->d_entries, s->d_chunk_start, s->d_site_chunks,
-                    s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status, s->d_queue, s->d_prep_moves, s->d_prep_trig,
+                    s->d_q64, s->d_g2, s->d_g4re, s->d_mask, s->d_sweep_counter, s->d_status, s->d_queue, s->d_prep_moves,
                     s->d_mid_spins, s->d_mid_perm,
                     s->d_beta_sched, s->d_perm, s->d_drand, s->d_ex_acc, s->d_ex_prop, s->d_trace,
                     s->d_tc_w, s->d_tc_x, s->d_tc_f, s->d_tc_ws, s->d_tc_h, s->d_f64_h, s->d_tc_e,
@@ -288,24 +289,54 @@ struct Carve {
     }
 };
 
-// The arrays of queued launches.  More blocks than run at once are cut in tasks only
-// where these exist: fewer than this many blocks always run at once (148 SMs, clusters
-// of 16), and where the device has no room the launch goes on without tasks.
-constexpr int kQueueUnits = 8;
+// What `lay` takes, or nothing (null pointers) where the device has no room.
 template <class Lay>
-static void alloc_mid(Lay lay) {
+static bool alloc_carved(Lay lay) {
     Carve count{nullptr};
     lay(count);
     void* p = nullptr;
     if (cudaMalloc(&p, count.used) != cudaSuccess) {
         cudaGetLastError();
-        return;
+        return false;
     }
     Carve place{static_cast<unsigned char*>(p)};
     lay(place);
+    return true;
 }
 
+// The arrays of queued launches.  More blocks than run at once are cut in tasks only
+// where these exist: this many blocks always run at once (148 SMs, clusters of 16),
+// and where the device has no room for the arrays a launch goes on without tasks.
+constexpr int kQueueUnits = 8;
+
 constexpr size_t kPrepBytes = (size_t)64 << 20;      // workspace of the list-resident kernel's prepared moves
+
+// The list-resident kernel's workspace: as many sweeps' prepared moves as kPrepBytes
+// hold, or as the device has room for.  Made where a shape with several warps is
+// chosen (set-up, the autotuner, a checkpoint), so that runs need no memory; false
+// where not even one sweep's fits.
+static bool ensure_prep(pspin_state* s) {
+    if (s->prep_sweeps > 0) return true;
+    const size_t steps = s->max_N / 2, per = steps * (s->units.size() * 7 * kRepBlock * sizeof(float) + s->S * sizeof(int4));
+    for (size_t n = std::max<size_t>(1, std::min<size_t>(kPrepBytes / std::max<size_t>(per, 1), 256)); n > 0; n /= 2) {
+        const bool made = alloc_carved([&](Carve& c) {
+            c.take(s->d_prep_moves, s->S * n * steps);
+            c.take(s->d_prep_trig, s->units.size() * n * steps * 7 * kRepBlock);
+        });
+        if (made) {
+            s->prep_sweeps = (int)n;
+            return true;
+        }
+    }
+    s->d_prep_moves = nullptr;
+    return false;
+}
+
+static void release_prep(pspin_state* s) {
+    cudaFree(s->d_prep_moves);
+    s->d_prep_moves = nullptr;
+    s->prep_sweeps = 0;
+}
 
 // ------------------------------------------------------------------ config
 extern "C" void pspin_default_config(pspin_config* c) {
@@ -1099,6 +1130,8 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
                 return bail(fail(PSPIN_ERR_ARG, "the site lists do not fit in shared memory (cluster_size -1)"));
             s->cluster = 0;
             s->warps = rw;
+            if (rw > 1 && !ensure_prep(s))
+                return bail(fail(PSPIN_ERR_ALLOC, "no room for the prepared moves of one sweep (cluster_size -1)"));
         } else {
             if (c != 1 && c != 2 && c != 4 && c != 8 && c != 16)
                 return bail(fail(PSPIN_ERR_ARG, "cluster_size must be -1, 1, 2, 4, 8 or 16"));
@@ -1130,7 +1163,7 @@ extern "C" int pspin_create_batch(const pspin_config* cfgs, int n, int variant, 
         (rc = dalloc(&s->d_units_k[1], s->units_k[1].size())))
         return bail(rc);
     if (s->units.size() > kQueueUnits)
-        alloc_mid([&](Carve& c) {
+        alloc_carved([&](Carve& c) {
             c.take(s->d_mid_spins, (size_t)s->spin_total);
             c.take(s->d_mid_E, s->R_tot);
             c.take(s->d_mid_acc, s->R_tot);
@@ -1320,27 +1353,11 @@ static int enqueue_ring(pspin_state* s, SweepParams& p, int pt_slots) {
     return PSPIN_OK;
 }
 
-// sweeps whose prepared moves fit the list-resident kernel's workspace
-static int resident_chunk(const pspin_state* s) {
-    const size_t per = (size_t)(s->max_N / 2) * (s->units.size() * 7 * kRepBlock * sizeof(float) + s->S * sizeof(int4));
-    return (int)std::max<size_t>(1, std::min<size_t>(kPrepBytes / std::max<size_t>(per, 1), 256));
-}
-
-static int ensure_prep(pspin_state* s) {
-    if (s->d_prep_trig) return PSPIN_OK;
-    const size_t moves = (size_t)resident_chunk(s) * (s->max_N / 2);
-    TRY(dalloc(&s->d_prep_moves, (size_t)s->S * moves));
-    return dalloc(&s->d_prep_trig, s->units.size() * moves * 7 * kRepBlock);
-}
-
-// The list-resident kernel (nsweeps <= resident_chunk unless it runs on one warp).
+// The list-resident kernel (nsweeps <= prep_sweeps unless it runs on one warp).
 static int enqueue_resident(pspin_state* s, SweepParams& p, int pt_slots) {
-    if (s->warps > 1) {
-        TRY(ensure_prep(s));
-        p.prep_moves = s->d_prep_moves;
-        p.prep_trig = s->d_prep_trig;
-        p.prep_stride = resident_chunk(s) * (s->max_N / 2);
-    }
+    p.prep_moves = s->d_prep_moves;
+    p.prep_trig = s->d_prep_trig;
+    p.prep_stride = s->prep_sweeps * (s->max_N / 2);
     p.exec = pt_slots > 0 ? (pt_slots + kRepBlock - 1) / kRepBlock : 1;
     CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, pt_slots, s->st));
     return PSPIN_OK;
@@ -1437,7 +1454,7 @@ static bool steps_in_launch(pspin_state* s) {
     const int slots = s->pt_NT * s->pt_nrep;
     if (s->cluster > 0) return n_units_of(s, s->rpl) == s->S && find_plan(s, slots);
     // list-resident: the blocks of a sample as one cluster (every sample has NT*nrep replicas)
-    return s->warps > 1 && slots <= 8 * kRepBlock && resident_chunk(s) >= s->pt_freq &&
+    return s->warps > 1 && slots <= 8 * kRepBlock && s->prep_sweeps >= s->pt_freq &&
            resident_smem_bytes_host(s->max_N, s->max_site_entries, s->warps, slots) <= 227 * 1024 - 64;
 }
 
@@ -1495,7 +1512,6 @@ static int capture_graph(pspin_state* s, int G) {
     drop_graph(s);
     if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster > 0) TRY(current_plan(s, 0));
     if (s->proposal != PSPIN_PROPOSAL_PLAIN) TRY(current_plan2(s));
-    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1) TRY(ensure_prep(s));
     cudaGraph_t graph = nullptr;
     CK(cudaStreamBeginCapture(s->st, cudaStreamCaptureModeThreadLocal));
     int rc = PSPIN_OK;
@@ -1530,7 +1546,8 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
     if (nsweeps < 0) return fail(PSPIN_ERR_ARG, "nsweeps < 0");
     int G = (pt && !s->profiling) ? graph_steps(s) : 0;
     const bool prepared = s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1;
-    if (prepared && pt && s->pt_freq > resident_chunk(s)) G = 0;
+    if (prepared && !ensure_prep(s)) return fail(PSPIN_ERR_ALLOC, "no room for the prepared moves of one sweep");
+    if (prepared && pt && s->pt_freq > s->prep_sweeps) G = 0;
     CK(cudaMemsetAsync(s->d_status, 0, sizeof(int), s->st));   // a time-out is reported by the call it happens in
     int left = nsweeps;
     while (left > 0) {
@@ -1540,7 +1557,7 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
             if (s->opt.resync_every > 0) room = std::min<long long>(room, s->opt.resync_every - s->since_resync);
             if (room >= s->pt_freq && steps_in_launch(s)) {
                 int steps = (int)std::max<long long>(1, std::min<long long>(room, kSweepsPerLaunch) / s->pt_freq);
-                if (s->cluster == 0) steps = std::min(steps, resident_chunk(s) / s->pt_freq);
+                if (s->cluster == 0) steps = std::min(steps, s->prep_sweeps / s->pt_freq);
                 TRY(launch_steps(s, steps));
                 left -= steps * s->pt_freq;
                 continue;
@@ -1567,8 +1584,8 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
                 ex = true;
             }
         }
-        if (prepared && chunk > resident_chunk(s)) {
-            chunk = resident_chunk(s);
+        if (prepared && chunk > s->prep_sweeps) {
+            chunk = s->prep_sweeps;
             ex = false;
         }
         if (chunk <= 0) chunk = 1;
@@ -1587,7 +1604,8 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
 static bool shape_fits(pspin_state* s, int warps, int cluster, int K = 1) {
     if (cluster == 0)
         return K == 1 && s->proposal == PSPIN_PROPOSAL_PLAIN &&
-               resident_smem_bytes_host(s->max_N, s->max_site_entries, warps, 0) <= 227 * 1024 - 64;
+               resident_smem_bytes_host(s->max_N, s->max_site_entries, warps, 0) <= 227 * 1024 - 64 &&
+               (warps == 1 || ensure_prep(s));
     if (cluster * warps > kSplit) return false;
     if (s->proposal == PSPIN_PROPOSAL_PLAIN) {
         RingPlan r;
@@ -1681,6 +1699,7 @@ static int autotune(pspin_state* s, int sweeps, int k_lo, int k_hi, int* chosen_
     Cl = good ? best_c : c0;
     if (plain) s->rpl = good ? best_k : k0;
     drop_graph(s);
+    if (s->cluster != 0 || s->warps == 1) release_prep(s);
     if (rc != PSPIN_OK) return rc;
     if (e != cudaSuccess) return fail(PSPIN_ERR_CUDA, "autotune: %s", cudaGetErrorString(e));
     if (status) return timeout_error(status);
@@ -1906,7 +1925,7 @@ extern "C" int pspin_pt_init(pspin_state* s, int NT, int nrep, const double* bet
         (rc = dalloc(&s->d_ex_prop, (size_t)s->S * (NT - 1))))
         return rc;
     if (s->units.size() > kQueueUnits)
-        alloc_mid([&](Carve& c) {
+        alloc_carved([&](Carve& c) {
             c.take(s->d_mid_perm, (size_t)s->S * NT * nrep);
             c.take(s->d_mid_beta, s->R_tot);
             c.take(s->d_mid_drand, s->S);
@@ -2766,6 +2785,8 @@ extern "C" int pspin_checkpoint_load(pspin_state* s, const char* path) {
     s->warps2 = warps2;
     s->cluster2 = cluster2;
     drop_graph(s);
+    if (s->cluster != 0 || s->warps == 1) release_prep(s);
+    else if (!ensure_prep(s)) return fail(PSPIN_ERR_ALLOC, "no room for the prepared moves of one sweep");
     return PSPIN_OK;
 }
 

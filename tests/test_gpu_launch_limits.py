@@ -63,3 +63,48 @@ def test_the_largest_N_of_a_block_shape_is_accepted_and_runs(N, warps, cluster, 
         eng.fill_betas(1.0)
         eng.sweep(1)
         assert np.all(eng.get_results()[2] == N // 2)
+
+
+def _resident(ps, warps):
+    c = ps.default_config(N=512, nrep=128, seed=11, fmc_mode=1)
+    c.gamma = 1.0
+    opts = ps.make_options(warps_per_unit=warps, cluster_size=-1, disorder_stream=True)
+    return ps.Engine(c, ps.PSPIN_SPARSE, opts)
+
+
+def test_a_list_resident_run_allocates_nothing(ps):
+    """The workspace of prepared moves (57 MB here) is made with the engine, given
+    back with it, and made again where a checkpoint brings the shape."""
+    import torch
+    free = lambda: torch.cuda.mem_get_info()[0]
+    _, betas = ps.temperature_schedule(32, 0.3, 1.5, True)
+    for _ in range(2):                      # (the first round loads kernels as well)
+        start = free()
+        with _resident(ps, 8) as eng:
+            eng.pt_init(32, 4, betas, 1)
+            before = free()
+            assert start - before > 50 << 20
+            eng.pt_run(3)
+            eng.sweep(2)
+            after = free()
+        end = free()
+    assert before - after < 4 << 20
+    assert start - end < 4 << 20
+
+
+def test_a_checkpoint_of_a_list_resident_shape_runs_on(ps, tmp_path):
+    _, betas = ps.temperature_schedule(32, 0.3, 1.5, True)
+    out = []
+    with _resident(ps, 8) as eng:
+        eng.pt_init(32, 4, betas, 1)
+        eng.pt_run(3)
+        eng.checkpoint_save(str(tmp_path / "c.bin"))
+        eng.pt_run(4)
+        out.append([eng.get_spins()[0], *eng.get_results(), *eng.pt_get(0)])
+    with _resident(ps, 1) as eng:           # made with one warp: no workspace
+        eng.pt_init(32, 4, betas, 1)
+        eng.checkpoint_load(str(tmp_path / "c.bin"))
+        eng.pt_run(4)
+        out.append([eng.get_spins()[0], *eng.get_results(), *eng.pt_get(0)])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
