@@ -655,7 +655,8 @@ cudaError_t DeviceLists::plan_fc(int N_, const double* g4, const uint8_t* mask, 
         for (int o = m + 1; o < N - 1; o++) add(o - 1, N - 1 - o);
         for (int o = 1; o < m; o++) add(N - 2 - o, o);
     }
-    if (n_fours >= (1ll << 27)) return cudaErrorMemoryAllocation;      // counts of entries stay below 2^31
+    // the kernels count entries in 31 bits, at most 2 (1 + kGroupMax) a four
+    if (n_fours * 2 * (1 + kGroupMax) >= (1ll << 31)) return cudaErrorInvalidValue;
     int* qcnt = nullptr;
     for (int pass = 0; pass < 2 && e == cudaSuccess; pass++) {
         size_t at = 0;

@@ -14,7 +14,8 @@ namespace pspin {
 // the sizes and whether tiles pay; write() puts everything in place:
 // the entries at `out` (entry `entry0` of the engine's), its chunk starts (chunk
 // `chunk0`), site-chunk table, quartets and neighbour masks.  g4 and mask stay
-// the caller's until then.
+// the caller's until then.  A plan fails where device memory is short, or (invalid
+// value) where a sample's entries are not counted in 31 bits: the host lays it out.
 struct DeviceLists {
     bool tiles = false;
     int64_t nominal = 0, entries = 0, chunks = 0, quartets = 0;
