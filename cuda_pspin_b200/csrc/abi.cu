@@ -1439,10 +1439,15 @@ static int account_sweeps(pspin_state* s, long long sweeps) {
     return PSPIN_OK;
 }
 
+// the list-resident kernel's preparation, a launch of its own
+static int prepares(const pspin_state* s) {
+    return s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1 ? 1 : 0;
+}
+
 // after `steps` steps of nsweeps sweeps each, one sweep launch a step
 static int account_steps(pspin_state* s, int steps, int nsweeps, bool exchange) {
     s->sweep_launches += steps;
-    s->kernel_launches += (long long)steps * (2 + ((exchange && s->obs_cap > 0) ? 1 : 0));
+    s->kernel_launches += (long long)steps * (2 + prepares(s) + ((exchange && s->obs_cap > 0) ? 1 : 0));
     return account_sweeps(s, (long long)steps * nsweeps);
 }
 
@@ -1473,7 +1478,7 @@ static int launch_steps(pspin_state* s, int steps) {
     else TRY(enqueue_resident(s, p, s->pt_NT * s->pt_nrep));
     TRY(enqueue_counter(s, steps * s->pt_freq, false));
     s->sweep_launches++;
-    s->kernel_launches += 2;
+    s->kernel_launches += 2 + prepares(s);
     return account_sweeps(s, (long long)steps * s->pt_freq);
 }
 

@@ -108,3 +108,17 @@ def test_a_checkpoint_of_a_list_resident_shape_runs_on(ps, tmp_path):
         out.append([eng.get_spins()[0], *eng.get_results(), *eng.pt_get(0)])
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("warps,launches", [(1, 2), (8, 3)])
+def test_every_launch_is_counted(ps, warps, launches):
+    """A list-resident sweep of several warps prepares its moves in a launch of its
+    own: prepare, sweep, sweep counter."""
+    _, betas = ps.temperature_schedule(32, 0.3, 1.5, True)
+    with _resident(ps, warps) as eng:
+        eng.get_profile()
+        eng.sweep(1)
+        assert eng.get_profile()[2] == launches
+        eng.pt_init(32, 4, betas, 1)
+        eng.pt_run(2)
+        assert eng.get_profile()[2] == (2 if warps == 1 else 1) * launches
