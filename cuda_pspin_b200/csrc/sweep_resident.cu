@@ -257,11 +257,11 @@ __global__ void __launch_bounds__(32) sweep_resident_one_kernel(const SweepParam
 // move {i0 | j0 << 16, slots of the earlier moves it does not commute with, 1 when
 // i0 and j0 share a term, 0}, per unit and move the proposal parts [7][32].
 __global__ void __launch_bounds__(128) resident_prepare_kernel(const SweepParams P, int variant) {
-    const Unit U = P.units[blockIdx.y];
+    const Unit U = P.units[blockIdx.x];          // (more units than a grid's y can count)
     const SampleDev S = P.samples[U.sample];
     const int N = S.N, steps = N / 2, total = P.nsweeps * steps;
     const int lane = threadIdx.x & 31;
-    const int m = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int m = blockIdx.y * 4 + (threadIdx.x >> 5);
     if (m >= total) return;
     const long long sweep0 = *P.sweep_counter;
     uint32_t k0 = 0, k1 = 0;
@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(128) resident_prepare_kernel(const SweepParams
     float tt[7];
     if (variant == 0) move_trig<0>(w, tt);
     else move_trig<1>(w, tt);
-    float* dst = P.prep_trig + ((size_t)blockIdx.y * P.prep_stride + m) * 7 * kRepBlock + lane;
+    float* dst = P.prep_trig + ((size_t)blockIdx.x * P.prep_stride + m) * 7 * kRepBlock + lane;
 #pragma unroll
     for (int q = 0; q < 7; q++) dst[q * kRepBlock] = tt[q];
     if (U.rep_begin != 0) return;
@@ -620,7 +620,7 @@ cudaError_t launch_sweep_resident(const SweepParams& p, int n_units, int variant
         return cudaGetLastError();
     }
     const int most = p.nsweeps * (max_N / 2);
-    resident_prepare_kernel<<<dim3((unsigned)((most + 3) / 4), (unsigned)n_units), 128, 0, st>>>(p, variant);
+    resident_prepare_kernel<<<dim3((unsigned)n_units, (unsigned)((most + 3) / 4)), 128, 0, st>>>(p, variant);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     auto kern = variant == 0 ? sweep_resident_kernel<0> : sweep_resident_kernel<1>;
