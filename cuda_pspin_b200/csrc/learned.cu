@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
                     sincosf(psi_j - argf(hj1), &s2, &c2);
                     ain = make_float2(mi * c1, mi * s1);
                     ajn = make_float2(mj * c2, mj * s2);
-                    // log q_L(x'|x) = log Beta + both mixtures, as log_learned_density
+                    // log q_L(x'|x) = log Beta + both mixtures
                     lq_fwd = log_beta_pdf_lg(tn, xch[X_A * 32 + lane], xch[X_B * 32 + lane], xch[X_LGA * 32 + lane],
                                              xch[X_LGB * 32 + lane], xch[X_LGAB * 32 + lane]) +
                              xch[X_VM0 * 32 + lane] + xch[X_VM1 * 32 + lane] - log_plain_density(tn);

@@ -52,11 +52,6 @@ __device__ __forceinline__ void pair_features(float2 ai, float2 aj, float2 hi, f
 __device__ __forceinline__ float softplusf(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-struct ProposalParams {
-    float a, b;               // Beta(a, b) for t'
-    float w[2][4], mu[2][4], kappa[2][4];   // mixtures for psi_i, psi_j
-};
-
 __device__ __forceinline__ float decode_beta_param(float o) { return 0.05f + softplusf(o); }
 
 // one site's mixture from its 12 outputs q: softmax weights, means, kappas
@@ -73,13 +68,6 @@ __device__ __forceinline__ void decode_site(const float* q, float* w, float* mu,
         mu[k] = q[4 + k];
         kappa[k] = kKappaMax * sigmoidf(q[8 + k]) + 0.01f;
     }
-}
-
-__device__ __forceinline__ void decode_outputs(const float* o, ProposalParams& p) {
-    p.a = decode_beta_param(o[0]);
-    p.b = decode_beta_param(o[1]);
-    #pragma unroll
-    for (int s = 0; s < 2; s++) decode_site(o + 2 + 12 * s, p.w[s], p.mu[s], p.kappa[s]);
 }
 
 // log I0(k) for 0 < k <= kKappaMax (CUDA's Bessel function, no overflow there)
@@ -111,14 +99,6 @@ __device__ __forceinline__ float log_vm_mix_site(const float* w, const float* mu
     #pragma unroll
     for (int k = 0; k < 4; k++) z += expf(v[k] - m);
     return m + logf(z);
-}
-
-__device__ __forceinline__ float log_vm_mix(const ProposalParams& p, int s, float psi) {
-    return log_vm_mix_site(p.w[s], p.mu[s], p.kappa[s], psi);
-}
-
-__device__ __forceinline__ float log_learned_density(const ProposalParams& p, float t, float psi_i, float psi_j) {
-    return log_beta_pdf(t, p.a, p.b) + log_vm_mix(p, 0, psi_i) + log_vm_mix(p, 1, psi_j);
 }
 
 // ------------------------------------------------------------------ sampling
@@ -267,8 +247,8 @@ __device__ __forceinline__ float digammaf_series(float x) {
 }
 
 // One record's -log q_L = -((log Beta + site 0) + site 1) and its gradient in
-// the outputs, in the three parts that are independent given the outputs
-// o[row * stride] (gradients to g[row * gstride]); each returns its part of
+// the outputs, in the three parts that are independent given the outputs: out(o)
+// reads output o, grad(o, v) takes the gradient in it; each returns its part of
 // log q_L.
 template <class Out, class Grad>
 __device__ __forceinline__ float loss_beta_grad(Out out, Grad grad, float t) {

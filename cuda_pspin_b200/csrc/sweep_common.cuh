@@ -62,10 +62,6 @@ __device__ __forceinline__ void propose(float2 ai, float2 aj, U4 w, float2& ain,
     propose_with<VARIANT>(ai, aj, t, ain, ajn);
 }
 
-// Static shared memory of the ring-fed cluster kernels (ring tags, the
-// stall-test barrier), kept free in their dynamic-size accounting.
-constexpr size_t kStaticSmem = 256;
-
 // ---------------------------------------------------------------- block state
 // Prologue copies into shared memory with kInFlight independent loads per
 // thread before their stores, so a CTA's state arrives in a few memory
@@ -116,14 +112,14 @@ __device__ __forceinline__ void load_block_range(T* dst, const T* src, int64_t n
 }
 
 // ---------------------------------------------------------------- TMA ring
-// Each warp streams the chunks of its share of the two site lists of every
-// move through a ring of kStages shared-memory slots.  Lane 0 issues 1-D
-// bulk copies (cp.async.bulk, completion counted on one mbarrier per slot)
-// kStages-1 chunks ahead of the chunk being read; the pair schedule is known
-// in advance, so the prefetch runs across move boundaries.  Waits are
-// bounded (SweepParams::wait_clocks): a wait that runs out raises the status
-// word, and the CTA (every CTA of a cluster) aborts the launch at the next
-// move barrier without writing anything back.
+// The streaming sweeps read the lists' chunks from rings of shared-memory slots,
+// filled by 1-D bulk copies (cp.async.bulk, completion counted on one mbarrier per
+// slot) ahead of the chunk being read; the pair schedule is known in advance, so
+// the copies run across move boundaries.  Who issues them is each kernel's: a
+// producer warp for all rings of a CTA (sweep_ring.cu), each warp for its own
+// (learned.cu).  Waits are bounded (SweepParams::wait_clocks): a wait that runs out
+// raises the status word, and the CTA (every CTA of a cluster) gives up without
+// writing anything back.
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -253,7 +249,7 @@ __device__ __forceinline__ void record_step(const int4 q, const float2 a, const 
     }
 }
 
-template <int kUnroll = 4, bool kSingle = false>
+template <int kUnroll>
 __device__ __forceinline__ void accumulate_records(const int2* __restrict__ R2, int n,
                                                    const float2* __restrict__ sp, int lane,
                                                    float& hx, float& hy) {
@@ -273,11 +269,11 @@ __device__ __forceinline__ void accumulate_records(const int2* __restrict__ R2, 
             ao[u] = sp[(q[u].z & 0xFFFF) * kRepBlock + lane];
         }
 #pragma unroll
-        for (int u = 0; u < kUnroll; u++) record_step<kSingle>(q[u], a[u], ap[u], ao[u], yx, yy, hx, hy);
+        for (int u = 0; u < kUnroll; u++) record_step<false>(q[u], a[u], ap[u], ao[u], yx, yy, hx, hy);
     }
     for (; r < nr; r++) {
         const int4 q = R[r];
-        record_step<kSingle>(q, sp[q.y * kRepBlock + lane], sp[(q.z >> 16) * kRepBlock + lane],
+        record_step<false>(q, sp[q.y * kRepBlock + lane], sp[(q.z >> 16) * kRepBlock + lane],
                              sp[(q.z & 0xFFFF) * kRepBlock + lane], yx, yy, hx, hy);
     }
 }
