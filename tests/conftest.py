@@ -13,6 +13,22 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: long CPU oracle runs")
 
 
+REF_DIR = os.path.join(ROOT, "oracle", "_ref")
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    """Tests that run the reference's own programs need its rebuild (make -C oracle
+    ref, where its sources are); without it they are skipped, with that reason."""
+    try:
+        return (yield)
+    except FileNotFoundError as e:
+        missing = os.path.realpath(str(e.filename or ""))
+        if os.path.dirname(missing) == os.path.realpath(REF_DIR) and not os.path.exists(missing):
+            pytest.skip(f"reference program not built: oracle/_ref/{os.path.basename(missing)}")
+        raise
+
+
 @pytest.fixture(scope="session")
 def orc():
     import oracle
