@@ -15,6 +15,7 @@
 #include <cstring>
 #include <string>
 #include <chrono>
+#include <climits>
 #include <unordered_map>
 #include <memory>
 #include <vector>
@@ -160,6 +161,8 @@ struct pspin_state {
     // (plan_key: warps, cluster, rpl, exchanging replicas it was made for)
     RingPlan plan[2] = {};
     int plan_key[2][4] = {};
+    int batched[2] = {};                // list-resident launches without and with exchanges inside: in batches?
+    int batched_key[2][2] = {};         //   (warps, exchanging replicas) it was asked for
     LearnPlan plan2 = {};               // of warps2, cluster2 (plan2_key)
     int plan2_key[2] = {};
     int4* d_prep_moves = nullptr;       // the list-resident kernel's prepared moves (workspace), one allocation
@@ -1353,13 +1356,36 @@ static int enqueue_ring(pspin_state* s, SweepParams& p, int pt_slots) {
     return PSPIN_OK;
 }
 
-// The list-resident kernel (nsweeps <= prep_sweeps unless it runs on one warp).
+// Which list-resident launches of the current shape run in the batched form, which
+// prepares nothing and holds no exchange.
+static int batched_form(pspin_state* s, int pt_slots) {
+    const int w = pt_slots > 0;
+    if (s->batched_key[w][0] != s->warps || s->batched_key[w][1] != pt_slots) {
+        s->batched[w] = resident_batched((int)s->units.size(), s->variant, s->max_N, s->max_site_entries, s->warps, pt_slots);
+        s->batched_key[w][0] = s->warps;
+        s->batched_key[w][1] = pt_slots;
+    }
+    return s->batched[w];
+}
+
+static bool batched_launch(pspin_state* s, int nsweeps) {
+    const int form = batched_form(s, 0);
+    return form == kBatchedAlways || (form == kBatchedShort && (long long)nsweeps * (s->max_N / 2) <= kShortLaunch);
+}
+
+// whether a launch of nsweeps sweeps is prepared, by a launch of its own
+static bool prepares(pspin_state* s, int nsweeps) {
+    return s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1 && !batched_launch(s, nsweeps);
+}
+
+// The list-resident kernel (nsweeps <= prep_sweeps unless its form prepares nothing).
 static int enqueue_resident(pspin_state* s, SweepParams& p, int pt_slots) {
     p.prep_moves = s->d_prep_moves;
     p.prep_trig = s->d_prep_trig;
     p.prep_stride = s->prep_sweeps * (s->max_N / 2);
     p.exec = pt_slots > 0 ? (pt_slots + kRepBlock - 1) / kRepBlock : 1;
-    CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, pt_slots, s->st));
+    CK(launch_sweep_resident(p, (int)s->units.size(), s->variant, s->max_N, s->max_site_entries, pt_slots,
+                             pt_slots == 0 && batched_launch(s, p.nsweeps), s->st));
     return PSPIN_OK;
 }
 
@@ -1439,15 +1465,10 @@ static int account_sweeps(pspin_state* s, long long sweeps) {
     return PSPIN_OK;
 }
 
-// the list-resident kernel's preparation, a launch of its own
-static int prepares(const pspin_state* s) {
-    return s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1 ? 1 : 0;
-}
-
 // after `steps` steps of nsweeps sweeps each, one sweep launch a step
 static int account_steps(pspin_state* s, int steps, int nsweeps, bool exchange) {
     s->sweep_launches += steps;
-    s->kernel_launches += (long long)steps * (2 + prepares(s) + ((exchange && s->obs_cap > 0) ? 1 : 0));
+    s->kernel_launches += (long long)steps * (2 + (prepares(s, nsweeps) ? 1 : 0) + ((exchange && s->obs_cap > 0) ? 1 : 0));
     return account_sweeps(s, (long long)steps * nsweeps);
 }
 
@@ -1460,6 +1481,7 @@ static bool steps_in_launch(pspin_state* s) {
     if (s->cluster > 0) return n_units_of(s, s->rpl) == s->S && find_plan(s, slots);
     // list-resident: the blocks of a sample as one cluster (every sample has NT*nrep replicas)
     return s->warps > 1 && slots <= 8 * kRepBlock && s->prep_sweeps >= s->pt_freq &&
+           batched_form(s, slots) != kBatchedAlways &&
            resident_smem_bytes_host(s->max_N, s->max_site_entries, s->warps, slots) <= 227 * 1024 - 64;
 }
 
@@ -1478,7 +1500,7 @@ static int launch_steps(pspin_state* s, int steps) {
     else TRY(enqueue_resident(s, p, s->pt_NT * s->pt_nrep));
     TRY(enqueue_counter(s, steps * s->pt_freq, false));
     s->sweep_launches++;
-    s->kernel_launches += 2 + prepares(s);
+    s->kernel_launches += s->cluster == 0 ? 3 : 2;     // (list-resident: its preparation)
     return account_sweeps(s, (long long)steps * s->pt_freq);
 }
 
@@ -1550,8 +1572,9 @@ static int run_sweeps(pspin_state* s, int nsweeps, bool pt) {
     if (!s) return fail(PSPIN_ERR_ARG, "null handle");
     if (nsweeps < 0) return fail(PSPIN_ERR_ARG, "nsweeps < 0");
     int G = (pt && !s->profiling) ? graph_steps(s) : 0;
-    const bool prepared = s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1;
-    if (prepared && !ensure_prep(s)) return fail(PSPIN_ERR_ALLOC, "no room for the prepared moves of one sweep");
+    if (s->proposal == PSPIN_PROPOSAL_PLAIN && s->cluster == 0 && s->warps > 1 && !ensure_prep(s))
+        return fail(PSPIN_ERR_ALLOC, "no room for the prepared moves of one sweep");
+    const bool prepared = prepares(s, INT_MAX);
     if (prepared && pt && s->pt_freq > s->prep_sweeps) G = 0;
     CK(cudaMemsetAsync(s->d_status, 0, sizeof(int), s->st));   // a time-out is reported by the call it happens in
     int left = nsweeps;

@@ -188,9 +188,13 @@ struct LearnPlan {
 bool plan_learned_sweep(LearnPlan& r, int warps, int cluster, int n_units, int max_N);
 // the list-resident kernel; warps > 1 runs moves that commute (no site of one in
 // the other's quartet neighbourhood, by the neighbour masks `nbmask`) at once, on
-// clusters of p.exec units; pt_slots: replicas that exchange inside the launch
+// clusters of p.exec units; pt_slots: replicas that exchange inside the launch;
+// batched: the form for many blocks (without exchanges, and nothing prepared)
 cudaError_t launch_sweep_resident(const SweepParams& p, int n_units, int variant, int max_N, int64_t max_entries,
-                                  int pt_slots, cudaStream_t st);
+                                  int pt_slots, bool batched, cudaStream_t st);
+enum { kBatchedNever, kBatchedShort, kBatchedAlways };
+constexpr int kShortLaunch = 64;      // moves
+int resident_batched(int n_units, int variant, int max_N, int64_t max_entries, int warps, int pt_slots);
 size_t resident_smem_bytes_host(int N, int64_t entries, int warps, int pt_slots);
 
 struct EnergyParams {

@@ -249,7 +249,7 @@ __device__ __forceinline__ void record_step(const int4 q, const float2 a, const 
     }
 }
 
-template <int kUnroll>
+template <int kUnroll, bool kSingle = false>
 __device__ __forceinline__ void accumulate_records(const int2* __restrict__ R2, int n,
                                                    const float2* __restrict__ sp, int lane,
                                                    float& hx, float& hy) {
@@ -269,11 +269,11 @@ __device__ __forceinline__ void accumulate_records(const int2* __restrict__ R2, 
             ao[u] = sp[(q[u].z & 0xFFFF) * kRepBlock + lane];
         }
 #pragma unroll
-        for (int u = 0; u < kUnroll; u++) record_step<false>(q[u], a[u], ap[u], ao[u], yx, yy, hx, hy);
+        for (int u = 0; u < kUnroll; u++) record_step<kSingle>(q[u], a[u], ap[u], ao[u], yx, yy, hx, hy);
     }
     for (; r < nr; r++) {
         const int4 q = R[r];
-        record_step<false>(q, sp[q.y * kRepBlock + lane], sp[(q.z >> 16) * kRepBlock + lane],
+        record_step<kSingle>(q, sp[q.y * kRepBlock + lane], sp[(q.z >> 16) * kRepBlock + lane],
                              sp[(q.z & 0xFFFF) * kRepBlock + lane], yx, yy, hx, hy);
     }
 }

@@ -31,7 +31,8 @@
 // of 32 moves prepared by the workers themselves, then cut in batches of
 // consecutive commuting moves with a CTA barrier each, took 7500 cycles of
 // preparation a window and 8.6 batches of 1950 cycles: 118 us a sweep launch and
-// 25 us of exchange; now 91 us for both.
+// 25 us of exchange; now 91 us for both.  Where many blocks share the SMs those
+// batches are the better form still, and run (resident_batched).
 #include <climits>
 
 #include "exchange.cuh"
@@ -602,14 +603,291 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
     }
 }
 
+// Many blocks (see resident_batched): windows of 32 moves, in batches.  The lanes of
+// warp 0 draw the window's pairs, every warp prepares its share of the proposals, and
+// the warps mark for every move the earlier moves of the window it does not commute
+// with; the window is cut, in move order, into batches of at most K moves that pairwise
+// commute, and warp w runs a batch's w-th move.  One CTA barrier per batch; the last
+// warp keeps the energies, in move order.
+inline size_t resident_batch_smem_bytes(int N, int64_t entries, int K) {
+    return (size_t)(N + 1) * kRepBlock * sizeof(float2) + (size_t)entries * sizeof(int2) + (size_t)N * sizeof(int2) +
+           2 * 32 * sizeof(int2) + 34 * sizeof(int) + 32 * sizeof(uint32_t) +
+           (size_t)2 * K * kRepBlock * (sizeof(float) + sizeof(int)) + (size_t)32 * 7 * kRepBlock * sizeof(float) +
+           (size_t)64 * ((N + 31) / 32) * sizeof(uint32_t);
+}
+
+template <int VARIANT>
+__global__ void __launch_bounds__(256, 2) sweep_resident_batch_kernel(const SweepParams P) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const Unit U = P.units[blockIdx.x];
+    const SampleDev S = P.samples[U.sample];
+    const int N = S.N, R = S.R;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int K = (int)(blockDim.x >> 5);
+    const int owner = K - 1;                   // keeps the running energy and counters
+    const int wpr = (N + 31) >> 5;             // words per neighbour-mask row
+    const uint32_t* nbm = P.nbmask + S.nb_off; // read through L1
+    const int* sc = P.site_chunks + S.split_off;
+    const int64_t e0 = __ldg(P.chunk_start + __ldg(sc));
+    const int64_t e1 = __ldg(P.chunk_start + __ldg(sc + (int64_t)(N - 1) * (kSplit + 1) + kSplit));
+    float2* sp = reinterpret_cast<float2*>(smem_raw);
+    int2* L = reinterpret_cast<int2*>(sp + (size_t)(N + 1) * kRepBlock);
+    int2* rng_site = L + (e1 - e0);
+    int2* picks = rng_site + N;
+    int2* mk = picks + 32;                                     // (sweep - sweep0, step) of each move
+    int* bounds = reinterpret_cast<int*>(mk + 32);             // [0..32] batch starts, [33] batch count
+    uint32_t* cm = reinterpret_cast<uint32_t*>(bounds + 34);   // [32]
+    float* dEx = reinterpret_cast<float*>(cm + 32);            // [2][K][32]
+    int* acx = reinterpret_cast<int*>(dEx + 2 * K * kRepBlock);  // [2][K][32]
+    float* tr = reinterpret_cast<float*>(acx + 2 * K * kRepBlock);  // [32][7][32]
+    uint32_t* nrow = reinterpret_cast<uint32_t*>(tr + 32 * 7 * kRepBlock);   // [32][2][wpr]
+    for (int m = threadIdx.x; m < N; m += blockDim.x) {
+        const int64_t b = __ldg(P.chunk_start + __ldg(sc + (int64_t)m * (kSplit + 1)));
+        const int64_t e = __ldg(P.chunk_start + __ldg(sc + (int64_t)m * (kSplit + 1) + kSplit));
+        rng_site[m] = make_int2((int)(b - e0), (int)(e - e0));
+    }
+    load_block_range(L, P.entries + e0, e1 - e0);
+    load_block_amplitudes(sp, P.spins + S.spin_off + U.rep_begin, R, N, kRepBlock, U.rep_count);
+    if (threadIdx.x < kRepBlock) sp[N * kRepBlock + threadIdx.x] = make_float2(1.f, 0.f);   // virtual site
+
+    const bool active = lane < U.rep_count;
+    const int64_t gr = S.rep_off + U.rep_begin + lane;
+    double E = 0.0, beta_d = 0.0;
+    float beta = 0.f;
+    long long nacc = 0, nprop = 0;
+    uint32_t k0 = 0, k1 = 0;
+    if (active) {
+        beta_d = P.beta[gr];
+        beta = (float)beta_d;
+        const uint64_t key = P.key[gr];
+        k0 = (uint32_t)key;
+        k1 = (uint32_t)(key >> 32);
+        if (warp == owner) E = P.energy[gr];
+    }
+    const long long sweep0 = *P.sweep_counter;
+    const int steps = N / 2, total = P.nsweeps * steps;
+    // is `site` a site of the window's move j or a neighbour of one?
+    auto in_reach = [&](int site, int j) {
+        const int2 q = picks[j];
+        const uint32_t* rows = nrow + 2 * j * wpr;
+        return site == q.x || site == q.y || (((rows[site >> 5] | rows[wpr + (site >> 5)]) >> (site & 31)) & 1u);
+    };
+    // the owner warp's running energy and counters take a batch's moves in move order
+    auto account = [&](int par, int n) {
+        for (int w = 0; w < n; w++) {
+            if (acx[(par * K + w) * kRepBlock + lane]) {
+                E += (double)dEx[(par * K + w) * kRepBlock + lane];
+                nacc++;
+            }
+            nprop++;
+        }
+    };
+    __syncthreads();
+
+    long long batches = 0;
+    int prev = 0;                              // moves in the previous batch
+    for (int m0 = 0; m0 < total; m0 += 32) {
+        const int n = min(32, total - m0);
+        if (warp == 0) {                       // the window's pairs
+            int i0 = 0, j0 = 1, sw = 0, kk = 0;
+            if (lane < n) {
+                sw = (m0 + lane) / steps;
+                kk = (m0 + lane) % steps;
+                pair_pick(S.pair_key0, S.pair_key1, (uint64_t)(sweep0 + sw), (uint32_t)kk, N, i0, j0);
+            }
+            picks[lane] = make_int2(i0, j0);
+            mk[lane] = make_int2(sw, kk);
+            cm[lane] = 0u;
+        }
+        // every warp: the state-independent parts of the proposals of its share
+        // of the window's moves (random words, sines and cosines), for its lanes
+        for (int t = warp; t < n; t += K) {
+            const int m = m0 + t;
+            float tt[7];
+            move_trig<VARIANT>(move_words(k0, k1, (uint64_t)(sweep0 + m / steps), (uint32_t)(m % steps)), tt);
+#pragma unroll
+            for (int q = 0; q < 7; q++) tr[(t * 7 + q) * kRepBlock + lane] = tt[q];
+        }
+        __syncthreads();
+        // the neighbour-mask rows of the window's sites, all loads in flight at once
+        const int tot = n * 2 * wpr;
+        for (int i0 = threadIdx.x; i0 < tot; i0 += kInFlight * blockDim.x) {
+            uint32_t v[kInFlight];
+#pragma unroll
+            for (int u = 0; u < kInFlight; u++) {
+                const int idx = i0 + u * (int)blockDim.x;
+                v[u] = 0u;
+                if (idx < tot) {
+                    const int j = idx / (2 * wpr), r = idx - j * 2 * wpr;
+                    const int2 q = picks[j];
+                    v[u] = __ldg(nbm + (r < wpr ? q.x * wpr + r : q.y * wpr + (r - wpr)));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kInFlight; u++) {
+                const int idx = i0 + u * (int)blockDim.x;
+                if (idx < tot) nrow[idx] = v[u];
+            }
+        }
+        __syncthreads();
+        // conflict masks: the earlier moves of the window that move `lane`
+        // does not commute with, the earlier moves shared out over the warps
+        uint32_t part = 0;
+        if (lane < n) {
+            const int2 me = picks[lane];
+            for (int j = warp; j < lane; j += K)
+                if (in_reach(me.x, j) || in_reach(me.y, j)) part |= 1u << j;
+        }
+        if (part) atomicOr(cm + lane, part);
+        __syncthreads();
+        if (warp == 0) {
+            // greedy cut in move order: a batch [s0, e) ends at the first move
+            // that does not commute with one of [s0, itself), or after K moves
+            const uint32_t mask = cm[lane];
+            int nb = 0;
+            for (int s0 = 0; s0 < n;) {
+                const unsigned bad = __ballot_sync(0xffffffffu, lane > s0 && lane < n && (mask >> s0) != 0u);
+                const int e = min(bad ? __ffs(bad) - 1 : n, min(n, s0 + K));
+                if (lane == 0) bounds[nb] = s0;
+                nb++;
+                s0 = e;
+            }
+            if (lane == 0) {
+                bounds[nb] = n;
+                bounds[33] = nb;
+            }
+        }
+        __syncthreads();
+        const int nb = bounds[33];
+        for (int b = 0; b < nb; b++) {
+            const int bs = bounds[b], be = bounds[b + 1];
+            const int par = (int)(batches & 1);
+            if (warp == owner && batches > 0) account(par ^ 1, prev);
+            if (warp < be - bs) {
+                const int t = bs + warp;
+                const int2 pq = picks[t], swk = mk[t];
+                const int i0 = pq.x, j0 = pq.y;
+                float tt[7];
+#pragma unroll
+                for (int q = 0; q < 7; q++) tt[q] = tr[(t * 7 + q) * kRepBlock + lane];
+                const float2 ai = sp[i0 * kRepBlock + lane], aj = sp[j0 * kRepBlock + lane];
+                float2 ain, ajn;
+                propose_with<VARIANT>(ai, aj, tt, ain, ajn);
+                const float cu = tt[6];
+                sp[j0 * kRepBlock + lane] = ajn;       // h_i is evaluated at the proposed a_j
+                __syncwarp();
+                float hix = 0.f, hiy = 0.f, hjx = 0.f, hjy = 0.f;
+                const int2 ri = rng_site[i0], rj = rng_site[j0];
+                if (S.tiles) {
+                    accumulate_tiles_1<2, 2, false>(L + ri.x, ri.y - ri.x, sp, lane, hix, hiy);
+                    accumulate_tiles_1<2, 2, false>(L + rj.x, rj.y - rj.x, sp, lane, hjx, hjy);
+                } else if (S.single_groups) {
+                    accumulate_records<4, true>(L + ri.x, ri.y - ri.x, sp, lane, hix, hiy);
+                    accumulate_records<4, true>(L + rj.x, rj.y - rj.x, sp, lane, hjx, hjy);
+                } else {
+                    accumulate_records<4>(L + ri.x, ri.y - ri.x, sp, lane, hix, hiy);
+                    accumulate_records<4>(L + rj.x, rj.y - rj.x, sp, lane, hjx, hjy);
+                }
+                const float dix = __fsub_rn(ain.x, ai.x), diy = __fsub_rn(ain.y, ai.y);
+                const float djx = __fsub_rn(ajn.x, aj.x), djy = __fsub_rn(ajn.y, aj.y);
+                const float dE = -fmaf(dix, hix, -diy * hiy) - fmaf(djx, hjx, -djy * hjy);
+                bool accept;
+                if (beta_d == 0.0) accept = true;
+                else accept = (dE <= 0.f) || (cu < expf(-beta * dE));
+                __syncwarp();
+                if (accept) sp[i0 * kRepBlock + lane] = ain;
+                else sp[j0 * kRepBlock + lane] = aj;
+                dEx[(par * K + warp) * kRepBlock + lane] = dE;
+                acx[(par * K + warp) * kRepBlock + lane] = accept ? 1 : 0;
+                if (P.trace != nullptr && U.sample == P.trace_sample && U.rep_begin + lane == P.trace_rep && active) {
+                    const long long idx = (long long)swk.x * steps + swk.y + (sweep0 - P.trace_sweep0) * steps;
+                    if (idx >= 0 && idx < P.trace_cap) {
+                        pspin_move_record* rec = reinterpret_cast<pspin_move_record*>(P.trace) + idx;
+                        rec->i0 = i0; rec->j0 = j0;
+                        rec->ai_old[0] = ai.x; rec->ai_old[1] = ai.y;
+                        rec->aj_old[0] = aj.x; rec->aj_old[1] = aj.y;
+                        rec->ai_new[0] = ain.x; rec->ai_new[1] = ain.y;
+                        rec->aj_new[0] = ajn.x; rec->aj_new[1] = ajn.y;
+                        rec->dE = dE;
+                        rec->accepted = accept ? 1 : 0;
+                        rec->log_q_ratio = 0.f;
+                        rec->log_u = logf(cu);
+                    }
+                }
+            }
+            __syncthreads();
+            prev = be - bs;
+            batches++;
+        }
+    }
+    if (warp == owner && batches > 0) account((int)((batches - 1) & 1), prev);
+    for (int idx = threadIdx.x; idx < N * kRepBlock; idx += blockDim.x) {
+        const int site = idx >> 5, l = idx & 31;
+        if (l < U.rep_count) P.spins[S.spin_off + (int64_t)site * R + U.rep_begin + l] = sp[idx];
+    }
+    if (warp == owner && active) {
+        P.energy[gr] = E;
+        P.accepted[gr] += nacc;
+        P.proposed[gr] += nprop;
+    }
+}
+
 size_t resident_smem_bytes_host(int N, int64_t entries, int warps, int pt_slots) {
     return resident_smem_bytes(N, entries, warps, pt_slots);
 }
 
+// Which launches run in the batched form.  The dataflow holds 168 registers a thread, a
+// warp more, and its prepared moves in global memory (some 900 bytes a move and block,
+// written and read) by a launch of their own; the batched form costs a barrier per
+// batch and its windows' preparation, but up to twice as many of its blocks share an
+// SM.  Samples of 96 replicas (three blocks), sweeps without exchanges, dataflow and
+// batched, us a sweep:
+//   many blocks, 8 warps: 50 samples N = 62 55 and 29, 200 samples 139 and 71, N = 128
+//     219 and 111; 2 warps: 100 samples N = 62 42 and 35;
+//   few, many moves: 8 warps, 16 samples N = 128 42 and 45, one sample N = 512 73 and 98;
+//   few, moves that mostly wait for one another: 8 warps, 8 samples N = 32 18.9 and
+//     17.8, N = 62 24.7 and 23.4; 2 warps N = 32 19.4 and 20.5;
+//   one sweep a launch: 8 samples, 8 warps N = 62 61 and 54, N = 128 71 and 69, N = 256
+//     89 and 90.
+// So the batched form takes every launch where it needs fewer waves of blocks than the
+// dataflow, or as many with more than two blocks per SM; and without exchanges those of
+// at least 4 warps at N <= 8 warps, and those of at most kShortLaunch moves.
+int resident_batched(int n_units, int variant, int max_N, int64_t max_entries, int warps, int pt_slots) {
+    if (warps == 1 || resident_batch_smem_bytes(max_N, max_entries, warps) > 227 * 1024 - 64) return kBatchedNever;
+    if (pt_slots == 0 && warps >= 4 && max_N <= 8 * warps) return kBatchedAlways;
+    const int otherwise = pt_slots == 0 ? kBatchedShort : kBatchedNever;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return otherwise;
+    }
+    if (n_units <= sms) return otherwise;
+    auto waves = [&](void (*kern)(const SweepParams), int threads, size_t smem) {
+        int blocks = 0;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kern, threads, smem);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && blocks > 0 ? (n_units + blocks * sms - 1) / (blocks * sms) : 1 << 30;
+    };
+    const int flow = waves(variant == 0 ? sweep_resident_kernel<0> : sweep_resident_kernel<1>, 32 * (warps + 1),
+                           resident_smem_bytes(max_N, max_entries, warps, pt_slots));
+    const int batch = waves(variant == 0 ? sweep_resident_batch_kernel<0> : sweep_resident_batch_kernel<1>, 32 * warps,
+                            resident_batch_smem_bytes(max_N, max_entries, warps));
+    return batch < flow || (pt_slots == 0 && batch == flow && n_units > 2 * sms) ? kBatchedAlways : otherwise;
+}
+
 cudaError_t launch_sweep_resident(const SweepParams& p, int n_units, int variant, int max_N, int64_t max_entries,
-                                  int pt_slots, cudaStream_t st) {
+                                  int pt_slots, bool batched, cudaStream_t st) {
     if (n_units <= 0) return cudaSuccess;
     if (p.warps < 1 || p.warps > 8 || (p.warps & (p.warps - 1)) != 0) return cudaErrorInvalidValue;
+    if (batched) {
+        const size_t smem = resident_batch_smem_bytes(max_N, max_entries, p.warps);
+        auto kern = variant == 0 ? sweep_resident_batch_kernel<0> : sweep_resident_batch_kernel<1>;
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<n_units, 32 * p.warps, smem, st>>>(p);
+        return cudaGetLastError();
+    }
     const size_t smem = resident_smem_bytes(max_N, max_entries, p.warps, pt_slots);
     if (smem > 227 * 1024 - 64) return cudaErrorInvalidValue;
     if (p.warps == 1) {

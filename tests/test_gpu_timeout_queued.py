@@ -81,7 +81,7 @@ def test_a_stall_beyond_the_launch_changes_nothing(ps, pt):
 @pytest.mark.parametrize("samples,N,NT,nrep,stall,pt", [
     (1, 96, 24, 4, 1, True), (3, 64, 24, 4, 70, True),       # three blocks a sample: one of a cluster gives up
     (2, 48, 10, 17, 144, True),                              # six, a ragged last, at the launch's last move
-    (2, 48, 4, 8, 100, True), (3, 64, 10, 4, 33, False),     # one block; blocks of their own
+    (2, 48, 4, 8, 100, True), (3, 96, 10, 4, 33, False),     # one block; blocks of their own
 ])
 def test_resident_blocks_of_a_sample_abort_together(ps, samples, N, NT, nrep, stall, pt, warps):
     with _engine(ps, (N,), samples, NT, nrep, stall, pt, sparse=True, warps_per_unit=warps, cluster_size=-1) as eng:
