@@ -127,6 +127,8 @@ struct SweepParams {
     int* status;                      // error word (kStatus* bits)
     long long wait_clocks;            // ring-wait limit in SM clocks
     int stall_move;                   // tests: move index of the stall wait (-1: none)
+    long long patience;               // sweep_resident_kernel: limit of its waits for other moves and blocks,
+                                      //   beyond any that is set for copies (tests: wait_clocks)
     // sweep_ring_kernel, launches of more than one task per unit: tasks of `chunk`
     // sweeps (the last one the rest of nsweeps), taken in order from *queue; done[u]:
     // tasks of unit u that are finished (-1: it aborted)

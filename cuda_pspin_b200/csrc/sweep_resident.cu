@@ -68,12 +68,6 @@ __device__ __forceinline__ void publish(int* p, int v) {
     *(volatile int*)p = v;
 }
 
-// What a move waits for other moves and blocks (clocks): beyond any limit set for a
-// copy, but for the test hook.
-__device__ __forceinline__ long long resident_patience(const SweepParams& P) {
-    return P.stall_move >= 0 ? P.wait_clocks : 2 * P.wait_clocks + kDrainClocks;
-}
-
 // Fields of two sites from their record lists, four records of each at a time with
 // all their loads in flight (a sparse site has ~4); the arithmetic of
 // accumulate_records on each.
@@ -304,7 +298,6 @@ template <int VARIANT>
 __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const SweepParams P) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int X = P.exec;                      // CTAs per cluster: the blocks of a sample, or 1
-    const uint32_t rank = X > 1 ? cluster_rank() : 0u;
     const Unit U = P.units[blockIdx.x];
     const SampleDev S = P.samples[U.sample];
     const int N = S.N, R = S.R;
@@ -374,7 +367,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
                 __syncwarp();
                 return true;
             }
-            const bool late = clock64() - t0 > resident_patience(P);
+            const bool late = clock64() - t0 > P.patience;
             if (__any_sync(0xffffffffu, late || stop != 0)) {
                 if (late) atomicOr(P.status, kStatusTimeout);
                 stop = 1;
@@ -431,7 +424,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
             // this slot's last dE is accounted for
             const int last = m - 1 - ((t - 1 - lane) & (kRing - 1));
             int need = ((uint32_t)mv.y >> lane) & 1u ? last : last - kRing;
-            if (m == P.stall_move && rank == (uint32_t)X - 1) need = INT_MAX;     // test hook, in one CTA of a cluster
+            if (m == P.stall_move && (X == 1 || cluster_rank() + 1 == (uint32_t)X)) need = INT_MAX;     // test hook, in one CTA of a cluster
             if (!wait([&]() { return peek(done + lane) >= need && peek(&counted) > m - kRing; })) break;
             const float2 ai = sp[i0 * kRepBlock + lane], aj = sp[j0 * kRepBlock + lane];
             float2 ain, ajn;
@@ -543,7 +536,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
                     const uint32_t dx = smem_u32(Ex + U.rep_begin + lane), db = smem_u32(ebar + par);
                     for (int q = 0; q < X; q++) st_async_f64(map_rank(dx, (uint32_t)q), E, map_rank(db, (uint32_t)q));
                 }
-                if (!__all_sync(0xffffffffu, mbar_wait(ebar + par, (uint32_t)(n_ex >> 1) & 1u, P.status, resident_patience(P)))) {
+                if (!__all_sync(0xffffffffu, mbar_wait(ebar + par, (uint32_t)(n_ex >> 1) & 1u, P.status, P.patience))) {
                     stop = 1;
                     break;
                 }
@@ -590,7 +583,7 @@ __global__ void __launch_bounds__((8 + 1) * 32) sweep_resident_kernel(const Swee
         P.proposed[gr] += nprop;
         if (RT > 0) P.beta_out[gr] = beta_d;
     }
-    if (warp == K && RT > 0 && rank == 0) {
+    if (warp == K && RT > 0 && (X == 1 || cluster_rank() == 0u)) {
         int* perm = P.perm + (int64_t)U.sample * RT;
         for (int i = lane; i < RT; i += 32) perm[i] = pt_slot[i];
         long long* acc = P.ex_acc + (int64_t)U.sample * (P.NT - 1);
@@ -897,6 +890,8 @@ cudaError_t launch_sweep_resident(const SweepParams& p, int n_units, int variant
         kern<<<n_units, 32, smem, st>>>(p);
         return cudaGetLastError();
     }
+    SweepParams q = p;
+    q.patience = p.stall_move >= 0 ? p.wait_clocks : 2 * p.wait_clocks + kDrainClocks;
     const int most = p.nsweeps * (max_N / 2);
     resident_prepare_kernel<<<dim3((unsigned)n_units, (unsigned)((most + 3) / 4)), 128, 0, st>>>(p, variant);
     cudaError_t e = cudaGetLastError();
@@ -916,7 +911,7 @@ cudaError_t launch_sweep_resident(const SweepParams& p, int n_units, int variant
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.exec > 1 ? 1 : 0;
-    e = cudaLaunchKernelEx(&cfg, kern, p);
+    e = cudaLaunchKernelEx(&cfg, kern, q);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
 }
