@@ -201,6 +201,11 @@ __device__ __noinline__ uint64_t ring_exchange(double* pt_E, int RT, int NT, int
     return drand;
 }
 
+// whether the task whose first sweep is `first` is a unit's last one
+__device__ __forceinline__ bool last_task(const SweepParams& P, int first) {
+    return P.queue == nullptr || P.nsweeps - first <= P.chunk;
+}
+
 // kLat: few blocks, at most kLatChains chain warps a CTA, so a warp has its
 // sub-partition's issue slots and registers to itself and deep batches of
 // loads in flight carry it; otherwise 16 chain warps share the SM.
@@ -365,8 +370,8 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
 #pragma unroll
             for (int q = 0; q < K; q++) hx[q] = hy[q] = 0.f;
             bool ok = true;
-            // test hook: the launch's move
-            if (P.stall_move >= 0 && (long long)first_s * steps + m == P.stall_move) ok = stall_wait(&stall_bar, P.status, P.wait_clocks);
+            // test hook, in a unit's last task
+            if (m == P.stall_move && last_task(P, first_s)) ok = stall_wait(&stall_bar, P.status, P.wait_clocks);
             for (bool last = false; ok && !last;) {
                 ok = ring_wait(fb + slot, phase, P.status, P.wait_clocks);
                 if (!ok) break;
@@ -394,7 +399,6 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
             __syncwarp();
             if (lane == 0) mbar_arrive(cbar);
         }
-        left_arrive(state_threads + 32);
     } else if (decider) {
         // ------------------------------------------------------------ decider
         const int W = P.warps, C = P.cluster;
@@ -517,7 +521,6 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
                 }
             }
         }
-        left_arrive(state_threads + 32);
     } else if (warp == c + K) {
         // ------------------------------------------------------------ producer: lane = chain of this CTA
         // chain g of the move: the groups alternate between the lists, group 2q
@@ -589,6 +592,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
         __syncwarp();
     }
 
+    if (warp < c + K) left_arrive(state_threads + 32);
     if (X > 1 && stop && threadIdx.x == 0)           // a CTA that gave up takes its cluster with it
         for (int q = 0; q < X; q++) st_cluster_u32((const void*)&stop, (uint32_t)q, 1u);
     if (X > 1) cluster_sync();                       // every final write; no store may still target a CTA
@@ -596,7 +600,7 @@ __global__ void __launch_bounds__(((kLat ? kLatChains : kMaxChains) + K + 1) * 3
     const bool good = stop == 0;
     if (rank == 0) {
         if (good) {
-            const bool head = first_s == 0, tail = !P.queue || P.nsweeps - first_s <= P.chunk;
+            const bool head = first_s == 0, tail = last_task(P, first_s);
             float2* spins = tail ? P.spins : P.mid_spins;
             for (int idx = threadIdx.x; idx < N * KB; idx += blockDim.x) {
                 const int site = idx / KB, r = idx % KB;

@@ -112,9 +112,10 @@ typedef struct pspin_options {
     int test_stall_move; /* tests of the time-out path: k > 0 makes every CTA
                             of the ring-fed sweep kernels (with the lists
                             resident and warps_per_unit > 1, one CTA of each
-                            cluster) wait, at move k-1 of each launch, for
-                            something that does not come, so the bounded wait
-                            runs out; 0: off */
+                            cluster) wait, at move k-1 of each launch (of its
+                            last task, where a replica block runs as several),
+                            for something that does not come, so the bounded
+                            wait runs out; 0: off */
     int disorder_stream; /* sparse set-up: 0 (default) the reference's couplings
                             bit for bit, from its single cuRAND call of
                             2*C(N,4) normals (2*8*C(N,4) bytes on the device:

@@ -39,10 +39,11 @@ def _engine(ps, Ns, samples, NT, nrep, stall, pt, sparse=False, **opts):
 
 @pytest.mark.parametrize("pt", [False, True])
 @pytest.mark.parametrize("Ns,samples,warps,cluster,lanes,stall", [
-    ((8,), 400, 8, 1, 3, 14),            # four moves a sweep, tasks of two sweeps: in the second task
-    ((8,), 400, 8, 4, 3, 21),            # in the third, on clusters
-    ((8, 20), 400, 8, 2, 3, 33),         # in the fifth of the small samples and the second of the large
-    ((8,), 400, 8, 1, 3, 24),            # at the launch's last move
+    ((8,), 400, 8, 1, 3, 1),             # four moves a sweep, the last of three tasks holds two sweeps
+    ((8,), 400, 8, 4, 3, 6),             # on clusters
+    ((8, 20), 400, 8, 2, 3, 5),          # samples of uneven size
+    ((8,), 400, 8, 1, 3, 8),             # at the launch's last move
+    ((8, 20), 400, 8, 1, 3, 15),         # only the larger samples' last tasks have that many moves
 ])
 def test_a_queued_launch_keeps_the_state_from_before_it(ps, Ns, samples, warps, cluster, lanes, stall, pt):
     NT, nrep, sweeps = 24, 4, 6
@@ -55,8 +56,9 @@ def test_a_queued_launch_keeps_the_state_from_before_it(ps, Ns, samples, warps, 
         assert ei.value.code == ps.PSPIN_ERR_TIMEOUT, str(ei.value)
         after = _state(eng, samples, pt)
         steps = np.repeat([Ns[k % len(Ns)] // 2 for k in range(samples)], NT * nrep)
-        reached = steps * sweeps >= stall                # the stall is a move of these samples' launch
+        reached = steps * 2 >= stall                     # the stall is a move of these samples' last task
         assert np.array_equal(before[3][reached], after[3][reached])
+        assert np.array_equal(before[1][reached], after[1][reached])
         if reached.all():
             for a, b in zip(before, after):
                 np.testing.assert_array_equal(a, b)
