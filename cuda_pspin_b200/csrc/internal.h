@@ -183,9 +183,10 @@ bool plan_sweep_ring(RingPlan& r, int warps, int cluster, int n_units, int varia
 cudaError_t launch_sweep_ring(const SweepParams& p, const RingPlan& r, int n_units, int variant, int max_N, int K,
                               int pt_slots, cudaStream_t st);
 // How the two-pass sweep spreads a unit's chains: `chains` of them on each of exec
-// CTAs; one: every CTA has an SM to itself.
+// CTAs; one: every CTA has an SM to itself; grouped: the CTAs exchange sums of the
+// shape's CTAs.
 struct LearnPlan {
-    int exec, chains, one;
+    int exec, chains, one, grouped;
 };
 bool plan_learned_sweep(LearnPlan& r, int warps, int cluster, int n_units, int max_N);
 // the list-resident kernel; warps > 1 runs moves that commute (no site of one in

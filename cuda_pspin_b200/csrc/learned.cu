@@ -160,7 +160,8 @@ constexpr int kLWarps = 8;
 struct LearnLayout {
     int rings;                                  // warps that read lists
     size_t ring, bars, buf, xch, parts, flag, total;
-    __host__ __device__ LearnLayout(int N, int all_chains, int exec, int chains) {
+    // sums: what the CTAs exchange, all chains or (grouped) the sums of the shape's CTAs
+    __host__ __device__ LearnLayout(int N, int sums, int exec, int chains, bool grouped) {
         rings = chains < kLWarps ? chains : kLWarps;
         size_t at = (size_t)(N + 1) * kRepBlock * sizeof(float2);           // amplitudes
         ring = at;
@@ -171,8 +172,8 @@ struct LearnLayout {
         at += (size_t)2 * kMlpBufWords * sizeof(uint32_t);
         xch = at;                               // the roles' exchange rows
         at += (size_t)kXchRows * kRepBlock * sizeof(float);
-        parts = (at + 15) & ~(size_t)15;        // partial fields, double-buffered across CTAs
-        at = parts + (size_t)(exec > 1 ? 2 : 1) * all_chains * kRepBlock * sizeof(float2);
+        parts = (at + 15) & ~(size_t)15;        // partial fields, double-buffered across CTAs; then, grouped, this CTA's
+        at = parts + (size_t)((exec > 1 ? 2 : 1) * sums + (grouped ? chains : 0)) * kRepBlock * sizeof(float2);
         flag = at;                              // the cluster's abort flag
         total = at + 16;
     }
@@ -234,7 +235,11 @@ struct LearnStream {
 // evaluates the network and takes the same decision on the same numbers, so the
 // amplitude copies stay identical; rank 0 writes records, trace and results.
 // kOne: one CTA has the SM (256 registers; loads of a tile ahead), else three share it.
-template <bool CL, bool kOne>
+// kGroup (full SMs, whole CTAs of the shape in a CTA): the sums of these go to the other
+// CTAs, not every chain.  60 samples of N = 28, 96 replicas, 8 warps x 4 CTAs: with 64
+// remote rows a pass into every CTA, summed by one warp, a sweep took 694 us (learned
+// 1492), now 468 (1001).
+template <bool CL, bool kOne, bool kGroup>
 __global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
     learned_sweep_kernel(const SweepParams P, const LearnParams L) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -248,7 +253,7 @@ __global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
     constexpr int W = kLWarps;
     const bool learned = L.mode == 2;
     float2* sp = reinterpret_cast<float2*>(smem_raw);
-    const LearnLayout Lo(N, 2 * CW, X, P.chains);
+    const LearnLayout Lo(N, kGroup ? 2 * P.cluster : 2 * CW, X, P.chains, kGroup);
     int2* ring = reinterpret_cast<int2*>(smem_raw + Lo.ring) + (size_t)warp * kLStages * kStage;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + Lo.bars) + warp * kLStages;
     uint32_t* bufA = reinterpret_cast<uint32_t*>(smem_raw + Lo.buf);
@@ -256,7 +261,7 @@ __global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
     const float* outs = reinterpret_cast<const float*>(bufB);
     float* xch = reinterpret_cast<float*>(smem_raw + Lo.xch);
     auto out_of = [&](int o) { return outs[o * kOutStride + lane]; };
-    float2* parts = reinterpret_cast<float2*>(smem_raw + Lo.parts);      // [parity][2 C W][32]
+    float2* parts = reinterpret_cast<float2*>(smem_raw + Lo.parts);      // [parity][2 C W][32] ([parity][2 C][32])
     int* cflag = reinterpret_cast<int*>(smem_raw + Lo.flag);             // cluster abort flags, by parity
 
     const bool active = lane < U.rep_count;
@@ -362,10 +367,43 @@ __global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
             }
         }
     };
+    // kGroup: the sums of this CTA's whole CTAs of the shape -> warp 0 of every CTA
+    auto reduce_groups = [&](const float (&h)[2][2]) {
+        float2* buf = parts + (size_t)(xchg & 1u) * 2 * P.cluster * kRepBlock;
+        float2* own = parts + (size_t)4 * P.cluster * kRepBlock;
+#pragma unroll
+        for (int q = 0; q < 2; q++)
+            if (q < st.n) own[(warp + q * kLWarps) * kRepBlock + lane] = make_float2(h[q][0], h[q][1]);
+        if (!ok_wait && lane == 0)
+            for (int r = 0; r < X; r++) st_cluster_u32(cflag + (xchg & 1u), (uint32_t)r, 1u);
+        __syncthreads();
+        const int groups = P.chains / P.warps;
+        for (int u = warp; u < groups; u += W) {
+            float2 s = make_float2(0.f, 0.f);
+            for (int w = u * P.warps; w < (u + 1) * P.warps; w++) {
+                const float2 a = own[w * kRepBlock + lane];
+                s.x += a.x;
+                s.y += a.y;
+            }
+            for (int r = 0; r < X; r++) st_cluster_f2(buf + ((int)rank * groups + u) * kRepBlock + lane, (uint32_t)r, s);
+        }
+        cluster_sync();
+        aborted = ((volatile int*)cflag)[xchg & 1u] != 0;
+        xchg++;
+        float4 hs = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (aborted || warp != 0) return hs;
+        for (int c = 0; c < P.cluster; c++) {
+            const float2 a = buf[c * kRepBlock + lane], b = buf[(P.cluster + c) * kRepBlock + lane];
+            if (c == 0) hs = make_float4(a.x, a.y, b.x, b.y);
+            else { hs.x += a.x; hs.y += a.y; hs.z += b.x; hs.w += b.y; }
+        }
+        return hs;
+    };
     // partial sums of all chains -> warp 0 of every CTA.  Also agrees on an abort:
     // a warp whose wait ran out makes the whole CTA (and, through the flag, the
     // whole cluster) set `aborted` here.
     auto reduce = [&](const float (&h)[2][2]) {
+        if constexpr (kGroup) return reduce_groups(h);
         float2* buf = parts + (CL ? (size_t)(xchg & 1u) * 2 * CW * kRepBlock : 0);
 #pragma unroll
         for (int q = 0; q < 2; q++) {
@@ -578,14 +616,18 @@ __global__ void __launch_bounds__(32 * kLWarps, kOne ? 1 : 3)
 
 using LearnKernel = void (*)(const SweepParams, const LearnParams);
 static LearnKernel learned_kernel(const LearnPlan& r) {
-    return r.exec > 1 ? (r.one ? learned_sweep_kernel<true, true> : learned_sweep_kernel<true, false>)
-                      : (r.one ? learned_sweep_kernel<false, true> : learned_sweep_kernel<false, false>);
+    if (r.grouped) return learned_sweep_kernel<true, false, true>;
+    return r.exec > 1 ? (r.one ? learned_sweep_kernel<true, true, false> : learned_sweep_kernel<true, false, false>)
+                      : (r.one ? learned_sweep_kernel<false, true, false> : learned_sweep_kernel<false, false, false>);
 }
 
 // The launch of a plan; `attr` is its cluster dimension.
-static cudaError_t learned_config(const LearnPlan& r, int all, int n_units, int max_N, cudaStream_t st,
+static size_t learned_smem(const LearnPlan& r, int warps, int C, int max_N) {
+    return LearnLayout(max_N, r.grouped ? 2 * C : 2 * C * warps, r.exec, r.chains, r.grouped != 0).total;
+}
+
+static cudaError_t learned_config(const LearnPlan& r, int n_units, size_t smem, cudaStream_t st,
                                   cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr) {
-    const size_t smem = LearnLayout(max_N, all, r.exec, r.chains).total;
     const LearnKernel kern = learned_kernel(r);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && r.exec > 8)
@@ -604,14 +646,17 @@ static cudaError_t learned_config(const LearnPlan& r, int all, int n_units, int 
     return e;
 }
 
-// As many CTAs per replica block as the blocks can all have at once with an SM
-// for each CTA (8 at most, no more than there are chains), and no fewer than the
-// shape has: chains on more SMs finish sooner, a second wave costs twice.  A move
+// As many CTAs per replica block as the blocks can all have at once with an SM for
+// each CTA (8 at most, no more than there are chains), or up to the shape's own where
+// these share SMs; else as few as hold the chains, two a warp: chains on more SMs
+// finish sooner, a second wave costs twice.  A move
 // of 24 blocks at N = 64 (gamma = 0.1, 8 warps x 2 CTAs) took 128 us on 2 CTAs
 // each, 84 on 6 (144 CTAs, but clusters of 6 do not tile the chip: two waves), 46
 // on the most that run at once; of 3 blocks 117 and 41 (8 CTAs); of 12 fully
-// connected blocks at N = 48 (one CTA's shape) 113 and 53.  Where the shape's own
-// CTAs are too few for the amplitudes beside their lists' share, the fewest that do.
+// connected blocks at N = 48 (one CTA's shape) 113 and 53; 60 samples of N = 28, 96
+// replicas, 4 warps x 8 CTAs, a sweep 1102 us on the shape's 8 CTAs, 474 on 4.  Where so
+// few CTAs have no room for the amplitudes beside their lists' share, the fewest that
+// have.
 bool plan_learned_sweep(LearnPlan& r, int warps, int cluster, int n_units, int max_N) {
     const int C = cluster > 1 ? cluster : 1, all = 2 * C * warps;
     if (warps < 1 || n_units < 1 || C > 16 || kSplit % (C * warps) != 0) return false;
@@ -622,22 +667,23 @@ bool plan_learned_sweep(LearnPlan& r, int warps, int cluster, int n_units, int m
     }
     // blocks that run at once on X CTAs each (0: they do not fit)
     auto resident = [&](int X) {
-        r = LearnPlan{X, (all + X - 1) / X, (long long)n_units * X <= sms};
+        r = LearnPlan{X, (all + X - 1) / X, (long long)n_units * X <= sms, 0};
         if (r.chains * (X - 1) >= all) return 0;                     // a CTA without a chain
-        if (LearnLayout(max_N, all, X, r.chains).total > kRingSmemMax) return 0;
+        r.grouped = X > 1 && !r.one && warps >= 4 && r.chains % warps == 0 && r.chains * X == all;
+        if (learned_smem(r, warps, C, max_N) > kRingSmemMax) return 0;
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         int fit = 1;
-        cudaError_t e = learned_config(r, all, n_units, max_N, nullptr, cfg, attr);
+        cudaError_t e = learned_config(r, n_units, learned_smem(r, warps, C, max_N), nullptr, cfg, attr);
         if (e == cudaSuccess && X > 1) e = cudaOccupancyMaxActiveClusters(&fit, learned_kernel(r), &cfg);
         if (e == cudaSuccess) return fit;
         cudaGetLastError();
         return 0;
     };
-    const int most = std::max(C, std::min({8, sms / n_units, all}));
-    for (int X = most; X > C; X--)
+    const int least = (all + 2 * kLWarps - 1) / (2 * kLWarps), most = std::max(C, std::min({8, sms / n_units, all}));
+    for (int X = most; X > least; X--)
         if (resident(X) >= n_units) return true;
-    for (int X = C; X <= 16 && X <= all; X++)
+    for (int X = least; X <= 16 && X <= all; X++)
         if (resident(X) > 0) return true;
     return false;
 }
@@ -652,7 +698,7 @@ cudaError_t launch_learned_sweep(const SweepParams& p, const LearnParams& l, con
     q.chains = r.chains;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    cudaError_t e = learned_config(r, 2 * q.cluster * p.warps, n_units, max_N, st, cfg, attr);
+    cudaError_t e = learned_config(r, n_units, learned_smem(r, p.warps, q.cluster, max_N), st, cfg, attr);
     if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, learned_kernel(r), q, l);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
