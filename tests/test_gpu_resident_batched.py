@@ -41,7 +41,7 @@ def test_the_form_does_not_change_the_chain(Ns, R, fmc, sparse, NT):
     variant = ps.PSPIN_SPARSE if sparse else ps.PSPIN_DENSE
     out, launches = [], {}
     for warps in (1, 2, 8):
-        launches[warps] = _run(ps, 400, Ns, R, fmc, variant, warps, NT, out)
+        launches[warps] = _run(ps, 170, Ns, R, fmc, variant, warps, NT, out)
     for other in out[1:]:
         for a, b in zip(out[0], other):
             np.testing.assert_array_equal(a, b)

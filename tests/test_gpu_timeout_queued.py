@@ -39,11 +39,11 @@ def _engine(ps, Ns, samples, NT, nrep, stall, pt, sparse=False, **opts):
 
 @pytest.mark.parametrize("pt", [False, True])
 @pytest.mark.parametrize("Ns,samples,warps,cluster,lanes,stall", [
-    ((8,), 400, 8, 1, 3, 1),             # four moves a sweep, the last of three tasks holds two sweeps
-    ((8,), 400, 8, 4, 3, 6),             # on clusters
-    ((8, 20), 400, 8, 2, 3, 5),          # samples of uneven size
-    ((8,), 400, 8, 1, 3, 8),             # at the launch's last move
-    ((8, 20), 400, 8, 1, 3, 15),         # only the larger samples' last tasks have that many moves
+    ((8,), 200, 8, 1, 3, 1),             # four moves a sweep, the last of three tasks holds two sweeps
+    ((8,), 200, 8, 4, 3, 6),             # on clusters
+    ((8, 20), 200, 8, 2, 3, 5),          # samples of uneven size
+    ((8,), 200, 8, 1, 3, 8),             # at the launch's last move
+    ((8, 20), 200, 8, 1, 3, 15),         # only the larger samples' last tasks have that many moves
 ])
 def test_a_queued_launch_keeps_the_state_from_before_it(ps, Ns, samples, warps, cluster, lanes, stall, pt):
     NT, nrep, sweeps = 24, 4, 6
@@ -71,9 +71,9 @@ def test_a_stall_beyond_the_launch_changes_nothing(ps, pt):
     out = []
     for stall in (0, 1000):
         opts = dict(warps_per_unit=8, cluster_size=2, replicas_per_lane=3)
-        with _engine(ps, (8, 12), 300, 12, 4, stall, pt, **opts) as eng:
+        with _engine(ps, (8, 12), 200, 12, 4, stall, pt, **opts) as eng:
             (eng.pt_run if pt else eng.sweep)(7)
-            out.append(_state(eng, 300, pt))
+            out.append(_state(eng, 200, pt))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
     assert out[0][2].sum() > 0
