@@ -31,7 +31,7 @@
 // of 32 moves prepared by the workers themselves, then cut in batches of
 // consecutive commuting moves with a CTA barrier each, took 7500 cycles of
 // preparation a window and 8.6 batches of 1950 cycles: 118 us a sweep launch and
-// 25 us of exchange; now 91 us for both.  Where many blocks share the SMs those
+// 25 us of exchange; now 89 us for both.  Where many blocks share the SMs those
 // batches are the better form still, and run (resident_batched).
 #include <climits>
 
